@@ -34,6 +34,10 @@ namespace pb {
 
 namespace {
 
+// tighten_levels runs when a ring of the early levels (gap + 1 of mean width) would hold
+// more than this many rows: below it the ring fits beside the stages as it is
+constexpr int64_t kTightenRing = 2048;
+
 inline int align4(int x) { return (x + 3) & ~3; }
 inline int64_t align16(int64_t x) { return (x + 15) & ~int64_t(15); }
 
@@ -65,6 +69,48 @@ void scatter_positions(int n, const int* pos, int* rowAt, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------------ host plan
+// Levels as late as their dependents allow, rows without dependents left where they are:
+// every row with dependents moves to one below its lowest dependent.  The number of levels and
+// the validity of the order are unchanged (the longest chain has no slack); what changes is
+// the largest level gap of a coupling.  A block that starts in the middle of a grid plane has
+// rows that could start at once but are only needed a hundred levels later; with the levels
+// taken as early as possible the ring of a 12,000-row block of a 61 x 53 x 47 stencil would
+// hold 58 levels, tightened it holds 2, as for a block of whole planes, and the grouped sweep
+// takes it instead of the general one, which gathers coupled values from global memory:
+// 147 -> 33 us per application there (16 blocks), 248 -> 53 us on 97 x 89 x 83 in 48 blocks.
+// Returns the new gap, or the old one (and the old levels) when it is no larger.
+static int tighten_levels(const HostCSR& A, int lo, int hi, int gap, int* lev, std::vector<int>& first,
+                   std::vector<int>& last, std::vector<int>& late) {
+  const int* rp = A.rowptr;
+  const int* ci = A.col;
+  const int cb = A.istart;
+  first.assign(hi - lo, INT_MAX);   // lowest and highest level of a row's dependents
+  last.assign(hi - lo, -1);
+  late.resize(hi - lo);
+  int g = 0;
+  for (int i = hi - 1; i >= lo; --i) {
+    int f = first[i - lo], l = last[i - lo];
+    for (int j = rp[i] - 1; j < rp[i + 1] - 1; ++j) {
+      const int c = ci[j] - cb;
+      if (c <= i || c >= hi) continue;
+      f = std::min(f, late[c - lo]);
+      l = std::max(l, late[c - lo]);
+    }
+    const int L = f == INT_MAX ? lev[i] : f - 1;
+    late[i - lo] = L;
+    if (l >= 0) g = std::max(g, l - L);
+    for (int j = rp[i] - 1; j < rp[i + 1] - 1; ++j) {
+      const int c = ci[j] - cb;
+      if (c < lo || c >= i) continue;
+      first[c - lo] = std::min(first[c - lo], L);
+      last[c - lo] = std::max(last[c - lo], L);
+    }
+  }
+  if (g >= gap) return gap;
+  std::copy(late.begin(), late.end(), lev + lo);
+  return g;
+}
+
 // Levels: row x waits for every in-block row y < x coupled to it in either direction
 // (a lower entry of x, or an upper entry (y, x) of y), so one level order serves the
 // forward and the backward sweep.  The dependency window W is the largest level gap of
@@ -99,7 +145,7 @@ void ilu_build_plan(const HostCSR& A, const BlockSplit& blocks, IluPlan& P, int*
   const int grain = std::max(1, nb / (32 * nthr));
 #pragma omp parallel num_threads(nthr)
   {
-    std::vector<int> lb, lsrc;   // this thread's scratch, reused across its blocks
+    std::vector<int> lb, lsrc, late;   // this thread's scratch, reused across its blocks
 #pragma omp for schedule(dynamic, grain)
     for (int b = 0; b < nb; ++b) {
       if (block_ready) block_ready(b);
@@ -145,6 +191,7 @@ void ilu_build_plan(const HostCSR& A, const BlockSplit& blocks, IluPlan& P, int*
         maxlev = std::max(maxlev, L);
         if (lmin != INT_MAX) g = std::max(g, L - lmin);
       }
+      if ((int64_t)(g + 1) * (hi - lo) > kTightenRing * (int64_t)(maxlev + 1)) g = tighten_levels(A, lo, hi, g, lev, lb, lsrc, late);
       nlev[b] = maxlev + 1;
       gap[b] = g;
     }
@@ -494,11 +541,11 @@ __global__ void k_ilu_pack(const IluChunk* __restrict__ ch, int nchunks,
 // the input vector fills one shared-memory stage, so the consumers wait on a stage
 // barrier once per group and, between levels, pass only the level barrier.  The rows of a
 // group are contiguous in the permuted layout ([sstart, sstart + sspan)).  Group record:
-//   int4 hdr              {nchunks, sstart, sspan, 0}
-//   int4 cd[kGrpMax][2]   per chunk in sweep order: {rec, w, ring, gs}, {xin, 0, 0, 0}:
-//                         stage byte offsets of the first row's row record and input
-//                         value, rows, ring byte offset of the first row, permuted
-//                         position of the first row
+//   int4 hdr              {nchunks, sstart, xoff, 0}: xoff is the byte offset of the input
+//                         slice in the stage
+//   int4 cd[kGrpMax]      per chunk in sweep order, ready to add: {byte offset of the first
+//                         row's record in the stage, rows - 1, ring byte offset of the first
+//                         row, byte offset of the first row in the input slice}
 //   row records           one per position of the span, `stride` bytes apart:
 //                           T dg        1/U_kk or D^-1 (backward sweep, forward D-ILU only)
 //                           T val[K]    coupled coefficients in the reference's order
@@ -508,8 +555,8 @@ __global__ void k_ilu_pack(const IluChunk* __restrict__ ch, int nchunks,
 //                         of a warp reading consecutive records hit distinct banks.
 // The stage holds T xin[sspan] (the input slice) after the records, 16-byte aligned.
 // Positions without a row (level padding) have zero records.
-constexpr int kGrpMax = 15;
-constexpr int kGrpHdr = 512;   // 16 + kGrpMax * 32, rounded up
+constexpr int kGrpMax = 31;
+constexpr int kGrpHdr = 16 + kGrpMax * 16;
 
 __host__ __device__ constexpr int rec_words(int tsize, bool has_dg, int K) {
   return ((has_dg ? 1 : 0) + K + (2 * K + tsize - 1) / tsize) | 1;
@@ -517,6 +564,15 @@ __host__ __device__ constexpr int rec_words(int tsize, bool has_dg, int K) {
 __host__ __device__ constexpr int rec_stride(int tsize, bool has_dg, int K) {
   return rec_words(tsize, has_dg, K) * tsize;
 }
+
+// Where a row's value sits in the shared-memory ring: the last W levels, or the whole block
+// by position (W = 0), whichever is smaller.
+struct RingMap {
+  int W, maxWp;
+  __host__ __device__ int at(int lvl, int off_in_level, int off_in_block) const {
+    return W > 0 ? (lvl % W) * maxWp + off_in_level : off_in_block;
+  }
+};
 
 // Packs the group records of the grouped sweep (layout above): one CTA per group;
 // gi[g] = {first chunk, end chunk, sstart, sspan}, goff[g] = byte offsets of the forward
@@ -529,10 +585,9 @@ __global__ void k_ilu_pack_grp(const int4* __restrict__ gi, const int64_t* __res
                                const int* __restrict__ pos, const int* __restrict__ lev,
                                const int* __restrict__ rp, const int* __restrict__ ci, int rbase, int cbase,
                                const double* __restrict__ vL, const double* __restrict__ vU,
-                               const double* __restrict__ Dinv, int dilu, int W, int maxWp, int K,
+                               const double* __restrict__ Dinv, int dilu, RingMap ring, int zslot, int K,
                                unsigned char* packF, unsigned char* packB) {
   const int sz = (int)sizeof(T);
-  const int zslot = W * maxWp * sz;   // byte offset of the ring's zero slot
   const int strF = rec_stride(sz, dilu != 0, K), strB = rec_stride(sz, true, K);
   for (int g = blockIdx.x; g < ngroups; g += gridDim.x) {
     const int4 G = gi[g];
@@ -540,28 +595,23 @@ __global__ void k_ilu_pack_grp(const int4* __restrict__ gi, const int64_t* __res
     const int nch = c1 - c0;
     const int blk = ch[c0].blk;
     const int lo = blk_lo[blk], hi = blk_hi[blk];
+    const int bstart = lvl_start[blk_lvl[blk]];   // the block's first position
     unsigned char* f = packF + goff[2 * g];
     unsigned char* bk = packB + goff[2 * g + 1];
     const int xF = kGrpHdr + (int)(((int64_t)sspan * strF + 15) & ~int64_t(15));
     const int xB = kGrpHdr + (int)(((int64_t)sspan * strB + 15) & ~int64_t(15));
     for (int t = threadIdx.x; t < kGrpHdr / 16; t += blockDim.x) {
       int4 hf = make_int4(0, 0, 0, 0), hb = make_int4(0, 0, 0, 0);
-      const int j = (t - 1) >> 1, half = (t - 1) & 1;
       if (t == 0) {
-        hf = make_int4(nch, sstart, sspan, 0);
-        hb = hf;
-      } else if (j < nch) {
-        const IluChunk& cf = ch[c0 + j];       // forward: increasing level
-        const IluChunk& cb = ch[c1 - 1 - j];   // backward: decreasing level
-        if (half == 0) {
-          hf = make_int4(kGrpHdr + (cf.start - sstart) * strF, cf.w,
-                         ((cf.lvl % W) * maxWp + cf.off_in_level) * sz, cf.start);
-          hb = make_int4(kGrpHdr + (cb.start - sstart) * strB, cb.w,
-                         ((cb.lvl % W) * maxWp + cb.off_in_level) * sz, cb.start);
-        } else {
-          hf = make_int4(xF + (cf.start - sstart) * sz, 0, 0, 0);
-          hb = make_int4(xB + (cb.start - sstart) * sz, 0, 0, 0);
-        }
+        hf = make_int4(nch, sstart, xF, 0);
+        hb = make_int4(nch, sstart, xB, 0);
+      } else if (t - 1 < nch) {
+        auto desc = [&](const IluChunk& c, int str) {
+          return make_int4(kGrpHdr + (c.start - sstart) * str, c.w - 1,
+                           ring.at(c.lvl, c.off_in_level, c.start - bstart) * sz, (c.start - sstart) * sz);
+        };
+        hf = desc(ch[c0 + t - 1], strF);   // forward: increasing level
+        hb = desc(ch[c1 - t], strB);       // backward: decreasing level
       }
       reinterpret_cast<int4*>(f)[t] = hf;
       reinterpret_cast<int4*>(bk)[t] = hb;
@@ -583,8 +633,8 @@ __global__ void k_ilu_pack_grp(const int4* __restrict__ gi, const int64_t* __res
       int ia, iz, idg;
       inblock_range(rp, ci, rbase, cbase, nat, lo, hi, &ia, &iz, &idg);
       auto slot_of = [&](int cnat) -> int {
-        const int l = lev[cnat];
-        return ((l % W) * maxWp + (pos[cnat] - lvl_start[blk_lvl[blk] + l])) * sz;
+        const int l = lev[cnat], q = pos[cnat];
+        return ring.at(l, q - lvl_start[blk_lvl[blk] + l], q - bstart) * sz;
       };
       // forward: strictly lower in-block entries, increasing column
       int k = 0;
@@ -666,193 +716,167 @@ struct GrpArgs {
   int* err;
 };
 
-// Operands of the R rows (p, p + NC, ...) a consumer thread owns in one chunk, staged in
-// registers one chunk ahead: coefficients, the input values, the shared-memory addresses
-// of the coupled ring values and of the row's own ring slot, and the output address.
-// Every chunk carries exactly KM coupled entries per row (shorter rows point at the ring's
-// zero slot), so the loops have compile-time trip counts.
-template <class T, int KM, int R>
-struct GOps {
-  T xin[R], dg[R];
-  T val[R][KM];
-  uint32_t gaddr[R][KM];
-  uint32_t waddr;
-  T* gout;
-  int w;
-};
-
 __device__ __forceinline__ void named_bar_arrive(int id, int nthreads) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
-// Shared-memory accesses that the compiler keeps in program order ("memory" clobber): the
-// ring gathers of a level are issued before the next chunk's operand loads, so they do not
-// queue behind them.
-__device__ __forceinline__ double lds_ord(uint32_t a, double) {
-  double v;
-  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ float lds_ord(uint32_t a, float) {
-  float v;
-  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ void sts(uint32_t a, double v) {
-  asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
-}
-__device__ __forceinline__ void sts(uint32_t a, float v) {
-  asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
-}
-
-
-// The K ring byte offsets of a row record, read as whole T-sized words.
+// Operands of the row a consumer thread owns in one chunk, staged in registers one chunk
+// ahead.  Every chunk carries exactly KM coupled entries per row (shorter rows point at the
+// ring's zero slot), and a thread past the chunk's last row repeats that row (the same
+// loads, the same result stored to the same place), so the level step has no branch and no
+// predicate.
 template <class T, int KM>
-__device__ __forceinline__ void load_slots(const unsigned char* sp, uint32_t ring_s, uint32_t (&ga)[KM]) {
+struct GOps {
+  T x, dg, v[KM];
+  uint32_t g[KM];       // ring byte offsets of the coupled rows
+  uint32_t w;           // ring byte offset of the row
+  uint32_t xo;          // byte offset of the row in the group's vector slice
+};
+
+// The K 16-bit ring offsets of a row record, read as whole T-sized words (no bank conflicts).
+template <class T, int KM>
+__device__ __forceinline__ void load_slots(const unsigned char* sp, uint32_t (&g)[KM]) {
   if constexpr (sizeof(T) == 8) {
-    const unsigned long long* w = reinterpret_cast<const unsigned long long*>(sp);
 #pragma unroll
     for (int k0 = 0; k0 < KM; k0 += 4) {
-      const unsigned long long v = w[k0 / 4];
+      const uint2 v = *reinterpret_cast<const uint2*>(sp + 2 * k0);
 #pragma unroll
-      for (int k = k0; k < KM && k < k0 + 4; ++k) ga[k] = ring_s + (uint32_t)((v >> (16 * (k - k0))) & 0xffffu);
+      for (int k = k0; k < KM && k < k0 + 4; ++k) {
+        const uint32_t h = k - k0 < 2 ? v.x : v.y;
+        g[k] = (k & 1) ? h >> 16 : h & 0xffffu;
+      }
     }
   } else {
-    const uint32_t* w = reinterpret_cast<const uint32_t*>(sp);
 #pragma unroll
     for (int k0 = 0; k0 < KM; k0 += 2) {
-      const uint32_t v = w[k0 / 2];
-      ga[k0] = ring_s + (v & 0xffffu);
-      if (k0 + 1 < KM) ga[k0 + 1] = ring_s + (v >> 16);
+      const uint32_t v = *reinterpret_cast<const uint32_t*>(sp + 2 * k0);
+      g[k0] = v & 0xffffu;
+      if (k0 + 1 < KM) g[k0 + 1] = v >> 16;
     }
   }
 }
 
-template <class T, bool HAS_DG, int KM, int R, int NC>
-__device__ __forceinline__ void gload(GOps<T, KM, R>& o, const unsigned char* sp, int j, int p, uint32_t ring_s,
-                                      T* vout) {
-  constexpr int STR = rec_stride((int)sizeof(T), HAS_DG, KM);
-  constexpr int VOFF = HAS_DG ? (int)sizeof(T) : 0;
-  constexpr int SOFF = VOFF + KM * (int)sizeof(T);
-  const int4 c0 = reinterpret_cast<const int4*>(sp)[1 + 2 * j];
-  const int xoff = reinterpret_cast<const int*>(sp)[4 * (2 + 2 * j)];
-  o.w = c0.y;
-  o.waddr = ring_s + (uint32_t)c0.z + (uint32_t)(p * (int)sizeof(T));
-  o.gout = vout + c0.w + p;
+template <class T, bool HAS_DG, int KM>
+__device__ __forceinline__ void gload(GOps<T, KM>& o, const int4& c, const unsigned char* sp, int xoff, int p) {
+  constexpr int SZ = (int)sizeof(T);
+  constexpr int STR = rec_stride(SZ, HAS_DG, KM);
+  constexpr int VOFF = HAS_DG ? SZ : 0;
+  const int i = min(p, c.y);
+  const unsigned char* rec = sp + c.x + i * STR;
+  o.xo = (uint32_t)(c.w + i * SZ);
+  o.w = (uint32_t)(c.z + i * SZ);
+  load_slots<T, KM>(rec + VOFF + KM * SZ, o.g);
+  o.x = *reinterpret_cast<const T*>(sp + xoff + o.xo);
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int q = p + r * NC;
-    if (q < o.w) {
-      const unsigned char* rec = sp + c0.x + q * STR;
-      o.xin[r] = *reinterpret_cast<const T*>(sp + xoff + q * (int)sizeof(T));
-      o.dg[r] = HAS_DG ? *reinterpret_cast<const T*>(rec) : T(1);
-#pragma unroll
-      for (int k = 0; k < KM; ++k) o.val[r][k] = reinterpret_cast<const T*>(rec + VOFF)[k];
-      load_slots<T, KM>(rec + SOFF, ring_s, o.gaddr[r]);
-    }
-  }
+  for (int k = 0; k < KM; ++k) o.v[k] = *reinterpret_cast<const T*>(rec + VOFF + k * SZ);
+  o.dg = HAS_DG ? *reinterpret_cast<const T*>(rec) : T(1);
 }
 
-template <class T, int KM, int R, int NC>
-__device__ __forceinline__ void ggather(const GOps<T, KM, R>& c, int p, T (&dv)[R][KM]) {
+template <class T, bool DILU, bool FWD, int KM>
+__device__ __forceinline__ T gsolve(const GOps<T, KM>& c, const T (&dv)[KM]) {
+  T acc = (FWD || !DILU) ? c.x : T(0);
 #pragma unroll
-  for (int r = 0; r < R; ++r)
-    if (p + r * NC < c.w) {
-#pragma unroll
-      for (int k = 0; k < KM; ++k) dv[r][k] = lds_ord(c.gaddr[r][k], T(0));
-    }
-}
-
-template <class T, bool DILU, bool FWD, int KM, int R, int NC>
-__device__ __forceinline__ void gsolve(const GOps<T, KM, R>& c, const T (&dv)[R][KM], int p) {
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    if (p + r * NC >= c.w) continue;
-    T acc = (FWD || !DILU) ? c.xin[r] : T(0);
-#pragma unroll
-    for (int k = 0; k < KM; ++k) {
-      if (FWD) acc = acc - c.val[r][k] * dv[r][k];
-      else if (DILU) acc = acc + dv[r][k] * c.val[r][k];
-      else acc = acc - dv[r][k] * c.val[r][k];
-    }
-    T out;
-    if (FWD) out = DILU ? c.dg[r] * acc : acc;
-    else if (DILU) out = c.xin[r] - c.dg[r] * acc;
-    else out = acc * c.dg[r];
-    sts(c.waddr + (uint32_t)(r * NC * (int)sizeof(T)), out);
-    c.gout[r * NC] = out;
+  for (int k = 0; k < KM; ++k) {
+    if (FWD) acc = acc - c.v[k] * dv[k];
+    else if (DILU) acc = acc + dv[k] * c.v[k];
+    else acc = acc - dv[k] * c.v[k];
   }
+  if (FWD) return DILU ? c.dg * acc : acc;
+  if (DILU) return c.x - c.dg * acc;
+  return acc * c.dg;
 }
 
 // Consumer side of one sweep over groups [g0, g0 + ng) of the sequence (NG groups over both
 // sweeps).  Per chunk: gather the coupled values from the ring, load the next chunk's
-// operands, finish the rows, and pass the level barrier.  A stage that never landed sets
-// the abort flag; every consumer reads it after the barrier that follows a stage wait, so
-// all return together (`arrived` tells how far each released stages).
-template <class T, bool DILU, bool FWD, int KM, int R, int NC>
+// operands (through its descriptor, read one chunk earlier still) and finish the row, then
+// pass the level barrier.  What a level costs is the number of instructions a warp issues
+// between two barriers -- each waits about four cycles for the one before it -- so
+// descriptors come ready to add, the group's bookkeeping runs once per group and threads
+// without a row repeat the last one instead of branching around the work (a warp-uniform
+// branch per level cost 14 us of the 84 below).  Measured, 128^3 convection-diffusion, 64
+// blocks, 2 x 256 levels: 125 us with the descriptors and records read in one dependent chain
+// under predicates, 84 us so (118 -> 72 us in FP32; 160^3 D-ILU, 80 blocks, 170 -> 128 us;
+// four 1,024-row blocks of a 16^3 grid, 18.5 -> 10.8 us).  The level's own chain (gather 29
+// cycles, four dependent FMAs 36, store and barrier about 45) is half of what remains.  A
+// stage that never landed sets the abort flag; every consumer reads it after the barrier that follows a
+// stage wait, so all return together (`arrived` tells how far each released stages).
+template <class T, bool DILU, bool FWD, int KM>
 __device__ __forceinline__ void gsweep(const GrpArgs<T>& a, uint64_t* full, volatile int* sflags,
-                                       unsigned char* stages, uint32_t ring_s, int g0, int ng, int NG, int p,
-                                       T* vout, int* arrived) {
+                                       const unsigned char* stages, unsigned char* ring, int NC, int g0, int ng,
+                                       int NG, int p, T* vout, int* arrived) {
   constexpr bool HAS_DG = DILU || !FWD;
-  constexpr int NT = NC + 32;
   const int NST = a.nstages;
   if (ng <= 0) return;
-  int g = g0, st = g0 % NST, ph = (g0 / NST) & 1, j = 0, nch = 0;
-  // Loads the chunk at the cursor into o (waiting for its group's stage when the cursor
-  // has just entered the group), then advances the cursor.  Returns 1 when loaded, 0 at
-  // the end of the sweep (the same for every thread), -1 when the stage did not land.
-  bool entered = false;   // the last next() waited for a stage (the same for every thread)
-  auto next = [&](GOps<T, KM, R>& o) -> int {
-    entered = false;
-    if (g >= g0 + ng) return 0;
-    const unsigned char* sp = stages + (size_t)st * a.stage_bytes;
-    if (j == 0) {
-      entered = true;
-      // warp-uniform outcome, so the aligned barrier instructions below never diverge
-      if (!__all_sync(kFull, mbar_wait(&full[st], ph, kWaitLimit))) {
-        atomicExch(a.err, 3);
-        sflags[0] = 1;
-        return -1;
-      }
-      nch = reinterpret_cast<const int*>(sp)[0];
+  int g = g0, st = g0 % NST, ph = (g0 / NST) & 1, j = 0, nch = 0, xoff = 0;
+  const unsigned char* sp = nullptr;
+  unsigned char *out = nullptr, *nout = nullptr;   // the staged and the next group's output slice
+  int4 h = make_int4(0, 0, 0, 0);                   // descriptor of chunk j of the group
+  enum { RUN = 0, CHECK = 1, LAST = 2 };
+  int state = RUN;
+  // Waits for group g's stage and loads its first chunk into o.
+  auto enter = [&](GOps<T, KM>& o) {
+    // warp-uniform outcome, so the aligned barrier instructions below never diverge
+    if (!__all_sync(kFull, mbar_wait(&full[st], ph, kWaitLimit))) {
+      atomicExch(a.err, 3);
+      sflags[0] = 1;
+      return;
     }
-    gload<T, HAS_DG, KM, R, NC>(o, sp, j, p, ring_s, vout);
-    if (++j == nch) {
+    sp = stages + (size_t)st * a.stage_bytes;
+    const int4 gh = *reinterpret_cast<const int4*>(sp);
+    nch = gh.x;
+    xoff = gh.z;
+    nout = reinterpret_cast<unsigned char*>(vout + gh.y);
+    gload<T, HAS_DG, KM>(o, reinterpret_cast<const int4*>(sp)[1], sp, xoff, p);
+    h = reinterpret_cast<const int4*>(sp)[2];
+    j = 1;
+  };
+  // One level: c is staged, n receives the next chunk.
+  auto step = [&](const GOps<T, KM>& c, GOps<T, KM>& n) -> bool {
+    T dv[KM];
+#pragma unroll
+    for (int k = 0; k < KM; ++k) dv[k] = *reinterpret_cast<const T*>(ring + c.g[k]);
+    if (j < nch) {
+      gload<T, HAS_DG, KM>(n, h, sp, xoff, p);
+      ++j;
+      h = reinterpret_cast<const int4*>(sp)[1 + j];   // past the last chunk: read, not used
+    } else {
       // every operand of the group is in this thread's registers: release the stage
-      if (g + NST < NG) named_bar_arrive(kBarStage0 + st, NT);
-      *arrived = g + 1;
-      j = 0;
-      ++g;
+      if (g + NST < NG) named_bar_arrive(kBarStage0 + st, NC + 32);
+      *arrived = ++g;
       if (++st == NST) { st = 0; ph ^= 1; }
+      if (g < g0 + ng) {
+        enter(n);
+        state = CHECK;
+      } else {
+        state = LAST;
+      }
     }
-    return 1;
-  };
-  // level barrier; after a stage wait every consumer also reads the abort flag, which a
-  // consumer whose wait failed has set before the barrier
-  auto level_barrier = [&]() -> bool {
+    const T r = gsolve<T, DILU, FWD, KM>(c, dv);
+    *reinterpret_cast<T*>(ring + c.w) = r;
+    *reinterpret_cast<T*>(out + c.xo) = r;
     named_bar_sync(kBarLevel, NC);
-    return !(entered && sflags[0]);
+    if (state != RUN) {
+      if (state == LAST || sflags[0]) return false;
+      state = RUN;
+      out = nout;
+    }
+    return true;
   };
-  GOps<T, KM, R> A, B;
-  T dv[R][KM];
-  int sA = next(A), sB = 0;
-  if (!level_barrier()) return;
-  while (sA > 0) {
-    ggather<T, KM, R, NC>(A, p, dv);
-    sB = next(B);
-    gsolve<T, DILU, FWD, KM, R, NC>(A, dv, p);
-    if (!level_barrier() || sB == 0) return;
-    ggather<T, KM, R, NC>(B, p, dv);
-    sA = next(A);
-    gsolve<T, DILU, FWD, KM, R, NC>(B, dv, p);
-    if (!level_barrier()) return;
+  GOps<T, KM> A, B;
+  enter(A);
+  out = nout;
+  named_bar_sync(kBarLevel, NC);
+  if (sflags[0]) return;
+  while (step(A, B) && step(B, A)) {
   }
 }
 
-template <class T, bool DILU, int KM, int R, int NC>
-__global__ void __launch_bounds__(NC + 32, 1) k_ilu_sweep_grp(GrpArgs<T> a) {
+// One CTA per block: NC consumer threads (a multiple of 32, at least the widest chunk, at
+// most MAXC) and a producer warp.
+template <class T, bool DILU, int KM, int MAXC>
+__global__ void __launch_bounds__(MAXC + 32, 1) k_ilu_sweep_grp(GrpArgs<T> a) {
   if (gated(a.gate)) return;
-  constexpr int NT = NC + 32;
+  const int NC = blockDim.x - 32, NT = blockDim.x;
   extern __shared__ __align__(128) unsigned char smem[];
   const int NST = a.nstages;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);
@@ -866,16 +890,16 @@ __global__ void __launch_bounds__(NC + 32, 1) k_ilu_sweep_grp(GrpArgs<T> a) {
   if (threadIdx.x == 0) {
     for (int i = 0; i < NST; ++i) mbar_init(&full[i], 1);
     sflags[0] = 0;
+    ring[a.ring_elems - 1] = T(0);   // the zero slot; every other entry is written before it is read
     mbar_fence_init();
   }
-  for (int i = threadIdx.x; i < a.ring_elems; i += blockDim.x) ring[i] = T(0);
   __syncthreads();
-  if (threadIdx.x >= NC) {
+  if ((int)threadIdx.x >= NC) {
     // Producer warp: lane 0 fills stage g % NST with group g once the consumers have
     // released the stage (named barrier kBarStage0 + stage: a hardware wait, no polling).
     // A backward group's slice of y can only be copied once the forward sweep has
     // written it (barrier kBarTurn), so before that only its record is copied.
-    const bool lead = threadIdx.x == NC;
+    const bool lead = (int)threadIdx.x == NC;
     int issued = 0;     // groups whose copies were issued
     bool turned = false;
     auto desc = [&](int g) -> GrpDesc { return g < nGF ? a.tabF[c0 + g] : a.tabB[c1 - 1 - (g - nGF)]; };
@@ -913,9 +937,9 @@ __global__ void __launch_bounds__(NC + 32, 1) k_ilu_sweep_grp(GrpArgs<T> a) {
     return;
   }
   const int p = threadIdx.x;
-  const uint32_t ring_s = smem_u32(ring);
+  unsigned char* ringb = reinterpret_cast<unsigned char*>(ring);
   int arrived = 0;   // groups (sequence index) whose stage this thread has released
-  gsweep<T, DILU, true, KM, R, NC>(a, full, sflags, stages, ring_s, 0, nGF, NG, p, a.y, &arrived);
+  gsweep<T, DILU, true, KM>(a, full, sflags, stages, ringb, NC, 0, nGF, NG, p, a.y, &arrived);
   // forward result written: make it visible to the producer's bulk copies
   fence_proxy_async_global();
   if (sflags[0]) {
@@ -926,7 +950,7 @@ __global__ void __launch_bounds__(NC + 32, 1) k_ilu_sweep_grp(GrpArgs<T> a) {
     named_bar_sync(kBarTurn, NT);
   } else {
     named_bar_arrive(kBarTurn, NT);
-    gsweep<T, DILU, false, KM, R, NC>(a, full, sflags, stages, ring_s, nGF, nGF, NG, p, a.s, &arrived);
+    gsweep<T, DILU, false, KM>(a, full, sflags, stages, ringb, NC, nGF, nGF, NG, p, a.s, &arrived);
   }
   if (sflags[0])
     for (int g = arrived; g < NG; ++g)
@@ -1394,17 +1418,25 @@ int ilu_setup_device(const IluPlan& P, const DevMat<double>& A, int ilu_method,
   int dev_smem = 0;
   PB_CUDA(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx().device));
   const int budget = std::min(dev_smem, 220 * 1024);
-  int64_t ring_bytes = ((int64_t)D.W * D.maxWp + 1) * sizeof(T);
-  D.ring = ring_bytes <= 64 * 1024;
-  int64_t ring_alloc = D.ring ? ((ring_bytes + 127) & ~int64_t(127)) : 0;
-  // consumer threads and rows per thread of the grouped sweep
-  // (one row per thread: a second row slot costs every level its predicated instructions,
-  // although few levels are wider than 256 rows)
-  if (maxw <= 128) { D.nc = 128; D.rows = 1; }
-  else if (maxw <= 256) { D.nc = 256; D.rows = 1; }
-  else if (maxw <= 384) { D.nc = 384; D.rows = 1; }
-  else { D.nc = 512; D.rows = 1; }   // chunks have at most kIluChunk = 512 rows
-  D.grp = D.ring && D.rows > 0 && kuni <= 8;
+  // ring of the grouped sweep: the last W levels or the largest block by position, whichever
+  // is smaller; its byte offsets are 16-bit and two stages of a widest chunk must fit beside it
+  int max_span = 0;
+  for (int b = 0; b < P.nb; ++b)
+    max_span = std::max(max_span, align4(P.lvl_end[P.blk_lvl[b + 1] - 1]) - P.lvl_start[P.blk_lvl[b]]);
+  const int64_t by_level = (int64_t)D.W * D.maxWp;
+  const RingMap ring = by_level <= max_span ? RingMap{D.W, D.maxWp} : RingMap{0, 0};
+  D.ring_elems = (int)std::min<int64_t>(by_level, max_span) + 1;
+  const int64_t grp_ring = ((int64_t)D.ring_elems * (int64_t)sizeof(T) + 127) & ~int64_t(127);
+  const int64_t widest = kGrpHdr + align4(maxw) * (int64_t)(rec_stride((int)sizeof(T), true, kuni) + sizeof(T)) + 256;
+  D.grp = kuni <= 8 && D.ring_elems * (int64_t)sizeof(T) <= 65536 && 128 + grp_ring + 2 * widest <= budget;
+  // consumer threads of the grouped sweep: one row per thread, as many warps as the widest
+  // chunk needs (chunks have at most kIluChunk = 512 rows): every warp more lengthens the
+  // level barrier
+  D.nc = std::max(32, (maxw + 31) & ~31);
+  // the general sweep's ring holds the last W levels
+  const int64_t ring_bytes = (by_level + 1) * (int64_t)sizeof(T);
+  D.ring = !D.grp && ring_bytes <= 64 * 1024;
+  const int64_t ring_alloc = D.grp ? grp_ring : (D.ring ? ((ring_bytes + 127) & ~int64_t(127)) : 0);
   if (D.grp) {
     // Groups of consecutive chunks of one block, each at most kGrpMax chunks and about a
     // quarter of the stage budget (a chunk larger than that forms a group of its own).
@@ -1413,7 +1445,8 @@ int ilu_setup_device(const IluPlan& P, const DevMat<double>& A, int ilu_method,
     auto grp_bytes = [&](int64_t span) {   // backward record (the larger) + vector slice
       return kGrpHdr + ((span * strB + 15) & ~int64_t(15)) + span * sz;
     };
-        const int64_t target = (budget - 128 - ring_alloc) / 4;
+    // at least two stages; four when a quarter still holds a widest chunk
+    const int64_t target = (budget - 128 - ring_alloc) / 4;
     std::vector<int4> gi;
     std::vector<int> blk_grp(P.nb + 1, 0);
     int64_t max_stage = 0;
@@ -1544,7 +1577,8 @@ int ilu_setup_device(const IluPlan& P, const DevMat<double>& A, int ilu_method,
     k_ilu_pack_grp<T><<<std::max(1, std::min(D.ngroups, 65535)), 256, 0, st>>>(
         dp<int4>(D.ginfo), dp<int64_t>(D.goff), D.ngroups, dp<IluChunk>(D.chunks), dp<int>(blo), dp<int>(bhi),
         dp<int>(blvl), dp<int>(lst), d_rowAt, d_pos, d_lev, A.rowptr, A.col, A.rbase, A.cbase, vL, vU,
-        D.dilu ? dp<double>(Di) : nullptr, D.dilu ? 1 : 0, D.W, D.maxWp, D.K, dp<unsigned char>(D.packF),
+        D.dilu ? dp<double>(Di) : nullptr, D.dilu ? 1 : 0, ring, (D.ring_elems - 1) * (int)sizeof(T), D.K,
+        dp<unsigned char>(D.packF),
         dp<unsigned char>(D.packB));
   } else {
     k_ilu_pack<T><<<std::min<int>((int)ch.size(), 65535) > 0 ? std::min<int>((int)ch.size(), 65535) : 1,
@@ -1623,15 +1657,15 @@ static void launch_ilu(const IluDev<T>& D, const IluSolveArgs<T>& a, cudaStream_
   kern<<<D.nb, kIluThreads, D.smem_bytes, st>>>(a);
 }
 
-template <class T, bool DILU, int KM, int R, int NC>
+template <class T, bool DILU, int KM, int MAXC>
 static void launch_grp(const IluDev<T>& D, const GrpArgs<T>& a, cudaStream_t st) {
-  auto kern = k_ilu_sweep_grp<T, DILU, KM, R, NC>;
+  auto kern = k_ilu_sweep_grp<T, DILU, KM, MAXC>;
   static bool configured = false;
   if (!configured) {
     PB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     configured = true;
   }
-  kern<<<D.nb, NC + 32, D.smem_bytes, st>>>(a);
+  kern<<<D.nb, D.nc + 32, D.smem_bytes, st>>>(a);
 }
 
 template <class T, bool DILU, int K, int LPB>
@@ -1696,23 +1730,22 @@ void ilu_apply(const IluDev<T>& D, const T* r, T* s, T* accum, const int* gate, 
     g.s = s;
     g.stage_bytes = D.stage_bytes;
     g.nstages = D.nstages;
-    g.ring_elems = D.W * D.maxWp + 1;
+    g.ring_elems = D.ring_elems;
     g.gate = gate;
     g.err = dp<int>(D.err);
-#define GRP_R(KM_, R_, NC_)                                                                        \
-  if (D.dilu) launch_grp<T, true, KM_, R_, NC_>(D, g, st); else launch_grp<T, false, KM_, R_, NC_>(D, g, st);
+    // 256 consumers leave each thread twice the registers of 512
+#define GRP_C(KM_, MAXC_)                                                                          \
+  if (D.dilu) launch_grp<T, true, KM_, MAXC_>(D, g, st); else launch_grp<T, false, KM_, MAXC_>(D, g, st);
 #define GRP(KM_)                                                                                   \
   case KM_:                                                                                        \
-    if (D.nc == 128) { GRP_R(KM_, 1, 128) }                                                        \
-    else if (D.nc == 256) { GRP_R(KM_, 1, 256) }                                                   \
-    else if (D.nc == 384) { GRP_R(KM_, 1, 384) } else { GRP_R(KM_, 1, 512) }                       \
+    if (D.nc <= 256) { GRP_C(KM_, 256) } else { GRP_C(KM_, 512) }                                  \
     break;
     switch (D.K) {
       GRP(1) GRP(2) GRP(3) GRP(4) GRP(6) GRP(8)
       default: PB_CHECK(false, PARCEL_B_E_ARG, "unsupported coupling count %d", D.K);
     }
 #undef GRP
-#undef GRP_R
+#undef GRP_C
     PB_CUDA(cudaGetLastError());
     return;
   }

@@ -97,11 +97,11 @@ template <class T>
 struct IluDev {
   int nb = 0, np = 0, n = 0;
   int W = 1, maxWp = 0;
-  bool ring = true;
+  bool ring = true;  // general sweep: its ring of W levels fits
   bool dilu = false;
-  bool grp = false;  // grouped sweep (ring mode, K <= 8, two stages fit); else the general one
-  int nc = 256;      // consumer threads of the grouped sweep (128 or 256)
-  int rows = 1;      // rows per consumer thread of the grouped sweep (1 or 2)
+  bool grp = false;  // grouped sweep (its ring and two stages fit, K <= 8); else the general one
+  int nc = 256;      // consumer threads of the grouped sweep
+  int ring_elems = 0;   // entries of the grouped sweep's ring, the zero slot included
   int K = 0;         // coupled entries per row in every record
   int ngroups = 0;
   int stage_bytes = 0, nstages = 0, smem_bytes = 0;

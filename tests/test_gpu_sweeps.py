@@ -1,0 +1,78 @@
+"""Block-Jacobi sweeps at the sizes where their layout changes: blocks that start inside a
+grid plane (levels tightened before the layout is made), blocks whose level gaps are so long
+that the shared-memory ring holds the whole block by position, levels wider than one chunk,
+levels narrower than a warp, and every supported coupling count.
+
+Tolerance: the sweeps evaluate the oracle's expressions with fused multiply-adds; 1e-11 of
+the largest entry, as the other preconditioner tests.
+"""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import oracle
+from parcel_b import _lib, api, problems
+
+pytestmark = pytest.mark.gpu
+
+
+def _apply_both(A, **pre):
+    r = np.random.default_rng(11).standard_normal(A.n)
+    s_ref = oracle.precon_apply(A, r, **pre)
+    s = np.zeros(A.n)
+    p = _lib.new_input(**pre)
+    rc = _lib.load().parcel_b_precon_apply(C.byref(p), C.byref(api.crs_struct(A)), r.ctypes.data, s.ctypes.data)
+    assert rc == 0, _lib.last_error()
+    return np.abs(s - s_ref).max() / np.abs(s_ref).max()
+
+
+def _symmetric_pattern(n, links, seed):
+    """A diagonally dominant matrix with the given number of long-range links per row (and
+    their transposes), nonsymmetric values."""
+    rng = np.random.default_rng(seed)
+    cols = [set((i,)) for i in range(n)]
+    for k in range(links):
+        p = rng.permutation(n)
+        for i in range(n):
+            cols[i].add(int(p[i]))
+            cols[int(p[i])].add(i)
+    rp, ci, va = [1], [], []
+    for i in range(n):
+        c = sorted(cols[i])
+        ci += [j + 1 for j in c]
+        va += [4.0 * len(c) if j == i else float(rng.uniform(-1, 1)) for j in c]
+        rp.append(len(ci) + 1)
+    return problems.CRS(n=n, rowptr=np.array(rp, np.int32), col=np.array(ci, np.int32), val=np.array(va))
+
+
+@pytest.mark.parametrize("ilu", [0, 1])
+@pytest.mark.parametrize("N,blocks", [(31, 1), (31, 7), (41, 3), (47, 5)])
+def test_blocks_that_start_inside_a_plane(N, blocks, ilu):
+    A = problems.convdiff3d_upwind(N)
+    assert _apply_both(A, ipreflag=2, ILU_method=ilu, precon_thblock=blocks) < 1e-11
+
+
+@pytest.mark.parametrize("n,blocks", [(700, 1), (6001, 3), (9000, 1)])
+def test_long_level_gaps(n, blocks):
+    """One link per row: at most four couplings; the blocks of 700, 2,000 and 9,000 rows keep
+    their whole solution, or too long a ring for 64 KB, which takes the general sweep."""
+    A = _symmetric_pattern(n, 1, n)
+    for ilu in (0, 1):
+        assert _apply_both(A, ipreflag=2, ILU_method=ilu, precon_thblock=blocks) < 1e-11
+
+
+@pytest.mark.parametrize("links", [1, 2, 3, 4])
+def test_coupling_counts(links):
+    """Up to eight couplings per row and sweep in the records, more in the general sweep."""
+    A = _symmetric_pattern(1500, links, 90 + links)
+    for ilu in (0, 1):
+        assert _apply_both(A, ipreflag=2, ILU_method=ilu, precon_thblock=2) < 1e-11
+
+
+@pytest.mark.parametrize("nx,ny", [(3, 900), (20, 20), (600, 600)])
+def test_level_widths(nx, ny):
+    """2D grids: levels of at most 3 rows, of 20, and of more than one 512-row chunk."""
+    A = problems.poisson2d_5pt(nx, ny)
+    for ilu in (0, 1):
+        assert _apply_both(A, ipreflag=2, ILU_method=ilu, precon_thblock=1) < 1e-11
