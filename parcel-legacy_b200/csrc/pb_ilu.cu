@@ -26,6 +26,7 @@
 #include <cmath>
 #include <memory>
 #include <numeric>
+#include <type_traits>
 
 #include "pb_device.cuh"
 #include "pb_ilu.cuh"
@@ -577,15 +578,38 @@ struct RingMap {
 // Packs the group records of the grouped sweep (layout above): one CTA per group;
 // gi[g] = {first chunk, end chunk, sstart, sspan}, goff[g] = byte offsets of the forward
 // and backward records.
+// Sweep coefficients of the packed records: L and U entries by position in the natural
+// matrix, and the diagonal factors of row nat (diagonal entry jd).
 template <class T>
+struct FpSrc {
+  const double *vL, *vU, *Dinv;   // Dinv: D-ILU only
+  __device__ T low(int j) const { return (T)vL[j]; }
+  __device__ T up(int j) const { return (T)vU[j]; }
+  __device__ T fwd(int nat) const { return (T)Dinv[nat]; }
+  // ILU(0): the reciprocal of U_kk, the sweep multiplies
+  __device__ T bwd(int nat, int jd) const { return Dinv ? (T)Dinv[nat] : (T)(1.0 / vU[jd]); }
+};
+struct DdSrc {
+  const double *ah, *al, *dih, *dil;   // al and dil null: low parts zero
+  __device__ dd low(int j) const { return dd{ah[j], al ? al[j] : 0.0}; }
+  __device__ dd up(int j) const { return low(j); }
+  __device__ dd fwd(int nat) const { return dd{dih[nat], dil ? dil[nat] : 0.0}; }
+  __device__ dd bwd(int nat, int) const { return fwd(nat); }
+};
+
+// Coefficient and ring value of a padding entry.  The sums add a zero product; the
+// double-double ones leave the entry out, and a factor of one keeps it on the short product.
+template <class T> __device__ __forceinline__ T pad_coef() { return T(0); }
+template <> __device__ __forceinline__ dd pad_coef<dd>() { return dd{1.0, 0.0}; }
+
+template <class T, class Src>
 __global__ void k_ilu_pack_grp(const int4* __restrict__ gi, const int64_t* __restrict__ goff, int ngroups,
                                const IluChunk* __restrict__ ch, const int* __restrict__ blk_lo,
                                const int* __restrict__ blk_hi, const int* __restrict__ blk_lvl,
                                const int* __restrict__ lvl_start, const int* __restrict__ rowAt,
                                const int* __restrict__ pos, const int* __restrict__ lev,
                                const int* __restrict__ rp, const int* __restrict__ ci, int rbase, int cbase,
-                               const double* __restrict__ vL, const double* __restrict__ vU,
-                               const double* __restrict__ Dinv, int dilu, RingMap ring, int zslot, int K,
+                               Src src, int dilu, RingMap ring, int zslot, int K,
                                unsigned char* packF, unsigned char* packB) {
   const int sz = (int)sizeof(T);
   const int strF = rec_stride(sz, dilu != 0, K), strB = rec_stride(sz, true, K);
@@ -639,28 +663,27 @@ __global__ void k_ilu_pack_grp(const int4* __restrict__ gi, const int64_t* __res
       // forward: strictly lower in-block entries, increasing column
       int k = 0;
       for (int j = ia; j < idg; ++j, ++k) {
-        valF[k] = (T)vL[j];
+        valF[k] = src.low(j);
         slF[k] = (unsigned short)slot_of(ci[j] - cbase);
       }
-      for (; k < K; ++k) slF[k] = (unsigned short)zslot;
-      if (dilu) *reinterpret_cast<T*>(rf) = (T)Dinv[nat];
+      for (; k < K; ++k) { valF[k] = pad_coef<T>(); slF[k] = (unsigned short)zslot; }
+      if (dilu) *reinterpret_cast<T*>(rf) = src.fwd(nat);
       // backward: strictly upper in-block entries; ILU(0) increasing column
       // (solve_LU_crs), D-ILU decreasing column (solve_ILU_crs runs Ustart down to Uend)
       k = 0;
       if (!dilu) {
         for (int j = idg + 1; j < iz; ++j, ++k) {
-          valB[k] = (T)vU[j];
+          valB[k] = src.up(j);
           slB[k] = (unsigned short)slot_of(ci[j] - cbase);
         }
-        *reinterpret_cast<T*>(rb) = (T)(1.0 / vU[idg]);   // reciprocal of U_kk: the sweep multiplies
       } else {
         for (int j = iz - 1; j > idg; --j, ++k) {
-          valB[k] = (T)vU[j];
+          valB[k] = src.up(j);
           slB[k] = (unsigned short)slot_of(ci[j] - cbase);
         }
-        *reinterpret_cast<T*>(rb) = (T)Dinv[nat];
       }
-      for (; k < K; ++k) slB[k] = (unsigned short)zslot;
+      *reinterpret_cast<T*>(rb) = src.bwd(nat, idg);
+      for (; k < K; ++k) { valB[k] = pad_coef<T>(); slB[k] = (unsigned short)zslot; }
     }
   }
 }
@@ -736,23 +759,21 @@ struct GOps {
 // The K 16-bit ring offsets of a row record, read as whole T-sized words (no bank conflicts).
 template <class T, int KM>
 __device__ __forceinline__ void load_slots(const unsigned char* sp, uint32_t (&g)[KM]) {
-  if constexpr (sizeof(T) == 8) {
+  constexpr int PER = (int)sizeof(T) / 2;   // offsets per word
 #pragma unroll
-    for (int k0 = 0; k0 < KM; k0 += 4) {
+  for (int k0 = 0; k0 < KM; k0 += PER) {
+    uint32_t w[PER / 2];
+    if constexpr (sizeof(T) == 16) {
+      const uint4 v = *reinterpret_cast<const uint4*>(sp + 2 * k0);
+      w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+    } else if constexpr (sizeof(T) == 8) {
       const uint2 v = *reinterpret_cast<const uint2*>(sp + 2 * k0);
-#pragma unroll
-      for (int k = k0; k < KM && k < k0 + 4; ++k) {
-        const uint32_t h = k - k0 < 2 ? v.x : v.y;
-        g[k] = (k & 1) ? h >> 16 : h & 0xffffu;
-      }
+      w[0] = v.x; w[1] = v.y;
+    } else {
+      w[0] = *reinterpret_cast<const uint32_t*>(sp + 2 * k0);
     }
-  } else {
 #pragma unroll
-    for (int k0 = 0; k0 < KM; k0 += 2) {
-      const uint32_t v = *reinterpret_cast<const uint32_t*>(sp + 2 * k0);
-      g[k0] = v & 0xffffu;
-      if (k0 + 1 < KM) g[k0 + 1] = v >> 16;
-    }
+    for (int k = k0; k < KM && k < k0 + PER; ++k) g[k] = (k & 1) ? w[(k - k0) / 2] >> 16 : w[(k - k0) / 2] & 0xffffu;
   }
 }
 
@@ -769,21 +790,40 @@ __device__ __forceinline__ void gload(GOps<T, KM>& o, const int4& c, const unsig
   o.x = *reinterpret_cast<const T*>(sp + xoff + o.xo);
 #pragma unroll
   for (int k = 0; k < KM; ++k) o.v[k] = *reinterpret_cast<const T*>(rec + VOFF + k * SZ);
-  o.dg = HAS_DG ? *reinterpret_cast<const T*>(rec) : T(1);
+  if constexpr (HAS_DG) o.dg = *reinterpret_cast<const T*>(rec);
 }
 
+// zslot: the ring offset of a padding entry.
 template <class T, bool DILU, bool FWD, int KM>
-__device__ __forceinline__ T gsolve(const GOps<T, KM>& c, const T (&dv)[KM]) {
-  T acc = (FWD || !DILU) ? c.x : T(0);
+__device__ __forceinline__ T gsolve(const GOps<T, KM>& c, const T (&dv)[KM], uint32_t zslot) {
+  if constexpr (std::is_same<T, dd>::value) {
+    // ddsolve_ILU_crs (ddmatrix.f90:4310-4680): products s_c a in the loop's order, padding
+    // entries left out (adding a zero would renormalise)
+    static_assert(DILU, "the double-double sweep is D-ILU");
+    dd v[KM];
 #pragma unroll
-  for (int k = 0; k < KM; ++k) {
-    if (FWD) acc = acc - c.v[k] * dv[k];
-    else if (DILU) acc = acc + dv[k] * c.v[k];
-    else acc = acc - dv[k] * c.v[k];
+    for (int k = 0; k < KM; ++k) v[k] = dd_mul(dv[k], c.v[k]);
+    dd z = FWD ? c.x : dd{0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < KM; ++k) {
+      const dd t = FWD ? dd_sub(z, v[k]) : dd_add(z, v[k]);
+      const bool on = c.g[k] != zslot;
+      z.hi = on ? t.hi : z.hi;
+      z.lo = on ? t.lo : z.lo;
+    }
+    return FWD ? dd_mul(z, c.dg) : dd_sub(c.x, dd_mul(c.dg, z));
+  } else {
+    T acc = (FWD || !DILU) ? c.x : T(0);
+#pragma unroll
+    for (int k = 0; k < KM; ++k) {
+      if (FWD) acc = acc - c.v[k] * dv[k];
+      else if (DILU) acc = acc + dv[k] * c.v[k];
+      else acc = acc - dv[k] * c.v[k];
+    }
+    if (FWD) return DILU ? c.dg * acc : acc;
+    if (DILU) return c.x - c.dg * acc;
+    return acc * c.dg;
   }
-  if (FWD) return DILU ? c.dg * acc : acc;
-  if (DILU) return c.x - c.dg * acc;
-  return acc * c.dg;
 }
 
 // Consumer side of one sweep over groups [g0, g0 + ng) of the sequence (NG groups over both
@@ -806,6 +846,7 @@ __device__ __forceinline__ void gsweep(const GrpArgs<T>& a, uint64_t* full, vola
                                        int NG, int p, T* vout, int* arrived) {
   constexpr bool HAS_DG = DILU || !FWD;
   const int NST = a.nstages;
+  const uint32_t zslot = (uint32_t)((a.ring_elems - 1) * (int)sizeof(T));
   if (ng <= 0) return;
   int g = g0, st = g0 % NST, ph = (g0 / NST) & 1, j = 0, nch = 0, xoff = 0;
   const unsigned char* sp = nullptr;
@@ -851,7 +892,7 @@ __device__ __forceinline__ void gsweep(const GrpArgs<T>& a, uint64_t* full, vola
         state = LAST;
       }
     }
-    const T r = gsolve<T, DILU, FWD, KM>(c, dv);
+    const T r = gsolve<T, DILU, FWD, KM>(c, dv, zslot);
     *reinterpret_cast<T*>(ring + c.w) = r;
     *reinterpret_cast<T*>(out + c.xo) = r;
     named_bar_sync(kBarLevel, NC);
@@ -890,7 +931,7 @@ __global__ void __launch_bounds__(MAXC + 32, 1) k_ilu_sweep_grp(GrpArgs<T> a) {
   if (threadIdx.x == 0) {
     for (int i = 0; i < NST; ++i) mbar_init(&full[i], 1);
     sflags[0] = 0;
-    ring[a.ring_elems - 1] = T(0);   // the zero slot; every other entry is written before it is read
+    ring[a.ring_elems - 1] = pad_coef<T>();   // the padding slot; every other entry is written before it is read
     mbar_fence_init();
   }
   __syncthreads();
@@ -1396,6 +1437,99 @@ k_ilu_small_staged(int nb, const int2* __restrict__ box, const int* __restrict__
 }
 
 // ------------------------------------------------------------------ host side
+static int sweep_smem_budget() {
+  int dev_smem = 0;
+  PB_CUDA(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx().device));
+  return std::min(dev_smem, 220 * 1024);
+}
+
+// Lays out the grouped sweep of plan P (chunks ch, kuni couplings per row and sweep) if it fits:
+// ring, groups, stages and the producer tables.  The ring holds the last W levels or the
+// largest block by position, whichever is smaller; its byte offsets are 16-bit and two
+// stages of a widest chunk must fit beside it.
+template <class T>
+static bool grp_layout(const IluPlan& P, const std::vector<IluChunk>& ch, int kuni, int maxw, IluDev<T>& D,
+                       RingMap& ring) {
+  const int budget = sweep_smem_budget();
+  int max_span = 0;
+  for (int b = 0; b < P.nb; ++b)
+    max_span = std::max(max_span, align4(P.lvl_end[P.blk_lvl[b + 1] - 1]) - P.lvl_start[P.blk_lvl[b]]);
+  const int64_t by_level = (int64_t)D.W * D.maxWp;
+  ring = by_level <= max_span ? RingMap{D.W, D.maxWp} : RingMap{0, 0};
+  const int64_t elems = std::min<int64_t>(by_level, max_span) + 1;
+  const int64_t ring_alloc = (elems * (int64_t)sizeof(T) + 127) & ~int64_t(127);
+  const int64_t widest = kGrpHdr + align4(maxw) * (int64_t)(rec_stride((int)sizeof(T), true, kuni) + sizeof(T)) + 256;
+  if (elems * (int64_t)sizeof(T) > 65536 || 128 + ring_alloc + 2 * widest > budget) return false;
+  D.ring_elems = (int)elems;
+  // consumer threads: one row per thread, as many warps as the widest chunk needs (chunks
+  // have at most kIluChunk = 512 rows): every warp more lengthens the level barrier
+  D.nc = std::max(32, (maxw + 31) & ~31);
+  // Groups of consecutive chunks of one block, each at most kGrpMax chunks and about a
+  // quarter of the stage budget (a chunk larger than that forms a group of its own).
+  const int64_t sz = sizeof(T);
+  const int64_t strF = rec_stride((int)sz, D.dilu, kuni), strB = rec_stride((int)sz, true, kuni);
+  auto grp_bytes = [&](int64_t span) {   // backward record (the larger) + vector slice
+    return kGrpHdr + ((span * strB + 15) & ~int64_t(15)) + span * sz;
+  };
+  // at least two stages; four when a quarter still holds a widest chunk
+  const int64_t target = (budget - 128 - ring_alloc) / 4;
+  std::vector<int4> gi;
+  std::vector<int> blk_grp(P.nb + 1, 0);
+  int64_t max_stage = 0;
+  for (int b = 0; b < P.nb; ++b) {
+    blk_grp[b] = (int)gi.size();
+    int c = P.blk_chunk[b];
+    while (c < P.blk_chunk[b + 1]) {
+      const int sstart = ch[c].start;
+      int e = c + 1;
+      auto span_to = [&](int ce) { return (int64_t)align4(ch[ce - 1].start + ch[ce - 1].w) - sstart; };
+      while (e < P.blk_chunk[b + 1] && e - c < kGrpMax && grp_bytes(span_to(e + 1)) <= target) ++e;
+      const int64_t span = span_to(e);
+      gi.push_back(make_int4(c, e, sstart, (int)span));
+      max_stage = std::max(max_stage, grp_bytes(span));
+      c = e;
+    }
+  }
+  blk_grp[P.nb] = (int)gi.size();
+  const int ng = (int)gi.size();
+  std::vector<int64_t> goff(2 * (size_t)std::max(ng, 1), 0);
+  std::vector<GrpDesc> tf(ng), tb(ng);
+  int64_t oF = 0, oB = 0;
+  for (int g = 0; g < ng; ++g) {
+    const int64_t span = gi[g].w;
+    const int64_t cbF = kGrpHdr + ((span * strF + 15) & ~int64_t(15));
+    const int64_t cbB = kGrpHdr + ((span * strB + 15) & ~int64_t(15));
+    goff[2 * g] = oF;
+    goff[2 * g + 1] = oB;
+    PB_CHECK(oF / 16 < INT32_MAX && oB / 16 < INT32_MAX, PARCEL_B_E_UNSUPPORTED,
+             "packed preconditioner larger than 32 GiB");
+    tf[g] = GrpDesc{(int)(oF / 16), (int)cbF, gi[g].z, (int)(span * sz)};
+    tb[g] = GrpDesc{(int)(oB / 16), (int)cbB, gi[g].z, (int)(span * sz)};
+    oF += align16(cbF);
+    oB += align16(cbB);
+  }
+  D.packF_bytes = std::max<int64_t>(oF, 16);
+  D.packB_bytes = std::max<int64_t>(oB, 16);
+  D.stage_bytes = (int)((max_stage + 127) & ~int64_t(127));
+  const int64_t room = budget - 128 - ring_alloc;
+  D.nstages = (int)std::min<int64_t>(kGrpMaxStages, room / D.stage_bytes);
+  PB_CHECK(D.nstages >= 2, PARCEL_B_E_UNSUPPORTED,
+           "block-Jacobi level too wide for shared memory (stage %d bytes)", D.stage_bytes);
+  D.smem_bytes = (int)(128 + ring_alloc + (int64_t)D.nstages * D.stage_bytes);
+  D.ngroups = ng;
+  D.tabF.alloc(sizeof(GrpDesc) * std::max(ng, 1));
+  D.tabB.alloc(sizeof(GrpDesc) * std::max(ng, 1));
+  h2d(D.tabF.p, tf.data(), sizeof(GrpDesc) * ng);
+  h2d(D.tabB.p, tb.data(), sizeof(GrpDesc) * ng);
+  D.blk_grp.alloc(sizeof(int) * (P.nb + 1));
+  h2d(D.blk_grp.p, blk_grp.data(), sizeof(int) * (P.nb + 1));
+  D.ginfo.alloc(sizeof(int4) * std::max(ng, 1));
+  h2d(D.ginfo.p, gi.data(), sizeof(int4) * ng);
+  D.goff.alloc(sizeof(int64_t) * goff.size());
+  h2d(D.goff.p, goff.data(), sizeof(int64_t) * goff.size());
+  return true;
+}
+
 template <class T>
 int ilu_setup_device(const IluPlan& P, const DevMat<double>& A, int ilu_method,
                      const int* d_pos, const int* d_rowAt, const int* d_lev, IluDev<T>& D) {
@@ -1414,94 +1548,14 @@ int ilu_setup_device(const IluPlan& P, const DevMat<double>& A, int ilu_method,
     if (kmax <= c) { kuni = c; break; }
   for (auto& c : ch) { c.KL = kuni; c.KU = kuni; }
   D.K = kuni;
-  // shared memory budget: barriers + ring + stages
-  int dev_smem = 0;
-  PB_CUDA(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx().device));
-  const int budget = std::min(dev_smem, 220 * 1024);
-  // ring of the grouped sweep: the last W levels or the largest block by position, whichever
-  // is smaller; its byte offsets are 16-bit and two stages of a widest chunk must fit beside it
-  int max_span = 0;
-  for (int b = 0; b < P.nb; ++b)
-    max_span = std::max(max_span, align4(P.lvl_end[P.blk_lvl[b + 1] - 1]) - P.lvl_start[P.blk_lvl[b]]);
-  const int64_t by_level = (int64_t)D.W * D.maxWp;
-  const RingMap ring = by_level <= max_span ? RingMap{D.W, D.maxWp} : RingMap{0, 0};
-  D.ring_elems = (int)std::min<int64_t>(by_level, max_span) + 1;
-  const int64_t grp_ring = ((int64_t)D.ring_elems * (int64_t)sizeof(T) + 127) & ~int64_t(127);
-  const int64_t widest = kGrpHdr + align4(maxw) * (int64_t)(rec_stride((int)sizeof(T), true, kuni) + sizeof(T)) + 256;
-  D.grp = kuni <= 8 && D.ring_elems * (int64_t)sizeof(T) <= 65536 && 128 + grp_ring + 2 * widest <= budget;
-  // consumer threads of the grouped sweep: one row per thread, as many warps as the widest
-  // chunk needs (chunks have at most kIluChunk = 512 rows): every warp more lengthens the
-  // level barrier
-  D.nc = std::max(32, (maxw + 31) & ~31);
-  // the general sweep's ring holds the last W levels
-  const int64_t ring_bytes = (by_level + 1) * (int64_t)sizeof(T);
-  D.ring = !D.grp && ring_bytes <= 64 * 1024;
-  const int64_t ring_alloc = D.grp ? grp_ring : (D.ring ? ((ring_bytes + 127) & ~int64_t(127)) : 0);
-  if (D.grp) {
-    // Groups of consecutive chunks of one block, each at most kGrpMax chunks and about a
-    // quarter of the stage budget (a chunk larger than that forms a group of its own).
-    const int64_t sz = sizeof(T);
-    const int64_t strF = rec_stride((int)sz, D.dilu, kuni), strB = rec_stride((int)sz, true, kuni);
-    auto grp_bytes = [&](int64_t span) {   // backward record (the larger) + vector slice
-      return kGrpHdr + ((span * strB + 15) & ~int64_t(15)) + span * sz;
-    };
-    // at least two stages; four when a quarter still holds a widest chunk
-    const int64_t target = (budget - 128 - ring_alloc) / 4;
-    std::vector<int4> gi;
-    std::vector<int> blk_grp(P.nb + 1, 0);
-    int64_t max_stage = 0;
-    for (int b = 0; b < P.nb; ++b) {
-      blk_grp[b] = (int)gi.size();
-      int c = P.blk_chunk[b];
-      while (c < P.blk_chunk[b + 1]) {
-        const int sstart = ch[c].start;
-        int e = c + 1;
-        auto span_to = [&](int ce) { return (int64_t)align4(ch[ce - 1].start + ch[ce - 1].w) - sstart; };
-        while (e < P.blk_chunk[b + 1] && e - c < kGrpMax && grp_bytes(span_to(e + 1)) <= target) ++e;
-        const int64_t span = span_to(e);
-        gi.push_back(make_int4(c, e, sstart, (int)span));
-        max_stage = std::max(max_stage, grp_bytes(span));
-        c = e;
-      }
-    }
-    blk_grp[P.nb] = (int)gi.size();
-    const int ng = (int)gi.size();
-    std::vector<int64_t> goff(2 * (size_t)std::max(ng, 1), 0);
-    std::vector<GrpDesc> tf(ng), tb(ng);
-    int64_t oF = 0, oB = 0;
-    for (int g = 0; g < ng; ++g) {
-      const int64_t span = gi[g].w;
-      const int64_t cbF = kGrpHdr + ((span * strF + 15) & ~int64_t(15));
-      const int64_t cbB = kGrpHdr + ((span * strB + 15) & ~int64_t(15));
-      goff[2 * g] = oF;
-      goff[2 * g + 1] = oB;
-      PB_CHECK(oF / 16 < INT32_MAX && oB / 16 < INT32_MAX, PARCEL_B_E_UNSUPPORTED,
-               "packed preconditioner larger than 32 GiB");
-      tf[g] = GrpDesc{(int)(oF / 16), (int)cbF, gi[g].z, (int)(span * sz)};
-      tb[g] = GrpDesc{(int)(oB / 16), (int)cbB, gi[g].z, (int)(span * sz)};
-      oF += align16(cbF);
-      oB += align16(cbB);
-    }
-    D.packF_bytes = std::max<int64_t>(oF, 16);
-    D.packB_bytes = std::max<int64_t>(oB, 16);
-    D.stage_bytes = (int)((max_stage + 127) & ~int64_t(127));
-    const int64_t room = budget - 128 - ring_alloc;
-    D.nstages = (int)std::min<int64_t>(kGrpMaxStages, room / D.stage_bytes);
-    PB_CHECK(D.nstages >= 2, PARCEL_B_E_UNSUPPORTED,
-             "block-Jacobi level too wide for shared memory (stage %d bytes)", D.stage_bytes);
-    D.smem_bytes = (int)(128 + ring_alloc + (int64_t)D.nstages * D.stage_bytes);
-    D.ngroups = ng;
-    D.tabF.alloc(sizeof(GrpDesc) * std::max(ng, 1));
-    D.tabB.alloc(sizeof(GrpDesc) * std::max(ng, 1));
-    h2d(D.tabF.p, tf.data(), sizeof(GrpDesc) * ng);
-    h2d(D.tabB.p, tb.data(), sizeof(GrpDesc) * ng);
-    D.blk_grp.alloc(sizeof(int) * (P.nb + 1));
-    h2d(D.blk_grp.p, blk_grp.data(), sizeof(int) * (P.nb + 1));
-    D.ginfo.alloc(sizeof(int4) * std::max(ng, 1));
-    h2d(D.ginfo.p, gi.data(), sizeof(int4) * ng);
-    D.goff.alloc(sizeof(int64_t) * goff.size());
-    h2d(D.goff.p, goff.data(), sizeof(int64_t) * goff.size());
-  } else {
+  RingMap ring;
+  D.grp = kuni <= 8 && grp_layout<T>(P, ch, kuni, maxw, D, ring);
+  if (!D.grp) {
+    // the general sweep: its ring holds the last W levels when they fit 64 KB
+    const int budget = sweep_smem_budget();
+    const int64_t ring_bytes = ((int64_t)D.W * D.maxWp + 1) * (int64_t)sizeof(T);
+    D.ring = ring_bytes <= 64 * 1024;
+    const int64_t ring_alloc = D.ring ? ((ring_bytes + 127) & ~int64_t(127)) : 0;
     // per-chunk records for the general sweep
     int64_t oF = 0, oB = 0;
     int64_t max_stage = 0;
@@ -1574,10 +1628,11 @@ int ilu_setup_device(const IluPlan& P, const DevMat<double>& A, int ilu_method,
   D.packF.alloc(D.packF_bytes);
   D.packB.alloc(D.packB_bytes);
   if (D.grp) {
-    k_ilu_pack_grp<T><<<std::max(1, std::min(D.ngroups, 65535)), 256, 0, st>>>(
+    const FpSrc<T> src{vL, vU, D.dilu ? dp<double>(Di) : nullptr};
+    k_ilu_pack_grp<T, FpSrc<T>><<<std::max(1, std::min(D.ngroups, 65535)), 256, 0, st>>>(
         dp<int4>(D.ginfo), dp<int64_t>(D.goff), D.ngroups, dp<IluChunk>(D.chunks), dp<int>(blo), dp<int>(bhi),
-        dp<int>(blvl), dp<int>(lst), d_rowAt, d_pos, d_lev, A.rowptr, A.col, A.rbase, A.cbase, vL, vU,
-        D.dilu ? dp<double>(Di) : nullptr, D.dilu ? 1 : 0, ring, (D.ring_elems - 1) * (int)sizeof(T), D.K,
+        dp<int>(blvl), dp<int>(lst), d_rowAt, d_pos, d_lev, A.rowptr, A.col, A.rbase, A.cbase, src,
+        D.dilu ? 1 : 0, ring, (D.ring_elems - 1) * (int)sizeof(T), D.K,
         dp<unsigned char>(D.packF),
         dp<unsigned char>(D.packB));
   } else {
@@ -1703,6 +1758,82 @@ static void launch_small(const IluDev<T>& D, const T* r, T* s, const int* gate, 
   else launch_small_lpb<T, DILU, K, 32>(D, r, s, gate, st);
 }
 
+bool ilu_setup_dd(const IluPlan& P, const DevMat<double>& A, const double* al, const double* dih, const double* dil,
+                  int precision, const int* d_pos, const int* d_rowAt, const int* d_lev, IluDev<dd>& D) {
+  cudaStream_t st = stream();
+  D.nb = P.nb; D.np = P.np; D.n = P.n;
+  D.dilu = true;
+  D.W = P.W;
+  D.maxWp = std::max(4, P.maxWp);
+  std::vector<IluChunk> ch = P.chunks;
+  int kmax = 0, maxw = 0;
+  for (const auto& c : ch) { kmax = std::max(kmax, std::max(c.KL, c.KU)); maxw = std::max(maxw, c.w); }
+  int kuni = 0;
+  for (int c : {6, 4, 3, 2, 1})
+    if (kmax <= c) kuni = c;
+  // a stage ring takes most of an SM: with eight blocks per SM and more the unstaged sweep,
+  // several CTAs to an SM, is the better one
+  if (kuni == 0 || P.nb >= 8 * num_sms()) return false;
+  for (auto& c : ch) { c.KL = kuni; c.KU = kuni; }
+  D.K = kuni;
+  RingMap ring;
+  if (!grp_layout<dd>(P, ch, kuni, maxw, D, ring)) return false;
+  D.grp = true;
+  DBuf chunks(sizeof(IluChunk) * std::max<size_t>(ch.size(), 1)), blo(sizeof(int) * P.nb), bhi(sizeof(int) * P.nb),
+      blvl(sizeof(int) * (P.nb + 1)), lst(sizeof(int) * std::max<size_t>(P.lvl_start.size(), 1));
+  h2d(chunks.p, ch.data(), sizeof(IluChunk) * ch.size());
+  h2d(blo.p, P.blk_lo.data(), sizeof(int) * P.nb);
+  h2d(bhi.p, P.blk_hi.data(), sizeof(int) * P.nb);
+  h2d(blvl.p, P.blk_lvl.data(), sizeof(int) * (P.nb + 1));
+  h2d(lst.p, P.lvl_start.data(), sizeof(int) * P.lvl_start.size());
+  D.packF.alloc(D.packF_bytes);
+  D.packB.alloc(D.packB_bytes);
+  const DdSrc src{A.val, precision == 2 ? al : nullptr, dih, precision == 2 ? dil : nullptr};
+  k_ilu_pack_grp<dd, DdSrc><<<std::max(1, std::min(D.ngroups, 65535)), 256, 0, st>>>(
+      dp<int4>(D.ginfo), dp<int64_t>(D.goff), D.ngroups, dp<IluChunk>(chunks), dp<int>(blo), dp<int>(bhi),
+      dp<int>(blvl), dp<int>(lst), d_rowAt, d_pos, d_lev, A.rowptr, A.col, A.rbase, A.cbase, src, 1, ring,
+      (D.ring_elems - 1) * (int)sizeof(dd), D.K, dp<unsigned char>(D.packF), dp<unsigned char>(D.packB));
+  PB_CUDA(cudaGetLastError());
+  D.ytmp.alloc(sizeof(dd) * (P.np + 4));
+  D.err.alloc(sizeof(int));
+  sync();   // the temporaries above are released on return
+  return true;
+}
+
+template <class T>
+static GrpArgs<T> grp_args(const IluDev<T>& D, const T* r, T* s, const int* gate) {
+  GrpArgs<T> g;
+  g.tabF = dp<GrpDesc>(D.tabF);
+  g.tabB = dp<GrpDesc>(D.tabB);
+  g.blk_grp = dp<int>(D.blk_grp);
+  g.packF = dp<unsigned char>(D.packF);
+  g.packB = dp<unsigned char>(D.packB);
+  g.r = r;
+  g.y = dp<T>(D.ytmp);
+  g.s = s;
+  g.stage_bytes = D.stage_bytes;
+  g.nstages = D.nstages;
+  g.ring_elems = D.ring_elems;
+  g.gate = gate;
+  g.err = dp<int>(D.err);
+  return g;
+}
+
+void ilu_apply_dd(const IluDev<dd>& D, const dd* r, dd* s, cudaStream_t st) {
+  const GrpArgs<dd> g = grp_args<dd>(D, r, s, nullptr);
+#define GRP_DD(KM_)                                                                                \
+  case KM_:                                                                                        \
+    if (D.nc <= 256) launch_grp<dd, true, KM_, 256>(D, g, st);                                     \
+    else launch_grp<dd, true, KM_, 512>(D, g, st);                                                 \
+    break;
+  switch (D.K) {
+    GRP_DD(1) GRP_DD(2) GRP_DD(3) GRP_DD(4) GRP_DD(6)
+    default: PB_CHECK(false, PARCEL_B_E_ARG, "unsupported coupling count %d", D.K);
+  }
+#undef GRP_DD
+  PB_CUDA(cudaGetLastError());
+}
+
 template <class T>
 void ilu_apply(const IluDev<T>& D, const T* r, T* s, T* accum, const int* gate, cudaStream_t st) {
   if (D.small && !accum) {
@@ -1719,20 +1850,7 @@ void ilu_apply(const IluDev<T>& D, const T* r, T* s, T* accum, const int* gate, 
     return;
   }
   if (D.grp && !accum) {
-    GrpArgs<T> g;
-    g.tabF = dp<GrpDesc>(D.tabF);
-    g.tabB = dp<GrpDesc>(D.tabB);
-    g.blk_grp = dp<int>(D.blk_grp);
-    g.packF = dp<unsigned char>(D.packF);
-    g.packB = dp<unsigned char>(D.packB);
-    g.r = r;
-    g.y = dp<T>(D.ytmp);
-    g.s = s;
-    g.stage_bytes = D.stage_bytes;
-    g.nstages = D.nstages;
-    g.ring_elems = D.ring_elems;
-    g.gate = gate;
-    g.err = dp<int>(D.err);
+    const GrpArgs<T> g = grp_args<T>(D, r, s, gate);
     // 256 consumers leave each thread twice the registers of 512
 #define GRP_C(KM_, MAXC_)                                                                          \
   if (D.dilu) launch_grp<T, true, KM_, MAXC_>(D, g, st); else launch_grp<T, false, KM_, MAXC_>(D, g, st);

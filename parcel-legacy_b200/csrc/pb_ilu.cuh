@@ -172,6 +172,17 @@ template <class T>
 int ilu_setup_device(const IluPlan& P, const DevMat<double>& A, int ilu_method,
                      const int* d_pos, const int* d_rowAt, const int* d_lev, IluDev<T>& D);
 
+// The double-double D-ILU sweep on the grouped records: lays out the sweep data of the natural
+// matrix (ah, al: value parts, al may be null) and the diagonal dih + dil (precision 1 drops
+// the low parts of both).  False when the sweep does not take this plan (more than six
+// couplings per row and sweep, levels too wide or too far apart for shared memory, or so many
+// blocks that one CTA per SM leaves the chip idle).
+struct dd;
+bool ilu_setup_dd(const IluPlan& P, const DevMat<double>& A, const double* al, const double* dih, const double* dil,
+                  int precision, const int* d_pos, const int* d_rowAt, const int* d_lev, IluDev<dd>& D);
+// s = M^-1 r on level-ordered vectors of np entries.
+void ilu_apply_dd(const IluDev<dd>& D, const dd* r, dd* s, cudaStream_t st);
+
 // s = M^-1 r on permuted vectors (np entries each).  If `accum` is non-null the result
 // is added into it instead of being written to s (s may then be null).
 template <class T>

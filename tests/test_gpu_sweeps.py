@@ -76,3 +76,39 @@ def test_level_widths(nx, ny):
     A = problems.poisson2d_5pt(nx, ny)
     for ilu in (0, 1):
         assert _apply_both(A, ipreflag=2, ILU_method=ilu, precon_thblock=1) < 1e-11
+
+
+# ---- double-double: bit for bit ----------------------------------------------------------------
+def _dd_both(A, b, **kw):
+    g = api.ddcg(A, b, **kw)
+    xh, xl, h, niter, _ = oracle.ddcg(A, b, **kw)
+    assert g["niter"] == niter
+    assert np.array_equal(g["reshistory"], h, equal_nan=True)
+    assert np.array_equal(g["x_hi"], xh, equal_nan=True) and np.array_equal(g["x_lo"], xl, equal_nan=True)
+
+
+@pytest.mark.parametrize("solver", [1, 2, 3])
+@pytest.mark.parametrize("N,blocks", [(21, 3), (13, 1), (24, 2000)])
+def test_dd_blocks(N, blocks, solver):
+    """Ragged blocks, one block, and so many that the sweep without staged records runs."""
+    A = problems.poisson3d_reference(N, N, N)[0] if solver == 1 else problems.convdiff3d_upwind(N)
+    _dd_both(A, problems.rhs_normal(A.n, N), solver=solver, itrmax=25, rtolmax=1e-13, GMRES_m=7, ipreflag=2,
+             ILU_method=1, precon_thblock=blocks)
+
+
+@pytest.mark.parametrize("links", [1, 2, 3, 4])
+def test_dd_coupling_counts(links):
+    """Up to six couplings per row and sweep in the records, more in the sweep without them."""
+    A = _symmetric_pattern(1500, links, 90 + links)
+    for ilu in (1, 2):
+        _dd_both(A, problems.rhs_normal(A.n, 5), solver=3, itrmax=12, rtolmax=1e-25, GMRES_m=5, ipreflag=2,
+                 ILU_method=ilu, precon_thblock=2)
+
+
+@pytest.mark.parametrize("exponent", [-520, -300, 0, 300, 505])
+def test_dd_products_near_the_ends_of_the_range(exponent):
+    """Right-hand sides scaled so far that products and their rounding errors leave the range in
+    which a fused multiply-subtract equals the split product."""
+    A = problems.poisson3d_reference(12, 12, 12)[0]
+    b = problems.rhs_normal(A.n, 3) * 2.0 ** exponent
+    _dd_both(A, b, solver=1, itrmax=20, rtolmax=1e-13, ipreflag=2, ILU_method=1, precon_thblock=3)
