@@ -10,8 +10,8 @@
 // Every dd operation is the reference's sequence of explicitly rounded double operations
 // (pb_device.cuh), every per-row loop runs in the reference's order (the CRS order for the
 // SpMV, L start..end and U start down to end for the D-ILU sweeps, the D-ILU diagonal
-// recurrence of ddDILU_DInv_crs), and the dot products sum in a fixed order (32,768
-// contiguous chunks in index order, their sums in 256 groups, the group sums in order), so
+// recurrence of ddDILU_DInv_crs), and the dot products sum in a fixed order (2^17 interleaved
+// streams folded by a binary tree), so
 // the solve is bit-for-bit reproducible and identical to the CPU oracle's restatement.
 // The D-ILU rows run level by level on the wavefront plan of the FP64 block-Jacobi path;
 // the level order changes no row's arithmetic.
@@ -27,8 +27,8 @@ namespace pb {
 namespace {
 
 constexpr int kDdStreams = 1 << 17;                 // dot-product streams (the oracle uses the same order)
-constexpr int kDdDotThreads = 256;
-constexpr int kDdDotCtas = kDdStreams / kDdDotThreads;   // 512
+constexpr int kDdDotThreads = 1024;
+constexpr int kDdDotCtas = kDdStreams / kDdDotThreads;   // 128
 constexpr int kDdThreads = 256;
 
 #define GRID_LOOP(i, n) \
@@ -93,61 +93,94 @@ __global__ void k_dd_cg_axpy2(int n, const DdScal* sc, double* __restrict__ xh, 
 // i = t, t + 2^17, ... in increasing i, from zero; the 2^17 stream sums are combined by a
 // complete binary tree (level by level, neighbours in pairs: s'[k] = s[2k] + s[2k+1]).
 // One launch: thread t of the grid owns stream t, so every load is coalesced; each CTA
-// folds its 256 streams (an aligned subtree) in shared memory and stores its sum; the last
-// CTA to finish (an atomic ticket, no waiting) folds the 512 CTA sums and stores the result.
-// The ticket counter is reset by that CTA for the next dot on the stream.
-__device__ __forceinline__ void dd_tree(dd* v, int count) {
-  // v[0..count) -> v[0], count a power of two, all threads of the CTA taking part
-  for (int h = count >> 1; h > 0; h >>= 1) {
-    dd r{0.0, 0.0};
-    for (int k = threadIdx.x; k < h; k += blockDim.x) r = dd_add(v[2 * k], v[2 * k + 1]);
-    __syncthreads();
-    for (int k = threadIdx.x; k < h; k += blockDim.x) v[k] = r;   // h <= blockDim.x after the first level
-    __syncthreads();
+// folds its 1,024 streams (an aligned subtree) and stores its sum; the last CTA to finish (an
+// atomic ticket, no waiting) folds the 128 CTA sums and stores the result.  The folds pair
+// lanes by shuffles: a level is one shuffle and one dd addition, where a fold through shared
+// memory paid two block barriers per level (512 CTAs of 256 threads, 8.9 us per dot of 64^3
+// entries).  The ticket counter is reset by the last CTA for the next dot on the stream.
+__device__ __forceinline__ dd dd_shfl_down(dd v, int o) {
+  return dd{__shfl_down_sync(kFull, v.hi, o), __shfl_down_sync(kFull, v.lo, o)};
+}
+// Lane 0: the binary tree of the warp's values.
+__device__ __forceinline__ dd dd_warp_tree(dd s) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) s = dd_add(s, dd_shfl_down(s, o));
+  return s;
+}
+// Thread 0: the tree of the 1,024 threads' values.  sm: 32 entries, free again after the
+// caller's next block barrier.
+__device__ __forceinline__ dd dd_block_tree(dd s, dd* sm) {
+  s = dd_warp_tree(s);
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) s = dd_warp_tree(sm[threadIdx.x]);
+  return s;
+}
+// Thread 0: the tree of the 128 CTA sums, those past ncta zero.  sm: 4 entries.
+__device__ __forceinline__ dd dd_grid_tree(const dd* part, int ncta, dd* sm) {
+  dd s{0.0, 0.0};
+  if (threadIdx.x < kDdDotCtas) {
+    if ((int)threadIdx.x < ncta) {
+      const double2 v = __ldcg(reinterpret_cast<const double2*>(part + threadIdx.x));
+      s = dd{v.x, v.y};
+    }
+    s = dd_warp_tree(s);
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
   }
+  __syncthreads();
+  if (threadIdx.x == 0) s = dd_add(dd_add(sm[0], sm[1]), dd_add(sm[2], sm[3]));
+  return s;
 }
 
+// MODE 0: out[0] = <x, y>; 1: and out2 = <y, y>; 2: and out2 = <x, x>, from the same loads.
+template <int MODE>
 __global__ void __launch_bounds__(kDdDotThreads) k_dd_dot(int64_t n, const double* __restrict__ xh,
                                                         const double* __restrict__ xl, const double* __restrict__ yh,
                                                         const double* __restrict__ yl, dd* part, unsigned* ticket,
-                                                        dd* out) {
-  __shared__ dd tr[2 * kDdDotThreads];
+                                                        dd* out, dd* out2) {
+  constexpr int ND = MODE ? 2 : 1;
+  __shared__ dd sm[ND][32];
   __shared__ bool last;
   const int64_t t = (int64_t)blockIdx.x * kDdDotThreads + threadIdx.x;
-  dd s{0.0, 0.0};
-  int64_t i = t;
-  for (; i + 3 * (int64_t)kDdStreams < n; i += 4 * (int64_t)kDdStreams) {
-    double ah[4], al[4], bh[4], bl[4];
+  dd s[ND];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+  for (int k = 0; k < ND; ++k) s[k] = dd{0.0, 0.0};
+  auto add = [&](dd a, dd b) {
+    s[0] = dd_add(s[0], dd_mul(a, b));
+    if constexpr (MODE == 1) s[1] = dd_add(s[1], dd_mul(b, b));
+    if constexpr (MODE == 2) s[1] = dd_add(s[1], dd_mul(a, a));
+  };
+  int64_t i = t;
+  constexpr int U = 2;
+  for (; i + (U - 1) * (int64_t)kDdStreams < n; i += U * (int64_t)kDdStreams) {
+    dd a[U], b[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
       const int64_t q = i + u * (int64_t)kDdStreams;
-      ah[u] = xh[q]; al[u] = xl[q]; bh[u] = yh[q]; bl[u] = yl[q];
+      a[u] = dd{xh[q], xl[q]};
+      b[u] = dd{yh[q], yl[q]};
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) s = dd_add(s, dd_mul(dd{ah[u], al[u]}, dd{bh[u], bl[u]}));
+    for (int u = 0; u < U; ++u) add(a[u], b[u]);
   }
-  for (; i < n; i += kDdStreams) s = dd_add(s, dd_mul(dd{xh[i], xl[i]}, dd{yh[i], yl[i]}));
-  tr[threadIdx.x] = s;
-  __syncthreads();
-  dd_tree(tr, kDdDotThreads);
+  for (; i < n; i += kDdStreams) add(dd{xh[i], xl[i]}, dd{yh[i], yl[i]});
+#pragma unroll
+  for (int k = 0; k < ND; ++k) s[k] = dd_block_tree(s[k], sm[k]);
   if (threadIdx.x == 0) {
-    part[blockIdx.x] = tr[0];
+#pragma unroll
+    for (int k = 0; k < ND; ++k) part[k * kDdDotCtas + blockIdx.x] = s[k];
     __threadfence();
     last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
-  for (int k = threadIdx.x; k < kDdDotCtas; k += kDdDotThreads) {
-    const double2 v = __ldcg(reinterpret_cast<const double2*>(part + k));
-    tr[k] = dd{v.x, v.y};
+#pragma unroll
+  for (int k = 0; k < ND; ++k) {
+    const dd v = dd_grid_tree(part + k * kDdDotCtas, gridDim.x, sm[k]);
+    if (threadIdx.x == 0) (k == 0 ? *out : *out2) = v;
   }
-  __syncthreads();
-  dd_tree(tr, kDdDotCtas);
-  if (threadIdx.x == 0) {
-    *out = tr[0];
-    *ticket = 0u;
-  }
+  if (threadIdx.x == 0) *ticket = 0u;
 }
 
 enum DdStep { DD_INIT_NORMS = 0, DD_INIT_RHO, DD_ALPHA, DD_RNORM, DD_BETA };
@@ -292,12 +325,10 @@ struct DdGm {
 
 enum DdStepG { DDG_BNORM = 0, DDG_START, DDG_NORM, DDG_SOLVE };
 
-// ddGivensRotations (ddpgmres.f90:147-250) on column i (1-based).
-__device__ void dd_givens(const DdGm& g, int i) {
-  dd* col = g.h + (int64_t)(i - 1) * (g.m + 1);
-  dd* c = g.c;
-  dd* s = g.s;
-  dd* e = g.e;
+// ddGivensRotations (ddpgmres.f90:147-250) on column i (1-based): col holds the column's
+// i + 1 entries, c and s the earlier rotations (all may be shared-memory copies), e0 and e1
+// the rotated right-hand side's entries i and i + 1.
+__device__ void dd_givens(int i, dd* col, dd* c, dd* s, dd& e0, dd& e1) {
   for (int k = 1; k <= i - 1; ++k) {
     const dd t1 = dd_sub(dd_mul(col[k - 1], c[k - 1]), dd_mul(col[k], s[k - 1]));
     const dd t2 = dd_add(dd_mul(col[k - 1], s[k - 1]), dd_mul(col[k], c[k - 1]));
@@ -309,10 +340,10 @@ __device__ void dd_givens(const DdGm& g, int i) {
   const dd q = dd_sqrt(dd_add(dd{1.0, 0.0}, dd_mul(t, t)));
   c[i - 1] = dd_div(dd{1.0, 0.0}, q);
   s[i - 1] = dd_mul(dd{-1.0, 0.0}, dd_mul(c[i - 1], t));
-  const dd e1 = dd_sub(dd_mul(c[i - 1], e[i - 1]), dd_mul(s[i - 1], e[i]));
-  const dd e2 = dd_add(dd_mul(s[i - 1], e[i - 1]), dd_mul(c[i - 1], e[i]));
-  e[i - 1] = e1;
-  e[i] = e2;
+  const dd f0 = dd_sub(dd_mul(c[i - 1], e0), dd_mul(s[i - 1], e1));
+  const dd f1 = dd_add(dd_mul(s[i - 1], e0), dd_mul(c[i - 1], e1));
+  e0 = f0;
+  e1 = f1;
   col[i - 1] = dd_sub(dd_mul(c[i - 1], col[i - 1]), dd_mul(s[i - 1], col[i]));
   col[i] = dd{0.0, 0.0};
 }
@@ -340,7 +371,7 @@ __global__ void k_dd_gm_scal(DdGm g, int step, int i, const dd* d) {
       dd* col = g.h + (int64_t)(i - 1) * ld;
       col[i] = dd_sqrt(*d);
       *g.t1 = dd_div(dd{1.0, 0.0}, col[i]);
-      dd_givens(g, i);
+      dd_givens(i, col, g.c, g.s, g.e[i - 1], g.e[i]);
       *g.rn = fabs(g.e[i].hi);
       break;
     }
@@ -367,6 +398,141 @@ __global__ void k_dd_axpy_nh(int n, const dd* hk, const double* __restrict__ vh,
     wh[i] = w.hi;
     wl[i] = w.lo;
   }
+}
+
+// ddMGS_Orthonormalization (ddQRDecomposition.f90:4-46) of column i (1-based) against
+// v_1..v_i, its norm, v_{i+1} and the column's rotation in one cooperative launch.  CTA c owns
+// streams 1024 c.. of the fixed-order dot, so a thread's elements of w are its stream's and are
+// updated and multiplied in one pass: step p applies w -= h_{p-1} v_{p-1} and sums <w, v_p> (the
+// last step <w, w>).  Up to kDdMgsElems elements per thread stay in registers, longer
+// vectors keep w in memory (REG false).  Every CTA folds the same CTA sums in the same
+// order after a bounded grid barrier, so all hold the same bits.  The operations and their
+// order are those of the separate dots and updates.  Measured, 64^3, GMRES(30): 98 us per
+// column on average (5.9 us per step), where a step took a dot (8.9 us) and an update
+// (3.9 us) in two launches.
+constexpr int kDdMgsElems = 4;
+constexpr unsigned kDdBarrierLimit = 1u << 22;
+
+template <bool REG>
+__global__ void __launch_bounds__(kDdDotThreads, 1) k_dd_mgs(int64_t n, int i, const double* __restrict__ Vh,
+                                                           const double* __restrict__ Vl, int64_t ldv, double* wh,
+                                                           double* wl, double* nh, double* nl, DdGm g, dd* parts,
+                                                           unsigned* ctr, int* err, bool staged) {
+  __shared__ dd sm[32], sg[4], stot;
+  extern __shared__ dd sgiv[];   // CTA 0: column, c, s
+  const int64_t t = (int64_t)blockIdx.x * kDdDotThreads + threadIdx.x;
+  const int ld = g.m + 1;
+  dd* col = g.h + (int64_t)(i - 1) * ld;
+  dd w[REG ? kDdMgsElems : 1];
+  if constexpr (REG) {
+#pragma unroll
+    for (int u = 0; u < kDdMgsElems; ++u) {
+      const int64_t q = t + u * (int64_t)kDdStreams;
+      if (q < n) w[u] = dd{wh[q], wl[q]};
+    }
+  }
+  dd hprev{0.0, 0.0};
+  for (int p = 1; p <= i + 1; ++p) {
+    const double *uh = Vh + (int64_t)(p - 2) * ldv, *ul = Vl + (int64_t)(p - 2) * ldv;   // v_{p-1}
+    const double *dh = Vh + (int64_t)(p - 1) * ldv, *dl = Vl + (int64_t)(p - 1) * ldv;   // v_p
+    const dd a = dd_mul(dd{-1.0, 0.0}, hprev);
+    dd s{0.0, 0.0};
+    auto elem = [&](dd x, dd v, dd y) -> dd {
+      if (p > 1) x = dd_add(dd_mul(a, v), dd_mul(dd{1.0, 0.0}, x));
+      s = dd_add(s, dd_mul(x, p <= i ? y : x));
+      return x;
+    };
+    if constexpr (REG) {
+#pragma unroll
+      for (int u0 = 0; u0 < kDdMgsElems; u0 += 2) {   // the loads of two elements in flight
+        dd v[2], y[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int64_t q = t + (u0 + u) * (int64_t)kDdStreams;
+          v[u] = (p > 1 && q < n) ? dd{uh[q], ul[q]} : dd{0.0, 0.0};
+          y[u] = (p <= i && q < n) ? dd{dh[q], dl[q]} : dd{0.0, 0.0};
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          if (t + (u0 + u) * (int64_t)kDdStreams < n) w[u0 + u] = elem(w[u0 + u], v[u], y[u]);
+      }
+    } else {
+      for (int64_t q = t; q < n; q += kDdStreams) {
+        dd v{0.0, 0.0}, y{0.0, 0.0};
+        if (p > 1) v = dd{uh[q], ul[q]};
+        if (p <= i) y = dd{dh[q], dl[q]};
+        const dd x = elem(dd{wh[q], wl[q]}, v, y);
+        if (p > 1) { wh[q] = x.hi; wl[q] = x.lo; }
+      }
+    }
+    s = dd_block_tree(s, sm);
+    dd* pt = parts + (p & 1) * kDdDotCtas;
+    if (threadIdx.x == 0) {
+      pt[blockIdx.x] = s;
+      __threadfence();
+      atomicAdd(ctr + (p - 1), 1u);
+      unsigned it = 0;
+      while (*(volatile unsigned*)(ctr + (p - 1)) < gridDim.x)
+        if (++it > kDdBarrierLimit) { atomicExch(err, 1); break; }
+      __threadfence();
+    }
+    __syncthreads();
+    const dd tot = dd_grid_tree(pt, gridDim.x, sg);
+    if (threadIdx.x == 0) {
+      stot = tot;
+      if (blockIdx.x == 0 && p <= i) col[p - 1] = tot;
+    }
+    __syncthreads();
+    hprev = stot;
+  }
+  // v_{i+1} = (1 / |w|) w  (ddaxpy with beta = 0)
+  const dd nrm = dd_sqrt(hprev);
+  const dd t1 = dd_div(dd{1.0, 0.0}, nrm);
+  auto put = [&](dd x, int64_t q) {
+    const dd y = dd_add(dd_mul(t1, x), dd_mul(dd{0.0, 0.0}, dd{nh[q], nl[q]}));
+    nh[q] = y.hi;
+    nl[q] = y.lo;
+  };
+  if constexpr (REG) {
+#pragma unroll
+    for (int u = 0; u < kDdMgsElems; ++u) {
+      const int64_t q = t + u * (int64_t)kDdStreams;
+      if (q < n) put(w[u], q);
+    }
+  } else {
+    for (int64_t q = t; q < n; q += kDdStreams) put(dd{wh[q], wl[q]}, q);
+  }
+  if (blockIdx.x != 0) return;
+  // DDG_NORM's work on this column, staged in shared memory when the launch gave it room
+  if (!staged) {
+    if (threadIdx.x == 0) {
+      *g.t1 = t1;
+      col[i] = nrm;
+      dd_givens(i, col, g.c, g.s, g.e[i - 1], g.e[i]);
+      *g.rn = fabs(g.e[i].hi);
+    }
+    return;
+  }
+  dd *sc = sgiv + ld, *ss = sgiv + 2 * ld;
+  for (int k = threadIdx.x; k < i; k += kDdDotThreads) {
+    sgiv[k] = col[k];   // written by this CTA's thread 0, ordered by the block barriers
+    sc[k] = g.c[k];
+    ss[k] = g.s[k];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    *g.t1 = t1;
+    sgiv[i] = nrm;
+    dd e0 = g.e[i - 1], e1 = g.e[i];
+    dd_givens(i, sgiv, sc, ss, e0, e1);
+    g.c[i - 1] = sc[i - 1];
+    g.s[i - 1] = ss[i - 1];
+    g.e[i - 1] = e0;
+    g.e[i] = e1;
+    *g.rn = fabs(e1.hi);
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k <= i; k += kDdDotThreads) col[k] = sgiv[k];
 }
 
 // The subtractions of ddCGS_Orthonormalization (ddQRDecomposition.f90:73-86),
@@ -826,11 +992,16 @@ struct DdSystem {
   const double* al = nullptr;   // null: A's low parts are zero
 };
 
-// part: kDdDotCtas CTA sums followed by the ticket counter (zero between dots).
-void dd_dot(const DdSystem& S, const double* xh, const double* xl, const double* yh, const double* yl, dd* part,
-            dd* out, cudaStream_t st) {
-  k_dd_dot<<<kDdDotCtas, kDdDotThreads, 0, st>>>(S.n, xh, xl, yh, yl, part,
-                                                reinterpret_cast<unsigned*>(part + kDdDotCtas), out);
+// part: 2 kDdDotCtas CTA sums followed by the ticket counter (zero between dots).
+inline int dd_dot_grid(int64_t n) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(kDdDotCtas, (n + kDdDotThreads - 1) / kDdDotThreads));
+}
+template <int MODE>
+void dd_dots(const DdSystem& S, const double* xh, const double* xl, const double* yh, const double* yl, dd* part,
+             dd* out, dd* out2, cudaStream_t st) {
+  k_dd_dot<MODE><<<dd_dot_grid(S.n), kDdDotThreads, 0, st>>>(S.n, xh, xl, yh, yl, part,
+                                                            reinterpret_cast<unsigned*>(part + 2 * kDdDotCtas), out,
+                                                            out2);
 }
 
 void dd_setup_precon(const Options& o, const parcel_b_crs& A, const DdSystem& S, int prec_M, DdPrecon& P) {
@@ -1003,9 +1174,16 @@ struct DdRun {
   }
   void spmv(const DdVec& x, DdVec& y) const { spmv(x.hi(), x.lo(), y.hi(), y.lo()); }
   void dot(const double* xh, const double* xl, const double* yh, const double* yl, dd* out) const {
-    dd_dot(S, xh, xl, yh, yl, part, out, st);
+    dd_dots<0>(S, xh, xl, yh, yl, part, out, nullptr, st);
   }
   void dot(const DdVec& u, const DdVec& v, DBuf& out) const { dot(u.hi(), u.lo(), v.hi(), v.lo(), dp<dd>(out)); }
+  // <u, v> and <v, v>, or <u, v> and <u, u>, in one pass
+  void dot_vv(const DdVec& u, const DdVec& v, DBuf& uv, DBuf& vv) const {
+    dd_dots<1>(S, u.hi(), u.lo(), v.hi(), v.lo(), part, dp<dd>(uv), dp<dd>(vv), st);
+  }
+  void dot_uu(const DdVec& u, const DdVec& v, DBuf& uv, DBuf& uu) const {
+    dd_dots<2>(S, u.hi(), u.lo(), v.hi(), v.lo(), part, dp<dd>(uv), dp<dd>(uu), st);
+  }
   // y = alpha x + beta y (ddaxpy)
   void axpy(const dd* alpha, const dd* beta, const double* xh, const double* xl, double* yh, double* yl) const {
     k_dd_axpy<<<g, kDdThreads, 0, st>>>(n, alpha, beta, xh, xl, yh, yl);
@@ -1063,8 +1241,7 @@ DdLoop dd_cg_loop(const DdRun& R, const Options& o, DdVec& x, const DdVec& b, do
     k_dd_scal<<<1, 32, 0, st>>>(sc, DD_ALPHA, dp<dd>(d1), nullptr);
     R.axpy(&sc->t1, R.one, q.hi(), q.lo(), r.hi(), r.lo());
     R.precon(r.hi(), r.lo(), s.hi(), s.lo());
-    R.dot(s, r, d1);
-    R.dot(r, r, d2);
+    R.dot_vv(s, r, d1, d2);
     k_dd_scal<<<1, 32, 0, st>>>(sc, DD_RNORM, dp<dd>(d1), dp<dd>(d2));
     PB_CUDA(cudaGetLastError());
     rnorm = read_double(&sc->rnorm.hi, st);
@@ -1110,13 +1287,11 @@ DdLoop dd_bicg_loop(const DdRun& R, const Options& o, DdVec& x, const DdVec& b, 
     k_dd_bicg_axpy3<<<g, kDdThreads, 0, st>>>(n, sb, r.hi(), r.lo(), q.hi(), q.lo(), e.hi(), e.lo());
     R.precon(e.hi(), e.lo(), pe.hi(), pe.lo());
     R.spmv(pe, v);
-    R.dot(e, v, d1);
-    R.dot(v, v, d2);
+    R.dot_vv(e, v, d1, d2);
     k_dd_scal_b<<<1, 32, 0, st>>>(sb, DDB_C3, dp<dd>(d1), dp<dd>(d2));
     k_dd_bicg_axpy4<<<g, kDdThreads, 0, st>>>(n, sb, x.hi(), x.lo(), pp.hi(), pp.lo(), pe.hi(), pe.lo());
     k_dd_bicg_axpy3r<<<g, kDdThreads, 0, st>>>(n, sb, e.hi(), e.lo(), v.hi(), v.lo(), r.hi(), r.lo());
-    R.dot(r, r0, d1);
-    R.dot(r, r, d2);
+    R.dot_uu(r, r0, d1, d2);
     k_dd_scal_b<<<1, 32, 0, st>>>(sb, DDB_RNORM, dp<dd>(d1), dp<dd>(d2));
     PB_CUDA(cudaGetLastError());
     double rn[2];
@@ -1174,6 +1349,28 @@ DdLoop dd_gmres_loop(const DdRun& R, const Options& o, DdVec& x, const DdVec& b,
   auto hist_at = [&](int k, double v) {   // 1-based entry k
     if (reshistory && k >= 1 && k <= o.itrmax) reshistory[k - 1] = v;
   };
+  // one launch per MGS column: two sets of CTA sums, a counter per grid barrier (zeroed before
+  // every launch) and the error flag of the barrier's bounded wait
+  DBuf mparts(sizeof(dd) * 2 * kDdDotCtas), mctr(sizeof(unsigned) * ((size_t)m + 2)), merr(sizeof(int));
+  auto mgs_column = [&](int i) {
+    PB_CUDA(cudaMemsetAsync(mctr.p, 0, sizeof(unsigned) * ((size_t)i + 1), st));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(dd_dot_grid(n));
+    cfg.blockDim = dim3(kDdDotThreads);
+    const size_t givens_bytes = sizeof(dd) * 3 * (size_t)ld;
+    const bool staged = givens_bytes <= 32 * 1024;
+    cfg.dynamicSmemBytes = staged ? givens_bytes : 0;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const bool reg = n <= kDdMgsElems * kDdStreams;
+    PB_CUDA(cudaLaunchKernelEx(&cfg, reg ? k_dd_mgs<true> : k_dd_mgs<false>, (int64_t)n, i,
+                               (const double*)dp<double>(Vh), (const double*)dp<double>(Vl), ldv, w.hi(), w.lo(), vh(i),
+                               vl(i), G, dp<dd>(mparts), dp<unsigned>(mctr), dp<int>(merr), staged));
+  };
   double rnorm = 0.0;
   int itr = 1, inner = 1, mm = 0;
   for (itr = 1; itr <= o.itrmax; itr += m) {
@@ -1190,20 +1387,18 @@ DdLoop dd_gmres_loop(const DdRun& R, const Options& o, DdVec& x, const DdVec& b,
       R.spmv(pv, w);
       dd* col = G.h + (int64_t)(inner - 1) * ld;
       if (mgs) {
-        for (int k = 1; k < inner; ++k) {
-          R.dot(w.hi(), w.lo(), vh(k - 1), vl(k - 1), col + (k - 1));
-          k_dd_axpy_nh<<<g, kDdThreads, 0, st>>>(n, col + (k - 1), vh(k - 1), vl(k - 1), w.hi(), w.lo());
-        }
-      } else if (inner > 1) {
+        mgs_column(inner);
+      } else {
         for (int k = 1; k < inner; ++k) R.dot(vh(k - 1), vl(k - 1), w.hi(), w.lo(), col + (k - 1));
-        k_dd_cgs_sub<<<g, kDdThreads, 0, st>>>(n, inner - 1, col, dp<double>(Vh), dp<double>(Vl), ldv, w.hi(),
-                                               w.lo());
+        if (inner > 1)
+          k_dd_cgs_sub<<<g, kDdThreads, 0, st>>>(n, inner - 1, col, dp<double>(Vh), dp<double>(Vl), ldv, w.hi(),
+                                                 w.lo());
+        R.dot(w.hi(), w.lo(), vh(inner - 1), vl(inner - 1), col + (inner - 1));
+        k_dd_axpy_nh<<<g, kDdThreads, 0, st>>>(n, col + (inner - 1), vh(inner - 1), vl(inner - 1), w.hi(), w.lo());
+        R.dot(w, w, d1);
+        k_dd_gm_scal<<<1, 32, 0, st>>>(G, DDG_NORM, inner, dp<dd>(d1));
+        R.axpy(G.t1, R.zero, w.hi(), w.lo(), vh(inner), vl(inner));   // v_{i+1} = w / |w|
       }
-      R.dot(w.hi(), w.lo(), vh(inner - 1), vl(inner - 1), col + (inner - 1));
-      k_dd_axpy_nh<<<g, kDdThreads, 0, st>>>(n, col + (inner - 1), vh(inner - 1), vl(inner - 1), w.hi(), w.lo());
-      R.dot(w, w, d1);
-      k_dd_gm_scal<<<1, 32, 0, st>>>(G, DDG_NORM, inner, dp<dd>(d1));
-      R.axpy(G.t1, R.zero, w.hi(), w.lo(), vh(inner), vl(inner));   // v_{i+1} = w / |w|
       PB_CUDA(cudaGetLastError());
       rnorm = read_double(G.rn, st);
       mm = inner;
@@ -1221,7 +1416,9 @@ DdLoop dd_gmres_loop(const DdRun& R, const Options& o, DdVec& x, const DdVec& b,
     if (rnorm / bnorm < o.rtol) break;
     if (itr + inner == o.itrmax) break;
   }
-  sync();
+  int merr_h = 0;
+  d2h(&merr_h, merr.p, sizeof(int));
+  PB_CHECK(merr_h == 0, PARCEL_B_E_CUDA, "dd MGS grid barrier timed out");
   L.used = std::min(o.itrmax, itr + inner);
   L.iret = (o.itrmax <= itr) ? 1 : 0;
   return L;
@@ -1269,7 +1466,7 @@ int dd_krylov(int solver, const parcel_b_input* prm, const parcel_b_crs* A, cons
     };
     load(x, x_hi, x_lo, precision_x == 2);
     load(b, b_hi, b_lo, precision_b == 2);
-    DBuf part(sizeof(dd) * (kDdDotCtas + 1)), cst(sizeof(dd) * 3);
+    DBuf part(sizeof(dd) * (2 * kDdDotCtas + 1)), cst(sizeof(dd) * 3);
     dd* dcst = dp<dd>(cst);
     {
       const dd h[3] = {dd{1.0, 0.0}, dd{-1.0, 0.0}, dd{0.0, 0.0}};

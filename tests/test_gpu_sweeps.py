@@ -112,3 +112,19 @@ def test_dd_products_near_the_ends_of_the_range(exponent):
     A = problems.poisson3d_reference(12, 12, 12)[0]
     b = problems.rhs_normal(A.n, 3) * 2.0 ** exponent
     _dd_both(A, b, solver=1, itrmax=20, rtolmax=1e-13, ipreflag=2, ILU_method=1, precon_thblock=3)
+
+
+@pytest.mark.parametrize("n,m,itrmax", [(524288, 3, 5), (524289, 3, 5), (700001, 4, 6), (1000, 700, 12), (3, 5, 4)])
+def test_dd_mgs_column_sizes(n, m, itrmax):
+    """Basis vectors at and past the register-resident length, a restart length whose rotations
+    do not fit shared memory, and fewer rows than a CTA has threads."""
+    i = np.arange(n)
+    cols, vals = [i - 1, i, i + 1], [-1.1, 4.0 + (i % 7) * 0.25, -0.9]
+    mask = [i > 0, i >= 0, i < n - 1]
+    C3 = np.stack(cols, 1)
+    V3 = np.stack([np.broadcast_to(v, n) for v in vals], 1)
+    M3 = np.stack(mask, 1)
+    rp = np.concatenate([[0], np.cumsum(M3.sum(1))]) + 1
+    A = problems.CRS(n=n, rowptr=rp.astype(np.int32), col=(C3[M3] + 1).astype(np.int32), val=V3[M3].astype(float))
+    _dd_both(A, problems.rhs_normal(n, 8), solver=3, itrmax=itrmax, rtolmax=1e-28, GMRES_m=m, GMRES_GSflag=1,
+             ipreflag=1)
