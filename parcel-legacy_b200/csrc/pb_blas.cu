@@ -270,8 +270,9 @@ __global__ void k_gm_backsolve(const double* h, const double* e, double* y, int 
 
 // After the restart cycle's update: exit test of pgmres.f90 (after update_xVec) and the
 // loop increment itr += m.
-__global__ void k_gm_post(KState* st, int m, int itrmax) {
+__global__ void k_gm_post(KState* st, int m) {
   if (st->done) return;
+  const int itrmax = st->itrmax;
   const int itr = st->itr;
   const int inner_end = st->stop_after_update ? st->inner : m + 1;
   if (st->stop_after_update) {
@@ -376,8 +377,8 @@ void gm_backsolve(const double* h, const double* e, double* y, int m0, KState* s
   PB_CUDA(cudaGetLastError());
 }
 
-void gm_post(KState* st, int m, int itrmax, cudaStream_t s_) {
-  k_gm_post<<<1, 1, 0, s_>>>(st, m, itrmax);
+void gm_post(KState* st, int m, cudaStream_t s_) {
+  k_gm_post<<<1, 1, 0, s_>>>(st, m);
   PB_CUDA(cudaGetLastError());
 }
 

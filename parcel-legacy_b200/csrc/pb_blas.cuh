@@ -42,7 +42,7 @@ void sum_vec(int64_t n, T* v0, const T* V, int64_t ldv, const double* y, const K
              const int* gate, cudaStream_t s_);
 void gm_backsolve(const double* h, const double* e, double* y, int m0, KState* st, const int* gate,
                   cudaStream_t s_);
-void gm_post(KState* st, int m, int itrmax, cudaStream_t s_);
+void gm_post(KState* st, int m, cudaStream_t s_);
 void fill(int64_t n, double* p, double v, cudaStream_t st);
 template <class TO, class TI>
 void convert(int64_t n, TO* o, const TI* in, cudaStream_t st);

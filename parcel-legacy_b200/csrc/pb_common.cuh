@@ -110,7 +110,8 @@ struct KState {
   int skip_inner;                          // GMRES: inner loop has exited this cycle
   int stop_after_update;                   // GMRES: exit the solve after update_xVec
   int last_inner;                          // GMRES: Fortran `inner` after the last cycle
-  int pad[5];
+  int itrmax;                              // iteration limit of this solve
+  int pad[4];
   __host__ __device__ int mm_prev_inner() const { return last_inner; }
 };
 

@@ -21,7 +21,6 @@ struct EpiArgs {
   double* sn = nullptr;
   double* out = nullptr;     // EPI_STORE destination
   int m = 0;
-  int itrmax = 0;
   double rtol = 0.0;
   double abstol = 0.0;
   int k = 0, j = 0;          // MGS indices of the value being reduced

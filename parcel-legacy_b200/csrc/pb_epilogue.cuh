@@ -61,7 +61,7 @@ static __device__ void epilogue(const double* S, int K, const Red& r) {
       st->done = 0;
       st->niter = 0;
       st->iret = 0;
-      if (a.itrmax < 1) { st->done = 1; st->iret = 1; break; }
+      if (st->itrmax < 1) { st->done = 1; st->iret = 1; break; }
       a.hist[0] = st->rnorm / st->bnorm;
       if (bad(st->rho0) || bad(st->bnorm)) { st->done = 1; st->breakdown = 1; st->niter = 1; }
       break;
@@ -78,18 +78,18 @@ static __device__ void epilogue(const double* S, int K, const Red& r) {
       const int itr = st->itr;
       double rel = rn / st->bnorm;
       if (rel < a.rtol) {
-        st->done = 1; st->niter = min(a.itrmax, itr); st->iret = (a.itrmax <= itr) ? 1 : 0;
+        st->done = 1; st->niter = min(st->itrmax, itr); st->iret = (st->itrmax <= itr) ? 1 : 0;
       } else if (rel > 1.0e8) {
-        st->done = 1; st->diverged = 1; st->niter = min(a.itrmax, itr);
-        st->iret = (a.itrmax <= itr) ? 1 : 0;
+        st->done = 1; st->diverged = 1; st->niter = min(st->itrmax, itr);
+        st->iret = (st->itrmax <= itr) ? 1 : 0;
       } else if (bad(rel) || bad(st->rho1)) {
-        st->done = 1; st->breakdown = 1; st->niter = min(a.itrmax, itr);
+        st->done = 1; st->breakdown = 1; st->niter = min(st->itrmax, itr);
         st->iret = PARCEL_B_E_BREAKDOWN;
       } else {
         st->beta = st->rho1 / st->rho0;
         st->rho0 = st->rho1;
-        if (itr + 1 > a.itrmax) {
-          st->done = 1; st->niter = a.itrmax; st->iret = 1;
+        if (itr + 1 > st->itrmax) {
+          st->done = 1; st->niter = st->itrmax; st->iret = 1;
         } else {
           st->itr = itr + 1;
           a.hist[itr] = rn / st->bnorm;
@@ -104,7 +104,7 @@ static __device__ void epilogue(const double* S, int K, const Red& r) {
       st->c1 = S[1];   // <r0, r0> with r0 = r
       st->c2 = 0.0; st->c3 = 0.0;
       st->itr = 1; st->done = 0; st->niter = 0; st->iret = 0;
-      if (a.itrmax < 1) { st->done = 1; st->iret = 1; break; }
+      if (st->itrmax < 1) { st->done = 1; st->iret = 1; break; }
       a.hist[0] = st->rnorm / st->bnorm;
       break;
     case EPI_BICG_C2:
@@ -125,15 +125,15 @@ static __device__ void epilogue(const double* S, int K, const Red& r) {
       const int itr = st->itr;
       double rel = rn / st->bnorm;
       if (rel < a.rtol) {
-        st->done = 1; st->niter = min(a.itrmax, itr); st->iret = (a.itrmax <= itr) ? 1 : 0;
+        st->done = 1; st->niter = min(st->itrmax, itr); st->iret = (st->itrmax <= itr) ? 1 : 0;
       } else if (bad(rel) || bad(st->c1)) {
-        st->done = 1; st->breakdown = 1; st->niter = min(a.itrmax, itr);
+        st->done = 1; st->breakdown = 1; st->niter = min(st->itrmax, itr);
         st->iret = PARCEL_B_E_BREAKDOWN;
       } else {
         st->beta = st->c1 / (st->c3 * st->c2);
         st->tmp[2] = -st->beta * st->c3;
-        if (itr + 1 > a.itrmax) {
-          st->done = 1; st->niter = a.itrmax; st->iret = 1;
+        if (itr + 1 > st->itrmax) {
+          st->done = 1; st->niter = st->itrmax; st->iret = 1;
         } else {
           st->itr = itr + 1;
           a.hist[itr] = rn / st->bnorm;
@@ -154,9 +154,9 @@ static __device__ void epilogue(const double* S, int K, const Red& r) {
       if (rn < a.abstol || rn / st->bnorm < a.rtol) {
         // exit at the top of the restart loop: niter = min(itrmax, itr + inner)
         st->done = 1;
-        st->niter = min(a.itrmax, itr + st->last_inner);
+        st->niter = min(st->itrmax, itr + st->last_inner);
         st->skip_inner = 1;
-        st->iret = (a.itrmax <= itr) ? 1 : 0;
+        st->iret = (st->itrmax <= itr) ? 1 : 0;
         break;
       }
       if (bad(rn)) { st->done = 1; st->skip_inner = 1; st->breakdown = 1; st->iret = PARCEL_B_E_BREAKDOWN; st->niter = itr; break; }
@@ -182,7 +182,7 @@ static __device__ void epilogue(const double* S, int K, const Red& r) {
       const int itr = st->itr;
       a.hist[itr + j - 1] = rn / st->bnorm;
       if (rn / st->bnorm < a.rtol) { st->skip_inner = 1; st->stop_after_update = 1; }
-      else if (itr + j == a.itrmax) { st->skip_inner = 1; st->stop_after_update = 1; }
+      else if (itr + j == st->itrmax) { st->skip_inner = 1; st->stop_after_update = 1; }
       else if (bad(rn)) { st->skip_inner = 1; st->stop_after_update = 1; st->breakdown = 1; }
       break;
     }

@@ -69,6 +69,7 @@ MixedResult solve_mixed_on(const Options& o, System<float>& S, const double* b, 
   if (setup_t) *setup_t = now_s();
   Options oi = o;
   oi.rtol = o.inner_rtol;
+  KrylovWork work;   // the corrections share their vectors and captured iterations
   int total = 0;
   hist.clear();
   double rel = 1.0;
@@ -92,7 +93,7 @@ MixedResult solve_mixed_on(const Options& o, System<float>& S, const double* b, 
     PB_CUDA(cudaMemsetAsync(d32.p, 0, sizeof(float) * np, st));
     oi.itrmax = o.itrmax - total;
     trace_mark("refine: outer residual");
-    SolveOut so = run_krylov<float>(oi, S, dp<float>(r32), dp<float>(d32), dp<double>(hist_dev));
+    SolveOut so = run_krylov<float>(oi, S, dp<float>(r32), dp<float>(d32), dp<double>(hist_dev), &work);
     trace_mark("refine: inner solve");
     res.launches += so.launches + 2;
     if (so.niter > 0) {

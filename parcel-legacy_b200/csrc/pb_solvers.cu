@@ -272,37 +272,6 @@ void build_system(const Options& o, const parcel_b_crs& A, bool dev, System<T>& 
 }
 
 // ------------------------------------------------------------------ graph replay
-struct GraphRunner {
-  cudaGraphExec_t exec = nullptr;
-  int launches = 0;
-  GraphRunner() = default;
-  GraphRunner(const GraphRunner&) = delete;
-  ~GraphRunner() { if (exec) cudaGraphExecDestroy(exec); }
-  template <class F>
-  void launch(F&& f, bool use_graph, cudaStream_t st) {
-    if (!use_graph) { f(); return; }
-    if (!exec) {
-      trace_mark(nullptr);
-      cudaGraph_t g = nullptr;
-      PB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-      try {
-        f();
-      } catch (...) {
-        cudaGraph_t g2 = nullptr;
-        cudaStreamEndCapture(st, &g2);
-        if (g2) cudaGraphDestroy(g2);
-        throw;
-      }
-      PB_CUDA(cudaStreamEndCapture(st, &g));
-      PB_CUDA(cudaGraphInstantiate(&exec, g, 0));
-      cudaGraphDestroy(g);
-      trace_mark("graph: capture + instantiate");
-    }
-    PB_CUDA(cudaGraphLaunch(exec, st));
-    trace_mark("graph: replay");
-  }
-};
-
 static int read_done(const KState* st, cudaStream_t s) {
   static int* pinned = nullptr;
   if (!pinned) PB_CUDA(cudaMallocHost(&pinned, sizeof(int)));
@@ -317,28 +286,30 @@ static KState read_state(const KState* st) {
   return h;
 }
 
-static void init_state(Workspace& W, int itr0) {
+static void init_state(Workspace& W, int itr0, int itrmax) {
   KState h;
   memset(&h, 0, sizeof(h));
   h.itr = itr0;
   h.last_inner = 1;
+  h.itrmax = itrmax;
   h2d(W.state.p, &h, sizeof(KState));
 }
 
 // ------------------------------------------------------------------ PCG
 template <class T>
 static SolveOut run_pcg(const Options& o, const System<T>& S, const T* b, T* x, double* hist,
-                        Workspace& W) {
+                        KrylovWork& kw) {
   cudaStream_t st = stream();
+  Workspace& W = kw.W;
   const int64_t np = S.np;
-  DBuf r(sizeof(T) * np), p(sizeof(T) * np), q(sizeof(T) * np), s(sizeof(T) * np);
-  T* R = dp<T>(r); T* P = dp<T>(p); T* Q = dp<T>(q); T* Sv = dp<T>(s);
+  const size_t vb = sizeof(T) * np;
+  T *R = kw.buf<T>(vb), *P = kw.buf<T>(vb), *Q = kw.buf<T>(vb), *Sv = kw.buf<T>(vb);
   KState* K = W.st();
-  init_state(W, 1);
+  init_state(W, 1, o.itrmax);
   const int* gdone = &K->done;
   auto red = [&](int epi) {
     Red rr = W.red(epi);
-    rr.ea.hist = hist; rr.ea.itrmax = o.itrmax; rr.ea.rtol = o.rtol; rr.ea.abstol = o.abstol;
+    rr.ea.hist = hist; rr.ea.rtol = o.rtol; rr.ea.abstol = o.abstol;
     return rr;
   };
   int launches = 0;
@@ -368,7 +339,7 @@ static SolveOut run_pcg(const Options& o, const System<T>& S, const T* b, T* x, 
                      red(EPI_CG_DOT2), gdone, st);
     }
   };
-  GraphRunner G;
+  GraphRunner& G = kw.G;
   const int max_chunks = o.itrmax / chunk + 2;
   for (int c = 0; c < max_chunks; ++c) {
     if (read_done(K, st)) break;
@@ -390,19 +361,19 @@ static SolveOut run_pcg(const Options& o, const System<T>& S, const T* b, T* x, 
 // ------------------------------------------------------------------ BiCGStab
 template <class T>
 static SolveOut run_bicg(const Options& o, const System<T>& S, const T* b, T* x, double* hist,
-                         Workspace& W) {
+                         KrylovWork& kw) {
   cudaStream_t st = stream();
+  Workspace& W = kw.W;
   const int64_t np = S.np;
   const size_t vb = sizeof(T) * np;
-  DBuf r(vb), r0(vb), p(vb), q(vb), pp(vb), e(vb), pe(vb), v(vb);
-  T *R = dp<T>(r), *R0 = dp<T>(r0), *P = dp<T>(p), *Q = dp<T>(q), *PP = dp<T>(pp),
-    *E = dp<T>(e), *PE = dp<T>(pe), *V = dp<T>(v);
+  T *R = kw.buf<T>(vb), *R0 = kw.buf<T>(vb), *P = kw.buf<T>(vb), *Q = kw.buf<T>(vb), *PP = kw.buf<T>(vb),
+    *E = kw.buf<T>(vb), *PE = kw.buf<T>(vb), *V = kw.buf<T>(vb);
   KState* K = W.st();
-  init_state(W, 1);
+  init_state(W, 1, o.itrmax);
   const int* gdone = &K->done;
   auto red = [&](int epi) {
     Red rr = W.red(epi);
-    rr.ea.hist = hist; rr.ea.itrmax = o.itrmax; rr.ea.rtol = o.rtol;
+    rr.ea.hist = hist; rr.ea.rtol = o.rtol;
     return rr;
   };
   int launches = 0;
@@ -434,7 +405,7 @@ static SolveOut run_bicg(const Options& o, const System<T>& S, const T* b, T* x,
       lincomb<T>(np, P, R, cimm(1.0), Q, cdev(&K->tmp[2]), P, cdev(&K->beta), gdone, st);  // p = r - beta c3 q + beta p
     }
   };
-  GraphRunner G;
+  GraphRunner& G = kw.G;
   const int max_chunks = o.itrmax / chunk + 2;
   for (int c = 0; c < max_chunks; ++c) {
     if (read_done(K, st)) break;
@@ -453,20 +424,20 @@ static SolveOut run_bicg(const Options& o, const System<T>& S, const T* b, T* x,
 // ------------------------------------------------------------------ GMRES(m)
 template <class T>
 static SolveOut run_gmres(const Options& o, const System<T>& S, const T* b, T* x, double* hist,
-                          Workspace& W) {
+                          KrylovWork& kw) {
   cudaStream_t st = stream();
+  Workspace& W = kw.W;
   const int64_t np = S.np;
   const int m = o.m;
   PB_CHECK(m >= 1 && m < kMaxRed, PARCEL_B_E_ARG, "GMRES restart length %d outside [1, %d)", m, kMaxRed);
   const int64_t ldv = (np + 31) & ~int64_t(31);
   const size_t vb = sizeof(T) * np;
-  DBuf r(vb), Vb(sizeof(T) * ldv * (m + 1)), pv(vb), w(vb), v0(vb), x0(vb);
+  T *R = kw.buf<T>(vb), *V = kw.buf<T>(sizeof(T) * ldv * (m + 1)), *PV = kw.buf<T>(vb), *Wv = kw.buf<T>(vb),
+    *V0 = kw.buf<T>(vb), *X0 = kw.buf<T>(vb);   // zero-filled: the tails past np stay zero
   // Flexible GMRES keeps z_j = M_j^-1 v_j (the preconditioner may change between
   // columns) and updates x with Z y instead of M^-1 V y.
   const bool flex = o.flexible || S.extra != nullptr;
-  DBuf Zb;
-  if (flex) Zb.alloc(sizeof(T) * ldv * m);
-  T* Z = dp<T>(Zb);
+  T* Z = flex ? kw.buf<T>(sizeof(T) * ldv * m) : nullptr;
   // precon(in, out, az): out = M^-1 in (+ the extra stage); with the extra stage and az
   // given, az = A out comes from the stage and the caller's SpMV is skipped.
   auto precon = [&](const T* in, T* out, T* az, const int* gate) {
@@ -475,20 +446,18 @@ static SolveOut run_gmres(const Options& o, const System<T>& S, const T* b, T* x
     if (S.extra) S.extra->apply(S, in, out, az, gate, st);
   };
   const int precon_launches = 1 + (S.extra ? S.extra->launches() : 0);
-  DBuf hb(sizeof(double) * (m + 1) * m), eb(sizeof(double) * (m + 1)), csb(sizeof(double) * (m + 1)),
-      snb(sizeof(double) * (m + 1)), yb(sizeof(double) * (m + 1));
-  T *R = dp<T>(r), *V = dp<T>(Vb), *PV = dp<T>(pv), *Wv = dp<T>(w), *V0 = dp<T>(v0),
-    *X0 = dp<T>(x0);
-  PB_CUDA(cudaMemsetAsync(V, 0, sizeof(T) * ldv * (m + 1), st));
+  const size_t mb = sizeof(double) * (m + 1);
+  double *hb = kw.buf<double>(mb * m), *eb = kw.buf<double>(mb), *csb = kw.buf<double>(mb), *snb = kw.buf<double>(mb),
+         *yb = kw.buf<double>(mb);
   KState* K = W.st();
-  init_state(W, 1);
+  init_state(W, 1, o.itrmax);
   const int* gdone = &K->done;
   const int* gskip = &K->skip_inner;
   auto red = [&](int epi, int k = 0, int j = 0) {
     Red rr = W.red(epi);
-    rr.ea.hist = hist; rr.ea.itrmax = o.itrmax; rr.ea.rtol = o.rtol; rr.ea.abstol = o.abstol;
-    rr.ea.h = dp<double>(hb); rr.ea.e = dp<double>(eb); rr.ea.cs = dp<double>(csb);
-    rr.ea.sn = dp<double>(snb); rr.ea.m = m; rr.ea.k = k; rr.ea.j = j;
+    rr.ea.hist = hist; rr.ea.rtol = o.rtol; rr.ea.abstol = o.abstol;
+    rr.ea.h = hb; rr.ea.e = eb; rr.ea.cs = csb;
+    rr.ea.sn = snb; rr.ea.m = m; rr.ea.k = k; rr.ea.j = j;
     return rr;
   };
   int launches = 0;
@@ -507,18 +476,19 @@ static SolveOut run_gmres(const Options& o, const System<T>& S, const T* b, T* x
   // cycle as all-ones bytes; the others through per-(column, pass) counters that start at 0.
   const bool staged_mgs = fused_mgs && mgs_staged<T>(np);
   const size_t nslots = (size_t)m * (m + 2) * (size_t)(num_sms() + 1);   // partials, then totals
-  DBuf mparts(sizeof(double) * 2 * (size_t)std::max(1, mgs_grid<T>())),
-      mctr(sizeof(unsigned) * (size_t)m * (m + 2)), merr(sizeof(int)),
-      mslots(staged_mgs ? sizeof(double) * nslots : 0);
-  PB_CUDA(cudaMemsetAsync(merr.p, 0, sizeof(int), st));
-  int per_cycle = 0;
+  double* mparts = kw.buf<double>(sizeof(double) * 2 * (size_t)std::max(1, mgs_grid<T>()));
+  unsigned* mctr = kw.buf<unsigned>(sizeof(unsigned) * (size_t)m * (m + 2));
+  int* merr = kw.buf<int>(sizeof(int));
+  double* mslots = staged_mgs ? kw.buf<double>(sizeof(double) * nslots) : nullptr;
+  PB_CUDA(cudaMemsetAsync(merr, 0, sizeof(int), st));
+  int& per_cycle = kw.per_cycle;   // counted when the cycle is captured
   auto cycle = [&] {
     per_cycle = 0;
     if (staged_mgs) {
-      PB_CUDA(cudaMemsetAsync(mslots.p, 0xFF, sizeof(double) * nslots, st));
+      PB_CUDA(cudaMemsetAsync(mslots, 0xFF, sizeof(double) * nslots, st));
       ++per_cycle;
     } else if (fused_mgs) {
-      PB_CUDA(cudaMemsetAsync(mctr.p, 0, sizeof(unsigned) * (size_t)m * (m + 2), st));
+      PB_CUDA(cudaMemsetAsync(mctr, 0, sizeof(unsigned) * (size_t)m * (m + 2), st));
       ++per_cycle;
     }
     int sa[2] = {0, 0}, sb[2] = {0, 0};
@@ -537,7 +507,7 @@ static SolveOut run_gmres(const Options& o, const System<T>& S, const T* b, T* x
       if (o.gs == PARCEL_B_GS_CGS) {
         spmv<T, T>(S.A, Pj, Wv, SPMV_Y, nullptr, gskip, st);
         multidot<T>(np, j, Wv, V, ldv, red(EPI_GM_HCGS, 0, j), gskip, st);
-        cgs_update<T>(np, j, Wv, V, ldv, dp<double>(hb) + (size_t)(j - 1) * (m + 1), red(EPI_GM_NORM, 0, j),
+        cgs_update<T>(np, j, Wv, V, ldv, hb + (size_t)(j - 1) * (m + 1), red(EPI_GM_NORM, 0, j),
                       gskip, st);
         per_cycle += 3;
       } else if (fused_mgs) {
@@ -545,13 +515,13 @@ static SolveOut run_gmres(const Options& o, const System<T>& S, const T* b, T* x
         MgsArgs<T> ma;
         ma.np = np; ma.j = j; ma.w = Wv; ma.V = V; ma.ldv = ldv;
         ma.vnext = (j < m) ? V + (size_t)j * ldv : nullptr;
-        ma.parts = dp<double>(mparts);
-        ma.ctr = dp<unsigned>(mctr) + (size_t)(j - 1) * (m + 2);
+        ma.parts = mparts;
+        ma.ctr = mctr + (size_t)(j - 1) * (m + 2);
         if (staged_mgs) {
-          ma.slots = dp<double>(mslots) + (size_t)(j - 1) * (m + 2) * num_sms();
-          ma.totals = dp<double>(mslots) + (size_t)m * (m + 2) * num_sms() + (size_t)(j - 1) * (m + 2);
+          ma.slots = mslots + (size_t)(j - 1) * (m + 2) * num_sms();
+          ma.totals = mslots + (size_t)m * (m + 2) * num_sms() + (size_t)(j - 1) * (m + 2);
         }
-        ma.err = dp<int>(merr);
+        ma.err = merr;
         ma.gate = gskip;
         ma.red = red(EPI_GM_NORM, 0, j);
         mgs_column<T>(ma, st);
@@ -577,19 +547,19 @@ static SolveOut run_gmres(const Options& o, const System<T>& S, const T* b, T* x
       }
     }
     // update_xVec: y = H^-1 e; v0 = V y; x0 = M^-1 v0; x = x0 + x
-    gm_backsolve(dp<double>(hb), dp<double>(eb), dp<double>(yb), m, K, gdone, st);
+    gm_backsolve(hb, eb, yb, m, K, gdone, st);
     if (flex) {
-      sum_vec<T>(np, X0, Z, ldv, dp<double>(yb), K, gdone, st);
+      sum_vec<T>(np, X0, Z, ldv, yb, K, gdone, st);
     } else {
-      sum_vec<T>(np, V0, V, ldv, dp<double>(yb), K, gdone, st);
+      sum_vec<T>(np, V0, V, ldv, yb, K, gdone, st);
       S.M.apply(np, V0, X0, gdone, st);
       ++per_cycle;
     }
     lincomb<T>(np, x, X0, cimm(1.0), x, cimm(1.0), nullptr, cimm(0), gdone, st);
-    gm_post(K, m, o.itrmax, st);
+    gm_post(K, m, st);
     per_cycle += 4;
   };
-  GraphRunner G;
+  GraphRunner& G = kw.G;
   const int max_cycles = o.itrmax / m + 2;
   for (int c = 0; c < max_cycles; ++c) {
     if (read_done(K, st)) break;
@@ -599,7 +569,7 @@ static SolveOut run_gmres(const Options& o, const System<T>& S, const T* b, T* x
   }
   KState h = read_state(K);
   int merr_h = 0;
-  d2h(&merr_h, merr.p, sizeof(int));
+  d2h(&merr_h, merr, sizeof(int));
   PB_CHECK(merr_h == 0, PARCEL_B_E_CUDA, "MGS grid barrier timed out");
   SolveOut out;
   out.niter = h.niter;
@@ -610,13 +580,14 @@ static SolveOut run_gmres(const Options& o, const System<T>& S, const T* b, T* x
 }
 
 template <class T>
-SolveOut run_krylov(const Options& o, const System<T>& S, const T* b, T* x, double* hist_dev) {
-  Workspace W;
-  W.init();
+SolveOut run_krylov(const Options& o, const System<T>& S, const T* b, T* x, double* hist_dev, KrylovWork* keep) {
+  KrylovWork own;
+  KrylovWork& kw = keep ? *keep : own;
+  kw.begin(&S, b, x, hist_dev);
   switch (o.solver) {
-    case PARCEL_B_SOLVER_CG: return run_pcg<T>(o, S, b, x, hist_dev, W);
-    case PARCEL_B_SOLVER_BICG: return run_bicg<T>(o, S, b, x, hist_dev, W);
-    case PARCEL_B_SOLVER_GMRES: return run_gmres<T>(o, S, b, x, hist_dev, W);
+    case PARCEL_B_SOLVER_CG: return run_pcg<T>(o, S, b, x, hist_dev, kw);
+    case PARCEL_B_SOLVER_BICG: return run_bicg<T>(o, S, b, x, hist_dev, kw);
+    case PARCEL_B_SOLVER_GMRES: return run_gmres<T>(o, S, b, x, hist_dev, kw);
     default:
       PB_CHECK(false, PARCEL_B_E_UNSUPPORTED, "solver %d is not provided by this build", o.solver);
   }
@@ -626,8 +597,8 @@ SolveOut run_krylov(const Options& o, const System<T>& S, const T* b, T* x, doub
 template void build_system<double>(const Options&, const parcel_b_crs&, bool, System<double>&);
 template void build_system<float>(const Options&, const parcel_b_crs&, bool, System<float>&);
 template SolveOut run_krylov<double>(const Options&, const System<double>&, const double*, double*,
-                                     double*);
+                                     double*, KrylovWork*);
 template SolveOut run_krylov<float>(const Options&, const System<float>&, const float*, float*,
-                                    double*);
+                                    double*, KrylovWork*);
 
 }  // namespace pb

@@ -2,6 +2,7 @@
 #pragma once
 
 #include <chrono>
+#include <deque>
 #include <functional>
 #include <memory>
 
@@ -107,11 +108,6 @@ struct SolveOut {
   int breakdown = 0;
 };
 
-// Runs the Krylov iteration on iteration-layout vectors x (in/out) and b.  hist_dev has
-// itrmax+1 entries on the device.
-template <class T>
-SolveOut run_krylov(const Options& o, const System<T>& S, const T* b, T* x, double* hist_dev);
-
 // Workspace shared by the drivers.
 struct Workspace {
   DBuf part, ticket, state;
@@ -119,6 +115,73 @@ struct Workspace {
   KState* st() const { return dp<KState>(state); }
   void init();
 };
+
+// A launch sequence captured into a CUDA graph the first time and replayed after that.
+struct GraphRunner {
+  cudaGraphExec_t exec = nullptr;
+  int launches = 0;
+  GraphRunner() = default;
+  GraphRunner(const GraphRunner&) = delete;
+  ~GraphRunner() { if (exec) cudaGraphExecDestroy(exec); }
+  template <class F>
+  void launch(F&& f, bool use_graph, cudaStream_t st) {
+    if (!use_graph) { f(); return; }
+    if (!exec) {
+      trace_mark(nullptr);
+      cudaGraph_t g = nullptr;
+      PB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+      try {
+        f();
+      } catch (...) {
+        cudaGraph_t g2 = nullptr;
+        cudaStreamEndCapture(st, &g2);
+        if (g2) cudaGraphDestroy(g2);
+        throw;
+      }
+      PB_CUDA(cudaStreamEndCapture(st, &g));
+      PB_CUDA(cudaGraphInstantiate(&exec, g, 0));
+      cudaGraphDestroy(g);
+      trace_mark("graph: capture + instantiate");
+    }
+    PB_CUDA(cudaGraphLaunch(exec, st));
+    trace_mark("graph: replay");
+  }
+};
+
+// What one Krylov solve keeps on the device: reduction workspace, vectors and the captured
+// iteration.  A caller that solves on the same system, right-hand side and solution buffers
+// again (the corrections of a refinement loop) passes the same object each time: the vectors
+// stay and the graph is replayed (instantiating and destroying one of a 40-column cycle with
+// the learned stage took 7 ms a time).  Options other than itrmax must be the same.
+struct KrylovWork {
+  Workspace W;
+  GraphRunner G;
+  int per_cycle = 0;
+  std::deque<DBuf> bufs;
+  size_t next = 0;
+  const void* key[4] = {};
+  void begin(const void* S, const void* b, const void* x, const void* hist) {
+    const void* k[4] = {S, b, x, hist};
+    if (!key[0]) {
+      W.init();
+      memcpy(key, k, sizeof(key));
+    }
+    PB_CHECK(memcmp(key, k, sizeof(key)) == 0, PARCEL_B_E_ARG, "Krylov workspace used with other vectors");
+    next = 0;
+  }
+  // The buffers are asked for in the same order every time; zero-filled when first allocated.
+  template <class T>
+  T* buf(size_t bytes) {
+    if (next == bufs.size()) bufs.emplace_back(bytes);
+    return dp<T>(bufs[next++]);
+  }
+};
+
+// Runs the Krylov iteration on iteration-layout vectors x (in/out) and b.  hist_dev has
+// itrmax+1 entries on the device.
+template <class T>
+SolveOut run_krylov(const Options& o, const System<T>& S, const T* b, T* x, double* hist_dev,
+                    KrylovWork* keep = nullptr);
 
 double now_s();
 
