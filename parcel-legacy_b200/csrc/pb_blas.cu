@@ -16,7 +16,7 @@
 namespace pb {
 
 // ------------------------------------------------------------------ kernels
-// Grid-stride helpers: the reduction kernels always run on the fixed grid red_blocks().
+// Grid-stride helpers: the reduction kernels run on the grid red_grid() gives for their length.
 #define GRID_LOOP(i, n) \
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += (int64_t)gridDim.x * blockDim.x)
 
@@ -328,7 +328,7 @@ template <class T>
 void lincomb_dot(int64_t n, T* out, const T* x0, Coef c0, const T* x1, Coef c1, const T* x2,
                  Coef c2, const T* d0, const T* d1, DotSel sel, int nd, const Red& red,
                  const int* gate, cudaStream_t st) {
-  const int g = red_blocks();
+  const int g = red.full_grid() ? red_blocks() : red_grid(n, 3 * kRedThreads);   // three elements per thread and step
   switch (nd) {
     case 1: k_lincomb_dot<T, 1><<<g, kRedThreads, 0, st>>>(n, out, x0, x1, x2, c0, c1, c2, d0, d1, sel, red, gate); break;
     case 2: k_lincomb_dot<T, 2><<<g, kRedThreads, 0, st>>>(n, out, x0, x1, x2, c0, c1, c2, d0, d1, sel, red, gate); break;
@@ -353,14 +353,14 @@ void scale(int64_t n, T* s, const T* d, const T* r, const int* gate, cudaStream_
 template <class T>
 void multidot(int64_t n, int j, const T* w, const T* V, int64_t ldv, const Red& red, const int* gate,
               cudaStream_t st) {
-  k_multidot<T><<<red_blocks(), kRedThreads, 0, st>>>(n, j, w, V, ldv, red, gate);
+  k_multidot<T><<<red_grid(n, 2 * kRedThreads), kRedThreads, 0, st>>>(n, j, w, V, ldv, red, gate);
   PB_CUDA(cudaGetLastError());
 }
 
 template <class T>
 void cgs_update(int64_t n, int j, T* w, const T* V, int64_t ldv, const double* hcol, const Red& red,
                 const int* gate, cudaStream_t st) {
-  k_cgs_update<T><<<red_blocks(), kRedThreads, 0, st>>>(n, j, w, V, ldv, hcol, red, gate);
+  k_cgs_update<T><<<red_grid(n, 2 * kRedThreads), kRedThreads, 0, st>>>(n, j, w, V, ldv, hcol, red, gate);
   PB_CUDA(cudaGetLastError());
 }
 

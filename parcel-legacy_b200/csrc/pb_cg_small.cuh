@@ -1,0 +1,29 @@
+// pb_cg_small.cuh -- PCG iterations of a short vector in one cooperative launch
+// (pb_cg_small.cu).
+#pragma once
+
+#include "pb_ilu.cuh"
+
+namespace pb {
+
+template <class T>
+struct CgSmallArgs {
+  DevMat<T> A;              // natural layout: the diagonal copy or the sliced-ELLPACK copy
+  const T* dinv = nullptr;  // point Jacobi, null: no preconditioner
+  T *x = nullptr, *r = nullptr, *s = nullptr;   // solution, residual, M^-1 r
+  T *p = nullptr, *p2 = nullptr;                // direction, and a second buffer for it
+  KState* st = nullptr;     // after EPI_CG_INIT; updated as the epilogues of the kernels do
+  double* hist = nullptr;
+  double rtol = 0.0;
+  int maxit = 0;            // iterations of this launch
+  unsigned long long* slots = nullptr;   // cg_small_slots() words, zeroed before the solve
+  unsigned tag0 = 0;        // iterations already tagged in the slots
+  int* err = nullptr;
+};
+
+// CTAs of the launch for n rows, 0 when the vector is too long for it.
+template <class T> int cg_small_grid(int64_t n);
+inline size_t cg_small_slots(int grid) { return (size_t)grid * 6; }
+template <class T> void cg_small(const CgSmallArgs<T>& a, cudaStream_t st);
+
+}  // namespace pb

@@ -80,7 +80,11 @@ template <class T> inline T* dp(const DBuf& b) { return reinterpret_cast<T*>(b.p
 // ------------------------------------------------------------------ launch shapes
 constexpr int kRedThreads = 256;     // threads of every reduction kernel
 int num_sms();
-int red_blocks();                    // fixed grid of the deterministic reductions
+int red_blocks();                    // largest grid of the deterministic reductions
+// Grid of a reduction over n elements, `per` of them to a block: every block takes a ticket
+// on one counter at its end (592 of them 5 us on vectors of a few thousand entries, where 6
+// blocks hold all the work), so a short vector gets as few as its elements fill.
+int red_grid(int64_t n, int per);
 
 // Deterministic multi-value reduction workspace: every reduction kernel writes one
 // partial per block and value, the last block to finish (ticket) sums them in block

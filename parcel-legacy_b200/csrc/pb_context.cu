@@ -78,6 +78,11 @@ int num_sms() { ensure_init(); return g_sms; }
 
 int red_blocks() { return 4 * num_sms(); }
 
+int red_grid(int64_t n, int per) {
+  const int64_t b = (n + per - 1) / per, cap = red_blocks();
+  return (int)(b < 1 ? 1 : (b < cap ? b : cap));
+}
+
 // ------------------------------------------------------------------ buffer cache
 // Released buffers are kept, keyed by their rounded size, and handed to the next request
 // of that size: a solve repeated on the same problem allocates nothing after the first,

@@ -47,6 +47,8 @@ struct Red {
   unsigned* ticket;
   EpiArgs ea;
   int epi;
+  // BiCGStab's sums keep one grid (and so one order) for every length: see run_bicg
+  bool full_grid() const { return epi >= EPI_BICG_INIT && epi <= EPI_BICG_END; }
 };
 
 // ------------------------------------------------------------------ gating

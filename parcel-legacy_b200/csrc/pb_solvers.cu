@@ -16,6 +16,7 @@
 #include <chrono>
 #include <type_traits>
 
+#include "pb_cg_small.cuh"
 #include "pb_mgs.cuh"
 
 #include <atomic>
@@ -324,6 +325,41 @@ static SolveOut run_pcg(const Options& o, const System<T>& S, const T* b, T* x, 
   lincomb_dot<T>(np, nullptr, b, cimm(0), R, cimm(0), Sv, cimm(0), nullptr, nullptr, sel, 3,
                  red(EPI_CG_INIT), nullptr, st);
   launches += 3;
+  auto finish = [&]() -> SolveOut {
+    // x = alpha p + x   (pcg.f90:733)
+    lincomb<T>(np, x, P, cdev(&K->alpha), x, cimm(1.0), nullptr, cimm(0), nullptr, st);
+    KState h = read_state(K);
+    SolveOut out;
+    out.niter = h.niter;
+    out.iret = h.iret;
+    out.breakdown = h.breakdown;
+    out.launches = launches + 1;
+    return out;
+  };
+  // short vectors in the natural layout: all iterations in cooperative launches
+  if (const int grid = S.permuted ? 0 : cg_small_grid<T>(np)) {
+    CgSmallArgs<T> ca;
+    ca.A = S.A;
+    ca.dinv = S.M.kind == PARCEL_B_PRECON_POINTJACOBI ? dp<T>(S.M.dinv) : nullptr;
+    ca.x = x; ca.r = R; ca.s = Sv; ca.p = P; ca.p2 = Q;
+    ca.st = K; ca.hist = hist; ca.rtol = o.rtol;
+    const size_t words = sizeof(unsigned long long) * cg_small_slots(grid);
+    ca.slots = kw.buf<unsigned long long>(words);
+    ca.err = kw.buf<int>(sizeof(int));
+    PB_CUDA(cudaMemsetAsync(ca.slots, 0, words, st));
+    PB_CUDA(cudaMemsetAsync(ca.err, 0, sizeof(int), st));
+    // a launch ends after 4,096 iterations (about 20 ms), so that one does not run for long
+    ca.maxit = 4096;
+    int err = 0;
+    for (int64_t it = 0; it <= o.itrmax && !err && !read_done(K, st); it += ca.maxit) {
+      ca.tag0 = (unsigned)it;
+      cg_small<T>(ca, st);
+      launches += 1;
+      d2h(&err, ca.err, sizeof(int));
+    }
+    PB_CHECK(err == 0, PARCEL_B_E_CUDA, "CG grid sum timed out");
+    return finish();
+  }
   const int chunk = 16;
   auto iterations = [&] {
     for (int it = 0; it < chunk; ++it) {
@@ -346,16 +382,7 @@ static SolveOut run_pcg(const Options& o, const System<T>& S, const T* b, T* x, 
     G.launch(iterations, o.use_graphs, st);
     launches += 5 * chunk;
   }
-  // x = alpha p + x   (pcg.f90:733)
-  lincomb<T>(np, x, P, cdev(&K->alpha), x, cimm(1.0), nullptr, cimm(0), nullptr, st);
-  launches += 1;
-  KState h = read_state(K);
-  SolveOut out;
-  out.niter = h.niter;
-  out.iret = h.iret;
-  out.breakdown = h.breakdown;
-  out.launches = launches;
-  return out;
+  return finish();
 }
 
 // ------------------------------------------------------------------ BiCGStab

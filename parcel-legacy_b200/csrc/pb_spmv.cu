@@ -227,7 +227,7 @@ static void launch_spmv(const DevMat<VT>& A, const XT* x, XT* y, const XT* b, co
                         const int* sa, const int* sb, const Red& red, const int* gate,
                         cudaStream_t st) {
   const int lpr = spmv_lanes(A.n, A.nnz);
-  const int grid = red_blocks();
+  const int grid = ND > 0 && red.full_grid() ? red_blocks() : red_grid(A.n, ND > 0 ? 2 * kRedThreads : kRedThreads);
   int a0 = sa ? sa[0] : 0, b0 = sb ? sb[0] : 0, a1 = sa ? sa[1] : 0, b1 = sb ? sb[1] : 0;
   if (A.d_val) {
     k_spmv_dia<VT, XT, ND, RES><<<grid, kRedThreads, 0, st>>>(A.n, A.ndiag, A.d_off, A.d_val, x, y, b, d, a0, b0,

@@ -78,6 +78,42 @@ def test_level_widths(nx, ny):
         assert _apply_both(A, ipreflag=2, ILU_method=ilu, precon_thblock=1) < 1e-11
 
 
+# ---- CG of short vectors in one launch -----------------------------------------------------------
+@pytest.mark.parametrize("ipreflag", [0, 1])
+@pytest.mark.parametrize("nx,ny", [(1, 1), (3, 2), (32, 16), (33, 16), (270, 281), (280, 271), (389, 390), (551, 550)])
+def test_short_vector_cg(nx, ny, ipreflag):
+    """One CTA, a partial one, and the row counts either side of 1, 2 and 4 rows per thread (151,552
+    and 303,104 rows on 148 SMs); past the last the separate kernels run."""
+    A = problems.poisson2d_5pt(nx, ny)
+    b = problems.rhs_normal(A.n, 1 + nx)
+    kw = dict(solver=1, itrmax=40, rtolmax=1e-10, ipreflag=ipreflag)
+    xo, ho, no, io = oracle.solve(A, b, **kw)
+    res = api.solve(A, b, **kw)
+    assert res["niter"] == no and res["iret"] == io
+    assert (np.abs(res["reshistory"][:no] - ho[:no]) / ho[:no]).max() < 1e-6
+    assert np.abs(res["x"] - xo).max() < 1e-7 * np.abs(xo).max()
+
+
+def test_short_vector_cg_without_a_diagonal_copy_and_past_one_launch():
+    """A matrix that has no diagonal copy (sliced ELLPACK), and more iterations than one launch
+    runs (4,096), ended by the iteration limit."""
+    A = _symmetric_pattern(900, 3, 4)
+    S = A.to_scipy()
+    S = (S + S.T).tocsr()
+    S.sort_indices()
+    B = problems.CRS(n=900, rowptr=(S.indptr + 1).astype(np.int32), col=(S.indices + 1).astype(np.int32),
+                     val=S.data.copy())
+    b = problems.rhs_normal(900, 5)
+    xo, ho, no, io = oracle.solve(B, b, solver=1, itrmax=300, rtolmax=1e-10, ipreflag=1)
+    res = api.solve(B, b, solver=1, itrmax=300, rtolmax=1e-10, ipreflag=1)
+    assert res["niter"] == no and res["iret"] == io and res["stats"]["spmv_diagonals"] == 0
+    assert np.abs(res["x"] - xo).max() < 1e-9 * np.abs(xo).max()
+    P = problems.poisson2d_5pt(300, 301)
+    res = api.solve(P, problems.rhs_normal(P.n, 5), solver=1, itrmax=5000, rtolmax=0.0, ipreflag=1)
+    # the true residual stagnates at the order of eps cond(A) = 2e-16 * 4e4
+    assert res["niter"] == 5000 and res["iret"] == 1 and res["stats"]["true_relres"] < 1e-11
+
+
 # ---- double-double: bit for bit ----------------------------------------------------------------
 def _dd_both(A, b, **kw):
     g = api.ddcg(A, b, **kw)
