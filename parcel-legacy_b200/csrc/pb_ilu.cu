@@ -22,6 +22,7 @@
 // barrier.  The arithmetic of every row is the reference's: same operands, same order.
 #include <algorithm>
 #include <omp.h>
+#include <cub/device/device_scan.cuh>
 #include <climits>
 #include <cmath>
 #include <memory>
@@ -29,6 +30,7 @@
 #include <type_traits>
 
 #include "pb_device.cuh"
+#include "pb_epilogue.cuh"
 #include "pb_ilu.cuh"
 
 namespace pb {
@@ -310,6 +312,11 @@ __device__ __forceinline__ void inblock_range(const int* rp, const int* ci, int 
 // is written back once.  Longer rows (or pivot rows) take the entry-by-entry path.
 constexpr int kFacCap = 8;
 
+// Levels [start, end) in the iteration layout; block b has levels blvl[b] .. blvl[b + 1] - 1.
+struct LevelTab {
+  const int *blvl, *start, *end;
+};
+
 __device__ __forceinline__ void ilu0_row_generic(const int* rp, const int* ci, int rbase, int cbase, int i, int lo, int hi,
                                  double* lu) {
   int ia, iz, idg;
@@ -332,16 +339,15 @@ __device__ __forceinline__ void ilu0_row_generic(const int* rp, const int* ci, i
   }
 }
 
-__global__ void k_ilu0_factor(const IluChunk* __restrict__ ch, const int* __restrict__ blk_chunk,
-                              const int* __restrict__ blk_lo, const int* __restrict__ blk_hi,
+__global__ void k_ilu0_factor(LevelTab tab, const int* __restrict__ blk_lo, const int* __restrict__ blk_hi,
                               const int* __restrict__ rowAt, const int* __restrict__ rp,
                               const int* __restrict__ ci, int rbase, int cbase, double* lu) {
   const int b = blockIdx.x;
   const int lo = blk_lo[b], hi = blk_hi[b];
-  for (int c = blk_chunk[b]; c < blk_chunk[b + 1]; ++c) {
-    const IluChunk C = ch[c];
-    for (int p = threadIdx.x; p < C.w; p += blockDim.x) {
-      const int i = rowAt[C.start + p];
+  for (int l = tab.blvl[b]; l < tab.blvl[b + 1]; ++l) {
+    const int e = tab.end[l];
+    for (int p = tab.start[l] + threadIdx.x; p < e; p += blockDim.x) {
+      const int i = rowAt[p];
       const int a = rp[i] - rbase, z = rp[i + 1] - rbase;
       if (z - a > kFacCap) {
         ilu0_row_generic(rp, ci, rbase, cbase, i, lo, hi, lu);
@@ -412,17 +418,16 @@ __global__ void k_ilu0_factor(const IluChunk* __restrict__ ch, const int* __rest
   }
 }
 
-__global__ void k_dilu_diag(const IluChunk* __restrict__ ch, const int* __restrict__ blk_chunk,
-                            const int* __restrict__ blk_lo, const int* __restrict__ blk_hi,
+__global__ void k_dilu_diag(LevelTab tab, const int* __restrict__ blk_lo, const int* __restrict__ blk_hi,
                             const int* __restrict__ rowAt, const int* __restrict__ rp,
                             const int* __restrict__ ci, const double* __restrict__ va, int rbase,
                             int cbase, int mlud, double* D, double* Dinv) {
   const int b = blockIdx.x;
   const int lo = blk_lo[b], hi = blk_hi[b];
-  for (int c = blk_chunk[b]; c < blk_chunk[b + 1]; ++c) {
-    const IluChunk C = ch[c];
-    for (int p = threadIdx.x; p < C.w; p += blockDim.x) {
-      int k = rowAt[C.start + p];
+  for (int l = tab.blvl[b]; l < tab.blvl[b + 1]; ++l) {
+    const int e = tab.end[l];
+    for (int p = tab.start[l] + threadIdx.x; p < e; p += blockDim.x) {
+      int k = rowAt[p];
       int ia, iz, idg;
       inblock_range(rp, ci, rbase, cbase, k, lo, hi, &ia, &iz, &idg);
       double d = va[idg];
@@ -1169,7 +1174,8 @@ __global__ void k_ilu_small_pack(int n, int nb, const int* __restrict__ blk_lo, 
                                  int rbase, int cbase, const double* __restrict__ vL, const double* __restrict__ vU,
                                  const double* __restrict__ Dinv, int dilu, int K, int* __restrict__ cF,
                                  T* __restrict__ vF, T* __restrict__ dF, int* __restrict__ cB, T* __restrict__ vB,
-                                 T* __restrict__ dB) {
+                                 T* __restrict__ dB, const int2* __restrict__ box, int KC,
+                                 unsigned short* __restrict__ hF, unsigned short* __restrict__ hB) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     int a = 0, z = nb - 1;   // block of row i: the last b with blk_lo[b] <= i
     while (a < z) {
@@ -1179,28 +1185,34 @@ __global__ void k_ilu_small_pack(int n, int nb, const int* __restrict__ blk_lo, 
     int ia, iz, idg;
     inblock_range(rp, ci, rbase, cbase, i, blk_lo[a], blk_hi[a], &ia, &iz, &idg);
     const int64_t p = pos[i];
+    // entry k of a sweep's record: permuted column (unstaged records) or position in the
+    // block's stretch (staged ones), -1 and 0xffff for none
+    auto put = [&](int* c, unsigned short* h, int k, int q) {
+      if (h) h[p * KC + k] = q < 0 ? (unsigned short)0xffff : (unsigned short)(q - box[a].x);
+      else c[p * K + k] = q;
+    };
     int k = 0;
     for (int j = ia; j < idg; ++j, ++k) {
-      cF[p * K + k] = pos[ci[j] - cbase];
+      put(cF, hF, k, pos[ci[j] - cbase]);
       vF[p * K + k] = (T)vL[j];
     }
-    for (; k < K; ++k) { cF[p * K + k] = -1; vF[p * K + k] = T(0); }
+    for (; k < K; ++k) { put(cF, hF, k, -1); vF[p * K + k] = T(0); }
     dF[p] = dilu ? (T)Dinv[i] : T(1);
     k = 0;
     if (!dilu) {
       for (int j = idg + 1; j < iz; ++j, ++k) {
-        cB[p * K + k] = pos[ci[j] - cbase];
+        put(cB, hB, k, pos[ci[j] - cbase]);
         vB[p * K + k] = (T)vU[j];
       }
       dB[p] = (T)(1.0 / vU[idg]);
     } else {
       for (int j = iz - 1; j > idg; --j, ++k) {
-        cB[p * K + k] = pos[ci[j] - cbase];
+        put(cB, hB, k, pos[ci[j] - cbase]);
         vB[p * K + k] = (T)vU[j];
       }
       dB[p] = (T)Dinv[i];
     }
-    for (; k < K; ++k) { cB[p * K + k] = -1; vB[p * K + k] = T(0); }
+    for (; k < K; ++k) { put(cB, hB, k, -1); vB[p * K + k] = T(0); }
   }
 }
 
@@ -1317,7 +1329,11 @@ k_ilu_small(int nb, const int* __restrict__ blvl, const int* __restrict__ lo, co
 // forward ones once the forward sweep is done: a smaller area per block lets more blocks be
 // in flight on an SM, which is what the sweep waits on.  Same records, same expressions, same
 // order as k_ilu_small.
+// The staged records hold a coupling as its 16-bit position in the stretch, a row's entries
+// padded to a multiple of four (small_kc): 8 bytes of indices per row and sweep instead of 12
+// for a 7-point stencil, read in one load, and a 4^3 box takes 3.9 KB instead of 4.3.
 constexpr int kStageWarps = 4;
+__host__ __device__ constexpr int small_kc(int K) { return (K + 3) & ~3; }
 constexpr int kStageBoxBytes = 12 * 1024;
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
@@ -1334,17 +1350,43 @@ __device__ __forceinline__ void group_stage(void* dst, const void* src, int byte
   for (int o = li * 16; o < bytes; o += lanes * 16) cp_async16(d + o, g + o);
 }
 
+template <int KC>
+__device__ __forceinline__ void small_cols16(unsigned short (&c)[KC], const unsigned short* p) {
+#pragma unroll
+  for (int k = 0; k < KC; k += 4) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p + k);
+    c[k] = (unsigned short)(v.x & 0xffffu);
+    c[k + 1] = (unsigned short)(v.x >> 16);
+    c[k + 2] = (unsigned short)(v.y & 0xffffu);
+    c[k + 3] = (unsigned short)(v.y >> 16);
+  }
+}
+
+// CG's step around the preconditioner: r += c q before the sweep, <s, r> and <r, r> after it.
+// The fused sweep reads q beside r (which it reads anyway) and writes r back; s is in shared
+// memory when its products are formed.  Apart they were three launches that moved five
+// vectors more.
+template <class T>
+struct SmallCg {
+  const T* q = nullptr;
+  T* r = nullptr;           // updated in place
+  const double* c = nullptr;
+  Red red{};
+};
+
 // LPB lanes per block, 32 / LPB blocks per warp (as k_ilu_small), each block with its own
 // area of box_bytes; blockDim.x / 32 warps per CTA.
-template <class T, bool DILU, int K, int LPB>
+template <class T, bool DILU, int K, int LPB, bool CG>
 __global__ void __launch_bounds__(kStageWarps * 32)
 k_ilu_small_staged(int nb, const int2* __restrict__ box, const int* __restrict__ blvl, const int* __restrict__ lo,
-                   const int* __restrict__ hi, const int* __restrict__ cF, const T* __restrict__ vF,
-                   const T* __restrict__ dF, const int* __restrict__ cB, const T* __restrict__ vB,
-                   const T* __restrict__ dB, const T* __restrict__ r, T* __restrict__ s, const int* gate, int span,
-                   int levcap, int box_bytes) {
+                   const int* __restrict__ hi, const unsigned short* __restrict__ cF, const T* __restrict__ vF,
+                   const T* __restrict__ dF, const unsigned short* __restrict__ cB, const T* __restrict__ vB,
+                   const T* __restrict__ dB, const T* r, T* __restrict__ s, const int* gate, int span,
+                   int levcap, int box_bytes, SmallCg<T> cg) {
   if (gated(gate)) return;
-  constexpr int BPW = 32 / LPB;
+  double acc2[2] = {0.0, 0.0};   // <s, r>, <r, r>
+  const T cgc = CG ? (T)*cg.c : T(0);
+  constexpr int BPW = 32 / LPB, KC = small_kc(K);
   extern __shared__ __align__(16) unsigned char stage_smem[];
   const int lane = threadIdx.x & 31, sub = lane / LPB, li = lane % LPB;
   const int wib = threadIdx.x >> 5, wpc = blockDim.x >> 5;
@@ -1354,8 +1396,8 @@ k_ilu_small_staged(int nb, const int2* __restrict__ box, const int* __restrict__
   T* Fd = X + span;
   T* Bd = DILU ? Fd : Fd + span;   // D-ILU: both sweeps scale by the same D^-1
   T* V = Fd + span + (DILU ? 0 : span);   // after Fd (D-ILU) or after Bd (ILU(0))
-  int* Cc = reinterpret_cast<int*>(V + (size_t)span * K);
-  int* Lo = Cc + (size_t)span * K;
+  unsigned short* Cc = reinterpret_cast<unsigned short*>(V + (size_t)span * K);
+  int* Lo = reinterpret_cast<int*>(Cc + (size_t)span * KC);
   int* Hi = Lo + levcap;
   const int nwarps = gridDim.x * wpc;
   const int ngroups = (nb + BPW - 1) / BPW;
@@ -1373,10 +1415,10 @@ k_ilu_small_staged(int nb, const int2* __restrict__ box, const int* __restrict__
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) maxlev = max(maxlev, __shfl_xor_sync(0xffffffffu, maxlev, o));
     if (b < nb) {
-      group_stage(X, r + P0, S * (int)sizeof(T), li, LPB);
+      if (!CG) group_stage(X, r + P0, S * (int)sizeof(T), li, LPB);
       group_stage(V, vF + (int64_t)P0 * K, S * K * (int)sizeof(T), li, LPB);
       group_stage(Fd, dF + P0, S * (int)sizeof(T), li, LPB);
-      group_stage(Cc, cF + (int64_t)P0 * K, S * K * 4, li, LPB);
+      group_stage(Cc, cF + (int64_t)P0 * KC, S * KC * 2, li, LPB);
       if (!DILU) group_stage(Bd, dB + P0, S * (int)sizeof(T), li, LPB);
       for (int t = li; t < nlev; t += LPB) {
         Lo[t] = lo[l0 + t] - P0;
@@ -1384,6 +1426,25 @@ k_ilu_small_staged(int nb, const int2* __restrict__ box, const int* __restrict__
       }
     }
     cp_async_commit();
+    if (CG && b < nb) {   // r += c q while the copies are under way (16 bytes at a time: S is a multiple of 4)
+      constexpr int E = 16 / (int)sizeof(T);
+      for (int o = li * E; o < S; o += LPB * E) {
+        const uint4 ru = *reinterpret_cast<const uint4*>(cg.r + P0 + o);
+        const uint4 qu = __ldcs(reinterpret_cast<const uint4*>(cg.q + P0 + o));
+        T rv[E], qv[E];
+        memcpy(rv, &ru, 16);
+        memcpy(qv, &qu, 16);
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          rv[e] = cgc * qv[e] + rv[e];
+          X[o + e] = rv[e];
+          acc2[1] += (double)(rv[e] * rv[e]);
+        }
+        uint4 wu;
+        memcpy(&wu, rv, 16);
+        *reinterpret_cast<uint4*>(cg.r + P0 + o) = wu;
+      }
+    }
     cp_async_wait<0>();   // this lane's copies
     __syncwarp();         // and everyone's
     // forward: y = D^-1 (r - L y) (D-ILU) or r - L y (ILU(0), unit L)
@@ -1392,11 +1453,11 @@ k_ilu_small_staged(int nb, const int2* __restrict__ box, const int* __restrict__
         const int e = Hi[t];
         for (int q = Lo[t] + li; q < e; q += LPB) {
           T acc = X[q];
+          unsigned short cc[KC];
+          small_cols16<KC>(cc, Cc + q * KC);
 #pragma unroll
-          for (int k = 0; k < K; ++k) {
-            const int c = Cc[q * K + k] - P0;   // -1 (no entry) falls outside [0, S)
-            if ((unsigned)c < (unsigned)S) acc = acc - V[q * K + k] * X[c];
-          }
+          for (int k = 0; k < K; ++k)
+            if (cc[k] != 0xffff) acc = acc - V[q * K + k] * X[cc[k]];
           X[q] = DILU ? Fd[q] * acc : acc;
         }
       }
@@ -1405,9 +1466,19 @@ k_ilu_small_staged(int nb, const int2* __restrict__ box, const int* __restrict__
     // the forward records are no longer read (the barrier above): the backward ones replace them
     if (b < nb) {
       group_stage(V, vB + (int64_t)P0 * K, S * K * (int)sizeof(T), li, LPB);
-      group_stage(Cc, cB + (int64_t)P0 * K, S * K * 4, li, LPB);
+      group_stage(Cc, cB + (int64_t)P0 * KC, S * KC * 2, li, LPB);
     }
     cp_async_commit();
+    // CG: the new r again, on its way (from L2) while the backward sweep runs
+    constexpr int E16 = 16 / (int)sizeof(T), RK = 3;
+    uint4 rk[RK];
+    if (CG) {
+#pragma unroll
+      for (int u = 0; u < RK; ++u) {
+        const int o = (li + u * LPB) * E16;
+        if (o < S) rk[u] = *reinterpret_cast<const uint4*>(cg.r + P0 + o);   // this lane's own stores
+      }
+    }
     cp_async_wait<0>();
     __syncwarp();
     // backward from the forward result
@@ -1418,22 +1489,46 @@ k_ilu_small_staged(int nb, const int2* __restrict__ box, const int* __restrict__
         for (int q = Lo[tl] + li; q < e; q += LPB) {
           const T xp = X[q], d = Bd[q];
           T acc = DILU ? T(0) : xp;
+          unsigned short cc[KC];
+          small_cols16<KC>(cc, Cc + q * KC);
 #pragma unroll
           for (int k = 0; k < K; ++k) {
-            const int c = Cc[q * K + k] - P0;
-            if ((unsigned)c < (unsigned)S) {
-              if (DILU) acc = acc + X[c] * V[q * K + k];
-              else acc = acc - X[c] * V[q * K + k];
+            if (cc[k] != 0xffff) {
+              if (DILU) acc = acc + X[cc[k]] * V[q * K + k];
+              else acc = acc - X[cc[k]] * V[q * K + k];
             }
           }
           const T o = DILU ? xp - d * acc : acc * d;
           X[q] = o;
-          s[P0 + q] = o;
+          if (!CG) s[P0 + q] = o;
         }
       }
       __syncwarp();
     }
+    if (CG && b < nb) {
+      auto finish = [&](int o, const uint4& ru) {
+        T rv[E16], sv[E16];
+        memcpy(rv, &ru, 16);
+#pragma unroll
+        for (int e = 0; e < E16; ++e) {
+          sv[e] = X[o + e];
+          acc2[0] += (double)(sv[e] * rv[e]);
+        }
+        uint4 wu;
+        memcpy(&wu, sv, 16);
+        *reinterpret_cast<uint4*>(s + P0 + o) = wu;
+      };
+#pragma unroll
+      for (int u = 0; u < RK; ++u) {
+        const int o = (li + u * LPB) * E16;
+        if (o < S) finish(o, rk[u]);
+      }
+      for (int o = (li + RK * LPB) * E16; o < S; o += LPB * E16)
+        finish(o, *reinterpret_cast<const uint4*>(cg.r + P0 + o));
+      __syncwarp();   // X is the next block's right-hand side
+    }
   }
+  if constexpr (CG) reduce_and_finish_wide<2>(acc2, cg.red);
 }
 
 // ------------------------------------------------------------------ host side
@@ -1530,6 +1625,31 @@ static bool grp_layout(const IluPlan& P, const std::vector<IluChunk>& ch, int ku
   return true;
 }
 
+// L and U values (ILU(0): lu; D-ILU: the matrix's) and D^-1 of every block, one CTA each.
+struct Factor {
+  DBuf lu, Dd, Di;
+  const double *vL = nullptr, *vU = nullptr, *dinv = nullptr;
+  void run(const DevMat<double>& A, int n, int nb, int maxw, int ilu_method, const LevelTab& tab, const int* blo,
+           const int* bhi, const int* d_rowAt, cudaStream_t st) {
+    vL = vU = A.val;
+    if (ilu_method == 0) {
+      lu.alloc(sizeof(double) * std::max<int64_t>(A.nnz, 1));
+      d2d(lu.p, A.val, sizeof(double) * A.nnz);
+      k_ilu0_factor<<<nb, ilu_factor_threads(maxw), 0, st>>>(tab, blo, bhi, d_rowAt, A.rowptr, A.col, A.rbase,
+                                                             A.cbase, dp<double>(lu));
+      vL = vU = dp<double>(lu);
+    } else {
+      Dd.alloc(sizeof(double) * n);
+      Di.alloc(sizeof(double) * n);
+      k_dilu_diag<<<nb, ilu_factor_threads(maxw), 0, st>>>(tab, blo, bhi, d_rowAt, A.rowptr, A.col, A.val, A.rbase,
+                                                           A.cbase, ilu_method == 2 ? 1 : 0, dp<double>(Dd),
+                                                           dp<double>(Di));
+      dinv = dp<double>(Di);
+    }
+    PB_CUDA(cudaGetLastError());
+  }
+};
+
 template <class T>
 int ilu_setup_device(const IluPlan& P, const DevMat<double>& A, int ilu_method,
                      const int* d_pos, const int* d_rowAt, const int* d_lev, IluDev<T>& D) {
@@ -1597,38 +1717,22 @@ int ilu_setup_device(const IluPlan& P, const DevMat<double>& A, int ilu_method,
   DBuf blo(sizeof(int) * P.nb), bhi(sizeof(int) * P.nb);
   h2d(blo.p, P.blk_lo.data(), sizeof(int) * P.nb);
   h2d(bhi.p, P.blk_hi.data(), sizeof(int) * P.nb);
-  DBuf blvl(sizeof(int) * (P.nb + 1)), lst(sizeof(int) * std::max<size_t>(P.lvl_start.size(), 1));
+  const size_t nl = std::max<size_t>(P.lvl_start.size(), 1);
+  DBuf blvl(sizeof(int) * (P.nb + 1)), lst(sizeof(int) * nl), lend(sizeof(int) * nl);
   h2d(blvl.p, P.blk_lvl.data(), sizeof(int) * (P.nb + 1));
   h2d(lst.p, P.lvl_start.data(), sizeof(int) * P.lvl_start.size());
+  h2d(lend.p, P.lvl_end.data(), sizeof(int) * P.lvl_end.size());
 
   trace_mark("ilu: tables to device");
   // factorisation in natural CSR order
-  const int64_t nnz = A.nnz;
-  DBuf lu, Dd, Di;
-  const double* vL = A.val;
-  const double* vU = A.val;
-  if (!D.dilu) {
-    lu.alloc(sizeof(double) * nnz);
-    d2d(lu.p, A.val, sizeof(double) * nnz);
-    k_ilu0_factor<<<P.nb, ilu_factor_threads(P.maxWp), 0, st>>>(dp<IluChunk>(D.chunks), dp<int>(D.blk_chunk), dp<int>(blo),
-                                        dp<int>(bhi), d_rowAt, A.rowptr, A.col, A.rbase, A.cbase,
-                                        dp<double>(lu));
-    PB_CUDA(cudaGetLastError());
-    vL = dp<double>(lu);
-    vU = dp<double>(lu);
-  } else {
-    Dd.alloc(sizeof(double) * P.n);
-    Di.alloc(sizeof(double) * P.n);
-    k_dilu_diag<<<P.nb, ilu_factor_threads(P.maxWp), 0, st>>>(dp<IluChunk>(D.chunks), dp<int>(D.blk_chunk), dp<int>(blo),
-                                      dp<int>(bhi), d_rowAt, A.rowptr, A.col, A.val, A.rbase, A.cbase,
-                                      ilu_method == 2 ? 1 : 0, dp<double>(Dd), dp<double>(Di));
-    PB_CUDA(cudaGetLastError());
-  }
+  Factor F;
+  F.run(A, P.n, P.nb, P.maxWp, ilu_method, LevelTab{dp<int>(blvl), dp<int>(lst), dp<int>(lend)}, dp<int>(blo),
+        dp<int>(bhi), d_rowAt, st);
   trace_mark("ilu: factor");
   D.packF.alloc(D.packF_bytes);
   D.packB.alloc(D.packB_bytes);
   if (D.grp) {
-    const FpSrc<T> src{vL, vU, D.dilu ? dp<double>(Di) : nullptr};
+    const FpSrc<T> src{F.vL, F.vU, F.dinv};
     k_ilu_pack_grp<T, FpSrc<T>><<<std::max(1, std::min(D.ngroups, 65535)), 256, 0, st>>>(
         dp<int4>(D.ginfo), dp<int64_t>(D.goff), D.ngroups, dp<IluChunk>(D.chunks), dp<int>(blo), dp<int>(bhi),
         dp<int>(blvl), dp<int>(lst), d_rowAt, d_pos, d_lev, A.rowptr, A.col, A.rbase, A.cbase, src,
@@ -1639,67 +1743,222 @@ int ilu_setup_device(const IluPlan& P, const DevMat<double>& A, int ilu_method,
     k_ilu_pack<T><<<std::min<int>((int)ch.size(), 65535) > 0 ? std::min<int>((int)ch.size(), 65535) : 1,
                     128, 0, st>>>(
         dp<IluChunk>(D.chunks), (int)ch.size(), dp<int>(blo), dp<int>(bhi), dp<int>(blvl),
-        dp<int>(lst), d_rowAt, d_pos, d_lev, A.rowptr, A.col, A.rbase, A.cbase, vL, vU,
-        D.dilu ? dp<double>(Di) : nullptr, D.dilu ? 1 : 0, D.ring ? 1 : 0, D.W, D.maxWp,
+        dp<int>(lst), d_rowAt, d_pos, d_lev, A.rowptr, A.col, A.rbase, A.cbase, F.vL, F.vU,
+        F.dinv, D.dilu ? 1 : 0, D.ring ? 1 : 0, D.W, D.maxWp,
         dp<unsigned char>(D.packF), dp<unsigned char>(D.packB));
   }
   PB_CUDA(cudaGetLastError());
-  // many small blocks: the warp-per-block records as well (the packed ones serve the
-  // accumulating apply)
-  int max_rows = 0;
-  for (int b = 0; b < P.nb; ++b) max_rows = std::max(max_rows, P.blk_hi[b] - P.blk_lo[b]);
-  D.small = max_rows <= kSmallMaxRows && P.nb >= 8 * num_sms() && D.K <= 8;
-  if (D.small) {
-    // lanes per block: the widest level, rounded up to 8, 16 or 32 (wider levels take
-    // several rows per lane)
-    D.s_lpb = maxw <= 8 ? 8 : (maxw <= 16 ? 16 : 32);
-    const size_t rk = (size_t)P.np * D.K;
-    D.s_cF.alloc(sizeof(int) * rk); D.s_vF.alloc(sizeof(T) * rk); D.s_dF.alloc(sizeof(T) * P.np);
-    D.s_cB.alloc(sizeof(int) * rk); D.s_vB.alloc(sizeof(T) * rk); D.s_dB.alloc(sizeof(T) * P.np);
-    const int totlev = (int)P.lvl_start.size();
-    D.s_blvl.alloc(sizeof(int) * (P.nb + 1));
-    D.s_lo.alloc(sizeof(int) * std::max(totlev, 1));
-    D.s_hi.alloc(sizeof(int) * std::max(totlev, 1));
-    h2d(D.s_blvl.p, P.blk_lvl.data(), sizeof(int) * (P.nb + 1));
-    h2d(D.s_lo.p, P.lvl_start.data(), sizeof(int) * totlev);
-    h2d(D.s_hi.p, P.lvl_end.data(), sizeof(int) * totlev);
-    const int g = (int)std::min<int64_t>(((int64_t)P.n + 255) / 256, 8LL * num_sms());
-    k_ilu_small_pack<T><<<std::max(g, 1), 256, 0, st>>>(
-        P.n, P.nb, dp<int>(blo), dp<int>(bhi), d_pos, A.rowptr, A.col, A.rbase, A.cbase, vL, vU,
-        D.dilu ? dp<double>(Di) : nullptr, D.dilu ? 1 : 0, D.K, dp<int>(D.s_cF), dp<T>(D.s_vF), dp<T>(D.s_dF),
-        dp<int>(D.s_cB), dp<T>(D.s_vB), dp<T>(D.s_dB));
-    PB_CUDA(cudaGetLastError());
-    // the staged variant: each block's stretch of the iteration layout, from its first level's
-    // start to its last level's end rounded up to 4 (the next block, or the end of the
-    // padded layout, starts there)
-    std::vector<int2> bxs(P.nb);
-    int span = 0;
-    for (int b = 0; b < P.nb; ++b) {
-      const int p0 = P.lvl_start[P.blk_lvl[b]], p1 = align4(P.lvl_end[P.blk_lvl[b + 1] - 1]);
-      bxs[b] = make_int2(p0, p1 - p0);
-      span = std::max(span, p1 - p0);
-    }
-    const int levcap = align4(std::max(P.max_levels, 1));
-    const int64_t tb = (int64_t)span * (2 + D.K + (D.dilu ? 0 : 1)) * (int64_t)sizeof(T) +
-                       (int64_t)span * D.K * 4 + 2LL * levcap * 4;
-    D.s_box_bytes = 0;
-    if (tb <= kStageBoxBytes) {   // a warp's blocks (at most 4) within the default 48 KB of a CTA
-      D.s_span = span;
-      D.s_levcap = levcap;
-      D.s_box_bytes = (int)tb;
-      D.s_box.alloc(sizeof(int2) * P.nb);
-      h2d(D.s_box.p, bxs.data(), sizeof(int2) * P.nb);
-    }
-  }
   D.ytmp.alloc(sizeof(T) * (P.np + 4));
   PB_CUDA(cudaMemsetAsync(D.ytmp.p, 0, sizeof(T) * (P.np + 4), st));
   D.err.alloc(sizeof(int));
   PB_CUDA(cudaMemsetAsync(D.err.p, 0, sizeof(int), st));
-  // temporaries (lu, Dd, Di, blo, ...) are freed when this function returns: make sure
+  // temporaries (the factors, blo, ...) are freed when this function returns: make sure
   // the kernels that read them have finished.
   sync();
   return 0;
 }
+
+// ------------------------------------------------------------------ many small blocks, set-up
+// The wavefront plan of tens of thousands of small blocks on the device, one thread per
+// block walking its rows as ilu_build_plan does: the sparsity structure does not come back to
+// the host and no per-chunk tables go out (64,000 boxes of 4^3: 28 ms on the host with its
+// copies).  A block's rows are few, so its thread's dependent loads (row pointer, column,
+// level: about 1.5 us a row) end after 0.1 to 1.5 ms whatever the number of blocks.
+struct SmallStat {
+  int maxw, max_levels, kmax, span, missing;   // missing: a block without a diagonal entry, or INT_MAX
+};
+
+__global__ void k_small_levels(int nb, const int* __restrict__ starts, const int* __restrict__ rp,
+                               const int* __restrict__ ci, int rbase, int cbase, int* lev, int* low, int* wid,
+                               int* __restrict__ nlev, int* __restrict__ span, SmallStat* stat) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= nb) return;
+  const int lo = starts[b], hi = starts[b + 1];
+  int maxlev = 0, kmax = 0;
+  bool missing = false;
+  for (int i = lo; i < hi; ++i) {   // low (zeroed): the level forced by upper entries of earlier rows
+    const int a = rp[i] - rbase, z = rp[i + 1] - rbase;
+    int L = low[i], nl = 0, nu = 0;
+    bool diag = false, fixed = false, unsorted = false;
+    for (int j = a; j < z; ++j) {
+      const int c = ci[j] - cbase;
+      if (c < lo || c >= hi) continue;
+      if (c < i) {
+        unsorted |= fixed;
+        L = max(L, lev[c] + 1);
+        ++nl;
+      } else if (c == i) {
+        diag = true;
+      } else {
+        fixed = true;
+        low[c] = max(low[c], L + 1);
+        ++nu;
+      }
+    }
+    if (unsorted)   // a lower entry after an upper one: redo the upper entries with the final level
+      for (int j = a; j < z; ++j) {
+        const int c = ci[j] - cbase;
+        if (c > i && c < hi) low[c] = max(low[c], L + 1);
+      }
+    missing |= !diag;
+    lev[i] = L;
+    wid[lo + L] += 1;   // zeroed; a block has no more levels than rows
+    maxlev = max(maxlev, L);
+    kmax = max(kmax, max(nl, nu));
+  }
+  int sp = 0, maxw = 0;
+  for (int l = 0; l <= maxlev; ++l) {
+    const int w = wid[lo + l];
+    sp += (w + 3) & ~3;
+    maxw = max(maxw, w);
+  }
+  nlev[b] = maxlev + 1;
+  span[b] = sp;
+  atomicMax(&stat->maxw, maxw);
+  atomicMax(&stat->max_levels, maxlev + 1);
+  atomicMax(&stat->kmax, kmax);
+  atomicMax(&stat->span, sp);
+  if (missing) atomicMin(&stat->missing, b);
+}
+
+// Level ranges and positions (stable by row within a level), block by block.
+__global__ void k_small_layout(int nb, const int* __restrict__ starts, const int* __restrict__ blvl,
+                               const int* __restrict__ first, const int* __restrict__ span,
+                               const int* __restrict__ lev, int* wid, int* __restrict__ lst, int* __restrict__ lend,
+                               int* __restrict__ pos, int* __restrict__ rowAt, int2* __restrict__ box) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= nb) return;
+  const int lo = starts[b], hi = starts[b + 1], l0 = blvl[b], nl = blvl[b + 1] - l0;
+  int cur = first[b];
+  for (int l = 0; l < nl; ++l) {
+    const int w = wid[lo + l];
+    lst[l0 + l] = cur;
+    lend[l0 + l] = cur + w;
+    wid[lo + l] = cur;   // from here on the level's next free position
+    cur = (cur + w + 3) & ~3;
+  }
+  for (int i = lo; i < hi; ++i) {
+    const int p = wid[lo + lev[i]]++;
+    pos[i] = p;
+    rowAt[p] = i;
+  }
+  box[b] = make_int2(first[b], span[b]);
+}
+
+bool ilu_small_blocks(const BlockSplit& bs, int n) {
+  if (bs.nb < 8 * num_sms() || 4 * (int64_t)n > INT_MAX) return false;
+  for (int b = 0; b < bs.nb; ++b) {
+    int lo, hi;
+    bs.rows(b, n, &lo, &hi);
+    if (hi - lo > kSmallMaxRows) return false;
+  }
+  return true;
+}
+
+bool ilu_small_plan(const BlockSplit& bs, const DevMat<double>& A, SmallPlan& P) {
+  cudaStream_t st = stream();
+  const int nb = bs.nb, n = A.n;
+  P.nb = nb;
+  P.n = n;
+  std::vector<int> starts(nb + 1, n);
+  for (int b = 0; b < nb; ++b) {
+    int hi;
+    bs.rows(b, n, &starts[b], &hi);
+  }
+  P.starts.alloc(sizeof(int) * (nb + 1));
+  h2d(P.starts.p, starts.data(), sizeof(int) * (nb + 1));
+  DBuf lev(sizeof(int) * n), low(sizeof(int) * n), wid(sizeof(int) * n), stat(sizeof(SmallStat)),
+      nlev(sizeof(int) * (nb + 1)), span(sizeof(int) * (nb + 1)), first(sizeof(int) * (nb + 1));   // zero-filled
+  SmallStat h{0, 0, 0, 0, INT_MAX};
+  h2d(stat.p, &h, sizeof(h));
+  const int grid = (nb + 127) / 128;
+  k_small_levels<<<grid, 128, 0, st>>>(nb, dp<int>(P.starts), A.rowptr, A.col, A.rbase, A.cbase, dp<int>(lev),
+                                       dp<int>(low), dp<int>(wid), dp<int>(nlev), dp<int>(span), dp<SmallStat>(stat));
+  PB_CUDA(cudaGetLastError());
+  P.blvl.alloc(sizeof(int) * (nb + 1));
+  size_t tmp_bytes = 0;
+  PB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, dp<int>(nlev), dp<int>(P.blvl), nb + 1, st));
+  DBuf tmp(std::max<size_t>(tmp_bytes, 16));
+  PB_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tmp_bytes, dp<int>(nlev), dp<int>(P.blvl), nb + 1, st));
+  PB_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tmp_bytes, dp<int>(span), dp<int>(first), nb + 1, st));
+  int totals[2];
+  PB_CUDA(cudaMemcpyAsync(&h, stat.p, sizeof(h), cudaMemcpyDeviceToHost, st));
+  PB_CUDA(cudaMemcpyAsync(&totals[0], dp<int>(P.blvl) + nb, sizeof(int), cudaMemcpyDeviceToHost, st));
+  PB_CUDA(cudaMemcpyAsync(&totals[1], dp<int>(first) + nb, sizeof(int), cudaMemcpyDeviceToHost, st));
+  sync();
+  PB_CHECK(h.missing == INT_MAX, PARCEL_B_E_ZERO_PIVOT,
+           "block-Jacobi block %d has a row without an in-block diagonal entry", h.missing);
+  if (h.kmax > 8) return false;   // more couplings than the records hold
+  P.totlev = totals[0];
+  P.np = totals[1];
+  P.maxw = h.maxw;
+  P.max_levels = h.max_levels;
+  P.kmax = h.kmax;
+  P.span = h.span;
+  P.lo.alloc(sizeof(int) * P.totlev);
+  P.hi.alloc(sizeof(int) * P.totlev);
+  P.pos.alloc(sizeof(int) * n);
+  P.rowAt.alloc(sizeof(int) * P.np);
+  PB_CUDA(cudaMemsetAsync(P.rowAt.p, 0xFF, sizeof(int) * P.np, st));   // padding: -1
+  P.box.alloc(sizeof(int2) * nb);
+  k_small_layout<<<grid, 128, 0, st>>>(nb, dp<int>(P.starts), dp<int>(P.blvl), dp<int>(first), dp<int>(span),
+                                       dp<int>(lev), dp<int>(wid), dp<int>(P.lo), dp<int>(P.hi), dp<int>(P.pos),
+                                       dp<int>(P.rowAt), dp<int2>(P.box));
+  PB_CUDA(cudaGetLastError());
+  sync();   // the temporaries above are released on return
+  return true;
+}
+
+template <class T>
+void ilu_small_setup(SmallPlan& P, const DevMat<double>& A, int ilu_method, const int* d_pos, const int* d_rowAt,
+                     IluDev<T>& D) {
+  cudaStream_t st = stream();
+  D.nb = P.nb; D.np = P.np; D.n = P.n;
+  D.dilu = ilu_method != 0;
+  D.small = true;
+  D.ring = D.grp = false;
+  D.K = 8;
+  for (int c : {6, 4, 3, 2, 1})
+    if (P.kmax <= c) D.K = c;
+  const int* blo = dp<int>(P.starts);
+  Factor F;
+  F.run(A, P.n, P.nb, P.maxw, ilu_method, LevelTab{dp<int>(P.blvl), dp<int>(P.lo), dp<int>(P.hi)}, blo, blo + 1,
+        d_rowAt, st);
+  // lanes per block: the widest level, rounded up to 8, 16 or 32 (wider levels take several
+  // rows per lane)
+  D.s_lpb = P.maxw <= 8 ? 8 : (P.maxw <= 16 ? 16 : 32);
+  // the staged variant when a block's area lets a warp's blocks (at most 4) fit the default
+  // 48 KB of a CTA
+  const int KC = small_kc(D.K);
+  const int levcap = align4(std::max(P.max_levels, 1));
+  const int64_t tb = (int64_t)P.span * (2 + D.K + (D.dilu ? 0 : 1)) * (int64_t)sizeof(T) +
+                     (int64_t)P.span * KC * 2 + 2LL * levcap * 4;
+  D.s_box_bytes = 0;
+  if (tb <= kStageBoxBytes) {
+    D.s_span = P.span;
+    D.s_levcap = levcap;
+    D.s_box_bytes = (int)tb;
+  }
+  const bool staged = D.s_box_bytes > 0;
+  const size_t rk = (size_t)P.np * D.K, ck = staged ? 2 * (size_t)P.np * KC : sizeof(int) * rk;
+  D.s_cF.alloc(ck); D.s_vF.alloc(sizeof(T) * rk); D.s_dF.alloc(sizeof(T) * P.np);
+  D.s_cB.alloc(ck); D.s_vB.alloc(sizeof(T) * rk); D.s_dB.alloc(sizeof(T) * P.np);
+  const int g = (int)std::min<int64_t>(((int64_t)P.n + 255) / 256, 8LL * num_sms());
+  k_ilu_small_pack<T><<<std::max(g, 1), 256, 0, st>>>(
+      P.n, P.nb, blo, blo + 1, d_pos, A.rowptr, A.col, A.rbase, A.cbase, F.vL, F.vU, F.dinv, D.dilu ? 1 : 0, D.K,
+      dp<int>(D.s_cF), dp<T>(D.s_vF), dp<T>(D.s_dF), dp<int>(D.s_cB), dp<T>(D.s_vB), dp<T>(D.s_dB), dp<int2>(P.box),
+      KC, staged ? dp<unsigned short>(D.s_cF) : nullptr, staged ? dp<unsigned short>(D.s_cB) : nullptr);
+  PB_CUDA(cudaGetLastError());
+  D.s_blvl = std::move(P.blvl);
+  D.s_lo = std::move(P.lo);
+  D.s_hi = std::move(P.hi);
+  D.s_box = std::move(P.box);
+  D.ytmp.alloc(sizeof(T) * (P.np + 4));
+  D.err.alloc(sizeof(int));
+  sync();   // the factors are released on return
+}
+template void ilu_small_setup<double>(SmallPlan&, const DevMat<double>&, int, const int*, const int*, IluDev<double>&);
+template void ilu_small_setup<float>(SmallPlan&, const DevMat<double>&, int, const int*, const int*, IluDev<float>&);
 
 template <class T, bool DILU, bool RING>
 static void launch_ilu(const IluDev<T>& D, const IluSolveArgs<T>& a, cudaStream_t st) {
@@ -1732,25 +1991,30 @@ static void launch_small_lpb(const IluDev<T>& D, const T* r, T* s, const int* ga
       dp<int>(D.s_cB), dp<T>(D.s_vB), dp<T>(D.s_dB), r, dp<T>(D.ytmp), s, gate);
 }
 
-template <class T, bool DILU, int K, int LPB>
-static void launch_staged(const IluDev<T>& D, const T* r, T* s, const int* gate, cudaStream_t st) {
+// Shared memory of a CTA besides its blocks' areas (the fused reduction's).
+constexpr int kStageStatic = 1024;
+
+template <class T, bool DILU, int K, int LPB, bool CG>
+static void launch_staged(const IluDev<T>& D, const T* r, T* s, const int* gate, cudaStream_t st,
+                          const SmallCg<T>& cg = {}) {
   constexpr int BPW = 32 / LPB;
   const int warp_bytes = BPW * D.s_box_bytes;
-  const int wpc = std::max(1, std::min(kStageWarps, 48 * 1024 / warp_bytes));
+  const int wpc = std::max(1, std::min(kStageWarps, (48 * 1024 - (CG ? kStageStatic : 0)) / warp_bytes));
   const int64_t groups = ((int64_t)D.nb + BPW - 1) / BPW;
   const int grid = (int)std::min<int64_t>((groups + wpc - 1) / wpc, 32LL * num_sms());
-  k_ilu_small_staged<T, DILU, K, LPB><<<grid, wpc * 32, (size_t)wpc * warp_bytes, st>>>(
-      D.nb, dp<int2>(D.s_box), dp<int>(D.s_blvl), dp<int>(D.s_lo), dp<int>(D.s_hi), dp<int>(D.s_cF),
-      dp<T>(D.s_vF), dp<T>(D.s_dF), dp<int>(D.s_cB), dp<T>(D.s_vB), dp<T>(D.s_dB), r, s, gate, D.s_span,
-      D.s_levcap, D.s_box_bytes);
+  k_ilu_small_staged<T, DILU, K, LPB, CG><<<grid, wpc * 32, (size_t)wpc * warp_bytes, st>>>(
+      D.nb, dp<int2>(D.s_box), dp<int>(D.s_blvl), dp<int>(D.s_lo), dp<int>(D.s_hi), dp<unsigned short>(D.s_cF),
+      dp<T>(D.s_vF), dp<T>(D.s_dF), dp<unsigned short>(D.s_cB), dp<T>(D.s_vB), dp<T>(D.s_dB), r, s, gate, D.s_span,
+      D.s_levcap, D.s_box_bytes, cg);
 }
 
 template <class T, bool DILU, int K>
 static void launch_small(const IluDev<T>& D, const T* r, T* s, const int* gate, cudaStream_t st) {
-  if (D.s_box_bytes > 0 && (reinterpret_cast<uintptr_t>(r) & 15) == 0) {
-    if (D.s_lpb == 8) launch_staged<T, DILU, K, 8>(D, r, s, gate, st);
-    else if (D.s_lpb == 16) launch_staged<T, DILU, K, 16>(D, r, s, gate, st);
-    else launch_staged<T, DILU, K, 32>(D, r, s, gate, st);
+  if (D.s_box_bytes > 0) {
+    PB_CHECK((reinterpret_cast<uintptr_t>(r) & 15) == 0, PARCEL_B_E_ARG, "right-hand side not 16-byte aligned");
+    if (D.s_lpb == 8) launch_staged<T, DILU, K, 8, false>(D, r, s, gate, st);
+    else if (D.s_lpb == 16) launch_staged<T, DILU, K, 16, false>(D, r, s, gate, st);
+    else launch_staged<T, DILU, K, 32, false>(D, r, s, gate, st);
     return;
   }
   if (D.s_lpb == 8) launch_small_lpb<T, DILU, K, 8>(D, r, s, gate, st);
@@ -1835,6 +2099,43 @@ void ilu_apply_dd(const IluDev<dd>& D, const dd* r, dd* s, cudaStream_t st) {
 }
 
 template <class T>
+bool ilu_apply_cg(const IluDev<T>& D, T* r, const T* q, const double* c, T* s, const Red& red, const int* gate,
+                  cudaStream_t st) {
+  // the staged sweep alone, with room for the reduction, 16-byte aligned vectors and block
+  // stretches that cover the whole layout
+  if (!D.small || D.s_box_bytes == 0) return false;
+  if ((32 / D.s_lpb) * D.s_box_bytes > 48 * 1024 - kStageStatic) return false;
+  if (((reinterpret_cast<uintptr_t>(r) | reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(s)) & 15) != 0)
+    return false;
+  SmallCg<T> cg;
+  cg.q = q; cg.r = r; cg.c = c; cg.red = red;
+#define SMALL_CG(K_)                                                                                            \
+  case K_:                                                                                                      \
+    if (D.s_lpb == 8) {                                                                                         \
+      if (D.dilu) launch_staged<T, true, K_, 8, true>(D, r, s, gate, st, cg);                                   \
+      else launch_staged<T, false, K_, 8, true>(D, r, s, gate, st, cg);                                         \
+    } else if (D.s_lpb == 16) {                                                                                 \
+      if (D.dilu) launch_staged<T, true, K_, 16, true>(D, r, s, gate, st, cg);                                  \
+      else launch_staged<T, false, K_, 16, true>(D, r, s, gate, st, cg);                                        \
+    } else {                                                                                                    \
+      if (D.dilu) launch_staged<T, true, K_, 32, true>(D, r, s, gate, st, cg);                                  \
+      else launch_staged<T, false, K_, 32, true>(D, r, s, gate, st, cg);                                        \
+    }                                                                                                           \
+    break;
+  switch (D.K) {
+    SMALL_CG(1) SMALL_CG(2) SMALL_CG(3) SMALL_CG(4) SMALL_CG(6) SMALL_CG(8)
+    default: return false;
+  }
+#undef SMALL_CG
+  PB_CUDA(cudaGetLastError());
+  return true;
+}
+template bool ilu_apply_cg<double>(const IluDev<double>&, double*, const double*, const double*, double*, const Red&,
+                                   const int*, cudaStream_t);
+template bool ilu_apply_cg<float>(const IluDev<float>&, float*, const float*, const double*, float*, const Red&,
+                                  const int*, cudaStream_t);
+
+template <class T>
 void ilu_apply(const IluDev<T>& D, const T* r, T* s, T* accum, const int* gate, cudaStream_t st) {
   if (D.small && !accum) {
 #define SMALL(K_)                                                                                  \
@@ -1867,7 +2168,7 @@ void ilu_apply(const IluDev<T>& D, const T* r, T* s, T* accum, const int* gate, 
     PB_CUDA(cudaGetLastError());
     return;
   }
-  PB_CHECK(!D.grp, PARCEL_B_E_UNSUPPORTED, "accumulating block-Jacobi apply needs the general sweep");
+  PB_CHECK(!D.grp && !D.small, PARCEL_B_E_UNSUPPORTED, "accumulating block-Jacobi apply needs the general sweep");
   IluSolveArgs<T> a;
   a.tabF = dp<ProdDesc>(D.tabF);
   a.tabB = dp<ProdDesc>(D.tabB);

@@ -172,6 +172,22 @@ template <class T>
 int ilu_setup_device(const IluPlan& P, const DevMat<double>& A, int ilu_method,
                      const int* d_pos, const int* d_rowAt, const int* d_lev, IluDev<T>& D);
 
+// Many small blocks (at least eight per SM, none above 1,024 rows): the wavefront plan built
+// on the device.  ilu_small_plan is false when a row has more couplings than the warp sweep's
+// records hold; the host plan takes such a matrix.
+struct SmallPlan {
+  int n = 0, nb = 0, np = 0, totlev = 0, maxw = 0, max_levels = 0, kmax = 0, span = 0;
+  DBuf starts;            // nb + 1 first rows
+  DBuf blvl, lo, hi;      // block -> first level; level -> [lo, hi) in the iteration layout
+  DBuf box;               // block -> {first position, stretch}
+  DBuf pos, rowAt;        // row -> position; position -> row or -1
+};
+bool ilu_small_blocks(const BlockSplit& bs, int n);
+bool ilu_small_plan(const BlockSplit& bs, const DevMat<double>& A, SmallPlan& P);
+template <class T>
+void ilu_small_setup(SmallPlan& P, const DevMat<double>& A, int ilu_method, const int* d_pos, const int* d_rowAt,
+                     IluDev<T>& D);
+
 // The double-double D-ILU sweep on the grouped records: lays out the sweep data of the natural
 // matrix (ah, al: value parts, al may be null) and the diagonal dih + dil (precision 1 drops
 // the low parts of both).  False when the sweep does not take this plan (more than six
@@ -182,6 +198,13 @@ bool ilu_setup_dd(const IluPlan& P, const DevMat<double>& A, const double* al, c
                   int precision, const int* d_pos, const int* d_rowAt, const int* d_lev, IluDev<dd>& D);
 // s = M^-1 r on level-ordered vectors of np entries.
 void ilu_apply_dd(const IluDev<dd>& D, const dd* r, dd* s, cudaStream_t st);
+
+// CG's r += c q, s = M^-1 r and the sums <s, r>, <r, r> (red's epilogue) in one launch; false
+// when this preconditioner has no such sweep (the caller then takes the separate kernels).
+struct Red;
+template <class T>
+bool ilu_apply_cg(const IluDev<T>& D, T* r, const T* q, const double* c, T* s, const Red& red, const int* gate,
+                  cudaStream_t st);
 
 // s = M^-1 r on permuted vectors (np entries each).  If `accum` is non-null the result
 // is added into it instead of being written to s (s may then be null).

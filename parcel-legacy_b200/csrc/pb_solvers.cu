@@ -161,12 +161,29 @@ void build_system(const Options& o, const parcel_b_crs& A, bool dev, System<T>& 
   S.M.kind = o.precon;
 
   if (o.precon == PARCEL_B_PRECON_BLOCKJACOBI) {
-    // The wavefront analysis runs on the host.  A device-resident structure comes back
+    // The wavefront analysis runs on the host unless there are many small blocks.  A device-resident structure comes back
     // through page-locked staging: the row pointers first, then the column indices in
     // block-aligned pieces, each with an event, so that the plan of the first blocks
     // overlaps the copy of the others.  The plan writes the permutation and the levels
     // into the same staging area, from where they go back to the device.
     const BlockSplit bs = block_split(o, A.n);
+    SmallPlan sp;
+    if (ilu_small_blocks(bs, A.n) && ilu_small_plan(bs, S.Anat, sp)) {
+      trace_mark("setup: wavefront plan (device)");
+      S.np = sp.np;
+      S.permuted = true;
+      S.ilu_levels_max = sp.max_levels;
+      S.ilu_nblocks = sp.nb;
+      S.pos = std::move(sp.pos);
+      S.rowAt = std::move(sp.rowAt);
+      S.A = DevMat<T>{};
+      S.A.nnz = A.nnz;
+      build_sell<T>(S.Anat, S.np, dp<int>(S.rowAt), dp<int>(S.pos), S.Asell, S.A);
+      trace_mark("setup: sliced ELLPACK");
+      ilu_small_setup<T>(sp, S.Anat, o.ilu_method, dp<int>(S.pos), dp<int>(S.rowAt), S.M.ilu);
+      trace_mark("setup: ILU factor + pack");
+      return;
+    }
     const int nb = bs.nb;
     const size_t n1 = (size_t)A.n + 1, nz = (size_t)A.nnz;
     int* pin = static_cast<int*>(pinned_staging(sizeof(int) * ((dev ? n1 + nz : 0) + 2 * (size_t)A.n)));
@@ -361,11 +378,19 @@ static SolveOut run_pcg(const Options& o, const System<T>& S, const T* b, T* x, 
     return finish();
   }
   const int chunk = 16;
+  int& per_chunk = kw.per_cycle;   // counted when the chunk is captured
   auto iterations = [&] {
+    per_chunk = 0;
     for (int it = 0; it < chunk; ++it) {
       cg_axpy2<T>(np, x, P, Sv, K, gdone, st);                            // x += alpha p; p = s + beta p
       int sa[2] = {1, 0}, sb[2] = {0, 0};
       spmv_dot<T, T>(S.A, P, Q, SPMV_Y, nullptr, nullptr, 1, sa, sb, red(EPI_CG_GAMMA), gdone, st);
+      if (S.M.kind == PARCEL_B_PRECON_BLOCKJACOBI &&
+          ilu_apply_cg<T>(S.M.ilu, R, Q, &K->tmp[0], Sv, red(EPI_CG_DOT2), gdone, st)) {
+        per_chunk += 3;
+        continue;
+      }
+      per_chunk += 5;
       lincomb<T>(np, R, Q, cdev(&K->tmp[0]), R, cimm(1.0), nullptr, cimm(0), gdone, st);  // r = -alpha q + r
       S.M.apply(np, R, Sv, gdone, st);                                    // s = M^-1 r
       DotSel d2;
@@ -380,7 +405,7 @@ static SolveOut run_pcg(const Options& o, const System<T>& S, const T* b, T* x, 
   for (int c = 0; c < max_chunks; ++c) {
     if (read_done(K, st)) break;
     G.launch(iterations, o.use_graphs, st);
-    launches += 5 * chunk;
+    launches += per_chunk;
   }
   return finish();
 }

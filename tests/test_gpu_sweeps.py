@@ -78,6 +78,71 @@ def test_level_widths(nx, ny):
         assert _apply_both(A, ipreflag=2, ILU_method=ilu, precon_thblock=1) < 1e-11
 
 
+# ---- many small blocks: plan on the device, CG's step fused into the sweep --------------------
+def _dense_blocks(nb, rows, seed):
+    """nb blocks of `rows` fully coupled rows each, linked to the next block by one entry."""
+    rng = np.random.default_rng(seed)
+    n = nb * rows
+    i = np.arange(n)
+    base = i // rows * rows
+    col = base[:, None] + np.arange(rows)[None, :]
+    val = rng.uniform(-1, 1, (n, rows))
+    val[i, i - base] = 2.0 * rows
+    col = np.concatenate([col, np.minimum(base + rows, n - 1)[:, None]], 1)
+    val = np.concatenate([val, np.full((n, 1), 0.5)], 1)
+    keep = np.ones_like(col, bool)
+    keep[:, -1] = base + rows < n
+    rp = np.concatenate([[0], np.cumsum(keep.sum(1))]) + 1
+    return problems.CRS(n=n, rowptr=rp.astype(np.int32), col=(col[keep] + 1).astype(np.int32), val=val[keep])
+
+
+@pytest.mark.parametrize("ilu", [0, 1, 2])
+@pytest.mark.parametrize("nb,rows", [(1300, 1), (1300, 3), (1400, 9), (1200, 12)])
+def test_small_dense_blocks(nb, rows, ilu):
+    """One-row blocks, one coupling count after the other, and more couplings than the records
+    hold (the host plan and the general sweep)."""
+    A = _dense_blocks(nb, rows, rows)
+    assert _apply_both(A, ipreflag=2, ILU_method=ilu, precon_thblock=nb) < 1e-11
+
+
+@pytest.mark.parametrize("ilu", [0, 1])
+@pytest.mark.parametrize("N,blocks", [(24, 1200), (24, 2000), (24, 5000), (61, 1500), (30, 27000)])
+def test_small_blocks_cg(N, blocks, ilu):
+    """CG through the fused sweep: 8, 16 and 32 lanes per block, staged and (61^3: 151 rows a
+    block) long stretches, one row per block; iterations and x against the oracle's."""
+    A = problems.poisson3d_reference(N, N, N)[0]
+    b = problems.rhs_normal(A.n, N)
+    kw = dict(solver=1, itrmax=60 if N > 40 else 400, rtolmax=1e-10, ipreflag=2, ILU_method=ilu,
+              precon_thblock=blocks)
+    xo, ho, no, io = oracle.solve(A, b, **kw)
+    res = api.solve(A, b, **kw)
+    assert abs(res["niter"] - no) <= 1
+    k = min(len(ho), len(res["reshistory"]))
+    assert (np.abs(res["reshistory"][:k] - ho[:k]) / ho[:k]).max() < 1e-6
+    assert np.abs(res["x"] - xo).max() < 1e-7 * np.abs(xo).max()
+
+
+def test_small_blocks_mixed_precision_cg():
+    A = problems.poisson3d_reference(24, 24, 24)[0]
+    b = problems.rhs_normal(A.n, 2)
+    res = api.solve(A, b, solver=1, itrmax=2000, rtolmax=1e-12, ipreflag=2, ILU_method=1, precon_thblock=2000,
+                    inner_precision=1, inner_rtol=1e-4, residual_dd=1, max_refine=50)
+    assert res["iret"] == 0 and res["stats"]["true_relres"] < 1e-12
+
+
+def test_small_blocks_missing_diagonal_is_an_error():
+    A = _dense_blocks(1300, 3, 1)
+    A.col[A.rowptr[700] - 1:A.rowptr[701] - 1][...] = np.clip(
+        A.col[A.rowptr[700] - 1:A.rowptr[701] - 1], 1, A.n)
+    row = slice(A.rowptr[700] - 1, A.rowptr[701] - 1)
+    keep = A.col[row] != 701
+    B = problems.CRS(n=A.n, rowptr=A.rowptr.copy(), col=np.delete(A.col, np.flatnonzero(~keep) + row.start),
+                     val=np.delete(A.val, np.flatnonzero(~keep) + row.start))
+    B.rowptr[701:] -= 1
+    with pytest.raises(RuntimeError, match="block 233 has a row without an in-block diagonal"):
+        api.solve(B, np.ones(B.n), solver=3, ipreflag=2, ILU_method=0, precon_thblock=1300)
+
+
 # ---- CG of short vectors in one launch -----------------------------------------------------------
 @pytest.mark.parametrize("ipreflag", [0, 1])
 @pytest.mark.parametrize("nx,ny", [(1, 1), (3, 2), (32, 16), (33, 16), (270, 281), (280, 271), (389, 390), (551, 550)])
