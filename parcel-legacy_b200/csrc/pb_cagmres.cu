@@ -304,6 +304,111 @@ __global__ void __launch_bounds__(256) k_tsqr_local(int64_t nrows, int c, const 
   }
 }
 
+// Structured Householder TSQR with the factor in a thread, for panels of at most kQrMaxC
+// columns.  A thread folds RB rows at a time (32 apart, so that a warp's loads are
+// contiguous) into its own upper triangular R: the norms and products of a column are sums
+// over the thread's registers, where one row per lane made each of them five shuffles (36
+// per 32 rows of an 8-column panel; 205 us per launch).  The threads' factors are then
+// folded pairwise by shuffles, the warps' through shared memory, so a CTA leaves one C x C
+// factor and two launches do: 148 CTAs, then one.  Bound by the FP64 pipe (about 1,700
+// operations per 8 rows of 8 columns) beside the panel's one read.
+constexpr int kQrMaxC = 10;
+constexpr int kQrThreads = 256;
+constexpr int qr_rows(int C) { return C <= 8 ? 8 : (C == 9 ? 6 : 5); }
+
+// [R; X] -> R by reflectors that touch R's diagonal entry and the rows of X.  TRI: X is upper
+// triangular too (row i starts at column i).
+template <int C, int RB, bool TRI>
+__device__ __forceinline__ void qr_fold(double (&R)[C][C], double (&X)[RB][C]) {
+#pragma unroll
+  for (int k = 0; k < C; ++k) {
+    double sig = 0.0;
+#pragma unroll
+    for (int i = 0; i < RB; ++i)
+      if (!TRI || i <= k) sig += X[i][k] * X[i][k];
+    const double alpha = R[k][k];
+    const double nrm = sqrt(alpha * alpha + sig);
+    const double beta = alpha >= 0.0 ? -nrm : nrm;
+    const bool on = sig != 0.0;   // a column of zeros: nothing to reflect
+    const double inv = on ? 1.0 / (alpha - beta) : 0.0, tau = on ? (beta - alpha) / beta : 0.0;
+#pragma unroll
+    for (int i = 0; i < RB; ++i)
+      if (!TRI || i <= k) X[i][k] *= inv;
+#pragma unroll
+    for (int j = k + 1; j < C; ++j) {
+      double w = R[k][j];
+#pragma unroll
+      for (int i = 0; i < RB; ++i)
+        if (!TRI || i <= k) w += X[i][k] * X[i][j];
+      w *= tau;
+      R[k][j] -= w;
+#pragma unroll
+      for (int i = 0; i < RB; ++i)
+        if (!TRI || i <= k) X[i][j] -= w * X[i][k];
+    }
+    R[k][k] = on ? beta : alpha;
+  }
+}
+
+// Folds lane l + o's factor into lane l's, o = 1, 2, .. below `lanes` (a power of two): lane 0 ends with all.
+template <int C>
+__device__ __forceinline__ void qr_fold_lanes(double (&R)[C][C], int lanes) {
+  for (int o = 1; o < lanes; o <<= 1) {
+    double X[C][C];
+#pragma unroll
+    for (int i = 0; i < C; ++i)
+#pragma unroll
+      for (int j = i; j < C; ++j) X[i][j] = __shfl_down_sync(kFull, R[i][j], o);
+    qr_fold<C, C, true>(R, X);
+  }
+}
+
+template <int C>
+__global__ void __launch_bounds__(kQrThreads, 1) k_tsqr_thread(int64_t n, int c, const double* __restrict__ A,
+                                                             int64_t lda, double* __restrict__ Rout, int64_t ldo) {
+  constexpr int RB = qr_rows(C), NW = kQrThreads / 32;
+  __shared__ double sr[NW][C * C];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double R[C][C];
+#pragma unroll
+  for (int i = 0; i < C; ++i)
+#pragma unroll
+    for (int j = 0; j < C; ++j) R[i][j] = 0.0;
+  const int64_t tiles = (n + 32 * RB - 1) / (32 * RB);
+  for (int64_t t = (int64_t)blockIdx.x * NW + warp; t < tiles; t += (int64_t)gridDim.x * NW) {
+    double X[RB][C];
+#pragma unroll
+    for (int j = 0; j < C; ++j)
+#pragma unroll
+      for (int i = 0; i < RB; ++i) {
+        const int64_t row = t * (32 * RB) + i * 32 + lane;
+        X[i][j] = (j < c && row < n) ? A[(size_t)j * lda + row] : 0.0;
+      }
+    qr_fold<C, RB, false>(R, X);
+  }
+  qr_fold_lanes<C>(R, 32);
+  if (lane == 0) {
+#pragma unroll
+    for (int i = 0; i < C; ++i)
+#pragma unroll
+      for (int j = 0; j < C; ++j) sr[warp][i * C + j] = j >= i ? R[i][j] : 0.0;
+  }
+  __syncthreads();
+  if (warp != 0) return;
+#pragma unroll
+  for (int i = 0; i < C; ++i)
+#pragma unroll
+    for (int j = 0; j < C; ++j) R[i][j] = lane < NW ? sr[lane][i * C + j] : 0.0;
+  qr_fold_lanes<C>(R, NW);
+  if (lane == 0) {
+#pragma unroll
+    for (int i = 0; i < C; ++i)
+#pragma unroll
+      for (int j = 0; j < C; ++j)
+        if (i < c && j < c) Rout[(size_t)j * ldo + (int64_t)blockIdx.x * c + i] = j >= i ? R[i][j] : 0.0;
+  }
+}
+
 // ------------------------------------------------------------------ host helpers
 namespace {
 
@@ -361,7 +466,30 @@ Mat tsqr_r(Dev& D, int64_t n, const double* A, int64_t lda, int c) {
   int64_t curld = lda, rows = n;
   DBuf bufs[2];
   int which = 0;
-  while (true) {
+  auto launch = [&](auto kern, int C) {
+    const int64_t tiles = (rows + 32 * qr_rows(C) - 1) / (32 * qr_rows(C));
+    // one CTA per SM, and one in all when its warps have few tiles each
+    const int grid = tiles <= 64 ? 1 : (int)std::min<int64_t>(num_sms(), (tiles + 7) / 8);
+    bufs[which].alloc(sizeof(double) * (size_t)grid * c * c);
+    kern<<<grid, kQrThreads, 0, st>>>(rows, c, cur, curld, dp<double>(bufs[which]), (int64_t)grid * c);
+    PB_CUDA(cudaGetLastError());
+    cur = dp<double>(bufs[which]);
+    curld = rows = (int64_t)grid * c;
+    which ^= 1;
+    return grid;
+  };
+  while (c <= kQrMaxC) {
+    int grid;
+    if (c <= 2) grid = launch(k_tsqr_thread<2>, 2);
+    else if (c <= 4) grid = launch(k_tsqr_thread<4>, 4);
+    else if (c <= 5) grid = launch(k_tsqr_thread<5>, 5);
+    else if (c <= 6) grid = launch(k_tsqr_thread<6>, 6);
+    else if (c <= 8) grid = launch(k_tsqr_thread<8>, 8);
+    else if (c <= 9) grid = launch(k_tsqr_thread<9>, 9);
+    else grid = launch(k_tsqr_thread<10>, 10);
+    if (grid == 1) break;
+  }
+  while (c > kQrMaxC) {
     const int64_t warps_max = (int64_t)num_sms() * 16;
     int64_t rpw = std::max<int64_t>(512, (rows + warps_max - 1) / warps_max);
     rpw = (rpw + 31) / 32 * 32;
@@ -370,10 +498,7 @@ Mat tsqr_r(Dev& D, int64_t n, const double* A, int64_t lda, int c) {
     bufs[which].alloc(sizeof(double) * (size_t)ldo * c);
     const int threads = 256;
     const int64_t blocks = (nw * 32 + threads - 1) / threads;
-    if (c <= 8)
-      k_tsqr_local<8><<<(unsigned)blocks, threads, 0, st>>>(rows, c, cur, curld, rpw, dp<double>(bufs[which]), ldo);
-    else
-      k_tsqr_local<16><<<(unsigned)blocks, threads, 0, st>>>(rows, c, cur, curld, rpw, dp<double>(bufs[which]), ldo);
+    k_tsqr_local<16><<<(unsigned)blocks, threads, 0, st>>>(rows, c, cur, curld, rpw, dp<double>(bufs[which]), ldo);
     PB_CUDA(cudaGetLastError());
     cur = dp<double>(bufs[which]);
     curld = ldo;
@@ -383,7 +508,8 @@ Mat tsqr_r(Dev& D, int64_t n, const double* A, int64_t lda, int c) {
   }
   Mat R(c, c);
   std::vector<double> h((size_t)c * c);
-  for (int j = 0; j < c; ++j) d2h(&R.a[(size_t)j * c], cur + (size_t)j * curld, sizeof(double) * c);
+  PB_CHECK(curld == c, PARCEL_B_E_ARG, "TSQR left %lld rows", (long long)curld);
+  d2h(R.a.data(), cur, sizeof(double) * c * c);
   for (int i = 0; i < c; ++i)
     for (int j = 0; j < i; ++j) R(i, j) = 0.0;
   for (int i = 0; i < c; ++i)
@@ -410,7 +536,7 @@ Mat qr_r_only(Dev& D, int64_t n, const double* V, int64_t ldv, int c, int flag) 
     Mat R1;
     if (dense::chol_upper(G, R1)) {
       if (flag == PARCEL_B_QR_CHOLQR) return R1;
-      D.tmp.alloc(sizeof(double) * (size_t)ldv * c);
+      D.tmp.alloc(sizeof(double) * (size_t)ldv * c, false);
       apply_rinv(D, n, V, ldv, dense::trinv_upper(R1), dp<double>(D.tmp), ldv);
       Mat G2 = tsgemm(D, n, dp<double>(D.tmp), ldv, c, dp<double>(D.tmp), ldv, c);
       Mat R2;
@@ -589,10 +715,13 @@ SolveOut solve_cagmres(const Options& o, System<double>& S, const double* b_nat,
     b = dp<double>(bb);
     x = dp<double>(xb);
   }
-  DBuf Vb(sizeof(double) * ldv * (s + 1)), Qb(sizeof(double) * ldv * (stt + 1)), rb(sizeof(double) * np),
+  // every column's np entries are written before they are read, so the panels (2.3 GB at 4M
+  // rows and 64 + 9 columns) are not zero-filled
+  DBuf Vb, Qb;
+  Vb.alloc(sizeof(double) * ldv * (s + 1), false);
+  Qb.alloc(sizeof(double) * ldv * (stt + 1), false);
+  DBuf rb(sizeof(double) * np),
       pvb(sizeof(double) * np), v0b(sizeof(double) * np), x0b(sizeof(double) * np), yb(sizeof(double) * (stt + 1));
-  PB_CUDA(cudaMemsetAsync(Vb.p, 0, Vb.bytes, st));
-  PB_CUDA(cudaMemsetAsync(Qb.p, 0, Qb.bytes, st));
   double* V = dp<double>(Vb);
   double* Q = dp<double>(Qb);
   double* r = dp<double>(rb);

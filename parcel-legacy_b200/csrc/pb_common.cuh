@@ -58,7 +58,8 @@ struct DBuf {
     return *this;
   }
   ~DBuf() { release(); }
-  void alloc(size_t b);    // zero-filled on the library stream; bytes may be rounded up
+  // zero-filled on the library stream unless zero is false; bytes may be rounded up
+  void alloc(size_t b, bool zero = true);
   void zero_fill();
   void release();          // returns the buffer to the library's cache
 };

@@ -134,7 +134,7 @@ void release_buffer_cache() {
   g_pin_bytes = 0;
 }
 
-void DBuf::alloc(size_t b) {
+void DBuf::alloc(size_t b, bool zero) {
   release();
   if (b == 0) return;
   ensure_init();
@@ -150,7 +150,7 @@ void DBuf::alloc(size_t b) {
   }
   if (p) {
     bytes = rb;
-    zero_fill();
+    if (zero) zero_fill();
     return;
   }
   cudaError_t e = cudaMalloc(&p, rb);
@@ -170,10 +170,10 @@ void DBuf::alloc(size_t b) {
     throw Error{PARCEL_B_E_NOMEM, "cudaMalloc failed"};
   }
   bytes = rb;
-  zero_fill();
+  if (zero) zero_fill();
 }
 
-// Every buffer starts zeroed (stream-ordered): layout padding positions that no kernel
+// Every buffer starts zeroed (stream-ordered) unless its user writes all it reads: layout padding positions that no kernel
 // writes (rows of the iteration layout that belong to no matrix row) must hold zeros, not
 // a previous solve's values.
 void DBuf::zero_fill() {
