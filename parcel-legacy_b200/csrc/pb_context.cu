@@ -109,29 +109,10 @@ void cache_trim_locked() {
 }
 }  // namespace
 
-namespace {
-void* g_pin = nullptr;
-size_t g_pin_bytes = 0;
-}  // namespace
-
-void* pinned_staging(size_t bytes) {
-  if (bytes > g_pin_bytes) {
-    if (g_pin) cudaFreeHost(g_pin);
-    g_pin = nullptr;
-    g_pin_bytes = 0;
-    PB_CUDA(cudaMallocHost(&g_pin, bytes));
-    g_pin_bytes = bytes;
-  }
-  return g_pin;
-}
-
 void release_buffer_cache() {
   std::lock_guard<std::mutex> lk(g_cache_mu);
   if (g_ctx.stream) cudaStreamSynchronize(g_ctx.stream);
   cache_trim_locked();
-  if (g_pin) cudaFreeHost(g_pin);
-  g_pin = nullptr;
-  g_pin_bytes = 0;
 }
 
 void DBuf::alloc(size_t b, bool zero) {

@@ -927,6 +927,16 @@ __global__ void __launch_bounds__(256, 1)
   }
 }
 
+// Ring slot of every row: level mod W, position within the level (widest level LW).
+__global__ void k_dd_ring_slots(int n, const int* __restrict__ blk_of, const int* __restrict__ blvl,
+                                const int* __restrict__ lst, const int* __restrict__ lev, const int* __restrict__ pos,
+                                int W, int LW, int* __restrict__ slot) {
+  GRID_LOOP(i, n) {
+    const int l = lev[i];
+    slot[i] = (l % W) * LW + pos[i] - lst[blvl[blk_of[i]] + l];
+  }
+}
+
 __global__ void k_block_of(int nb, const int* __restrict__ blk_lo, const int* __restrict__ blk_hi, int* blk_of) {
   const int b = blockIdx.x;
   if (b >= nb) return;
@@ -1021,35 +1031,19 @@ void dd_setup_precon(const Options& o, const parcel_b_crs& A, const DdSystem& S,
            "ipreflag=%d: the dd CG provides none, point Jacobi and block Jacobi", o.precon);
   PB_CHECK(o.ilu_method == 1 || o.ilu_method == 2, PARCEL_B_E_UNSUPPORTED,
            "ILU_method=%d: the dd CG's block-Jacobi preconditioner is D-ILU (1 or 2)", o.ilu_method);
-  // wavefront plan on the host (the structure comes back from the device if it lives there)
-  std::vector<int> hrp, hci;
-  const int* hrpp = A.rowptr;
-  const int* hcip = A.col;
-  if (is_device_ptr(A.rowptr)) {
-    hrp.resize((size_t)A.n + 1);
-    hci.resize((size_t)A.nnz);
-    d2h(hrp.data(), A.rowptr, sizeof(int) * hrp.size());
-    d2h(hci.data(), A.col, sizeof(int) * hci.size());
-    hrpp = hrp.data();
-    hcip = hci.data();
-  }
-  HostCSR H;
-  H.n = A.n; H.nnz = A.nnz; H.istart = A.istart; H.rowptr = hrpp; H.col = hcip;
-  std::vector<int> pos(A.n), lev(A.n);
+  DevMat<double> M;
+  M.n = S.n; M.nnz = A.nnz; M.rowptr = S.rp; M.col = S.ci; M.val = S.ah; M.rbase = 1; M.cbase = S.cbase;
   IluPlan plan;
-  ilu_build_plan(H, block_split(o, A.n), plan, pos.data(), lev.data());
+  DBuf dpos, dlev;
+  ilu_build_plan(M, block_split(o, A.n), true, plan, dpos, P.rowAt, dlev);
   P.nb = plan.nb;
   P.chunks.alloc(sizeof(IluChunk) * std::max<size_t>(plan.chunks.size(), 1));
   h2d(P.chunks.p, plan.chunks.data(), sizeof(IluChunk) * plan.chunks.size());
   P.blk_chunk.alloc(sizeof(int) * (plan.nb + 1));
   h2d(P.blk_chunk.p, plan.blk_chunk.data(), sizeof(int) * (plan.nb + 1));
-  DBuf dpos(sizeof(int) * A.n), blo(sizeof(int) * plan.nb), bhi(sizeof(int) * plan.nb), bof(sizeof(int) * A.n);
-  h2d(dpos.p, pos.data(), sizeof(int) * A.n);
+  DBuf blo(sizeof(int) * plan.nb), bhi(sizeof(int) * plan.nb), bof(sizeof(int) * A.n);
   h2d(blo.p, plan.blk_lo.data(), sizeof(int) * plan.nb);
   h2d(bhi.p, plan.blk_hi.data(), sizeof(int) * plan.nb);
-  P.rowAt.alloc(sizeof(int) * plan.np);
-  PB_CUDA(cudaMemsetAsync(P.rowAt.p, 0xFF, sizeof(int) * plan.np, st));
-  scatter_positions(A.n, dp<int>(dpos), dp<int>(P.rowAt), st);
   k_block_of<<<plan.nb, 256, 0, st>>>(plan.nb, dp<int>(blo), dp<int>(bhi), dp<int>(bof));
   P.rng.alloc(sizeof(int4) * A.n);
   k_dd_ranges<<<grid_for(A.n), kDdThreads, 0, st>>>(A.n, plan.nb, dp<int>(blo), dp<int>(bhi), dp<int>(bof), S.rp,
@@ -1063,10 +1057,6 @@ void dd_setup_precon(const Options& o, const parcel_b_crs& A, const DdSystem& S,
   const int np = plan.np;
   P.np = np;
   {
-    DBuf dlev(sizeof(int) * A.n);
-    h2d(dlev.p, lev.data(), sizeof(int) * A.n);
-    DevMat<double> M;
-    M.n = S.n; M.nnz = A.nnz; M.rowptr = S.rp; M.col = S.ci; M.val = S.ah; M.rbase = 1; M.cbase = S.cbase;
     if (ilu_setup_dd(plan, M, S.al, dp<double>(P.dih), dp<double>(P.dil), prec_M, dp<int>(dpos), dp<int>(P.rowAt),
                      dp<int>(dlev), P.grp)) {
       P.rq.alloc(sizeof(dd) * np);
@@ -1080,14 +1070,13 @@ void dd_setup_precon(const Options& o, const parcel_b_crs& A, const DdSystem& S,
   const int64_t ring_rows = (int64_t)plan.W * LW;
   DBuf drs;
   if (ring_rows > 0 && 2 * ring_rows * (int64_t)sizeof(double) <= kDdRingBytes) {
-    std::vector<int> rslot(A.n);
-    for (int b = 0; b < plan.nb; ++b)
-      for (int c = plan.blk_lo[b]; c < plan.blk_hi[b]; ++c) {
-        const int l = lev[c];
-        rslot[c] = (l % plan.W) * LW + (pos[c] - plan.lvl_start[plan.blk_lvl[b] + l]);
-      }
+    DBuf blvl(sizeof(int) * (plan.nb + 1)), lst(sizeof(int) * std::max<size_t>(plan.lvl_start.size(), 1));
+    h2d(blvl.p, plan.blk_lvl.data(), sizeof(int) * (plan.nb + 1));
+    h2d(lst.p, plan.lvl_start.data(), sizeof(int) * plan.lvl_start.size());
     drs.alloc(sizeof(int) * A.n);
-    h2d(drs.p, rslot.data(), sizeof(int) * A.n);
+    k_dd_ring_slots<<<grid_for(A.n), kDdThreads, 0, st>>>(A.n, dp<int>(bof), dp<int>(blvl), dp<int>(lst), dp<int>(dlev),
+                                                          dp<int>(dpos), plan.W, LW, dp<int>(drs));
+    PB_CUDA(cudaGetLastError());
     P.ring_rows = (int)ring_rows;
   }
   const size_t nq = (size_t)np, nt = (size_t)kPre * np;

@@ -21,7 +21,6 @@
 // a shared-memory ring, so a level step costs shared-memory latency and one named
 // barrier.  The arithmetic of every row is the reference's: same operands, same order.
 #include <algorithm>
-#include <omp.h>
 #include <cub/device/device_scan.cuh>
 #include <climits>
 #include <cmath>
@@ -37,8 +36,8 @@ namespace pb {
 
 namespace {
 
-// tighten_levels runs when a ring of the early levels (gap + 1 of mean width) would hold
-// more than this many rows: below it the ring fits beside the stages as it is
+// the plan looks for later levels when a ring of the early ones (gap + 1 of mean width) would
+// hold more than this many rows: below it the ring fits beside the stages as it is
 constexpr int64_t kTightenRing = 2048;
 
 inline int align4(int x) { return (x + 3) & ~3; }
@@ -60,200 +59,324 @@ void ilu_block_rows(int b, int nb, int n, int* lo, int* hi) {
   *hi = (int)h;
 }
 
-__global__ void k_scatter_rowat(int n, const int* __restrict__ pos, int* __restrict__ rowAt) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) rowAt[pos[i]] = i;
-}
-
-void scatter_positions(int n, const int* pos, int* rowAt, cudaStream_t st) {
-  if (n <= 0) return;
-  const int grid = (int)std::min<int64_t>(((int64_t)n + 255) / 256, 8LL * num_sms());
-  k_scatter_rowat<<<grid, 256, 0, st>>>(n, pos, rowAt);
-  PB_CUDA(cudaGetLastError());
-}
-
-// ------------------------------------------------------------------ host plan
-// Levels as late as their dependents allow, rows without dependents left where they are:
-// every row with dependents moves to one below its lowest dependent.  The number of levels and
-// the validity of the order are unchanged (the longest chain has no slack); what changes is
-// the largest level gap of a coupling.  A block that starts in the middle of a grid plane has
-// rows that could start at once but are only needed a hundred levels later; with the levels
-// taken as early as possible the ring of a 12,000-row block of a 61 x 53 x 47 stencil would
-// hold 58 levels, tightened it holds 2, as for a block of whole planes, and the grouped sweep
-// takes it instead of the general one, which gathers coupled values from global memory:
-// 147 -> 33 us per application there (16 blocks), 248 -> 53 us on 97 x 89 x 83 in 48 blocks.
-// Returns the new gap, or the old one (and the old levels) when it is no larger.
-static int tighten_levels(const HostCSR& A, int lo, int hi, int gap, int* lev, std::vector<int>& first,
-                   std::vector<int>& last, std::vector<int>& late) {
-  const int* rp = A.rowptr;
-  const int* ci = A.col;
-  const int cb = A.istart;
-  first.assign(hi - lo, INT_MAX);   // lowest and highest level of a row's dependents
-  last.assign(hi - lo, -1);
-  late.resize(hi - lo);
-  int g = 0;
-  for (int i = hi - 1; i >= lo; --i) {
-    int f = first[i - lo], l = last[i - lo];
-    for (int j = rp[i] - 1; j < rp[i + 1] - 1; ++j) {
-      const int c = ci[j] - cb;
-      if (c <= i || c >= hi) continue;
-      f = std::min(f, late[c - lo]);
-      l = std::max(l, late[c - lo]);
-    }
-    const int L = f == INT_MAX ? lev[i] : f - 1;
-    late[i - lo] = L;
-    if (l >= 0) g = std::max(g, l - L);
-    for (int j = rp[i] - 1; j < rp[i + 1] - 1; ++j) {
-      const int c = ci[j] - cb;
-      if (c < lo || c >= i) continue;
-      first[c - lo] = std::min(first[c - lo], L);
-      last[c - lo] = std::max(last[c - lo], L);
-    }
-  }
-  if (g >= gap) return gap;
-  std::copy(late.begin(), late.end(), lev + lo);
-  return g;
-}
-
+// ------------------------------------------------------------------ wavefront plan
 // Levels: row x waits for every in-block row y < x coupled to it in either direction
 // (a lower entry of x, or an upper entry (y, x) of y), so one level order serves the
-// forward and the backward sweep.  The dependency window W is the largest level gap of
-// any coupling + 1; it is found in the same pass: lower couplings compare with rows whose
-// level is final, upper couplings (y, x) through the lowest level among x's upper-entry
-// sources, known once x is reached.
-void ilu_build_plan(const HostCSR& A, const BlockSplit& blocks, IluPlan& P, int* pos_out, int* lev_out,
-                    const std::function<void(int)>& block_ready) {
-  const int n = A.n;
-  const int nb = blocks.nb;
-  P.n = n;
-  P.nb = nb;
-  P.lev = lev_out;
-  P.pos = pos_out;
-  P.blk_lo.resize(nb);
-  P.blk_hi.resize(nb);
-  for (int b = 0; b < nb; ++b) blocks.rows(b, n, &P.blk_lo[b], &P.blk_hi[b]);
-  std::vector<int> nlev(nb, 0), gap(nb, 0), missing_diag(nb, 0);
-  // per-row coupling counts, written for every row by the level pass (no zero fill: first
-  // touched by the threads that use them)
-  std::unique_ptr<int[]> cL(new int[std::max(n, 1)]), cU(new int[std::max(n, 1)]);
-  const int* rp = A.rowptr;
-  const int* ci = A.col;
-  const int cb = A.istart;
-  int* lev = lev_out;
-  // one core is left to the caller's other threads: a plan thread that the scheduler
-  // pre-empts for a time slice would hold up the whole loop
-  const int nthr = std::max(1, omp_get_num_procs() - 1);
-  // blocks are handed out in runs: one at a time when there are few (large) blocks, about
-  // 32 runs per thread when there are tens of thousands of small ones, so that the
-  // per-level counters of neighbouring blocks are mostly written by one thread
-  const int grain = std::max(1, nb / (32 * nthr));
-#pragma omp parallel num_threads(nthr)
-  {
-    std::vector<int> lb, lsrc, late;   // this thread's scratch, reused across its blocks
-#pragma omp for schedule(dynamic, grain)
-    for (int b = 0; b < nb; ++b) {
-      if (block_ready) block_ready(b);
-      const int lo = P.blk_lo[b], hi = P.blk_hi[b];
-      lb.assign(hi - lo, 0);
-      lsrc.assign(hi - lo, INT_MAX);
-      int maxlev = 0, g = 0;
-      for (int i = lo; i < hi; ++i) {
-        // columns are sorted: the lower entries come first, so the row's level is final at
-        // its first upper entry and one walk over the row suffices
-        int L = lb[i - lo];
-        int nl = 0, nu = 0, lmin = lsrc[i - lo];
-        bool diag = false, fixed = false, unsorted = false;
-        for (int j = rp[i] - 1; j < rp[i + 1] - 1; ++j) {
-          const int c = ci[j] - cb;
-          if (c < lo || c >= hi) continue;
-          if (c < i) {
-            unsorted |= fixed;
-            L = std::max(L, lev[c] + 1);
-            lmin = std::min(lmin, lev[c]);
-            ++nl;
-          } else if (c == i) {
-            diag = true;
-          } else {
-            fixed = true;
-            // an upper entry (i, c) makes c wait for i in the backward sweep order as well
-            lb[c - lo] = std::max(lb[c - lo], L + 1);
-            lsrc[c - lo] = std::min(lsrc[c - lo], L);
-            ++nu;
-          }
-        }
-        if (unsorted)   // a lower entry after an upper one: redo the upper entries with the final level
-          for (int j = rp[i] - 1; j < rp[i + 1] - 1; ++j) {
-            const int c = ci[j] - cb;
-            if (c > i && c < hi) {
-              lb[c - lo] = std::max(lb[c - lo], L + 1);
-              lsrc[c - lo] = std::min(lsrc[c - lo], L);   // an earlier, smaller L only widens W
-            }
-          }
-        if (!diag) missing_diag[b] = 1;
-        lev[i] = L;
-        cL[i] = nl; cU[i] = nu;
-        maxlev = std::max(maxlev, L);
-        if (lmin != INT_MAX) g = std::max(g, L - lmin);
-      }
-      if ((int64_t)(g + 1) * (hi - lo) > kTightenRing * (int64_t)(maxlev + 1)) g = tighten_levels(A, lo, hi, g, lev, lb, lsrc, late);
-      nlev[b] = maxlev + 1;
-      gap[b] = g;
+// forward and the backward sweep.  The dependency window W is the largest level gap of any
+// coupling + 1.
+//
+// One CTA per block walks the block's rows kPlanRows at a time.  Levels of earlier rows are
+// final; among the rows at hand, every row takes the largest level of what it waits for plus
+// one until nothing changes.  The equations are acyclic and the levels only grow, so the
+// reads of rows that change at the same time do no harm.  A chunk takes as many rounds as the
+// longest chain in it, about the line length for a stencil.  The same work on the host
+// cores, with the structure's copy back and the maps' copy out, was 3 to 11 ms of a solve's
+// set-up (128^3 to 160^3, 16 cores).
+//
+// When the early levels' gap makes the ring too long, they are moved as late as the rows'
+// dependents allow, rows without dependents left where they are (every row with dependents to
+// one below its lowest dependent).  The number of levels and the validity of the order are
+// unchanged (the longest chain has no slack); what changes is the largest gap.  A block that
+// starts in the middle of a grid plane has rows that could start at once but are only needed
+// a hundred levels later; with the levels taken as early as possible the ring of a
+// 12,000-row block of a 61 x 53 x 47 stencil would hold 58 levels, tightened it holds 2, as for
+// a block of whole planes, and the grouped sweep takes it instead of the general one, which
+// gathers coupled values from global memory: 147 -> 33 us per application there (16 blocks),
+// 248 -> 53 us on 97 x 89 x 83 in 48 blocks.  The late levels are kept when they shorten the gap.
+constexpr int kPlanRows = 1024;
+constexpr int kPlanReg = 8;   // entries of a row kept in registers
+
+struct PlanStat {
+  int kmax, gap, missing;   // missing: a block without a diagonal entry, or INT_MAX
+  int long_ring;            // a block's early levels make its ring too long
+};
+
+// The in-block entries of a row, from registers when it has at most kPlanReg entries.
+struct PlanRow {
+  int col[kPlanReg];
+  int a, z;
+  template <class F>
+  __device__ __forceinline__ void each(const int* ci, int cbase, F&& f) const {
+    if (z - a <= kPlanReg) {
+#pragma unroll
+      for (int e = 0; e < kPlanReg; ++e)
+        if (col[e] >= 0) f(col[e]);
+    } else {
+      for (int j = a; j < z; ++j) f(ci[j] - cbase);
     }
   }
-  for (int b = 0; b < nb; ++b)
-    if (missing_diag[b]) {
-      set_last_error(PARCEL_B_E_ZERO_PIVOT,
-                     "block-Jacobi block %d has a row without an in-block diagonal entry", b);
-      throw Error{PARCEL_B_E_ZERO_PIVOT, "missing diagonal"};
+};
+
+// lev: levels out.  low (zeroed), first (all INT_MAX) and late: scratch, one int per row; dep
+// (zeroed): one byte.  wid (zeroed): level widths, block b's from its first row on.
+__global__ void __launch_bounds__(kPlanRows) k_plan_levels(const int* __restrict__ starts, const int* __restrict__ rp,
+                                                           const int* __restrict__ ci, int rbase, int cbase, int* lev,
+                                                           int* low, int* first, int* late, unsigned char* dep,
+                                                           int* wid, int* __restrict__ nlev, PlanStat* stat, bool tighten) {
+  __shared__ volatile int cur[kPlanRows];   // level of the chunk's rows
+  __shared__ int push[kPlanRows];           // forced on them by rows whose entries point at them
+  __shared__ int s_max, s_gap, s_kmax;
+  const int b = blockIdx.x, t = threadIdx.x;
+  const int lo = starts[b], hi = starts[b + 1];
+  if (t == 0) s_max = s_gap = s_kmax = 0;
+  __syncthreads();
+  auto row_at = [&](int i, PlanRow& R) {
+    R.a = R.z = 0;
+    if (i < hi) {
+      R.a = rp[i] - rbase;
+      R.z = rp[i + 1] - rbase;
     }
-  // level widths and coupling counts
+#pragma unroll
+    for (int e = 0; e < kPlanReg; ++e) {
+      const int c = e < R.z - R.a ? ci[R.a + e] - cbase : -1;
+      R.col[e] = c;
+    }
+  };
+  int kmax = 0, maxlev = 0;
+  bool missing = false;
+  // ---- early levels, chunk by chunk
+  for (int base = lo; base < hi; base += kPlanRows) {
+    const int i = base + t;
+    const bool on = i < hi;
+    PlanRow R;
+    row_at(i, R);
+    int L0 = on ? __ldcg(low + i) : 0;
+    int nl = 0, nu = 0;
+    bool diag = false;
+    R.each(ci, cbase, [&](int c) {
+      if (c < lo || c >= hi) return;
+      if (c < i) {
+        ++nl;
+        if (c < base) L0 = max(L0, __ldcg(lev + c) + 1);
+      } else if (c > i) {
+        ++nu;
+      } else {
+        diag = true;
+      }
+    });
+    kmax = max(kmax, max(nl, nu));
+    missing |= on && !diag;
+    cur[t] = -1;
+    push[t] = L0;
+    __syncthreads();
+    int mine = -1;
+    int changed;
+    do {
+      changed = 0;
+      if (on) {
+        int L = *(volatile int*)&push[t];
+        R.each(ci, cbase, [&](int c) {
+          if (c >= base && c < i) L = max(L, cur[c - base] + 1);
+        });
+        if (L > mine) {
+          mine = L;
+          cur[t] = L;
+          changed = 1;
+          R.each(ci, cbase, [&](int c) {
+            if (c > i && c < hi && c < base + kPlanRows) atomicMax(&push[c - base], L + 1);
+          });
+        }
+      }
+    } while (__syncthreads_or(changed));
+    if (on) {
+      lev[i] = mine;
+      maxlev = max(maxlev, mine);
+      R.each(ci, cbase, [&](int c) {
+        if (c >= base + kPlanRows && c < hi) atomicMax(low + c, mine + 1);
+      });
+    }
+    __syncthreads();
+  }
+  atomicMax(&s_max, maxlev);
+  atomicMax(&s_kmax, kmax);
+  if (missing) atomicMin(&stat->missing, b);
+  __syncthreads();
+  maxlev = s_max;
+  // largest gap of a coupling; which rows have dependents
+  auto gap_of = [&](const int* lv) {
+    int g = 0;
+    for (int base = lo; base < hi; base += kPlanRows) {
+      const int i = base + t;
+      if (i >= hi) continue;
+      PlanRow R;
+      row_at(i, R);
+      const int L = __ldcg(lv + i);
+      R.each(ci, cbase, [&](int c) {
+        if (c < lo || c >= hi || c == i) return;
+        g = max(g, abs(__ldcg(lv + c) - L));
+        dep[min(c, i)] = 1;
+      });
+    }
+    __syncthreads();
+    if (t == 0) s_gap = 0;
+    __syncthreads();
+    atomicMax(&s_gap, g);
+    __syncthreads();
+    return s_gap;
+  };
+  int gap = gap_of(lev);
+  const int* use = lev;
+  const bool long_ring = (int64_t)(gap + 1) * (hi - lo) > kTightenRing * (int64_t)(maxlev + 1);
+  if (long_ring && t == 0) stat->long_ring = 1;
+  if (long_ring && tighten) {
+    // ---- late levels, from the last chunk back; they fall from the largest level
+    const int nch = (hi - lo + kPlanRows - 1) / kPlanRows;
+    for (int k = nch - 1; k >= 0; --k) {
+      const int base = lo + k * kPlanRows, i = base + t;
+      const bool on = i < hi;
+      PlanRow R;
+      row_at(i, R);
+      const bool has = on && *(volatile unsigned char*)(dep + i) != 0;
+      const int own = on ? __ldcg(lev + i) : 0;
+      int F = on ? __ldcg(first + i) : INT_MAX;
+      R.each(ci, cbase, [&](int c) {
+        if (c >= base + kPlanRows && c < hi) F = min(F, __ldcg(late + c));
+      });
+      cur[t] = has ? maxlev : own;
+      push[t] = F;
+      __syncthreads();
+      int mine = INT_MAX;
+      int changed;
+      do {
+        changed = 0;
+        if (on) {
+          int m = *(volatile int*)&push[t];
+          R.each(ci, cbase, [&](int c) {
+            if (c > i && c < hi && c < base + kPlanRows) m = min(m, cur[c - base]);
+          });
+          const int L = has ? m - 1 : own;
+          if (L < mine) {
+            mine = L;
+            cur[t] = L;
+            changed = 1;
+            R.each(ci, cbase, [&](int c) {
+              if (c >= base && c < i) atomicMin(&push[c - base], L);
+            });
+          }
+        }
+      } while (__syncthreads_or(changed));
+      if (on) {
+        late[i] = mine;
+        R.each(ci, cbase, [&](int c) {
+          if (c >= lo && c < base) atomicMin(first + c, mine);
+        });
+      }
+      __syncthreads();
+    }
+    const int g2 = gap_of(late);
+    if (g2 < gap) {
+      gap = g2;
+      use = late;
+    }
+  }
+  // level widths
+  for (int i = lo + t; i < hi; i += kPlanRows) {
+    const int L = __ldcg(use + i);
+    if (use != lev) lev[i] = L;
+    atomicAdd(wid + lo + L, 1);
+  }
+  if (t == 0) {
+    nlev[b] = maxlev + 1;
+    atomicMax(&stat->gap, gap);
+    atomicMax(&stat->kmax, s_kmax);
+  }
+}
+
+// Block b's level widths from wid (from its first row on) to width[blvl[b]..].
+__global__ void k_plan_widths(const int* __restrict__ starts, const int* __restrict__ blvl,
+                              const int* __restrict__ wid, int* __restrict__ width) {
+  const int b = blockIdx.x, l0 = blvl[b], n = blvl[b + 1] - l0;
+  for (int l = threadIdx.x; l < n; l += blockDim.x) width[l0 + l] = wid[starts[b] + l];
+}
+
+// Positions: the rows of a level in natural order.  One warp per block takes 32 rows at a time;
+// rows of one level among them are ranked by lane, and next[level] is where the level goes on.
+__global__ void __launch_bounds__(32) k_plan_pos(const int* __restrict__ starts, const int* __restrict__ blvl,
+                                                 const int* __restrict__ lev, int* next, int* __restrict__ pos,
+                                                 int* __restrict__ rowAt) {
+  const int b = blockIdx.x, lane = threadIdx.x;
+  const int lo = starts[b], hi = starts[b + 1];
+  int* nx = next + blvl[b];
+  int L = lo + lane < hi ? lev[lo + lane] : -1;
+  for (int base = lo; base < hi; base += 32) {
+    const int i = base + lane;
+    const int Ln = i + 32 < hi ? lev[i + 32] : -1;   // on its way while this step runs
+    const unsigned same = __match_any_sync(kFull, L);
+    const int lead = __ffs(same) - 1, rank = __popc(same & ((1u << lane) - 1u));
+    int at = 0;
+    if (lane == lead && L >= 0) {   // one lane per level, this warp alone on the block's counters
+      at = *(volatile int*)(nx + L);
+      *(volatile int*)(nx + L) = at + __popc(same);
+    }
+    at = __shfl_sync(kFull, at, lead) + rank;
+    if (L >= 0) {
+      pos[i] = at;
+      rowAt[at] = i;
+    }
+    __syncwarp();
+    L = Ln;
+  }
+}
+
+bool ilu_build_plan(const DevMat<double>& A, const BlockSplit& blocks, bool tighten, IluPlan& P, DBuf& pos,
+                    DBuf& rowAt, DBuf& lev) {
+  cudaStream_t st = stream();
+  const int n = A.n, nb = blocks.nb;
+  P.n = n;
+  P.nb = nb;
+  P.blk_lo.resize(nb);
+  P.blk_hi.resize(nb);
+  std::vector<int> starts(nb + 1, n);
+  for (int b = 0; b < nb; ++b) {
+    blocks.rows(b, n, &P.blk_lo[b], &P.blk_hi[b]);
+    starts[b] = P.blk_lo[b];
+  }
+  const size_t ib = sizeof(int) * (size_t)n;
+  DBuf dstarts(sizeof(int) * (nb + 1)), low(ib), dep(n), wid(ib), dnlev(sizeof(int) * nb), dstat(sizeof(PlanStat)),
+      first, late;
+  first.alloc(ib, false);
+  late.alloc(ib, false);
+  lev.alloc(ib, false);
+  PB_CUDA(cudaMemsetAsync(first.p, 0x7f, ib, st));   // 0x7f7f7f7f: above every level
+  PlanStat h{0, 0, INT_MAX, 0};
+  h2d(dstarts.p, starts.data(), sizeof(int) * (nb + 1));
+  h2d(dstat.p, &h, sizeof(h));
+  k_plan_levels<<<nb, kPlanRows, 0, st>>>(dp<int>(dstarts), A.rowptr, A.col, A.rbase, A.cbase, dp<int>(lev),
+                                          dp<int>(low), dp<int>(first), dp<int>(late), dp<unsigned char>(dep),
+                                          dp<int>(wid), dp<int>(dnlev), dp<PlanStat>(dstat), tighten);
+  PB_CUDA(cudaGetLastError());
+  std::vector<int> nlev(nb);
+  PB_CUDA(cudaMemcpyAsync(nlev.data(), dnlev.p, sizeof(int) * nb, cudaMemcpyDeviceToHost, st));
+  d2h(&h, dstat.p, sizeof(h));
+  PB_CHECK(h.missing == INT_MAX, PARCEL_B_E_ZERO_PIVOT,
+           "block-Jacobi block %d has a row without an in-block diagonal entry", h.missing);
   P.blk_lvl.assign(nb + 1, 0);
   for (int b = 0; b < nb; ++b) P.blk_lvl[b + 1] = P.blk_lvl[b] + nlev[b];
   const int totlev = P.blk_lvl[nb];
-  std::unique_ptr<int[]> width(new int[std::max(totlev, 1)]), kl(new int[std::max(totlev, 1)]),
-      ku(new int[std::max(totlev, 1)]);   // zeroed block by block below
-  // per block: its span in the permuted layout (every level starts on a multiple of 4, so a
-  // block that starts on one spans the sum of its rounded-up widths) and its chunks (a level
-  // split at kIluChunk rows)
-  std::vector<int64_t> span(nb + 1, 0);
-  std::vector<int> nchunk(nb + 1, 0);
-#pragma omp parallel for schedule(dynamic, grain) num_threads(nthr)
-  for (int b = 0; b < nb; ++b) {   // blocks own disjoint level ranges
-    const int l0 = P.blk_lvl[b];
-    for (int l = 0; l < nlev[b]; ++l) width[l0 + l] = kl[l0 + l] = ku[l0 + l] = 0;
-    for (int i = P.blk_lo[b]; i < P.blk_hi[b]; ++i) {
-      const int gl = l0 + lev[i];
-      width[gl]++;
-      kl[gl] = std::max(kl[gl], cL[i]);
-      ku[gl] = std::max(ku[gl], cU[i]);
-    }
-    int64_t sp = 0;
-    int nc = 0;
-    for (int l = 0; l < nlev[b]; ++l) {
-      sp += align4(width[l0 + l]);
-      nc += (width[l0 + l] + kIluChunk - 1) / kIluChunk;
-    }
-    span[b + 1] = sp;
-    nchunk[b + 1] = nc;
+  DBuf dblvl(sizeof(int) * (nb + 1)), dwidth(sizeof(int) * std::max(totlev, 1));
+  h2d(dblvl.p, P.blk_lvl.data(), sizeof(int) * (nb + 1));
+  k_plan_widths<<<nb, 256, 0, st>>>(dp<int>(dstarts), dp<int>(dblvl), dp<int>(wid), dp<int>(dwidth));
+  PB_CUDA(cudaGetLastError());
+  std::vector<int> width(totlev);
+  d2h(width.data(), dwidth.p, sizeof(int) * totlev);
+  // level starts (multiples of 4) and chunks (a level split at kIluChunk rows), in block order
+  int64_t total = 0;
+  size_t nchunk = 0;
+  for (int w : width) {
+    total += align4(w);
+    nchunk += (w + kIluChunk - 1) / kIluChunk;
   }
+  PB_CHECK(total <= INT_MAX - 3, PARCEL_B_E_ARG, "the permuted layout of %d rows exceeds 2^31 entries", n);
+  P.lvl_start.resize(totlev);
+  P.lvl_end.resize(totlev);
+  P.blk_chunk.assign(nb + 1, 0);
+  P.chunks.resize(nchunk);
+  int cursor = 0, c = 0, maxw = 0, maxl = 0;
   for (int b = 0; b < nb; ++b) {
-    span[b + 1] += span[b];
-    nchunk[b + 1] += nchunk[b];
-  }
-  PB_CHECK(span[nb] <= INT_MAX - 3, PARCEL_B_E_ARG, "the permuted layout of %d rows exceeds 2^31 entries", n);
-  P.lvl_start.assign(totlev, 0);
-  P.lvl_end.assign(totlev, 0);
-  P.blk_chunk.assign(nchunk.begin(), nchunk.end());
-  P.chunks.resize(nchunk[nb]);
-  int maxw = 0;
-  // level starts, positions (stable by natural index within a level) and chunks, in block
-  // order
-#pragma omp parallel for schedule(dynamic, grain) num_threads(nthr) reduction(max : maxw)
-  for (int b = 0; b < nb; ++b) {
-    const int l0 = P.blk_lvl[b];
-    int cursor = (int)span[b];
-    int c = P.blk_chunk[b];
+    P.blk_chunk[b] = c;
+    maxl = std::max(maxl, nlev[b]);
     for (int l = 0; l < nlev[b]; ++l) {
-      const int gl = l0 + l, w = width[gl];
+      const int gl = P.blk_lvl[b] + l, w = width[gl];
       P.lvl_start[gl] = cursor;
       P.lvl_end[gl] = cursor + w;
       maxw = std::max(maxw, w);
@@ -262,8 +385,7 @@ void ilu_build_plan(const HostCSR& A, const BlockSplit& blocks, IluPlan& P, int*
         C.start = cursor + o;
         C.w = std::min(kIluChunk, w - o);
         C.wpad = align4(C.w);
-        C.KL = kl[gl];
-        C.KU = ku[gl];
+        C.KL = C.KU = h.kmax;
         C.lvl = l;
         C.off_in_level = o;
         C.blk = b;
@@ -272,19 +394,23 @@ void ilu_build_plan(const HostCSR& A, const BlockSplit& blocks, IluPlan& P, int*
       }
       cursor = align4(cursor + w);
     }
-    for (int l = 0; l < nlev[b]; ++l) width[l0 + l] = 0;   // reused as the fill counters
-    for (int i = P.blk_lo[b]; i < P.blk_hi[b]; ++i) {
-      const int gl = l0 + lev[i];
-      pos_out[i] = P.lvl_start[gl] + width[gl]++;
-    }
   }
-  // the last level of the last block is not padded at its end
-  P.np = nb > 0 ? align4(P.lvl_end[totlev - 1]) : 0;
+  P.blk_chunk[nb] = c;
+  P.np = (int)total;   // the last level is padded as well
   P.maxWp = align4(maxw);
-  P.max_levels = nb > 0 ? *std::max_element(nlev.begin(), nlev.end()) : 0;
-  P.W = (nb > 0 ? *std::max_element(gap.begin(), gap.end()) : 0) + 1;
+  P.max_levels = maxl;
+  P.W = h.gap + 1;
+  pos.alloc(ib, false);
+  rowAt.alloc(sizeof(int) * (size_t)P.np, false);
+  PB_CUDA(cudaMemsetAsync(rowAt.p, 0xFF, sizeof(int) * (size_t)P.np, st));   // padding: -1
+  DBuf next(sizeof(int) * std::max(totlev, 1));
+  h2d(next.p, P.lvl_start.data(), sizeof(int) * totlev);
+  k_plan_pos<<<nb, 32, 0, st>>>(dp<int>(dstarts), dp<int>(dblvl), dp<int>(lev), dp<int>(next), dp<int>(pos),
+                                dp<int>(rowAt));
+  PB_CUDA(cudaGetLastError());
+  sync();   // the temporaries above are released on return
+  return h.long_ring != 0;
 }
-
 
 // ------------------------------------------------------------------ factorisation
 // In-block column range of natural row i (columns sorted): [first, last) positions.
@@ -1759,10 +1885,9 @@ int ilu_setup_device(const IluPlan& P, const DevMat<double>& A, int ilu_method,
 }
 
 // ------------------------------------------------------------------ many small blocks, set-up
-// The wavefront plan of tens of thousands of small blocks on the device, one thread per
-// block walking its rows as ilu_build_plan does: the sparsity structure does not come back to
-// the host and no per-chunk tables go out (64,000 boxes of 4^3: 28 ms on the host with its
-// copies).  A block's rows are few, so its thread's dependent loads (row pointer, column,
+// The wavefront plan of tens of thousands of small blocks, one thread per block walking its
+// rows in order; no per-chunk tables go out (64,000 boxes of 4^3: 28 ms with the plan and the
+// tables made on the host, 0.8 ms so).  A block's rows are few, so its thread's dependent loads (row pointer, column,
 // level: about 1.5 us a row) end after 0.1 to 1.5 ms whatever the number of blocks.
 struct SmallStat {
   int maxw, max_levels, kmax, span, missing;   // missing: a block without a diagonal entry, or INT_MAX
@@ -2135,8 +2260,65 @@ template bool ilu_apply_cg<double>(const IluDev<double>&, double*, const double*
 template bool ilu_apply_cg<float>(const IluDev<float>&, float*, const float*, const double*, float*, const Red&,
                                   const int*, cudaStream_t);
 
+// Iteration layout <-> sweep order (D.perm), where the two differ.
+template <class T>
+__global__ void k_to_sweep(int np, const int* __restrict__ perm, const T* __restrict__ r, T* __restrict__ q,
+                           const int* gate) {
+  if (gated(gate)) return;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
+    const int p = perm[i];
+    q[i] = p >= 0 ? r[p] : T(0);
+  }
+}
+template <class T>
+__global__ void k_from_sweep(int np, const int* __restrict__ perm, const T* __restrict__ q, T* __restrict__ s,
+                             const int* gate) {
+  if (gated(gate)) return;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
+    const int p = perm[i];
+    if (p >= 0) s[p] = q[i];
+  }
+}
+
+__global__ void k_sweep_perm(int np, const int* __restrict__ rowAt, const int* __restrict__ pos,
+                             int* __restrict__ perm) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
+    const int k = rowAt[i];
+    perm[i] = k >= 0 ? pos[k] : -1;
+  }
+}
+
+template <class T>
+void ilu_reorder(IluDev<T>& D, const int* sweep_rowAt, const int* layout_pos) {
+  D.perm.alloc(sizeof(int) * (size_t)D.np, false);
+  D.rq.alloc(sizeof(T) * (size_t)(D.np + 4));
+  D.sq.alloc(sizeof(T) * (size_t)(D.np + 4));
+  const int grid = std::max(1, std::min((D.np + 255) / 256, 8 * num_sms()));
+  k_sweep_perm<<<grid, 256, 0, stream()>>>(D.np, sweep_rowAt, layout_pos, dp<int>(D.perm));
+  PB_CUDA(cudaGetLastError());
+}
+template void ilu_reorder<double>(IluDev<double>&, const int*, const int*);
+template void ilu_reorder<float>(IluDev<float>&, const int*, const int*);
+
+template <class T>
+static void ilu_sweep(const IluDev<T>& D, const T* r, T* s, T* accum, const int* gate, cudaStream_t st);
+
 template <class T>
 void ilu_apply(const IluDev<T>& D, const T* r, T* s, T* accum, const int* gate, cudaStream_t st) {
+  if (!D.perm.p) {
+    ilu_sweep<T>(D, r, s, accum, gate, st);
+    return;
+  }
+  PB_CHECK(!accum, PARCEL_B_E_UNSUPPORTED, "accumulating block-Jacobi apply on a reordered sweep");
+  const int grid = std::max(1, std::min((D.np + 255) / 256, 8 * num_sms()));
+  k_to_sweep<T><<<grid, 256, 0, st>>>(D.np, dp<int>(D.perm), r, dp<T>(D.rq), gate);
+  ilu_sweep<T>(D, dp<T>(D.rq), dp<T>(D.sq), nullptr, gate, st);
+  k_from_sweep<T><<<grid, 256, 0, st>>>(D.np, dp<int>(D.perm), dp<T>(D.sq), s, gate);
+  PB_CUDA(cudaGetLastError());
+}
+
+template <class T>
+static void ilu_sweep(const IluDev<T>& D, const T* r, T* s, T* accum, const int* gate, cudaStream_t st) {
   if (D.small && !accum) {
 #define SMALL(K_)                                                                                  \
   case K_:                                                                                         \

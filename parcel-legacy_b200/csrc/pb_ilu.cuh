@@ -1,7 +1,6 @@
 // pb_ilu.cuh -- block-Jacobi ILU(0) / D-ILU preconditioner on the level-major layout.
 #pragma once
 
-#include <functional>
 #include <vector>
 
 #include "pb_common.cuh"
@@ -74,16 +73,14 @@ struct IluChunk {
 constexpr int kIluChunk = 512;      // rows per chunk (multiple of 4)
 constexpr int kIluHeader = 32;      // bytes of the per-chunk header in the packed data
 
-// Host-side plan: wavefront levels of every block and the permuted, padded layout.
+// Wavefront levels of every block and the permuted, padded layout: what the host keeps of it.
 struct IluPlan {
   int n = 0;            // natural rows
   int np = 0;           // permuted length incl. padding
   int nb = 0;           // blocks
   int W = 1;            // ring depth in levels
-  int maxWp = 0;        // widest chunk (padded)
+  int maxWp = 0;        // widest level (padded)
   int max_levels = 0;
-  int* pos = nullptr;           // natural row -> permuted position (caller's storage, n)
-  int* lev = nullptr;           // natural row -> level within its block (caller's storage, n)
   std::vector<IluChunk> chunks;
   std::vector<int> blk_chunk;   // nb + 1
   std::vector<int> blk_lo, blk_hi;   // natural row ranges [lo, hi)
@@ -114,6 +111,9 @@ struct IluDev {
   int64_t packF_bytes = 0, packB_bytes = 0;
   DBuf ytmp;        // forward result, np + 1 entries
   DBuf err;         // int error flag
+  // set by ilu_reorder when the sweep order is not the iteration layout: sweep position ->
+  // layout position (-1: padding), and the sweep's input and output
+  DBuf perm, rq, sq;
   // Many small blocks (k_ilu_small): one warp per block, per-row records in the iteration
   // layout: K coupled entries (permuted column or -1, value) and a diagonal factor for each
   // sweep, forward (F) and backward (B).
@@ -126,15 +126,6 @@ struct IluDev {
   // memory of one block (0: the stretches are too long, the unstaged sweep runs)
   DBuf s_box;
   int s_span = 0, s_levcap = 0, s_box_bytes = 0;
-};
-
-// Sparsity structure of the natural matrix on the host (for the wavefront plan).
-struct HostCSR {
-  int n = 0;
-  int64_t nnz = 0;
-  int istart = 1;
-  const int* rowptr = nullptr;   // 1-based
-  const int* col = nullptr;      // 1-based global
 };
 
 // Natural rows [lo, hi) of block-Jacobi block b of nb (0-based).
@@ -157,14 +148,12 @@ struct BlockSplit {
 // gives the same result; small blocks with narrow levels then fit many more CTAs per SM).
 inline int ilu_factor_threads(int maxWp) { return std::min(256, std::max(32, (maxWp + 31) & ~31)); }
 
-// rowAt[pos[i]] = i for i < n (entries not hit keep their value).
-void scatter_positions(int n, const int* pos, int* rowAt, cudaStream_t st);
-
-// Wavefront plan of the block-Jacobi blocks.  pos_out and lev_out (n entries each) receive
-// the permutation and the levels.  block_ready(b), when given, is called before block b's
-// rows are read (the structure may still be arriving from the device).
-void ilu_build_plan(const HostCSR& A, const BlockSplit& blocks, IluPlan& P, int* pos_out, int* lev_out,
-                    const std::function<void(int)>& block_ready = {});
+// Wavefront plan of the block-Jacobi blocks of the natural matrix A (device arrays).  pos and
+// lev (n entries) receive every row's permuted position and its level within its block, rowAt
+// (np entries) the row at every position, -1 for padding.  Returns whether the early levels of
+// a block make its sweep's ring too long; with tighten they are then moved later.
+bool ilu_build_plan(const DevMat<double>& A, const BlockSplit& blocks, bool tighten, IluPlan& P, DBuf& pos,
+                    DBuf& rowAt, DBuf& lev);
 
 // Factorises (ILU(0)) or computes the D-ILU diagonal on the device and packs the sweep
 // data.  ilu_method: 0 ILU(0), 1 ILUD, 2 MLUD (define.f90:40-42).  Returns a status.
@@ -205,6 +194,10 @@ struct Red;
 template <class T>
 bool ilu_apply_cg(const IluDev<T>& D, T* r, const T* q, const double* c, T* s, const Red& red, const int* gate,
                   cudaStream_t st);
+
+// Makes ilu_apply take and give vectors in another layout than the sweep's own order.
+template <class T>
+void ilu_reorder(IluDev<T>& D, const int* sweep_rowAt, const int* layout_pos);
 
 // s = M^-1 r on permuted vectors (np entries each).  If `accum` is non-null the result
 // is added into it instead of being written to s (s may then be null).

@@ -19,7 +19,6 @@
 #include "pb_cg_small.cuh"
 #include "pb_mgs.cuh"
 
-#include <atomic>
 #include <functional>
 #include "pb_solvers.cuh"
 
@@ -123,7 +122,7 @@ void Precon<T>::apply(int64_t np, const T* r, T* s, const int* gate, cudaStream_
       break;
     case PARCEL_B_PRECON_BLOCKJACOBI:
       // the sweeps may read r over the whole padded iteration layout
-      PB_CHECK(np >= ilu.np, PARCEL_B_E_ARG, "vector of %lld entries, the iteration layout has %d", (long long)np,
+      PB_CHECK(ilu.perm.p || np >= ilu.np, PARCEL_B_E_ARG, "vector of %lld entries, the iteration layout has %d", (long long)np,
                ilu.np);
       ilu_apply<T>(ilu, r, s, nullptr, gate, st);
       break;
@@ -161,15 +160,10 @@ void build_system(const Options& o, const parcel_b_crs& A, bool dev, System<T>& 
   S.M.kind = o.precon;
 
   if (o.precon == PARCEL_B_PRECON_BLOCKJACOBI) {
-    // The wavefront analysis runs on the host unless there are many small blocks.  A device-resident structure comes back
-    // through page-locked staging: the row pointers first, then the column indices in
-    // block-aligned pieces, each with an event, so that the plan of the first blocks
-    // overlaps the copy of the others.  The plan writes the permutation and the levels
-    // into the same staging area, from where they go back to the device.
     const BlockSplit bs = block_split(o, A.n);
     SmallPlan sp;
     if (ilu_small_blocks(bs, A.n) && ilu_small_plan(bs, S.Anat, sp)) {
-      trace_mark("setup: wavefront plan (device)");
+      trace_mark("setup: wavefront plan");
       S.np = sp.np;
       S.permuted = true;
       S.ilu_levels_max = sp.max_levels;
@@ -184,85 +178,30 @@ void build_system(const Options& o, const parcel_b_crs& A, bool dev, System<T>& 
       trace_mark("setup: ILU factor + pack");
       return;
     }
-    const int nb = bs.nb;
-    const size_t n1 = (size_t)A.n + 1, nz = (size_t)A.nnz;
-    int* pin = static_cast<int*>(pinned_staging(sizeof(int) * ((dev ? n1 + nz : 0) + 2 * (size_t)A.n)));
-    int* hpos = pin + (dev ? n1 + nz : 0);
-    int* hlev = hpos + A.n;
-    const int* hrpp = A.rowptr;
-    const int* hcip = A.col;
-    constexpr int kPieces = 4;
-    cudaEvent_t ev[kPieces] = {};
-    std::vector<int> piece_of(nb, 0);
-    std::atomic<int> copy_failed{0};
-    std::atomic<int> piece_done[kPieces];
-    for (auto& d : piece_done) d.store(0);
-    std::function<void(int)> ready;
-    auto destroy_events = [&] {
-      for (auto& e : ev)
-        if (e) { cudaEventDestroy(e); e = nullptr; }
-    };
-    if (dev) {
-      d2h(pin, A.rowptr, sizeof(int) * n1);   // synchronous: the row pointers size the pieces
-      hrpp = pin;
-      hcip = pin + n1;
-      for (int k = 0; k < kPieces; ++k) {
-        const int b0 = (int)((int64_t)nb * k / kPieces), b1 = (int)((int64_t)nb * (k + 1) / kPieces);
-        for (int b = b0; b < b1; ++b) piece_of[b] = k;
-        cudaError_t e = cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming);
-        if (e == cudaSuccess && b1 > b0) {
-          int lo0, hi0, lo1, hi1;
-          bs.rows(b0, A.n, &lo0, &hi0);
-          bs.rows(b1 - 1, A.n, &lo1, &hi1);
-          const size_t j0 = (size_t)(hrpp[lo0] - 1), j1 = (size_t)(hrpp[hi1] - 1);   // 1-based
-          if (j1 > j0) e = cudaMemcpyAsync(pin + n1 + j0, A.col + j0, sizeof(int) * (j1 - j0), cudaMemcpyDeviceToHost, st);
-        }
-        if (e == cudaSuccess) e = cudaEventRecord(ev[k], st);
-        if (e != cudaSuccess) {
-          destroy_events();
-          PB_CUDA(e);
-        }
-      }
-      // called from the plan's parallel loop: no exception may leave it.  A piece is waited
-      // for once (with tens of thousands of blocks a wait per block costs more than the plan).
-      ready = [&](int b) {
-        const int k = piece_of[b];
-        if (piece_done[k].load(std::memory_order_acquire)) return;
-        if (cudaEventSynchronize(ev[k]) != cudaSuccess) copy_failed = 1;
-        piece_done[k].store(1, std::memory_order_release);
-      };
-    }
-    HostCSR H;
-    H.n = A.n; H.nnz = A.nnz; H.istart = A.istart; H.rowptr = hrpp; H.col = hcip;
     IluPlan P;
-    trace_mark("setup: row pointers to host");
-    try {
-      ilu_build_plan(H, bs, P, hpos, hlev, ready);
-    } catch (...) {
-      destroy_events();
-      throw;
-    }
-    destroy_events();
-    PB_CHECK(!copy_failed, PARCEL_B_E_CUDA, "copy of the sparsity structure to the host failed");
-    trace_mark("setup: wavefront plan (host)");
+    // BiCGStab's recurrences amplify the order of a sum to 1e-3 of its residual history, so its
+    // vectors keep the early levels' order whatever order the sweep takes; the two copies per
+    // application are 6 of 60 us where levels are moved at all (97 x 89 x 83, 48 blocks)
+    const bool keep_order = o.solver == PARCEL_B_SOLVER_BICG;
+    const bool long_ring = ilu_build_plan(S.Anat, bs, !keep_order, P, S.pos, S.rowAt, S.lev);
+    trace_mark("setup: wavefront plan");
     S.np = P.np;
     S.permuted = true;
     S.ilu_levels_max = P.max_levels;
     S.ilu_nblocks = P.nb;
-    S.pos.alloc(sizeof(int) * A.n);
-    S.lev.alloc(sizeof(int) * A.n);
-    S.rowAt.alloc(sizeof(int) * P.np);
-    h2d(S.pos.p, hpos, sizeof(int) * A.n);
-    h2d(S.lev.p, hlev, sizeof(int) * A.n);
-    PB_CUDA(cudaMemsetAsync(S.rowAt.p, 0xFF, sizeof(int) * P.np, st));   // padding: -1
-    scatter_positions(A.n, dp<int>(S.pos), dp<int>(S.rowAt), st);
-    trace_mark("setup: layout maps to device");
     S.A = DevMat<T>{};
     S.A.nnz = A.nnz;
     build_sell<T>(S.Anat, P.np, dp<int>(S.rowAt), dp<int>(S.pos), S.Asell, S.A);
     trace_mark("setup: sliced ELLPACK");
-    ilu_setup_device<T>(P, S.Anat, o.ilu_method, dp<int>(S.pos), dp<int>(S.rowAt),
-                        dp<int>(S.lev), S.M.ilu);
+    if (keep_order && long_ring) {
+      IluPlan Q;
+      DBuf pos, rowAt, lev;
+      ilu_build_plan(S.Anat, bs, true, Q, pos, rowAt, lev);
+      ilu_setup_device<T>(Q, S.Anat, o.ilu_method, dp<int>(pos), dp<int>(rowAt), dp<int>(lev), S.M.ilu);
+      ilu_reorder<T>(S.M.ilu, dp<int>(rowAt), dp<int>(S.pos));
+    } else {
+      ilu_setup_device<T>(P, S.Anat, o.ilu_method, dp<int>(S.pos), dp<int>(S.rowAt), dp<int>(S.lev), S.M.ilu);
+    }
     trace_mark("setup: ILU factor + pack");
   } else {
     S.np = A.n;
