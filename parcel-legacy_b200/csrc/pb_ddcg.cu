@@ -927,6 +927,16 @@ __global__ void __launch_bounds__(256, 1)
   }
 }
 
+// D^-1 (a zero D replaced by 1e-100).
+__global__ void k_dd_dilu_inv(int n, const dd* __restrict__ D, double* __restrict__ dih, double* __restrict__ dil) {
+  GRID_LOOP(k, n) {
+    const dd d = D[k];
+    const dd di = dd_div(dd{1.0, 0.0}, (d.hi == 0.0 && d.lo == 0.0) ? dd{1.0e-100, 0.0} : d);
+    dih[k] = di.hi;
+    dil[k] = di.lo;
+  }
+}
+
 // Ring slot of every row: level mod W, position within the level (widest level LW).
 __global__ void k_dd_ring_slots(int n, const int* __restrict__ blk_of, const int* __restrict__ blvl,
                                 const int* __restrict__ lst, const int* __restrict__ lev, const int* __restrict__ pos,
@@ -1048,11 +1058,17 @@ void dd_setup_precon(const Options& o, const parcel_b_crs& A, const DdSystem& S,
   P.rng.alloc(sizeof(int4) * A.n);
   k_dd_ranges<<<grid_for(A.n), kDdThreads, 0, st>>>(A.n, plan.nb, dp<int>(blo), dp<int>(bhi), dp<int>(bof), S.rp,
                                                      S.ci, S.cbase, dp<int4>(P.rng));
-  DBuf Dh(sizeof(double) * A.n), Dl(sizeof(double) * A.n);
-  k_dd_dilu_diag<<<plan.nb, ilu_factor_threads(plan.maxWp), 0, st>>>(dp<IluChunk>(P.chunks), dp<int>(P.blk_chunk), dp<int>(blo),
-                                                 dp<int>(bhi), dp<int>(P.rowAt), S.rp, S.ci, S.ah, S.al, S.cbase,
-                                                 o.ilu_method == 2 ? 1 : 0, dp<double>(Dh), dp<double>(Dl),
-                                                 dp<double>(P.dih), dp<double>(P.dil));
+  DBuf Dd(o.ilu_method == 1 ? sizeof(dd) * A.n : 0);
+  if (o.ilu_method == 1 && ilu_dd_diag(plan, M, S.al, dp<int>(blo), dp<int>(bhi), dp<int>(dpos), dp<int>(P.rowAt),
+                                       dp<int>(dlev), dp<dd>(Dd))) {
+    k_dd_dilu_inv<<<grid_for(A.n), kDdThreads, 0, st>>>(A.n, dp<dd>(Dd), dp<double>(P.dih), dp<double>(P.dil));
+  } else {
+    DBuf Dh(sizeof(double) * A.n), Dl(sizeof(double) * A.n);
+    k_dd_dilu_diag<<<plan.nb, ilu_factor_threads(plan.maxWp), 0, st>>>(
+        dp<IluChunk>(P.chunks), dp<int>(P.blk_chunk), dp<int>(blo), dp<int>(bhi), dp<int>(P.rowAt), S.rp, S.ci, S.ah,
+        S.al, S.cbase, o.ilu_method == 2 ? 1 : 0, dp<double>(Dh), dp<double>(Dl), dp<double>(P.dih),
+        dp<double>(P.dil));
+  }
   PB_CUDA(cudaGetLastError());
   const int np = plan.np;
   P.np = np;

@@ -686,7 +686,7 @@ __global__ void k_ilu_pack(const IluChunk* __restrict__ ch, int nchunks,
 //                         padded to an odd number of T-sized words, so that the 32 lanes
 //                         of a warp reading consecutive records hit distinct banks.
 // The stage holds T xin[sspan] (the input slice) after the records, 16-byte aligned.
-// Positions without a row (level padding) have zero records.
+// Positions without a row (level padding) have no record contents.
 constexpr int kGrpMax = 31;
 constexpr int kGrpHdr = 16 + kGrpMax * 16;
 
@@ -774,17 +774,12 @@ __global__ void k_ilu_pack_grp(const int4* __restrict__ gi, const int64_t* __res
     for (int i = threadIdx.x; i < sspan; i += blockDim.x) {
       unsigned char* rf = f + kGrpHdr + (size_t)i * strF;
       unsigned char* rb = bk + kGrpHdr + (size_t)i * strB;
-      for (int o = 0; o < strF; o += 4) *reinterpret_cast<int*>(rf + o) = 0;
-      for (int o = 0; o < strB; o += 4) *reinterpret_cast<int*>(rb + o) = 0;
       T* valF = reinterpret_cast<T*>(rf + (dilu ? sz : 0));
       unsigned short* slF = reinterpret_cast<unsigned short*>(rf + (dilu ? sz : 0) + K * sz);
       T* valB = reinterpret_cast<T*>(rb + sz);
       unsigned short* slB = reinterpret_cast<unsigned short*>(rb + sz + K * sz);
       const int nat = rowAt[sstart + i];
-      if (nat < 0) {
-        for (int k = 0; k < K; ++k) { slF[k] = (unsigned short)zslot; slB[k] = (unsigned short)zslot; }
-        continue;
-      }
+      if (nat < 0) continue;   // level padding: never read
       int ia, iz, idg;
       inblock_range(rp, ci, rbase, cbase, nat, lo, hi, &ia, &iz, &idg);
       auto slot_of = [&](int cnat) -> int {
@@ -1751,10 +1746,279 @@ static bool grp_layout(const IluPlan& P, const std::vector<IluChunk>& ch, int ku
   return true;
 }
 
+// ------------------------------------------------------------------ diagonal recurrences
+// D-ILU (ILUD): D_k = a_kk - sum over the lower in-block entries of (a_kr a_rk) / D_r.
+// ILU(0) of a matrix without triangles (no entry of row k right of the diagonal meets row i's
+// pattern except at the diagonal, as in 5- and 7-point stencils): U_ii = a_ii - sum of
+// (a_ik / U_kk) a_ki, and L_ik = a_ik / U_kk; everything right of the diagonal stays.  Only the
+// recurrence is sequential, so one parallel pass collects its operands in level order (the
+// products a_kr a_rk, or both factors) and the recurrence reads them by position, the next
+// level's while the current one is worked on, with the diagonals of earlier levels in a
+// shared-memory ring (the sweep's).  Searching the transposed entries inside the recurrence
+// made every level several dependent loads.  Operands + recurrence, before the split and now:
+// D-ILU of 160^3 in 80 blocks 3.6 -> 0.55 + 0.25 ms, ILU(0) of 128^3 2.0 -> 0.35 + 0.21 ms,
+// double-double D-ILU of 80^3 1.3 ms -> 0.1 + 0.27 ms.
+// The operations and their order are those of the general kernels.
+enum { FAC_DILU = 0, FAC_ILU0 = 1 };
+constexpr int kFacMaxK = 4;
+constexpr int kFacThreads = 512;
+
+__device__ __forceinline__ double fac_val(const double* h, const double*, int j, double) { return h[j]; }
+__device__ __forceinline__ dd fac_val(const double* h, const double* l, int j, dd) { return dd{h[j], l ? l[j] : 0.0}; }
+__device__ __forceinline__ double fac_mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ dd fac_mul(dd a, dd b) { return dd_mul(a, b); }
+__device__ __forceinline__ double fac_sub(double a, double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ dd fac_sub(dd a, dd b) { return dd_sub(a, b); }
+__device__ __forceinline__ double fac_div(double a, double b) { return __ddiv_rn(a, b); }
+// ddDILU_DInv_crs replaces a zero D by 1e-100
+__device__ __forceinline__ dd fac_div(dd a, dd b) {
+  return dd_div(a, (b.hi == 0.0 && b.lo == 0.0) ? dd{1.0e-100, 0.0} : b);
+}
+
+// Operands of position q: x (the diagonal entry), K couplings (c, and c2 for ILU(0)) at
+// k * np + q with the ring index of the coupled row, -1 for none.  *other is set when the
+// matrix needs the general kernel (unsorted rows or no diagonal entry; triangles under ILU(0)).
+template <class S, int MODE>
+__global__ void k_fac_operands(int np, int nb, int K, const int* __restrict__ rowAt, const int* __restrict__ pos,
+                               const int* __restrict__ lev, const int* __restrict__ blo, const int* __restrict__ bhi,
+                               const int* __restrict__ blvl, const int* __restrict__ lst, const int* __restrict__ rp,
+                               const int* __restrict__ ci, int rbase, int cbase, const double* __restrict__ vh,
+                               const double* __restrict__ vl, RingMap ring, S* __restrict__ x, S* __restrict__ c,
+                               S* __restrict__ c2, int* __restrict__ slot, int* __restrict__ other) {
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < np; q += gridDim.x * blockDim.x) {
+    const int i = rowAt[q];
+    if (i < 0) continue;
+    int a = 0, z = nb - 1;   // block of row i: the last b with blo[b] <= i
+    while (a < z) {
+      const int mid = (a + z + 1) >> 1;
+      if (blo[mid] <= i) a = mid; else z = mid - 1;
+    }
+    const int lo = blo[a], hi = bhi[a], l0 = blvl[a], bstart = lst[l0];
+    const int ra = rp[i] - rbase, rz = rp[i + 1] - rbase;
+    bool bad = false, diag = false;
+    int k = 0, prev = -1;
+    for (int j = ra; j < rz; ++j) {
+      const int r = ci[j] - cbase;
+      bad |= r <= prev;
+      prev = r;
+      if (r == i) {
+        x[q] = fac_val(vh, vl, j, S{});
+        diag = true;
+      }
+      if (r < lo || r >= i) continue;
+      // the transposed entry a_ri, and (ILU(0)) whether row r's other entries meet row i's
+      int ja = -1;
+      const int sa = rp[r] - rbase, sz = rp[r + 1] - rbase;
+      for (int s = sa; s < sz; ++s) {
+        const int cc = ci[s] - cbase;
+        if (cc == i) ja = s;
+        if (MODE == FAC_ILU0 && cc > r && cc < hi && cc != i)
+          for (int m = ra; m < rz; ++m) bad |= ci[m] - cbase == cc;
+      }
+      const int64_t o = (int64_t)k * np + q;
+      if (k < K) {
+        int sl = -1;
+        if (ja >= 0) {
+          const S v = fac_val(vh, vl, j, S{}), t = fac_val(vh, vl, ja, S{});
+          if (MODE == FAC_DILU) {
+            c[o] = fac_mul(v, t);
+          } else {
+            c[o] = v;
+            c2[o] = t;
+          }
+          const int l = lev[r], pr = pos[r];
+          sl = ring.at(l, pr - lst[l0 + l], pr - bstart);
+        }
+        slot[o] = sl;
+      }
+      ++k;
+    }
+    for (; k < K; ++k) slot[(int64_t)k * np + q] = -1;
+    if (bad || !diag) *other = 1;
+  }
+}
+
+template <class S, int MODE, int K>
+struct FacOps {
+  S x, c[K], c2[MODE == FAC_ILU0 ? K : 1];
+  int sl[K], nat, ring;
+};
+
+// One CTA per block; diag: D or U_ii by natural row.
+template <class S, int MODE, int K>
+__global__ void __launch_bounds__(kFacThreads, 1) k_fac_sweep(int np, LevelTab tab, const int* __restrict__ rowAt,
+                                                            RingMap ring, const S* __restrict__ x,
+                                                            const S* __restrict__ c, const S* __restrict__ c2,
+                                                            const int* __restrict__ slot, S* __restrict__ diag) {
+  extern __shared__ __align__(16) unsigned char fac_smem[];
+  S* R = reinterpret_cast<S*>(fac_smem);
+  const int b = blockIdx.x, l0 = tab.blvl[b], l1 = tab.blvl[b + 1];
+  if (l0 == l1) return;
+  const int bstart = tab.start[l0];
+  auto load = [&](FacOps<S, MODE, K>& o, int q, int l, int off) {
+    o.nat = rowAt[q];
+    o.x = x[q];
+    o.ring = ring.at(l - l0, off, q - bstart);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int64_t at = (int64_t)k * np + q;
+      o.sl[k] = slot[at];
+      o.c[k] = c[at];
+      if (MODE == FAC_ILU0) o.c2[MODE == FAC_ILU0 ? k : 0] = c2[at];
+    }
+  };
+  auto solve = [&](const FacOps<S, MODE, K>& o) {
+    S d = o.x;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (o.sl[k] >= 0) {
+        const S t = fac_div(o.c[k], R[o.sl[k]]);
+        d = fac_sub(d, MODE == FAC_ILU0 ? fac_mul(t, o.c2[MODE == FAC_ILU0 ? k : 0]) : t);
+      }
+    R[o.ring] = d;
+    diag[o.nat] = d;
+  };
+  const int t = threadIdx.x;
+  FacOps<S, MODE, K> cur, nxt;
+  int s = tab.start[l0], e = tab.end[l0];
+  bool on = s + t < e;
+  if (on) load(cur, s + t, l0, t);
+  for (int l = l0; l < l1; ++l) {
+    int sn = 0, en = 0;
+    if (l + 1 < l1) {
+      sn = tab.start[l + 1];
+      en = tab.end[l + 1];
+    }
+    const bool onn = sn + t < en;
+    if (onn) load(nxt, sn + t, l + 1, t);
+    if (on) solve(cur);
+    for (int p = t + blockDim.x; s + p < e; p += blockDim.x) {   // levels wider than the CTA
+      FacOps<S, MODE, K> o;
+      load(o, s + p, l, p);
+      solve(o);
+    }
+    __syncthreads();
+    cur = nxt;
+    on = onn;
+    s = sn;
+    e = en;
+  }
+}
+
+// L_ik = a_ik / U_kk, U_ii, and the rest as it is (lu is a copy of the values).
+__global__ void k_ilu0_finish(int n, int nb, const int* __restrict__ blo, const int* __restrict__ rp,
+                              const int* __restrict__ ci, int rbase, int cbase, const double* __restrict__ diag,
+                              double* __restrict__ lu) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    int a = 0, z = nb - 1;
+    while (a < z) {
+      const int mid = (a + z + 1) >> 1;
+      if (blo[mid] <= i) a = mid; else z = mid - 1;
+    }
+    const int lo = blo[a];
+    for (int j = rp[i] - rbase; j < rp[i + 1] - rbase; ++j) {
+      const int c = ci[j] - cbase;
+      if (c == i) lu[j] = diag[i];
+      else if (c >= lo && c < i) lu[j] = __ddiv_rn(lu[j], diag[c]);
+    }
+  }
+}
+
+__global__ void k_dilu_inv(int n, const double* __restrict__ D, double* __restrict__ Dinv) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    Dinv[i] = __ddiv_rn(1.0, D[i]);
+}
+
+// Runs the recurrence into diag; false when the matrix or the plan needs the general kernels.
+template <class S, int MODE>
+static bool fac_run(const IluPlan& P, int kmax, const DevMat<double>& A, const double* vlo, const LevelTab& tab,
+                    const int* blo, const int* bhi, const int* d_pos, const int* d_rowAt, const int* d_lev, S* diag) {
+  if (kmax > kFacMaxK) return false;
+  int max_span = 0;
+  for (int b = 0; b < P.nb; ++b)
+    if (P.blk_lvl[b + 1] > P.blk_lvl[b])
+      max_span = std::max(max_span, align4(P.lvl_end[P.blk_lvl[b + 1] - 1]) - P.lvl_start[P.blk_lvl[b]]);
+  const int maxWp = std::max(4, P.maxWp);
+  const int64_t by_level = (int64_t)P.W * maxWp;
+  const RingMap ring = by_level <= max_span ? RingMap{P.W, maxWp} : RingMap{0, 0};
+  const int64_t smem = std::min<int64_t>(by_level, max_span) * (int64_t)sizeof(S);
+  if (smem > 200 * 1024) return false;
+  cudaStream_t st = stream();
+  const int np = P.np, K = kmax <= 3 ? 3 : kFacMaxK;
+  const size_t nk = (size_t)K * np;
+  DBuf x, c, c2, slot, other(sizeof(int));
+  x.alloc(sizeof(S) * (size_t)np, false);
+  c.alloc(sizeof(S) * nk, false);
+  if (MODE == FAC_ILU0) c2.alloc(sizeof(S) * nk, false);
+  slot.alloc(sizeof(int) * nk, false);
+  const int grid = std::max(1, std::min((np + 255) / 256, 8 * num_sms()));
+  k_fac_operands<S, MODE><<<grid, 256, 0, st>>>(np, P.nb, K, d_rowAt, d_pos, d_lev, blo, bhi, tab.blvl, tab.start,
+                                                A.rowptr, A.col, A.rbase, A.cbase, A.val, vlo, ring, dp<S>(x),
+                                                dp<S>(c), dp<S>(c2), dp<int>(slot), dp<int>(other));
+  PB_CUDA(cudaGetLastError());
+  int no = 0;
+  d2h(&no, other.p, sizeof(int));
+  if (no) return false;
+  const int threads = std::min(kFacThreads, std::max(32, (P.maxWp + 31) & ~31));
+  auto go = [&](auto kern) {
+    PB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    kern<<<P.nb, threads, (size_t)smem, st>>>(np, tab, d_rowAt, ring, dp<S>(x), dp<S>(c), dp<S>(c2), dp<int>(slot),
+                                              diag);
+    PB_CUDA(cudaGetLastError());
+  };
+  if (K == 3) go(k_fac_sweep<S, MODE, 3>); else go(k_fac_sweep<S, MODE, kFacMaxK>);
+  return true;
+}
+
+bool ilu_dd_diag(const IluPlan& P, const DevMat<double>& A, const double* al, const int* blo, const int* bhi,
+                 const int* d_pos, const int* d_rowAt, const int* d_lev, dd* diag) {
+  int kmax = 0;
+  for (const auto& c : P.chunks) kmax = std::max(kmax, std::max(c.KL, c.KU));
+  const size_t nl = std::max<size_t>(P.lvl_start.size(), 1);
+  DBuf blvl(sizeof(int) * (P.nb + 1)), lst(sizeof(int) * nl), lend(sizeof(int) * nl);
+  h2d(blvl.p, P.blk_lvl.data(), sizeof(int) * (P.nb + 1));
+  h2d(lst.p, P.lvl_start.data(), sizeof(int) * P.lvl_start.size());
+  h2d(lend.p, P.lvl_end.data(), sizeof(int) * P.lvl_end.size());
+  return fac_run<dd, FAC_DILU>(P, kmax, A, al, LevelTab{dp<int>(blvl), dp<int>(lst), dp<int>(lend)}, blo, bhi, d_pos,
+                               d_rowAt, d_lev, diag);
+}
+
 // L and U values (ILU(0): lu; D-ILU: the matrix's) and D^-1 of every block, one CTA each.
 struct Factor {
   DBuf lu, Dd, Di;
   const double *vL = nullptr, *vU = nullptr, *dinv = nullptr;
+  // The recurrence in level order where it applies (plan, kmax couplings a row), then the rest
+  // in parallel; otherwise the general kernels.
+  void run_plan(const IluPlan& P, int kmax, const DevMat<double>& A, int ilu_method, const LevelTab& tab,
+                const int* blo, const int* bhi, const int* d_pos, const int* d_rowAt, const int* d_lev,
+                cudaStream_t st) {
+    const int n = P.n, grid = std::max(1, std::min((n + 255) / 256, 8 * num_sms()));
+    if (ilu_method != 2) {
+      Dd.alloc(sizeof(double) * n);
+      const bool done = ilu_method == 0
+                            ? fac_run<double, FAC_ILU0>(P, kmax, A, nullptr, tab, blo, bhi, d_pos, d_rowAt, d_lev, dp<double>(Dd))
+                            : fac_run<double, FAC_DILU>(P, kmax, A, nullptr, tab, blo, bhi, d_pos, d_rowAt, d_lev, dp<double>(Dd));
+      if (done && ilu_method == 0) {
+        lu.alloc(sizeof(double) * std::max<int64_t>(A.nnz, 1), false);
+        d2d(lu.p, A.val, sizeof(double) * A.nnz);
+        k_ilu0_finish<<<grid, 256, 0, st>>>(n, P.nb, blo, A.rowptr, A.col, A.rbase, A.cbase, dp<double>(Dd),
+                                            dp<double>(lu));
+        PB_CUDA(cudaGetLastError());
+        vL = vU = dp<double>(lu);
+        return;
+      }
+      if (done) {
+        Di.alloc(sizeof(double) * n, false);
+        k_dilu_inv<<<grid, 256, 0, st>>>(n, dp<double>(Dd), dp<double>(Di));
+        PB_CUDA(cudaGetLastError());
+        vL = vU = A.val;
+        dinv = dp<double>(Di);
+        return;
+      }
+    }
+    run(A, n, P.nb, P.maxWp, ilu_method, tab, blo, bhi, d_rowAt, st);
+  }
+
   void run(const DevMat<double>& A, int n, int nb, int maxw, int ilu_method, const LevelTab& tab, const int* blo,
            const int* bhi, const int* d_rowAt, cudaStream_t st) {
     vL = vU = A.val;
@@ -1852,11 +2116,12 @@ int ilu_setup_device(const IluPlan& P, const DevMat<double>& A, int ilu_method,
   trace_mark("ilu: tables to device");
   // factorisation in natural CSR order
   Factor F;
-  F.run(A, P.n, P.nb, P.maxWp, ilu_method, LevelTab{dp<int>(blvl), dp<int>(lst), dp<int>(lend)}, dp<int>(blo),
-        dp<int>(bhi), d_rowAt, st);
+  F.run_plan(P, kmax, A, ilu_method, LevelTab{dp<int>(blvl), dp<int>(lst), dp<int>(lend)}, dp<int>(blo), dp<int>(bhi),
+             d_pos, d_rowAt, d_lev, st);
   trace_mark("ilu: factor");
-  D.packF.alloc(D.packF_bytes);
-  D.packB.alloc(D.packB_bytes);
+  // every byte of them that is read is packed below
+  D.packF.alloc(D.packF_bytes, false);
+  D.packB.alloc(D.packB_bytes, false);
   if (D.grp) {
     const FpSrc<T> src{F.vL, F.vU, F.dinv};
     k_ilu_pack_grp<T, FpSrc<T>><<<std::max(1, std::min(D.ngroups, 65535)), 256, 0, st>>>(
@@ -2175,8 +2440,8 @@ bool ilu_setup_dd(const IluPlan& P, const DevMat<double>& A, const double* al, c
   h2d(bhi.p, P.blk_hi.data(), sizeof(int) * P.nb);
   h2d(blvl.p, P.blk_lvl.data(), sizeof(int) * (P.nb + 1));
   h2d(lst.p, P.lvl_start.data(), sizeof(int) * P.lvl_start.size());
-  D.packF.alloc(D.packF_bytes);
-  D.packB.alloc(D.packB_bytes);
+  D.packF.alloc(D.packF_bytes, false);
+  D.packB.alloc(D.packB_bytes, false);
   const DdSrc src{A.val, precision == 2 ? al : nullptr, dih, precision == 2 ? dil : nullptr};
   k_ilu_pack_grp<dd, DdSrc><<<std::max(1, std::min(D.ngroups, 65535)), 256, 0, st>>>(
       dp<int4>(D.ginfo), dp<int64_t>(D.goff), D.ngroups, dp<IluChunk>(chunks), dp<int>(blo), dp<int>(bhi),

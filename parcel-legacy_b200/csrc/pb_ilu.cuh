@@ -185,6 +185,10 @@ void ilu_small_setup(SmallPlan& P, const DevMat<double>& A, int ilu_method, cons
 struct dd;
 bool ilu_setup_dd(const IluPlan& P, const DevMat<double>& A, const double* al, const double* dih, const double* dil,
                   int precision, const int* d_pos, const int* d_rowAt, const int* d_lev, IluDev<dd>& D);
+// The double-double D-ILU (ILUD) diagonal by natural row, recurrence in level order; false when
+// the general kernel has to compute it.
+bool ilu_dd_diag(const IluPlan& P, const DevMat<double>& A, const double* al, const int* blo, const int* bhi,
+                 const int* d_pos, const int* d_rowAt, const int* d_lev, dd* diag);
 // s = M^-1 r on level-ordered vectors of np entries.
 void ilu_apply_dd(const IluDev<dd>& D, const dd* r, dd* s, cudaStream_t st);
 

@@ -140,9 +140,9 @@ void build_system(const Options& o, const parcel_b_crs& A, bool dev, System<T>& 
   const int* ci = A.col;
   const double* va = A.val;
   if (!dev) {
-    S.up_rowptr.alloc(sizeof(int) * (A.n + 1));
-    S.up_col.alloc(sizeof(int) * std::max<int64_t>(A.nnz, 1));
-    S.up_val.alloc(sizeof(double) * std::max<int64_t>(A.nnz, 1));
+    S.up_rowptr.alloc(sizeof(int) * (A.n + 1), false);
+    S.up_col.alloc(sizeof(int) * std::max<int64_t>(A.nnz, 1), false);
+    S.up_val.alloc(sizeof(double) * std::max<int64_t>(A.nnz, 1), false);
     h2d(S.up_rowptr.p, A.rowptr, sizeof(int) * (A.n + 1));
     h2d(S.up_col.p, A.col, sizeof(int) * A.nnz);
     h2d(S.up_val.p, A.val, sizeof(double) * A.nnz);

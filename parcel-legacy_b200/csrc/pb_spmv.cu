@@ -367,8 +367,8 @@ void build_sell(const DevMat<double>& A, int np, const int* rowAt_d, const int* 
   d2h(&total, tot.p, sizeof(long long));
   PB_CHECK(total < INT32_MAX, PARCEL_B_E_UNSUPPORTED, "matrix too large for int32 SELL");
   total = std::max(total, 1LL);
-  buf.col.alloc(sizeof(int) * total);
-  buf.val.alloc(sizeof(VT) * total);
+  buf.col.alloc(sizeof(int) * total, false);   // written whole below
+  buf.val.alloc(sizeof(VT) * total, false);
   k_fill_sell<VT><<<8 * num_sms(), 256, 0, st>>>(np, rowAt_d, pos_d, A.rowptr, A.col, A.val, A.rbase,
                                                  A.cbase, dp<int>(buf.off), dp<int>(buf.w),
                                                  dp<int>(buf.col), dp<VT>(buf.val));

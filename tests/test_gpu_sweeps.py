@@ -78,6 +78,27 @@ def test_level_widths(nx, ny):
         assert _apply_both(A, ipreflag=2, ILU_method=ilu, precon_thblock=1) < 1e-11
 
 
+def _lattice(nx, ny, diagonals):
+    """nx x ny grid, five-point links plus the first `diagonals` of the two diagonal directions."""
+    i = np.arange(nx * ny).reshape(ny, nx)
+    pairs = [(i[:, :-1], i[:, 1:]), (i[:-1], i[1:]), (i[:-1, :-1], i[1:, 1:]), (i[:-1, 1:], i[1:, :-1])][:2 + diagonals]
+    r = np.concatenate([i.ravel()] + [np.concatenate([a.ravel(), b.ravel()]) for a, b in pairs])
+    c = np.concatenate([i.ravel()] + [np.concatenate([b.ravel(), a.ravel()]) for a, b in pairs])
+    v = np.random.default_rng(nx).uniform(-1, 1, r.size)
+    v[:nx * ny] = 9.0
+    o = np.lexsort((c, r))
+    rp = np.concatenate([[0], np.cumsum(np.bincount(r, minlength=nx * ny))]) + 1
+    return problems.CRS(n=nx * ny, rowptr=rp.astype(np.int32), col=(c[o] + 1).astype(np.int32), val=v[o])
+
+
+@pytest.mark.parametrize("ilu", [0, 1])
+@pytest.mark.parametrize("nx,ny,diagonals,blocks", [(40, 30, 1, 1), (40, 30, 2, 3), (700, 700, 0, 1), (700, 700, 1, 2)])
+def test_factor_recurrences(nx, ny, diagonals, blocks, ilu):
+    """Three and four couplings; levels wider than the recurrence's CTA; triangles, which send
+    ILU(0) to the general elimination but not D-ILU."""
+    assert _apply_both(_lattice(nx, ny, diagonals), ipreflag=2, ILU_method=ilu, precon_thblock=blocks) < 1e-11
+
+
 # ---- many small blocks: plan on the device, CG's step fused into the sweep --------------------
 def _dense_blocks(nb, rows, seed):
     """nb blocks of `rows` fully coupled rows each, linked to the next block by one entry."""
