@@ -12,8 +12,9 @@
 //
 // Grid sum without a counter: a CTA stores each 64-bit partial as two 64-bit words of 32
 // value bits and a 32-bit tag (the iteration number), so a word is either this iteration's or
-// visibly not, and every CTA reads all CTAs' words until the tags match: one L2 round trip
-// after the last store.  Only the second sum also publishes the vectors: p and s are gathered
+// visibly not.  Up to kCgDirect CTAs read all CTAs' words until the tags match, one L2 round
+// trip after the last store; of more, CTA 0 does and stores the total in kCgCopies lines for
+// the others, because lines that many CTAs poll hold up the stores into them.  Only the second sum also publishes the vectors: p and s are gathered
 // after it, and what the first sum orders (s may be overwritten) rests on loads whose values
 // went into it.  The two sums of an iteration use different words, so a CTA can only
 // overwrite words that every CTA has finished reading.  Waits are bounded; one that runs
@@ -29,23 +30,50 @@ constexpr int kCgThreads = 512;
 constexpr int kCgWarps = kCgThreads / 32;
 constexpr int kCgMaxElems = 4;             // rows per thread
 constexpr unsigned kCgWaitLimit = 1u << 21;
+constexpr int kCgDirect = 32;
 
-__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long* p) {
-  unsigned long long v;
-  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+// Both words of a value in one access; each word is single-copy atomic by itself, and each
+// carries its tag.
+__device__ __forceinline__ ulonglong2 ld_words(const unsigned long long* p) {
+  ulonglong2 v;
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long long v) {
-  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+__device__ __forceinline__ void st_words(unsigned long long* p, unsigned long long x, unsigned long long y) {
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(x), "l"(y) : "memory");
 }
 
 // Sums K per-thread values over the grid; every thread of every CTA gets the same bits.
-// words: 2 K per CTA, [CTA][2 K].  PUBLISH: the CTA's vector stores are visible to every CTA
-// that has the sum.  False when a wait ran out.
+// words: 2 K per CTA, then the total's copies, 2 K words in a line each.  PUBLISH: the CTA's
+// vector stores are visible to every CTA that has the sum.  False when a wait ran out.
 template <int K, bool PUBLISH>
 __device__ __forceinline__ bool grid_sum(double (&v)[K], unsigned long long* words, unsigned tag,
                                          double (*wsum)[kCgWarps], double (*csum)[8], int* sbad) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5, G = gridDim.x;
+  unsigned long long* tot = words + (size_t)((G * 2 * K + kCgLine - 1) & ~(kCgLine - 1));
+  auto put = [&](unsigned long long* w, double x) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    st_words(w, (b & 0xffffffff00000000ull) | tag, (b << 32) | tag);
+  };
+  // waits for K values in consecutive words; false when it gave up
+  auto get = [&](const unsigned long long* w, double (&x)[K]) -> bool {
+    ulonglong2 u[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) u[k] = ld_words(w + 2 * k);
+    for (unsigned it = 0;; ++it) {
+      bool pending = false;
+#pragma unroll
+      for (int k = 0; k < K; ++k) pending |= (unsigned)u[k].x != tag || (unsigned)u[k].y != tag;
+      if (!pending) break;
+      if (it >= kCgWaitLimit) return false;
+#pragma unroll
+      for (int k = 0; k < K; ++k) u[k] = ld_words(w + 2 * k);
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      x[k] = __longlong_as_double((long long)((u[k].x & 0xffffffff00000000ull) | (u[k].y >> 32)));
+    return true;
+  };
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     double x = v[k];
@@ -57,51 +85,55 @@ __device__ __forceinline__ bool grid_sum(double (&v)[K], unsigned long long* wor
   if (warp < K) {    // warp k stores this CTA's k-th sum
     double x = lane < kCgWarps ? wsum[warp][lane] : 0.0;
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(kFull, x, o);
+    for (int o = kCgWarps / 2; o > 0; o >>= 1) x += __shfl_xor_sync(kFull, x, o);
     if (lane == 0) {
-      const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-      unsigned long long* w = words + (size_t)blockIdx.x * 2 * K + 2 * warp;
       if (PUBLISH) __threadfence();   // the block barrier above put the CTA's stores before it
-      st_relaxed(w, (b & 0xffffffff00000000ull) | tag);
-      st_relaxed(w + 1, (b << 32) | tag);
+      put(words + (size_t)blockIdx.x * 2 * K + 2 * warp, x);
     }
   }
-  const int nw = (G + 31) >> 5;   // warps that read: at most 8 (G <= 256)
-  if (warp < nw) {
-    double x[K];
+  const bool direct = G <= kCgDirect;
+  if (direct || blockIdx.x == 0) {
+    const int nw = (G + 31) >> 5;   // warps that read: at most 8 (G <= 256)
+    if (warp < nw) {
+      double x[K];
 #pragma unroll
-    for (int k = 0; k < K; ++k) x[k] = 0.0;
-    bool bad = false;
-    if (t < G) {
-      const unsigned long long* w = words + (size_t)t * 2 * K;
+      for (int k = 0; k < K; ++k) x[k] = 0.0;
+      const bool bad = t < G && !get(words + (size_t)t * 2 * K, x);
+      if (PUBLISH) __threadfence();
 #pragma unroll
       for (int k = 0; k < K; ++k) {
-        unsigned long long hi = ld_relaxed(w + 2 * k), lo = ld_relaxed(w + 2 * k + 1);
-        unsigned it = 0;
-        while ((unsigned)hi != tag || (unsigned)lo != tag) {
-          if (++it > kCgWaitLimit) { bad = true; break; }
-          hi = ld_relaxed(w + 2 * k);
-          lo = ld_relaxed(w + 2 * k + 1);
-        }
-        x[k] = __longlong_as_double((long long)((hi & 0xffffffff00000000ull) | (lo >> 32)));
+        double y = x[k];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) y += __shfl_xor_sync(kFull, y, o);
+        if (lane == 0) csum[k][warp] = y;
       }
+      if (__any_sync(kFull, bad) && lane == 0) *sbad = 1;
     }
-    if (PUBLISH) __threadfence();
+    __syncthreads();
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-      double y = x[k];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) y += __shfl_xor_sync(kFull, y, o);
-      if (lane == 0) csum[k][warp] = y;
+      double y = 0.0;
+      for (int w = 0; w < nw; ++w) y += csum[k][w];
+      v[k] = y;
     }
-    if (__any_sync(kFull, bad) && lane == 0) *sbad = 1;
-  }
-  __syncthreads();
+    if (!direct && t < kCgCopies && *sbad == 0) {
+      if (PUBLISH) __threadfence();
 #pragma unroll
-  for (int k = 0; k < K; ++k) {
-    double y = 0.0;
-    for (int w = 0; w < nw; ++w) y += csum[k][w];
-    v[k] = y;
+      for (int k = 0; k < K; ++k) put(tot + t * kCgLine + 2 * k, v[k]);
+    }
+  } else {
+    if (t == 0) {
+      double x[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) x[k] = 0.0;
+      if (!get(tot + (blockIdx.x % kCgCopies) * kCgLine, x)) *sbad = 1;
+      if (PUBLISH) __threadfence();
+#pragma unroll
+      for (int k = 0; k < K; ++k) csum[k][0] = x[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] = csum[k][0];
   }
   const bool ok = *sbad == 0;
   __syncthreads();
@@ -136,7 +168,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) k_cg_small(CgSmallArgs<T> a) {
   int itr = a.st->itr, done = 0, niter = 0, iret = 0, diverged = 0, breakdown = 0;
   const T *pold = a.p;
   T* pnew = a.p2;
-  unsigned long long *w1 = a.slots, *w2 = a.slots + (size_t)gridDim.x * 2;
+  unsigned long long *w1 = a.slots, *w2 = a.slots + cg_small_slots(gridDim.x) / 2;
   bool ok = true;
   for (int k = 0; k < a.maxit && !done; ++k) {
     const unsigned tag = a.tag0 + (unsigned)k + 1u;

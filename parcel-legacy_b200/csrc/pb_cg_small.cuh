@@ -23,7 +23,11 @@ struct CgSmallArgs {
 
 // CTAs of the launch for n rows, 0 when the vector is too long for it.
 template <class T> int cg_small_grid(int64_t n);
-inline size_t cg_small_slots(int grid) { return (size_t)grid * 6; }
+constexpr int kCgCopies = 16, kCgLine = 16;   // copies of a grid sum's total, a 128-byte line each
+// Words of both sums: at most four per CTA and the total's copies, each.
+__host__ __device__ constexpr size_t cg_small_slots(int grid) {
+  return 2 * ((((size_t)grid * 4 + kCgLine - 1) & ~(size_t)(kCgLine - 1)) + kCgCopies * kCgLine);
+}
 template <class T> void cg_small(const CgSmallArgs<T>& a, cudaStream_t st);
 
 }  // namespace pb
