@@ -252,26 +252,29 @@ __device__ __forceinline__ bool reduce_block(double (&v)[K], const Red& r, doubl
 
 // Block-reduces K per-thread values, and lets the last block sum all partials in block order
 // and run the epilogue.  Every thread of the block must call it.  Deterministic for a fixed
-// grid size.  The last block's threads bring all partials into shared memory side by side:
-// summed by one warp per value straight from L2, four loads at a time, 592 partials took 3 of
-// the 5 us that a sum added to a short kernel.
-constexpr int kRedStage = 640;   // partials of the largest grid (four blocks on each of 148 SMs) and some
+// grid size.  Warp k sums value k, a lane's loads (19 for four blocks on each of 148 SMs) all
+// in flight before the first is added: four at a time straight from L2 they took 3 of the 5 us
+// that a sum added to a short kernel.  (Staged in 5 KB of shared memory they were as fast, but
+// the space came out of the L1 cache: a product on the diagonal copy went from 61 to 65 us at
+// 160^3.)
 template <int K>
 __device__ __forceinline__ void reduce_and_finish(double (&v)[K], const Red& r) {
   __shared__ double sm[K][32];
   __shared__ double S[K > 0 ? K : 1];
-  __shared__ double sp[K * kRedStage];
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
   if (!reduce_block<K>(v, r, sm)) return;
   const int G = gridDim.x;
-  const bool staged = G <= kRedStage;
-  if (staged) {
-    for (int i = threadIdx.x; i < G * K; i += blockDim.x) sp[i] = __ldcg(r.part + i);
-    __syncthreads();
-  }
+  constexpr int U = 20;
   for (int k = w; k < K; k += nw) {
     double s = 0.0;
-    for (int b = l; b < G; b += 32) s += staged ? sp[b * K + k] : __ldcg(r.part + (size_t)b * K + k);
+    for (int b0 = l; b0 < G; b0 += 32 * U) {
+      double y[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) y[u] = b0 + 32 * u < G ? __ldcg(r.part + (size_t)(b0 + 32 * u) * K + k) : 0.0;
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (b0 + 32 * u < G) s += y[u];
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
     if (l == 0) S[k] = s;
