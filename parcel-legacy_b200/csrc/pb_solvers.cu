@@ -260,7 +260,10 @@ static SolveOut run_pcg(const Options& o, const System<T>& S, const T* b, T* x, 
   Workspace& W = kw.W;
   const int64_t np = S.np;
   const size_t vb = sizeof(T) * np;
-  T *R = kw.buf<T>(vb), *P = kw.buf<T>(vb), *Q = kw.buf<T>(vb), *Sv = kw.buf<T>(vb);
+  const int small_grid = S.permuted ? 0 : cg_small_grid<T>(np);
+  const bool none = S.M.kind == PARCEL_B_PRECON_NONE;
+  T *R = kw.buf<T>(vb), *P = kw.buf<T>(vb), *Q = kw.buf<T>(vb);
+  T* Sv = none && !small_grid ? R : kw.buf<T>(vb);   // s = M^-1 r
   KState* K = W.st();
   init_state(W, 1, o.itrmax);
   const int* gdone = &K->done;
@@ -272,7 +275,7 @@ static SolveOut run_pcg(const Options& o, const System<T>& S, const T* b, T* x, 
   int launches = 0;
   // r = b - A x; s = M^-1 r; bnorm, rnorm, rho0 = <s, r>   (pcg.f90:442-478)
   spmv<T, T>(S.A, x, R, SPMV_RES, b, nullptr, st);
-  S.M.apply(np, R, Sv, nullptr, st);
+  if (Sv != R) S.M.apply(np, R, Sv, nullptr, st);
   PB_CUDA(cudaMemsetAsync(P, 0, sizeof(T) * np, st));
   DotSel sel;
   sel.a[0] = 1; sel.b[0] = 1;   // <b, b>
@@ -293,7 +296,7 @@ static SolveOut run_pcg(const Options& o, const System<T>& S, const T* b, T* x, 
     return out;
   };
   // short vectors in the natural layout: all iterations in cooperative launches
-  if (const int grid = S.permuted ? 0 : cg_small_grid<T>(np)) {
+  if (const int grid = small_grid) {
     CgSmallArgs<T> ca;
     ca.A = S.A;
     ca.dinv = S.M.kind == PARCEL_B_PRECON_POINTJACOBI ? dp<T>(S.M.dinv) : nullptr;
@@ -326,6 +329,12 @@ static SolveOut run_pcg(const Options& o, const System<T>& S, const T* b, T* x, 
       spmv_dot<T, T>(S.A, P, Q, SPMV_Y, nullptr, nullptr, 1, sa, sb, red(EPI_CG_GAMMA), gdone, st);
       if (S.M.kind == PARCEL_B_PRECON_BLOCKJACOBI &&
           ilu_apply_cg<T>(S.M.ilu, R, Q, &K->tmp[0], Sv, red(EPI_CG_DOT2), gdone, st)) {
+        per_chunk += 3;
+        continue;
+      }
+      if (none || S.M.kind == PARCEL_B_PRECON_POINTJACOBI) {
+        cg_step<T>(np, R, Q, none ? nullptr : dp<T>(S.M.dinv), none ? nullptr : Sv, &K->tmp[0], red(EPI_CG_DOT2),
+                   gdone, st);
         per_chunk += 3;
         continue;
       }

@@ -180,6 +180,21 @@ def test_short_vector_cg(nx, ny, ipreflag):
     assert np.abs(res["x"] - xo).max() < 1e-7 * np.abs(xo).max()
 
 
+@pytest.mark.parametrize("ipreflag", [0, 1])
+@pytest.mark.parametrize("nx,ny", [(551, 551), (673, 677)])
+def test_cg_step(nx, ny, ipreflag):
+    """The smallest vector past the one-launch CG, and one with elements over in the last step of
+    a thread (a step takes three elements of each of 151,552 threads)."""
+    A = problems.poisson2d_5pt(nx, ny)
+    b = problems.rhs_normal(A.n, nx)
+    kw = dict(solver=1, itrmax=40, rtolmax=1e-10, ipreflag=ipreflag)
+    xo, ho, no, io = oracle.solve(A, b, **kw)
+    res = api.solve(A, b, **kw)
+    assert res["niter"] == no and res["iret"] == io
+    assert (np.abs(res["reshistory"][:no] - ho[:no]) / ho[:no]).max() < 1e-6
+    assert np.abs(res["x"] - xo).max() < 1e-7 * np.abs(xo).max()
+
+
 def test_short_vector_cg_without_a_diagonal_copy_and_past_one_launch():
     """A matrix that has no diagonal copy (sliced ELLPACK), and more iterations than one launch
     runs (4,096), ended by the iteration limit."""
