@@ -187,6 +187,35 @@ __global__ void __launch_bounds__(kRedThreads, 4) k_cg_step(int64_t n, T* __rest
   reduce_and_finish<2>(acc, red);
 }
 
+// <s, r> and <r, r>.  Bound by HBM, with eight elements per thread and step: lincomb_dot's
+// three keep too few bytes in flight when there are only two vectors to read: 160^3 20.1 -> 16.5 us,
+// FP32 128^3 11.3 -> 8.1 us.
+// Elements and sum order are lincomb_dot's.
+template <class T>
+__global__ void __launch_bounds__(kRedThreads, 4) k_cg_dots(int64_t n, const T* __restrict__ s, const T* __restrict__ r,
+                                                         Red red, const int* gate) {
+  if (gated(gate)) return;
+  double acc[2] = {0.0, 0.0};
+  constexpr int kUD = 8;
+  const int64_t st = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += kUD * st) {
+    T sv[kUD], rv[kUD];
+#pragma unroll
+    for (int u = 0; u < kUD; ++u) {
+      const int64_t i = i0 + u * st;
+      sv[u] = i < n ? s[i] : T(0);
+      rv[u] = i < n ? r[i] : T(0);
+    }
+#pragma unroll
+    for (int u = 0; u < kUD; ++u) {
+      if (i0 + u * st >= n) continue;
+      acc[0] += (double)(sv[u] * rv[u]);
+      acc[1] += (double)(rv[u] * rv[u]);
+    }
+  }
+  reduce_and_finish<2>(acc, red);
+}
+
 // s = D^-1 r (pointJacobi, matrix.f90:4452-4468)
 template <class T>
 __global__ void k_scale(int64_t n, T* __restrict__ s, const T* __restrict__ d, const T* __restrict__ r,
@@ -398,6 +427,12 @@ void cg_step(int64_t n, T* r, const T* q, const T* dinv, T* s, const double* na,
 }
 
 template <class T>
+void cg_dots(int64_t n, const T* s, const T* r, const Red& red, const int* gate, cudaStream_t st) {
+  k_cg_dots<T><<<red_grid(n, 3 * kRedThreads), kRedThreads, 0, st>>>(n, s, r, red, gate);
+  PB_CUDA(cudaGetLastError());
+}
+
+template <class T>
 void scale(int64_t n, T* s, const T* d, const T* r, const int* gate, cudaStream_t st) {
   k_scale<T><<<eb(n), 256, 0, st>>>(n, s, d, r, gate);
   PB_CUDA(cudaGetLastError());
@@ -466,6 +501,7 @@ void gather_perm(int n, double* out, const T* inp, const int* perm, cudaStream_t
   template void cg_axpy2<T>(int64_t, T*, T*, const T*, const KState*, const int*, cudaStream_t); \
   template void cg_step<T>(int64_t, T*, const T*, const T*, T*, const double*, const Red&,      \
                            const int*, cudaStream_t);                                            \
+  template void cg_dots<T>(int64_t, const T*, const T*, const Red&, const int*, cudaStream_t);    \
   template void scale<T>(int64_t, T*, const T*, const T*, const int*, cudaStream_t);             \
   template void multidot<T>(int64_t, int, const T*, const T*, int64_t, const Red&, const int*,   \
                             cudaStream_t);                                                       \

@@ -29,6 +29,9 @@ void lincomb_dot(int64_t n, T* out, const T* x0, Coef c0, const T* x1, Coef c1, 
                  const int* gate, cudaStream_t st);
 template <class T>
 void cg_axpy2(int64_t n, T* x, T* p, const T* s, const KState* st, const int* gate, cudaStream_t s_);
+// {<s, r>, <r, r>} into red's epilogue.
+template <class T>
+void cg_dots(int64_t n, const T* s, const T* r, const Red& red, const int* gate, cudaStream_t st);
 // r += *na q; s = dinv r (dinv null: none); {<s, r>, <r, r>} into red's epilogue.
 template <class T>
 void cg_step(int64_t n, T* r, const T* q, const T* dinv, T* s, const double* na, const Red& red, const int* gate,

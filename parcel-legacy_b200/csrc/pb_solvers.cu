@@ -341,11 +341,7 @@ static SolveOut run_pcg(const Options& o, const System<T>& S, const T* b, T* x, 
       per_chunk += 5;
       lincomb<T>(np, R, Q, cdev(&K->tmp[0]), R, cimm(1.0), nullptr, cimm(0), gdone, st);  // r = -alpha q + r
       S.M.apply(np, R, Sv, gdone, st);                                    // s = M^-1 r
-      DotSel d2;
-      d2.a[0] = 1; d2.b[0] = 2;   // <s, r>
-      d2.a[1] = 2; d2.b[1] = 2;   // <r, r>
-      lincomb_dot<T>(np, nullptr, Sv, cimm(0), R, cimm(0), nullptr, cimm(0), nullptr, nullptr, d2, 2,
-                     red(EPI_CG_DOT2), gdone, st);
+      cg_dots<T>(np, Sv, R, red(EPI_CG_DOT2), gdone, st);                  // <s, r>, <r, r>
     }
   };
   GraphRunner& G = kw.G;
