@@ -132,12 +132,80 @@ __device__ __forceinline__ dd dd_grid_tree(const dd* part, int ncta, dd* sm) {
   return s;
 }
 
+enum DdStep { DD_NONE = -1, DD_INIT_NORMS = 0, DD_INIT_RHO, DD_ALPHA, DD_RNORM, DD_BETA };
+
+// Scalar updates of ddKSP_pCG, by the thread that finishes the dot products they need.
+__device__ __forceinline__ void dd_scal(DdScal* sc, int step, const dd* bdot, const dd* rdot) {
+  switch (step) {
+    case DD_INIT_NORMS:
+      sc->bnorm = dd_sqrt(*bdot);
+      sc->rnorm = dd_sqrt(*rdot);
+      sc->alpha = dd{0.0, 0.0};
+      sc->beta = dd{0.0, 0.0};
+      break;
+    case DD_INIT_RHO:
+      sc->rho0 = *bdot;
+      break;
+    case DD_ALPHA:
+      sc->gamma = *bdot;
+      sc->alpha = dd_div(sc->rho0, sc->gamma);
+      sc->t1 = dd_mul(dd{-1.0, 0.0}, sc->alpha);
+      break;
+    case DD_RNORM:
+      sc->rnorm = dd_sqrt(*rdot);
+      break;
+    case DD_BETA:
+      sc->rho1 = *bdot;
+      sc->beta = dd_div(sc->rho1, sc->rho0);
+      sc->rho0 = sc->rho1;
+      break;
+  }
+}
+
+// Scalars of ddKSP_pBiCG (ddpbicg.f90:496-875); hist = high part of dd_div(rnorm, bnorm).
+struct DdScalB {
+  dd bnorm, rnorm, c1, c2, c3, alpha, beta;
+  double hist;
+};
+
+enum DdStepB { DDB_INIT = 0, DDB_ALPHA, DDB_C3, DDB_RNORM };
+
+__device__ __forceinline__ void dd_scal(DdScalB* sc, int step, const dd* d1, const dd* d2) {
+  switch (step) {
+    case DDB_INIT:   // d1 = <b, b>, d2 = <r0, r0>
+      sc->bnorm = dd_sqrt(*d1);
+      sc->c1 = *d2;
+      sc->rnorm = dd_sqrt(sc->c1);
+      sc->hist = dd_div(sc->rnorm, sc->bnorm).hi;
+      sc->c2 = dd{0.0, 0.0};
+      sc->c3 = dd{0.0, 0.0};
+      break;
+    case DDB_ALPHA:   // d1 = <r0, q>
+      sc->c2 = *d1;
+      sc->alpha = dd_div(sc->c1, sc->c2);
+      break;
+    case DDB_C3:   // d1 = <e, v>, d2 = <v, v>
+      sc->c3 = dd_div(*d1, *d2);
+      break;
+    case DDB_RNORM:   // d1 = <r, r0>, d2 = <r, r>
+      sc->c1 = *d1;
+      sc->rnorm = dd_sqrt(*d2);
+      sc->hist = dd_div(sc->rnorm, sc->bnorm).hi;
+      // for the next iteration: c1 / (c3 c2)
+      sc->beta = dd_div(sc->c1, dd_mul(sc->c3, sc->c2));
+      break;
+  }
+}
+
 // MODE 0: out[0] = <x, y>; 1: and out2 = <y, y>; 2: and out2 = <x, x>, from the same loads.
-template <int MODE>
+// The thread that finishes them runs the solver's scalar step on them (sc null: none): a launch
+// of its own took 2 us and the gap before it, three times an iteration.
+template <int MODE, class Scal>
 __global__ void __launch_bounds__(kDdDotThreads) k_dd_dot(int64_t n, const double* __restrict__ xh,
                                                         const double* __restrict__ xl, const double* __restrict__ yh,
                                                         const double* __restrict__ yl, dd* part, unsigned* ticket,
-                                                        dd* out, dd* out2) {
+                                                        dd* out, dd* out2, Scal* sc, int step, const dd* d1,
+                                                        const dd* d2) {
   constexpr int ND = MODE ? 2 : 1;
   __shared__ dd sm[ND][32];
   __shared__ bool last;
@@ -180,78 +248,13 @@ __global__ void __launch_bounds__(kDdDotThreads) k_dd_dot(int64_t n, const doubl
     const dd v = dd_grid_tree(part + k * kDdDotCtas, gridDim.x, sm[k]);
     if (threadIdx.x == 0) (k == 0 ? *out : *out2) = v;
   }
-  if (threadIdx.x == 0) *ticket = 0u;
-}
-
-enum DdStep { DD_INIT_NORMS = 0, DD_INIT_RHO, DD_ALPHA, DD_RNORM, DD_BETA };
-
-// Scalar updates of ddKSP_pCG, one thread.
-__global__ void k_dd_scal(DdScal* sc, int step, const dd* bdot, const dd* rdot) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  switch (step) {
-    case DD_INIT_NORMS:
-      sc->bnorm = dd_sqrt(*bdot);
-      sc->rnorm = dd_sqrt(*rdot);
-      sc->alpha = dd{0.0, 0.0};
-      sc->beta = dd{0.0, 0.0};
-      break;
-    case DD_INIT_RHO:
-      sc->rho0 = *bdot;
-      break;
-    case DD_ALPHA:
-      sc->gamma = *bdot;
-      sc->alpha = dd_div(sc->rho0, sc->gamma);
-      sc->t1 = dd_mul(dd{-1.0, 0.0}, sc->alpha);
-      break;
-    case DD_RNORM:
-      sc->rho1 = *bdot;
-      sc->rnorm = dd_sqrt(*rdot);
-      break;
-    case DD_BETA:
-      sc->beta = dd_div(sc->rho1, sc->rho0);
-      sc->rho0 = sc->rho1;
-      break;
+  if (threadIdx.x == 0) {
+    *ticket = 0u;
+    if (sc) dd_scal(sc, step, d1, d2);
   }
 }
 
 // ------------------------------------------------------------------ BiCGStab (ddKSP_pBiCG)
-// Scalars of ddKSP_pBiCG (ddpbicg.f90:496-875); hist = high part of dd_div(rnorm, bnorm).
-struct DdScalB {
-  dd bnorm, rnorm, c1, c2, c3, alpha, beta;
-  double hist;
-};
-
-enum DdStepB { DDB_INIT = 0, DDB_ALPHA, DDB_C3, DDB_RNORM, DDB_BETA };
-
-__global__ void k_dd_scal_b(DdScalB* sc, int step, const dd* d1, const dd* d2) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  switch (step) {
-    case DDB_INIT:   // d1 = <b, b>, d2 = <r0, r0>
-      sc->bnorm = dd_sqrt(*d1);
-      sc->c1 = *d2;
-      sc->rnorm = dd_sqrt(sc->c1);
-      sc->hist = dd_div(sc->rnorm, sc->bnorm).hi;
-      sc->c2 = dd{0.0, 0.0};
-      sc->c3 = dd{0.0, 0.0};
-      break;
-    case DDB_ALPHA:   // d1 = <r0, q>
-      sc->c2 = *d1;
-      sc->alpha = dd_div(sc->c1, sc->c2);
-      break;
-    case DDB_C3:   // d1 = <e, v>, d2 = <v, v>
-      sc->c3 = dd_div(*d1, *d2);
-      break;
-    case DDB_RNORM:   // d1 = <r, r0>, d2 = <r, r>
-      sc->c1 = *d1;
-      sc->rnorm = dd_sqrt(*d2);
-      sc->hist = dd_div(sc->rnorm, sc->bnorm).hi;
-      break;
-    case DDB_BETA:
-      sc->beta = dd_div(sc->c1, dd_mul(sc->c3, sc->c2));
-      break;
-  }
-}
-
 // ddBiCG_axpy3 (ddpbicg.f90:8-43): e = r - alpha q
 __global__ void k_dd_bicg_axpy3(int n, const DdScalB* sc, const double* __restrict__ rh, const double* __restrict__ rl,
                                 const double* __restrict__ qh, const double* __restrict__ ql, double* __restrict__ eh,
@@ -1016,12 +1019,19 @@ struct DdSystem {
 inline int dd_dot_grid(int64_t n) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(kDdDotCtas, (n + kDdDotThreads - 1) / kDdDotThreads));
 }
-template <int MODE>
+// A scalar step after a dot: the dot products it takes are d1 and d2.
+template <class Scal>
+struct DdThen {
+  Scal* sc = nullptr;
+  int step = 0;
+  const dd *d1 = nullptr, *d2 = nullptr;
+};
+template <int MODE, class Scal>
 void dd_dots(const DdSystem& S, const double* xh, const double* xl, const double* yh, const double* yl, dd* part,
-             dd* out, dd* out2, cudaStream_t st) {
-  k_dd_dot<MODE><<<dd_dot_grid(S.n), kDdDotThreads, 0, st>>>(S.n, xh, xl, yh, yl, part,
-                                                            reinterpret_cast<unsigned*>(part + 2 * kDdDotCtas), out,
-                                                            out2);
+             dd* out, dd* out2, const DdThen<Scal>& then, cudaStream_t st) {
+  k_dd_dot<MODE, Scal><<<dd_dot_grid(S.n), kDdDotThreads, 0, st>>>(
+      S.n, xh, xl, yh, yl, part, reinterpret_cast<unsigned*>(part + 2 * kDdDotCtas), out, out2, then.sc, then.step,
+      then.d1, then.d2);
 }
 
 void dd_setup_precon(const Options& o, const parcel_b_crs& A, const DdSystem& S, int prec_M, DdPrecon& P) {
@@ -1178,16 +1188,23 @@ struct DdRun {
     k_dd_spmv<<<g, kDdThreads, 0, st>>>(n, S.rp, S.ci, S.ah, S.al, S.cbase, xh, xl, yh, yl);
   }
   void spmv(const DdVec& x, DdVec& y) const { spmv(x.hi(), x.lo(), y.hi(), y.lo()); }
-  void dot(const double* xh, const double* xl, const double* yh, const double* yl, dd* out) const {
-    dd_dots<0>(S, xh, xl, yh, yl, part, out, nullptr, st);
+  template <class Scal = DdScal>
+  void dot(const double* xh, const double* xl, const double* yh, const double* yl, dd* out,
+           const DdThen<Scal>& then = {}) const {
+    dd_dots<0>(S, xh, xl, yh, yl, part, out, nullptr, then, st);
   }
-  void dot(const DdVec& u, const DdVec& v, DBuf& out) const { dot(u.hi(), u.lo(), v.hi(), v.lo(), dp<dd>(out)); }
+  template <class Scal = DdScal>
+  void dot(const DdVec& u, const DdVec& v, DBuf& out, const DdThen<Scal>& then = {}) const {
+    dot(u.hi(), u.lo(), v.hi(), v.lo(), dp<dd>(out), then);
+  }
   // <u, v> and <v, v>, or <u, v> and <u, u>, in one pass
-  void dot_vv(const DdVec& u, const DdVec& v, DBuf& uv, DBuf& vv) const {
-    dd_dots<1>(S, u.hi(), u.lo(), v.hi(), v.lo(), part, dp<dd>(uv), dp<dd>(vv), st);
+  template <class Scal>
+  void dot_vv(const DdVec& u, const DdVec& v, DBuf& uv, DBuf& vv, const DdThen<Scal>& then) const {
+    dd_dots<1>(S, u.hi(), u.lo(), v.hi(), v.lo(), part, dp<dd>(uv), dp<dd>(vv), then, st);
   }
-  void dot_uu(const DdVec& u, const DdVec& v, DBuf& uv, DBuf& uu) const {
-    dd_dots<2>(S, u.hi(), u.lo(), v.hi(), v.lo(), part, dp<dd>(uv), dp<dd>(uu), st);
+  template <class Scal>
+  void dot_uu(const DdVec& u, const DdVec& v, DBuf& uv, DBuf& uu, const DdThen<Scal>& then) const {
+    dd_dots<2>(S, u.hi(), u.lo(), v.hi(), v.lo(), part, dp<dd>(uv), dp<dd>(uu), then, st);
   }
   // y = alpha x + beta y (ddaxpy)
   void axpy(const dd* alpha, const dd* beta, const double* xh, const double* xl, double* yh, double* yl) const {
@@ -1208,12 +1225,37 @@ struct DdLoop {
   double setup_end = 0.0;
 };
 
-double read_double(const double* dev, cudaStream_t st) {
-  double v;
-  PB_CUDA(cudaMemcpyAsync(&v, dev, sizeof(double), cudaMemcpyDeviceToHost, st));
-  PB_CUDA(cudaStreamSynchronize(st));
-  return v;
-}
+// A device scalar that the host waits for while kernels queued behind it run: the stop test
+// of an iteration needs a norm that is known before the iteration's last kernels (CG), or the
+// next iteration's first kernels change nothing the result depends on (BiCGStab, GMRES).  With
+// the read at the end the device idled 30 us in each iteration.
+struct DdReadback {
+  double* p = nullptr;
+  cudaEvent_t ev = nullptr;
+  DdReadback() {
+    PB_CUDA(cudaMallocHost(&p, 2 * sizeof(double)));
+    if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
+      cudaFreeHost(p);
+      PB_CHECK(false, PARCEL_B_E_CUDA, "no event for the dd solver's stop test");
+    }
+  }
+  ~DdReadback() {
+    cudaEventSynchronize(ev);
+    cudaEventDestroy(ev);
+    cudaFreeHost(p);
+  }
+  DdReadback(const DdReadback&) = delete;
+  DdReadback& operator=(const DdReadback&) = delete;
+  void post(const double* d0, const double* d1, cudaStream_t st) {
+    PB_CUDA(cudaMemcpyAsync(p, d0, sizeof(double), cudaMemcpyDeviceToHost, st));
+    if (d1) PB_CUDA(cudaMemcpyAsync(p + 1, d1, sizeof(double), cudaMemcpyDeviceToHost, st));
+    PB_CUDA(cudaEventRecord(ev, st));
+  }
+  double wait() {
+    PB_CUDA(cudaEventSynchronize(ev));
+    return p[0];
+  }
+};
 
 // ddKSP_pCG (ddpcg.f90:247-563).
 DdLoop dd_cg_loop(const DdRun& R, const Options& o, DdVec& x, const DdVec& b, double* reshistory) {
@@ -1224,12 +1266,12 @@ DdLoop dd_cg_loop(const DdRun& R, const Options& o, DdVec& x, const DdVec& b, do
   DBuf scal(sizeof(DdScal)), d1(sizeof(dd)), d2(sizeof(dd));
   DdScal* sc = dp<DdScal>(scal);
   R.residual(x, b, r);
+  DdReadback back;
+  auto then = [&](int step) { return DdThen<DdScal>{sc, step, dp<dd>(d1), dp<dd>(d2)}; };
   R.dot(b, b, d1);
-  R.dot(r, r, d2);
-  k_dd_scal<<<1, 32, 0, st>>>(sc, DD_INIT_NORMS, dp<dd>(d1), dp<dd>(d2));
+  R.dot(r, r, d2, then(DD_INIT_NORMS));
   R.precon(r.hi(), r.lo(), s.hi(), s.lo());
-  R.dot(s, r, d1);
-  k_dd_scal<<<1, 32, 0, st>>>(sc, DD_INIT_RHO, dp<dd>(d1), nullptr);
+  R.dot(s, r, d1, then(DD_INIT_RHO));
   PB_CUDA(cudaGetLastError());
   L.setup_end = now_s();
   DdScal h;
@@ -1242,16 +1284,15 @@ DdLoop dd_cg_loop(const DdRun& R, const Options& o, DdVec& x, const DdVec& b, do
     if (reshistory) reshistory[itr - 1] = rnorm / bnorm;
     k_dd_cg_axpy2<<<g, kDdThreads, 0, st>>>(n, sc, x.hi(), x.lo(), p.hi(), p.lo(), s.hi(), s.lo());
     R.spmv(p, q);
-    R.dot(p, q, d1);
-    k_dd_scal<<<1, 32, 0, st>>>(sc, DD_ALPHA, dp<dd>(d1), nullptr);
+    R.dot(p, q, d1, then(DD_ALPHA));
     R.axpy(&sc->t1, R.one, q.hi(), q.lo(), r.hi(), r.lo());
+    R.dot(r, r, d2, then(DD_RNORM));
+    back.post(&sc->rnorm.hi, nullptr, st);
     R.precon(r.hi(), r.lo(), s.hi(), s.lo());
-    R.dot_vv(s, r, d1, d2);
-    k_dd_scal<<<1, 32, 0, st>>>(sc, DD_RNORM, dp<dd>(d1), dp<dd>(d2));
+    R.dot(s, r, d1, then(DD_BETA));
     PB_CUDA(cudaGetLastError());
-    rnorm = read_double(&sc->rnorm.hi, st);
+    rnorm = back.wait();
     if (rnorm / bnorm < o.rtol) break;
-    k_dd_scal<<<1, 32, 0, st>>>(sc, DD_BETA, nullptr, nullptr);
   }
   // x = alpha p + 1 x
   R.axpy(&sc->alpha, R.one, p.hi(), p.lo(), x.hi(), x.lo());
@@ -1269,44 +1310,42 @@ DdLoop dd_bicg_loop(const DdRun& R, const Options& o, DdVec& x, const DdVec& b, 
   DdVec r(n), p(n), q(n), r0(n), pp(n), e(n), pe(n), v(n);
   DBuf scb(sizeof(DdScalB)), d1(sizeof(dd)), d2(sizeof(dd));
   DdScalB* sb = dp<DdScalB>(scb);
+  DdReadback back;
+  auto then = [&](int step) { return DdThen<DdScalB>{sb, step, dp<dd>(d1), dp<dd>(d2)}; };
   R.residual(x, b, r);
   k_dd_copy<<<g, kDdThreads, 0, st>>>(n, r.hi(), r.lo(), r0.hi(), r0.lo());
   k_dd_copy<<<g, kDdThreads, 0, st>>>(n, r.hi(), r.lo(), p.hi(), p.lo());
   R.dot(b, b, d1);
-  R.dot(r0, r0, d2);
-  k_dd_scal_b<<<1, 32, 0, st>>>(sb, DDB_INIT, dp<dd>(d1), dp<dd>(d2));
+  R.dot(r0, r0, d2, then(DDB_INIT));
   PB_CUDA(cudaGetLastError());
   L.setup_end = now_s();
   DdScalB h;
   PB_CUDA(cudaMemcpyAsync(&h, sb, sizeof(DdScalB), cudaMemcpyDeviceToHost, st));
   sync();
   const double bnorm = h.bnorm.hi;
-  double hist = h.hist;
+  double hist = h.hist, rnorm;
   int itr;
   for (itr = 1; itr <= o.itrmax; ++itr) {
     if (reshistory) reshistory[itr - 1] = hist;
-    R.precon(p.hi(), p.lo(), pp.hi(), pp.lo());
+    if (itr == 1) R.precon(p.hi(), p.lo(), pp.hi(), pp.lo());
     R.spmv(pp, q);
-    R.dot(r0, q, d1);
-    k_dd_scal_b<<<1, 32, 0, st>>>(sb, DDB_ALPHA, dp<dd>(d1), nullptr);
+    R.dot(r0, q, d1, then(DDB_ALPHA));
     k_dd_bicg_axpy3<<<g, kDdThreads, 0, st>>>(n, sb, r.hi(), r.lo(), q.hi(), q.lo(), e.hi(), e.lo());
     R.precon(e.hi(), e.lo(), pe.hi(), pe.lo());
     R.spmv(pe, v);
-    R.dot_vv(e, v, d1, d2);
-    k_dd_scal_b<<<1, 32, 0, st>>>(sb, DDB_C3, dp<dd>(d1), dp<dd>(d2));
+    R.dot_vv(e, v, d1, d2, then(DDB_C3));
     k_dd_bicg_axpy4<<<g, kDdThreads, 0, st>>>(n, sb, x.hi(), x.lo(), pp.hi(), pp.lo(), pe.hi(), pe.lo());
     k_dd_bicg_axpy3r<<<g, kDdThreads, 0, st>>>(n, sb, e.hi(), e.lo(), v.hi(), v.lo(), r.hi(), r.lo());
-    R.dot_uu(r, r0, d1, d2);
-    k_dd_scal_b<<<1, 32, 0, st>>>(sb, DDB_RNORM, dp<dd>(d1), dp<dd>(d2));
+    R.dot_uu(r, r0, d1, d2, then(DDB_RNORM));
+    back.post(&sb->rnorm.hi, &sb->hist, st);
+    if (itr < o.itrmax) {   // the next iteration's p and M^-1 p, while the host reads the norm
+      k_dd_bicg_axpy4p<<<g, kDdThreads, 0, st>>>(n, sb, p.hi(), p.lo(), r.hi(), r.lo(), q.hi(), q.lo());
+      R.precon(p.hi(), p.lo(), pp.hi(), pp.lo());
+    }
     PB_CUDA(cudaGetLastError());
-    double rn[2];
-    PB_CUDA(cudaMemcpyAsync(&rn[0], &sb->rnorm.hi, sizeof(double), cudaMemcpyDeviceToHost, st));
-    PB_CUDA(cudaMemcpyAsync(&rn[1], &sb->hist, sizeof(double), cudaMemcpyDeviceToHost, st));
-    sync();
-    hist = rn[1];
-    if (rn[0] / bnorm < o.rtol) break;
-    k_dd_scal_b<<<1, 32, 0, st>>>(sb, DDB_BETA, nullptr, nullptr);
-    k_dd_bicg_axpy4p<<<g, kDdThreads, 0, st>>>(n, sb, p.hi(), p.lo(), r.hi(), r.lo(), q.hi(), q.lo());
+    rnorm = back.wait();
+    hist = back.p[1];
+    if (rnorm / bnorm < o.rtol) break;
   }
   PB_CUDA(cudaGetLastError());
   L.used = std::min(o.itrmax, itr);
@@ -1376,6 +1415,7 @@ DdLoop dd_gmres_loop(const DdRun& R, const Options& o, DdVec& x, const DdVec& b,
                                (const double*)dp<double>(Vh), (const double*)dp<double>(Vl), ldv, w.hi(), w.lo(), vh(i),
                                vl(i), G, dp<dd>(mparts), dp<unsigned>(mctr), dp<int>(merr), staged));
   };
+  DdReadback back;
   double rnorm = 0.0;
   int itr = 1, inner = 1, mm = 0;
   for (itr = 1; itr <= o.itrmax; itr += m) {
@@ -1384,12 +1424,16 @@ DdLoop dd_gmres_loop(const DdRun& R, const Options& o, DdVec& x, const DdVec& b,
     k_dd_gm_scal<<<1, 32, 0, st>>>(G, DDG_START, 0, dp<dd>(d1));
     R.axpy(G.t1, R.zero, r.hi(), r.lo(), vh(0), vl(0));   // v_1 = -r / |r|
     PB_CUDA(cudaGetLastError());
-    rnorm = read_double(G.rn, st);
+    back.post(G.rn, nullptr, st);
+    auto next = [&](int i) {   // w = A M^-1 v_i
+      R.precon(vh(i - 1), vl(i - 1), pv.hi(), pv.lo());
+      R.spmv(pv, w);
+    };
+    next(1);
+    rnorm = back.wait();
     if (itr == 1) hist_at(itr, rnorm / bnorm);
     bool exit_inner = false;
     for (inner = 1; inner <= m; ++inner) {
-      R.precon(vh(inner - 1), vl(inner - 1), pv.hi(), pv.lo());
-      R.spmv(pv, w);
       dd* col = G.h + (int64_t)(inner - 1) * ld;
       if (mgs) {
         mgs_column(inner);
@@ -1405,7 +1449,10 @@ DdLoop dd_gmres_loop(const DdRun& R, const Options& o, DdVec& x, const DdVec& b,
         R.axpy(G.t1, R.zero, w.hi(), w.lo(), vh(inner), vl(inner));   // v_{i+1} = w / |w|
       }
       PB_CUDA(cudaGetLastError());
-      rnorm = read_double(G.rn, st);
+      back.post(G.rn, nullptr, st);
+      if (inner < m && itr + inner != o.itrmax) next(inner + 1);   // while the host reads the norm
+      PB_CUDA(cudaGetLastError());
+      rnorm = back.wait();
       mm = inner;
       hist_at(itr + inner, rnorm / bnorm);
       if (rnorm / bnorm < o.rtol || itr + inner == o.itrmax) { exit_inner = true; break; }
