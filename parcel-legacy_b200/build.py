@@ -23,7 +23,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
 def flags(debug: bool):
-    f = ARCH + ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC,-fopenmp", "-ccbin", "/usr/bin/g++",
+    f = ARCH + ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-ccbin", "/usr/bin/g++",
                 "-I", os.path.join(HERE, "..", "include"), "--expt-relaxed-constexpr", "-Xptxas", "-v" if debug else "-O3"]
     return f
 
@@ -48,7 +48,7 @@ def build(jobs: int = 8, debug: bool = False) -> str:
     srcs = sorted(glob.glob(os.path.join(CSRC, "*.cu")))
     with cf.ThreadPoolExecutor(max_workers=jobs) as ex:
         objs = list(ex.map(lambda s: compile_one(s, debug), srcs))
-    cmd = [NVCC] + ARCH + ["-shared", "-Xcompiler", "-fPIC,-fopenmp", "-ccbin", "/usr/bin/g++", "-o", LIB] + objs + ["-lgomp"]
+    cmd = [NVCC] + ARCH + ["-shared", "-Xcompiler", "-fPIC", "-ccbin", "/usr/bin/g++", "-o", LIB] + objs
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         sys.stderr.write(r.stdout + r.stderr)

@@ -14,9 +14,10 @@
 // B200 design.  Rows of every block are grouped into wavefront levels (row i depends on
 // the in-block rows it couples to with a smaller index), and the library stores every
 // Krylov vector in a permuted, level-major layout where each level is contiguous and
-// starts on a 16-byte boundary.  One CTA sweeps one block.  A producer warp streams each
-// level's packed coefficients and its input-vector slice into a ring of shared-memory
-// stages with bulk asynchronous copies (cp.async.bulk + mbarrier); the consumer warps
+// starts on a 16-byte boundary.  The plan and the layout are made on the device.  One CTA sweeps
+// one block (many small blocks: a warp for one, two or four).  A producer warp streams groups
+// of levels, packed coefficients and input-vector slice, into a ring of shared-memory stages
+// with bulk asynchronous copies (cp.async.bulk + mbarrier); the consumer warps
 // solve the level's rows from shared memory, keeping the last W levels of the solution in
 // a shared-memory ring, so a level step costs shared-memory latency and one named
 // barrier.  The arithmetic of every row is the reference's: same operands, same order.
@@ -1760,6 +1761,9 @@ static bool grp_layout(const IluPlan& P, const std::vector<IluChunk>& ch, int ku
 // double-double D-ILU of 80^3 1.3 ms -> 0.1 + 0.27 ms.
 // The operations and their order are those of the general kernels.
 enum { FAC_DILU = 0, FAC_ILU0 = 1 };
+// Lower couplings per row: three of the 5- and 7-point stencils, four of a 9-point one under
+// D-ILU.  Wider stencils have triangles, so ILU(0) could not take this path; D-ILU on them keeps
+// the general kernel because no solve here needed more instances (not measured).
 constexpr int kFacMaxK = 4;
 constexpr int kFacThreads = 512;
 

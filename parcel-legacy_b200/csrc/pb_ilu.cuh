@@ -163,7 +163,7 @@ int ilu_setup_device(const IluPlan& P, const DevMat<double>& A, int ilu_method,
 
 // Many small blocks (at least eight per SM, none above 1,024 rows): the wavefront plan built
 // on the device.  ilu_small_plan is false when a row has more couplings than the warp sweep's
-// records hold; the host plan takes such a matrix.
+// records hold; the general plan takes such a matrix.
 struct SmallPlan {
   int n = 0, nb = 0, np = 0, totlev = 0, maxw = 0, max_levels = 0, kmax = 0, span = 0;
   DBuf starts;            // nb + 1 first rows

@@ -121,7 +121,7 @@ def _dense_blocks(nb, rows, seed):
 @pytest.mark.parametrize("nb,rows", [(1300, 1), (1300, 3), (1400, 9), (1200, 12)])
 def test_small_dense_blocks(nb, rows, ilu):
     """One-row blocks, one coupling count after the other, and more couplings than the records
-    hold (the host plan and the general sweep)."""
+    hold (the general plan and the general sweep)."""
     A = _dense_blocks(nb, rows, rows)
     assert _apply_both(A, ipreflag=2, ILU_method=ilu, precon_thblock=nb) < 1e-11
 
