@@ -1229,20 +1229,27 @@ struct DdLoop {
 // of an iteration needs a norm that is known before the iteration's last kernels (CG), or the
 // next iteration's first kernels change nothing the result depends on (BiCGStab, GMRES).  With
 // the read at the end the device idled 30 us in each iteration.
+// The two page-locked doubles belong to the host thread (a thread runs one solve at a time)
+// and are given back when it ends: locking pages is a driver call that waits for whoever else
+// talks to the driver.
+struct DdPinned {
+  double* p = nullptr;
+  ~DdPinned() {
+    if (p) cudaFreeHost(p);
+  }
+};
 struct DdReadback {
   double* p = nullptr;
   cudaEvent_t ev = nullptr;
   DdReadback() {
-    PB_CUDA(cudaMallocHost(&p, 2 * sizeof(double)));
-    if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
-      cudaFreeHost(p);
-      PB_CHECK(false, PARCEL_B_E_CUDA, "no event for the dd solver's stop test");
-    }
+    static thread_local DdPinned mine;
+    if (!mine.p) PB_CUDA(cudaMallocHost(&mine.p, 2 * sizeof(double)));
+    p = mine.p;
+    PB_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   }
   ~DdReadback() {
-    cudaEventSynchronize(ev);
+    cudaEventSynchronize(ev);   // no copy into p is left when the next solve takes it
     cudaEventDestroy(ev);
-    cudaFreeHost(p);
   }
   DdReadback(const DdReadback&) = delete;
   DdReadback& operator=(const DdReadback&) = delete;
