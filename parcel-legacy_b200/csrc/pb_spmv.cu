@@ -239,7 +239,14 @@ static void launch_spmv(const DevMat<VT>& A, const XT* x, XT* y, const XT* b, co
                         const int* sa, const int* sb, const Red& red, const int* gate,
                         cudaStream_t st) {
   const int lpr = spmv_lanes(A.n, A.nnz);
-  const int grid = ND > 0 && red.full_grid() ? red_blocks() : red_grid(A.n, ND > 0 ? 2 * kRedThreads : kRedThreads);
+  // A block for as many rows as its warps hold at once, so that no warp does twice what another
+  // could do beside it; a fused dot takes two rounds of a copy's slices per block where rows are
+  // short (fewer CTAs take its ticket), one where a slice lasts longer than a ticket.  CRS rows are
+  // split over lpr lanes, so a block holds 512 rows of two entries but 8 of more than 20.
+  const bool copy = A.d_val || A.s_val, long_rows = A.nnz > 16 * (int64_t)A.n;
+  const int unr = lpr <= 8 ? 4 : (lpr == 16 ? 2 : 1);   // as launched below
+  const int rows = copy ? (ND > 0 && !long_rows ? 2 * kRedThreads : kRedThreads) : kRedThreads / lpr * unr;
+  const int grid = ND > 0 && red.full_grid() ? red_blocks() : red_grid(A.n, rows);
   int a0 = sa ? sa[0] : 0, b0 = sb ? sb[0] : 0, a1 = sa ? sa[1] : 0, b1 = sb ? sb[1] : 0;
   if (A.d_val) {
     k_spmv_dia<VT, XT, ND, RES><<<grid, kRedThreads, 0, st>>>(A.n, A.ndiag, A.d_off, A.d_val, x, y, b, d, a0, b0,

@@ -265,3 +265,45 @@ def test_dd_mgs_column_sizes(n, m, itrmax):
     A = problems.CRS(n=n, rowptr=rp.astype(np.int32), col=(C3[M3] + 1).astype(np.int32), val=V3[M3].astype(float))
     _dd_both(A, problems.rhs_normal(n, 8), solver=3, itrmax=itrmax, rtolmax=1e-28, GMRES_m=m, GMRES_GSflag=1,
              ipreflag=1)
+
+
+# ---- times that a launch shape decides ------------------------------------------------------------
+def _spread_rows(n, k, seed):
+    """n rows of k entries spread over a quarter of the columns, the diagonal among them."""
+    rng = np.random.default_rng(seed)
+    w = max(n // 4, k)
+    c = (np.arange(n)[:, None] + np.arange(k) * (w // k) + rng.integers(0, max(1, w // k), (n, k))) % n
+    c[:, 0] = np.arange(n)
+    c.sort(1)
+    v = -rng.random((n, k))
+    v[c == np.arange(n)[:, None]] = 1.2 * k
+    keep = np.ones_like(c, bool)
+    keep[:, 1:] = c[:, 1:] != c[:, :-1]
+    rp = np.concatenate([[0], np.cumsum(keep.sum(1))]) + 1
+    return problems.CRS(n=n, rowptr=rp.astype(np.int32), col=(c[keep] + 1).astype(np.int32), val=v[keep])
+
+
+def _spmv_ms(A):
+    import time
+    import torch
+    L = _lib.load()
+    rp, ci, va, x = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (A.rowptr, A.col, A.val, np.ones(A.n)))
+    y = torch.empty_like(x)
+    S = api.crs_struct(A, rp, ci, va)
+    best = np.inf
+    torch.cuda.synchronize()
+    for _ in range(8):
+        t = time.perf_counter()
+        for _ in range(20):
+            assert L.parcel_b_spmv(C.byref(S), x.data_ptr(), y.data_ptr()) == 0, _lib.last_error()
+        torch.cuda.synchronize()
+        best = min(best, (time.perf_counter() - t) / 20)
+    assert np.abs(y.cpu().numpy() - A.to_scipy() @ np.ones(A.n)).max() < 1e-11 * np.abs(A.val).max()
+    return best
+
+
+def test_product_of_few_long_rows_fills_the_chip():
+    """Rows of 400 entries are split over a warp each, so 2,000 of them need 250 CTAs; with a CTA for
+    256 rows (8 CTAs) their product took five times as long as the call, which the same number of
+    short rows measures."""
+    assert _spmv_ms(_spread_rows(2000, 400, 1)) < 2.0 * _spmv_ms(_spread_rows(2000, 9, 1))
