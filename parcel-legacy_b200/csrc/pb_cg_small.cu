@@ -307,24 +307,34 @@ inline int elems(int64_t n) {   // rows per thread: the fewest that need at most
 
 }  // namespace
 
+// Which matrices take the launch.  Its 512 threads per SM walk their rows alone and gather two
+// vectors per entry, so it wins while an iteration is launches and latency and loses once it is
+// bandwidth: per iteration, one launch against three kernels (200 iterations, one B200, point
+// Jacobi): 20,000 rows of 100 entries 23.3 / 24.9 us, 60,000 of 27 20.2 / 20.9, 300,000 of 9 29.1 /
+// 32.1; 60,000 of 100 38.3 / 32.8, 150,000 of 27 37.9 / 32.5, 300,000 of 27 68.8 / 50.8, 150,000
+// of 100 103 / 49.6.
+constexpr int64_t kCgMaxEntries = 2000000;
+constexpr int64_t kCgShortRow = 12;
+
 template <class T>
-int cg_small_grid(int64_t n) {
+int cg_small_grid(int64_t n, int64_t nnz) {
+  if (nnz > kCgMaxEntries && nnz > kCgShortRow * n) return 0;
   const int e = elems(n);
   return e ? (int)((n + (int64_t)e * kCgThreads - 1) / ((int64_t)e * kCgThreads)) : 0;
 }
 
 template <class T>
 void cg_small(const CgSmallArgs<T>& a, cudaStream_t st) {
-  const int e = elems(a.A.n), g = cg_small_grid<T>(a.A.n);
-  PB_CHECK(e > 0 && (a.A.d_val || a.A.s_val), PARCEL_B_E_ARG, "short-vector CG on %d rows", a.A.n);
+  const int e = elems(a.A.n), g = cg_small_grid<T>(a.A.n, a.A.nnz);
+  PB_CHECK(g > 0 && (a.A.d_val || a.A.s_val), PARCEL_B_E_ARG, "short-vector CG on %d rows", a.A.n);
 #define CG_E(E_)                                                                    \
   if (a.A.d_val) launch<T, E_, true>(a, g, st); else launch<T, E_, false>(a, g, st);
   if (e == 1) { CG_E(1) } else if (e == 2) { CG_E(2) } else { CG_E(4) }
 #undef CG_E
 }
 
-template int cg_small_grid<double>(int64_t);
-template int cg_small_grid<float>(int64_t);
+template int cg_small_grid<double>(int64_t, int64_t);
+template int cg_small_grid<float>(int64_t, int64_t);
 template void cg_small<double>(const CgSmallArgs<double>&, cudaStream_t);
 template void cg_small<float>(const CgSmallArgs<float>&, cudaStream_t);
 

@@ -21,8 +21,8 @@ struct CgSmallArgs {
   int* err = nullptr;
 };
 
-// CTAs of the launch for n rows, 0 when the vector is too long for it.
-template <class T> int cg_small_grid(int64_t n);
+// CTAs of the launch for n rows with nnz entries, 0 when the separate kernels are for them.
+template <class T> int cg_small_grid(int64_t n, int64_t nnz);
 constexpr int kCgCopies = 16, kCgLine = 16;   // copies of a grid sum's total, a 128-byte line each
 // Words of both sums: at most four per CTA and the total's copies, each.
 __host__ __device__ constexpr size_t cg_small_slots(int grid) {

@@ -260,7 +260,7 @@ static SolveOut run_pcg(const Options& o, const System<T>& S, const T* b, T* x, 
   Workspace& W = kw.W;
   const int64_t np = S.np;
   const size_t vb = sizeof(T) * np;
-  const int small_grid = S.permuted ? 0 : cg_small_grid<T>(np);
+  const int small_grid = S.permuted ? 0 : cg_small_grid<T>(np, S.A.nnz);
   const bool none = S.M.kind == PARCEL_B_PRECON_NONE;
   T *R = kw.buf<T>(vb), *P = kw.buf<T>(vb), *Q = kw.buf<T>(vb);
   T* Sv = none && !small_grid ? R : kw.buf<T>(vb);   // s = M^-1 r

@@ -307,3 +307,17 @@ def test_product_of_few_long_rows_fills_the_chip():
     256 rows (8 CTAs) their product took five times as long as the call, which the same number of
     short rows measures."""
     assert _spmv_ms(_spread_rows(2000, 400, 1)) < 2.0 * _spmv_ms(_spread_rows(2000, 9, 1))
+
+
+@pytest.mark.parametrize("n,k,one_launch", [(20000, 100, True), (20400, 100, False), (180000, 11, True), (180000, 14, False)])
+def test_short_vector_cg_is_for_few_entries(n, k, one_launch):
+    """Either side of two million entries, and of twelve a row past that: the launch count tells which
+    kernels ran (the separate ones are three an iteration)."""
+    A = _spread_rows(n, k, 3)
+    b = problems.rhs_normal(A.n, 4)
+    kw = dict(solver=1, itrmax=30, rtolmax=1e-200, ipreflag=1)
+    xo, _, no, _ = oracle.solve(A, b, **kw)
+    res = api.solve(A, b, **kw)
+    assert res["niter"] == no == 30
+    assert (res["stats"]["kernel_launches"] < 20) == one_launch
+    assert np.abs(res["x"] - xo).max() < 1e-9 * np.abs(xo).max()
