@@ -664,7 +664,7 @@ __global__ void k_dd_dilu_diag(const IluChunk* __restrict__ ch, const int* __res
             if (rc >= hi) break;
             const bool take = mlud ? kr < rc : rc == k;
             if (!take) continue;
-            dd t = dd_mul(av(jr), av(i));
+            dd t = dd_mul_split(av(jr), av(i));
             t = (Dr.hi == 0.0 && Dr.lo == 0.0) ? dd_div(t, dd{1.0e-100, 0.0}) : dd_div(t, Dr);
             D = dd_sub(D, t);
             if (!mlud) break;
@@ -830,17 +830,17 @@ __device__ __forceinline__ dd dd_row(int k, int n, int j0, const int* col, const
 #pragma unroll
   for (int t = 0; t < kPre; ++t)
     if (t < n) {
-      const dd v = RING ? dd_mul(dd{ringh[col[t]], ringl[col[t]]}, a[t]) : dd_mul(dd{sh[col[t]], sl[col[t]]}, a[t]);
+      const dd v = RING ? dd_mul_split(dd{ringh[col[t]], ringl[col[t]]}, a[t]) : dd_mul_split(dd{sh[col[t]], sl[col[t]]}, a[t]);
       z = DIR == 0 ? dd_sub(z, v) : dd_add(z, v);
     }
   for (int t = kPre; t < n; ++t) {   // couplings past the records, straight from the CRS
     const int j = DIR == 0 ? j0 + t : j0 - t;
     const int c = ci[j] - cbase;
-    const dd v = dd_mul(dd{sh[c], sl[c]}, dd{ah[j], (prec == 2 && al) ? al[j] : 0.0});
+    const dd v = dd_mul_split(dd{sh[c], sl[c]}, dd{ah[j], (prec == 2 && al) ? al[j] : 0.0});
     z = DIR == 0 ? dd_sub(z, v) : dd_add(z, v);
   }
   (void)k;
-  return DIR == 0 ? dd_mul(z, di) : dd_sub(x, dd_mul(di, z));
+  return DIR == 0 ? dd_mul_split(z, di) : dd_sub(x, dd_mul_split(di, z));
 }
 
 // The rows of one level: the staged ones, then any past kRowsPer per thread.

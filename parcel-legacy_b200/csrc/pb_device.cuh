@@ -136,15 +136,8 @@ __device__ __forceinline__ dd dd_sub(dd a, dd b) {
   return dd{s1, t1l};
 }
 
-// The rounding error of t = fl(a b).  The reference computes it from Veltkamp halves, 16
-// operations that are all exact unless something over- or underflows, so the fused
-// multiply-subtract gives the same bits; where an exponent is near either end of the range (or
-// a factor is zero) the halves are used as written.  Bounds: with biased exponents ea + eb >=
-// 1134 the last bit of the product is at least 2^-1016; below 2010 and 3034 neither the split
-// (a 2^27) nor a partial product overflows.  25 -> 9 operations per product.
-__device__ __forceinline__ double two_prod_err(double a, double b, double t) {
-  const unsigned ea = ((unsigned)__double2hiint(a) >> 20) & 0x7ffu, eb = ((unsigned)__double2hiint(b) >> 20) & 0x7ffu;
-  if (ea + eb - 1134u <= 1900u && max(ea, eb) < 2010u) return __fma_rn(a, b, -t);
+// The rounding error of t = fl(a b) from Veltkamp halves, as the reference computes it.
+__device__ __forceinline__ double two_prod_err_split(double a, double b, double t) {
   double u1 = __dmul_rn(134217729.0, a);
   const double p1 = __dsub_rn(u1, __dsub_rn(u1, a));
   const double p2 = __dsub_rn(a, p1);
@@ -154,14 +147,35 @@ __device__ __forceinline__ double two_prod_err(double a, double b, double t) {
   return __dadd_rn(__dadd_rn(__dadd_rn(__dsub_rn(__dmul_rn(p1, r1), t), __dmul_rn(p1, r2)), __dmul_rn(p2, r1)),
                    __dmul_rn(p2, r2));
 }
+// The same with fewer operations: the halves' 16 operations are all exact unless something over-
+// or underflows, so the fused multiply-subtract gives the same bits; where an exponent is near
+// either end of the range (or a factor is zero) the halves are used as written.  Bounds: with
+// biased exponents ea + eb >= 1134 the last bit of the product is at least 2^-1016; below 2010
+// and 3034 neither the split (a 2^27) nor a partial product overflows.  25 -> 9 operations per
+// product.
+__device__ __forceinline__ double two_prod_err(double a, double b, double t) {
+  const unsigned ea = ((unsigned)__double2hiint(a) >> 20) & 0x7ffu, eb = ((unsigned)__double2hiint(b) >> 20) & 0x7ffu;
+  if (ea + eb - 1134u <= 1900u && max(ea, eb) < 2010u) return __fma_rn(a, b, -t);
+  return two_prod_err_split(a, b, t);
+}
 
-__device__ __forceinline__ dd dd_mul(dd a, dd b) {
-  const double t1h = __dmul_rn(a.hi, b.hi);
-  double t1l = two_prod_err(a.hi, b.hi, t1h);
+__device__ __forceinline__ dd dd_mul_from(dd a, dd b, double t1h, double t1l) {
   t1l = __dadd_rn(t1l, __dadd_rn(__dmul_rn(a.hi, b.lo), __dmul_rn(a.lo, b.hi)));
   double s1 = __dadd_rn(t1h, t1l);
   t1l = __dsub_rn(t1l, __dsub_rn(s1, t1h));
   return dd{s1, t1l};
+}
+
+__device__ __forceinline__ dd dd_mul(dd a, dd b) {
+  const double t1h = __dmul_rn(a.hi, b.hi);
+  return dd_mul_from(a, b, t1h, two_prod_err(a.hi, b.hi, t1h));
+}
+// The same bits without the branch: for chains of products in which a warp waits for each one's
+// outcome and for memory, not for the issue of its operations (the sweep and the diagonal
+// without staged records: 48^3 27-point D-ILU sweep 1.19 -> 1.04 ms, diagonal 9.5 -> 8.1 ms).
+__device__ __forceinline__ dd dd_mul_split(dd a, dd b) {
+  const double t1h = __dmul_rn(a.hi, b.hi);
+  return dd_mul_from(a, b, t1h, two_prod_err_split(a.hi, b.hi, t1h));
 }
 
 // dd_div (dd_func.f90:99-142): q1 = a.hi / b.hi, the product b * q1 formed exactly with
