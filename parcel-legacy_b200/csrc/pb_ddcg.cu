@@ -630,11 +630,14 @@ __global__ void k_dd_ranges(int n, int nb, const int* __restrict__ blk_lo, const
   }
 }
 
+// Up to kIluChunk rows of one level: first permuted position, rows.
+struct DdChunk { int start, w; };
+
 // ddDILU_DInv_crs (ddmatrix.f90:1451-1640), independ_nvec = 1, one CTA per block, level by
 // level: D_k = a_kk - sum over the lower in-block entries a_kr (kr < k) of a_kr a_rk / D_r
 // (ILUD: the entry of row r in column k only; MLUD: every entry of row r right of r), then
 // D^-1 = 1 / D (a zero D replaced by 1e-100).
-__global__ void k_dd_dilu_diag(const IluChunk* __restrict__ ch, const int* __restrict__ blk_chunk,
+__global__ void k_dd_dilu_diag(const DdChunk* __restrict__ ch, const int* __restrict__ blk_chunk,
                                const int* __restrict__ blk_lo, const int* __restrict__ blk_hi,
                                const int* __restrict__ rowAt, const int* __restrict__ rp,
                                const int* __restrict__ ci, const double* __restrict__ ah,
@@ -644,7 +647,7 @@ __global__ void k_dd_dilu_diag(const IluChunk* __restrict__ ch, const int* __res
   const int lo = blk_lo[b], hi = blk_hi[b];
   auto av = [&](int j) { return dd{ah[j], al ? al[j] : 0.0}; };
   for (int c = blk_chunk[b]; c < blk_chunk[b + 1]; ++c) {
-    const IluChunk C = ch[c];
+    const DdChunk C = ch[c];
     for (int p = threadIdx.x; p < C.w; p += blockDim.x) {
       const int k = rowAt[C.start + p];
       dd D{0.0, 0.0};
@@ -792,7 +795,7 @@ struct DdStage {
 };
 
 template <int DIR>
-__device__ __forceinline__ void dd_stage(DdStage& S, const IluChunk& C, const DdRecords& R, const double* xh,
+__device__ __forceinline__ void dd_stage(DdStage& S, const DdChunk& C, const DdRecords& R, const double* xh,
                                          const double* xl) {
 #pragma unroll
   for (int u = 0; u < kRowsPer; ++u) {
@@ -845,7 +848,7 @@ __device__ __forceinline__ dd dd_row(int k, int n, int j0, const int* col, const
 
 // The rows of one level: the staged ones, then any past kRowsPer per thread.
 template <int DIR, bool RING>
-__device__ __forceinline__ void dd_level(const DdStage& S, const IluChunk& C, const DdRecords& R, const double* xh,
+__device__ __forceinline__ void dd_level(const DdStage& S, const DdChunk& C, const DdRecords& R, const double* xh,
                                          const double* xl, const int* __restrict__ ci, const double* __restrict__ ah,
                                          const double* __restrict__ al, int cbase, int prec, double* sh, double* sl,
                                          double* fqh, double* fql, double* ringh, double* ringl) {
@@ -899,7 +902,7 @@ __device__ __forceinline__ void dd_level(const DdStage& S, const IluChunk& C, co
 // shared-memory loads instead of L2 round trips.
 template <bool RING>
 __global__ void __launch_bounds__(256, 1)
-    k_dd_dilu_sweep(const IluChunk* __restrict__ ch, const int* __restrict__ blk_chunk, DdRecords R,
+    k_dd_dilu_sweep(const DdChunk* __restrict__ ch, const int* __restrict__ blk_chunk, DdRecords R,
                     const int* __restrict__ ci, const double* __restrict__ ah, const double* __restrict__ al, int cbase,
                     int prec, const double* __restrict__ rqh, const double* __restrict__ rql, double* fqh, double* fql,
                     double* sh, double* sl, int ring_rows) {
@@ -913,7 +916,7 @@ __global__ void __launch_bounds__(256, 1)
   // forward: input r in level order; the results also go to level order for the backward
   dd_stage<0>(A, ch[c0], R, rqh, rql);
   for (int c = c0; c < c1; ++c) {
-    const IluChunk C = ch[c];
+    const DdChunk C = ch[c];
     if (c + 1 < c1) dd_stage<0>(B, ch[c + 1], R, rqh, rql);
     dd_level<0, RING>(A, C, R, rqh, rql, ci, ah, al, cbase, prec, sh, sl, fqh, fql, ringh, ringl);
     __syncthreads();
@@ -922,7 +925,7 @@ __global__ void __launch_bounds__(256, 1)
   // backward: input the forward result (complete after the barrier above)
   dd_stage<1>(A, ch[c1 - 1], R, fqh, fql);
   for (int c = c1 - 1; c >= c0; --c) {
-    const IluChunk C = ch[c];
+    const DdChunk C = ch[c];
     if (c - 1 >= c0) dd_stage<1>(B, ch[c - 1], R, fqh, fql);
     dd_level<1, RING>(A, C, R, fqh, fql, ci, ah, al, cbase, prec, sh, sl, nullptr, nullptr, ringh, ringl);
     __syncthreads();
@@ -1034,6 +1037,26 @@ void dd_dots(const DdSystem& S, const double* xh, const double* xl, const double
       then.d1, then.d2);
 }
 
+// The chunk tables of the sweep and the diagonal without staged records, made where they run:
+// blocks of a few rows have as many levels as rows (262,144 chunks at 64^3 in 4,096 lines).
+void dd_chunks(const IluPlan& plan, DdPrecon& P) {
+  if (P.chunks.p) return;
+  std::vector<DdChunk> ch;
+  std::vector<int> first(plan.nb + 1, 0);
+  ch.reserve(plan.lvl_start.size());
+  for (int b = 0; b < plan.nb; ++b) {
+    first[b] = (int)ch.size();
+    for (int l = plan.blk_lvl[b]; l < plan.blk_lvl[b + 1]; ++l)
+      for (int s = plan.lvl_start[l]; s < plan.lvl_end[l]; s += kIluChunk)
+        ch.push_back(DdChunk{s, std::min(kIluChunk, plan.lvl_end[l] - s)});
+  }
+  first[plan.nb] = (int)ch.size();
+  P.chunks.alloc(sizeof(DdChunk) * std::max<size_t>(ch.size(), 1), false);
+  h2d(P.chunks.p, ch.data(), sizeof(DdChunk) * ch.size());
+  P.blk_chunk.alloc(sizeof(int) * first.size(), false);
+  h2d(P.blk_chunk.p, first.data(), sizeof(int) * first.size());
+}
+
 void dd_setup_precon(const Options& o, const parcel_b_crs& A, const DdSystem& S, int prec_M, DdPrecon& P) {
   cudaStream_t st = stream();
   P.kind = o.precon == PARCEL_B_PRECON_ADDITIVESCHWARZ ? PARCEL_B_PRECON_BLOCKJACOBI : o.precon;
@@ -1057,10 +1080,6 @@ void dd_setup_precon(const Options& o, const parcel_b_crs& A, const DdSystem& S,
   DBuf dpos, dlev;
   ilu_build_plan(M, block_split(o, A.n), true, plan, dpos, P.rowAt, dlev);
   P.nb = plan.nb;
-  P.chunks.alloc(sizeof(IluChunk) * std::max<size_t>(plan.chunks.size(), 1));
-  h2d(P.chunks.p, plan.chunks.data(), sizeof(IluChunk) * plan.chunks.size());
-  P.blk_chunk.alloc(sizeof(int) * (plan.nb + 1));
-  h2d(P.blk_chunk.p, plan.blk_chunk.data(), sizeof(int) * (plan.nb + 1));
   DBuf blo(sizeof(int) * plan.nb), bhi(sizeof(int) * plan.nb), bof(sizeof(int) * A.n);
   h2d(blo.p, plan.blk_lo.data(), sizeof(int) * plan.nb);
   h2d(bhi.p, plan.blk_hi.data(), sizeof(int) * plan.nb);
@@ -1074,8 +1093,9 @@ void dd_setup_precon(const Options& o, const parcel_b_crs& A, const DdSystem& S,
     k_dd_dilu_inv<<<grid_for(A.n), kDdThreads, 0, st>>>(A.n, dp<dd>(Dd), dp<double>(P.dih), dp<double>(P.dil));
   } else {
     DBuf Dh(sizeof(double) * A.n), Dl(sizeof(double) * A.n);
+    dd_chunks(plan, P);
     k_dd_dilu_diag<<<plan.nb, ilu_factor_threads(plan.maxWp), 0, st>>>(
-        dp<IluChunk>(P.chunks), dp<int>(P.blk_chunk), dp<int>(blo), dp<int>(bhi), dp<int>(P.rowAt), S.rp, S.ci, S.ah,
+        dp<DdChunk>(P.chunks), dp<int>(P.blk_chunk), dp<int>(blo), dp<int>(bhi), dp<int>(P.rowAt), S.rp, S.ci, S.ah,
         S.al, S.cbase, o.ilu_method == 2 ? 1 : 0, dp<double>(Dh), dp<double>(Dl), dp<double>(P.dih),
         dp<double>(P.dil));
   }
@@ -1090,6 +1110,7 @@ void dd_setup_precon(const Options& o, const parcel_b_crs& A, const DdSystem& S,
       return;
     }
   }
+  dd_chunks(plan, P);
   // ring: slot of natural row c = (level % W) * LW + (position - the level's first position),
   // LW the widest level; used when its hi and lo parts fit kDdRingBytes of shared memory
   const int LW = plan.maxWp;   // the widest level (rows, rounded up to 4)
@@ -1153,10 +1174,10 @@ void dd_apply_precon(const DdSystem& S, const DdPrecon& P, const double* rh, con
           attr = true;
         }
         k_dd_dilu_sweep<true><<<P.nb, kDdThreads, 2 * sizeof(double) * P.ring_rows, st>>>(
-            dp<IluChunk>(P.chunks), dp<int>(P.blk_chunk), P.rec(), S.ci, S.ah, S.al, S.cbase, P.prec,
+            dp<DdChunk>(P.chunks), dp<int>(P.blk_chunk), P.rec(), S.ci, S.ah, S.al, S.cbase, P.prec,
             dp<double>(P.rqh), dp<double>(P.rql), dp<double>(P.fqh), dp<double>(P.fql), sh, sl, P.ring_rows);
       } else {
-        k_dd_dilu_sweep<false><<<P.nb, kDdThreads, 0, st>>>(dp<IluChunk>(P.chunks), dp<int>(P.blk_chunk), P.rec(),
+        k_dd_dilu_sweep<false><<<P.nb, kDdThreads, 0, st>>>(dp<DdChunk>(P.chunks), dp<int>(P.blk_chunk), P.rec(),
                                                             S.ci, S.ah, S.al, S.cbase, P.prec, dp<double>(P.rqh),
                                                             dp<double>(P.rql), dp<double>(P.fqh), dp<double>(P.fql),
                                                             sh, sl, 0);

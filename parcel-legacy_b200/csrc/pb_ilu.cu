@@ -360,46 +360,24 @@ bool ilu_build_plan(const DevMat<double>& A, const BlockSplit& blocks, bool tigh
   PB_CUDA(cudaGetLastError());
   std::vector<int> width(totlev);
   d2h(width.data(), dwidth.p, sizeof(int) * totlev);
-  // level starts (multiples of 4) and chunks (a level split at kIluChunk rows), in block order
+  // level starts (multiples of 4), in block order
   int64_t total = 0;
-  size_t nchunk = 0;
-  for (int w : width) {
-    total += align4(w);
-    nchunk += (w + kIluChunk - 1) / kIluChunk;
-  }
+  for (int w : width) total += align4(w);
   PB_CHECK(total <= INT_MAX - 3, PARCEL_B_E_ARG, "the permuted layout of %d rows exceeds 2^31 entries", n);
   P.lvl_start.resize(totlev);
   P.lvl_end.resize(totlev);
-  P.blk_chunk.assign(nb + 1, 0);
-  P.chunks.resize(nchunk);
-  int cursor = 0, c = 0, maxw = 0, maxl = 0;
-  for (int b = 0; b < nb; ++b) {
-    P.blk_chunk[b] = c;
-    maxl = std::max(maxl, nlev[b]);
-    for (int l = 0; l < nlev[b]; ++l) {
-      const int gl = P.blk_lvl[b] + l, w = width[gl];
-      P.lvl_start[gl] = cursor;
-      P.lvl_end[gl] = cursor + w;
-      maxw = std::max(maxw, w);
-      for (int o = 0; o < w; o += kIluChunk) {
-        IluChunk& C = P.chunks[c++];
-        C.start = cursor + o;
-        C.w = std::min(kIluChunk, w - o);
-        C.wpad = align4(C.w);
-        C.KL = C.KU = h.kmax;
-        C.lvl = l;
-        C.off_in_level = o;
-        C.blk = b;
-        C.offF = 0;
-        C.offB = 0;
-      }
-      cursor = align4(cursor + w);
-    }
+  int cursor = 0, maxw = 0, maxl = 0;
+  for (int b = 0; b < nb; ++b) maxl = std::max(maxl, nlev[b]);
+  for (int l = 0; l < totlev; ++l) {
+    P.lvl_start[l] = cursor;
+    P.lvl_end[l] = cursor + width[l];
+    maxw = std::max(maxw, width[l]);
+    cursor = align4(cursor + width[l]);
   }
-  P.blk_chunk[nb] = c;
   P.np = (int)total;   // the last level is padded as well
   P.maxWp = align4(maxw);
   P.max_levels = maxl;
+  P.kmax = h.kmax;
   P.W = h.gap + 1;
   pos.alloc(ib, false);
   rowAt.alloc(sizeof(int) * (size_t)P.np, false);
@@ -411,6 +389,36 @@ bool ilu_build_plan(const DevMat<double>& A, const BlockSplit& blocks, bool tigh
   PB_CUDA(cudaGetLastError());
   sync();   // the temporaries above are released on return
   return h.long_ring != 0;
+}
+
+// The plan's chunks (a level split at kIluChunk rows), in block order; K couplings per row in
+// their records.  blk_chunk: nb + 1.
+static std::vector<IluChunk> plan_chunks(const IluPlan& P, int K, std::vector<int>& blk_chunk) {
+  size_t n = 0;
+  for (size_t l = 0; l < P.lvl_start.size(); ++l) n += (P.lvl_end[l] - P.lvl_start[l] + kIluChunk - 1) / kIluChunk;
+  std::vector<IluChunk> ch(n);
+  blk_chunk.assign(P.nb + 1, 0);
+  int c = 0;
+  for (int b = 0; b < P.nb; ++b) {
+    blk_chunk[b] = c;
+    for (int gl = P.blk_lvl[b]; gl < P.blk_lvl[b + 1]; ++gl) {
+      const int w = P.lvl_end[gl] - P.lvl_start[gl];
+      for (int o = 0; o < w; o += kIluChunk) {
+        IluChunk& C = ch[c++];
+        C.start = P.lvl_start[gl] + o;
+        C.w = std::min(kIluChunk, w - o);
+        C.wpad = align4(C.w);
+        C.KL = C.KU = K;
+        C.lvl = gl - P.blk_lvl[b];
+        C.off_in_level = o;
+        C.blk = b;
+        C.offF = 0;
+        C.offB = 0;
+      }
+    }
+  }
+  blk_chunk[P.nb] = c;
+  return ch;
 }
 
 // ------------------------------------------------------------------ factorisation
@@ -1665,9 +1673,10 @@ static int sweep_smem_budget() {
 // largest block by position, whichever is smaller; its byte offsets are 16-bit and two
 // stages of a widest chunk must fit beside it.
 template <class T>
-static bool grp_layout(const IluPlan& P, const std::vector<IluChunk>& ch, int kuni, int maxw, IluDev<T>& D,
-                       RingMap& ring) {
+static bool grp_layout(const IluPlan& P, const std::vector<IluChunk>& ch, const std::vector<int>& blk_chunk, int kuni,
+                       IluDev<T>& D, RingMap& ring) {
   const int budget = sweep_smem_budget();
+  const int maxw = std::min(P.maxWp, kIluChunk);
   int max_span = 0;
   for (int b = 0; b < P.nb; ++b)
     max_span = std::max(max_span, align4(P.lvl_end[P.blk_lvl[b + 1] - 1]) - P.lvl_start[P.blk_lvl[b]]);
@@ -1695,12 +1704,12 @@ static bool grp_layout(const IluPlan& P, const std::vector<IluChunk>& ch, int ku
   int64_t max_stage = 0;
   for (int b = 0; b < P.nb; ++b) {
     blk_grp[b] = (int)gi.size();
-    int c = P.blk_chunk[b];
-    while (c < P.blk_chunk[b + 1]) {
+    int c = blk_chunk[b];
+    while (c < blk_chunk[b + 1]) {
       const int sstart = ch[c].start;
       int e = c + 1;
       auto span_to = [&](int ce) { return (int64_t)align4(ch[ce - 1].start + ch[ce - 1].w) - sstart; };
-      while (e < P.blk_chunk[b + 1] && e - c < kGrpMax && grp_bytes(span_to(e + 1)) <= target) ++e;
+      while (e < blk_chunk[b + 1] && e - c < kGrpMax && grp_bytes(span_to(e + 1)) <= target) ++e;
       const int64_t span = span_to(e);
       gi.push_back(make_int4(c, e, sstart, (int)span));
       max_stage = std::max(max_stage, grp_bytes(span));
@@ -1976,14 +1985,13 @@ static bool fac_run(const IluPlan& P, int kmax, const DevMat<double>& A, const d
 
 bool ilu_dd_diag(const IluPlan& P, const DevMat<double>& A, const double* al, const int* blo, const int* bhi,
                  const int* d_pos, const int* d_rowAt, const int* d_lev, dd* diag) {
-  int kmax = 0;
-  for (const auto& c : P.chunks) kmax = std::max(kmax, std::max(c.KL, c.KU));
+  if (P.kmax > kFacMaxK) return false;
   const size_t nl = std::max<size_t>(P.lvl_start.size(), 1);
   DBuf blvl(sizeof(int) * (P.nb + 1)), lst(sizeof(int) * nl), lend(sizeof(int) * nl);
   h2d(blvl.p, P.blk_lvl.data(), sizeof(int) * (P.nb + 1));
   h2d(lst.p, P.lvl_start.data(), sizeof(int) * P.lvl_start.size());
   h2d(lend.p, P.lvl_end.data(), sizeof(int) * P.lvl_end.size());
-  return fac_run<dd, FAC_DILU>(P, kmax, A, al, LevelTab{dp<int>(blvl), dp<int>(lst), dp<int>(lend)}, blo, bhi, d_pos,
+  return fac_run<dd, FAC_DILU>(P, P.kmax, A, al, LevelTab{dp<int>(blvl), dp<int>(lst), dp<int>(lend)}, blo, bhi, d_pos,
                                d_rowAt, d_lev, diag);
 }
 
@@ -2054,16 +2062,14 @@ int ilu_setup_device(const IluPlan& P, const DevMat<double>& A, int ilu_method,
   D.maxWp = std::max(4, P.maxWp);
   // every chunk carries the same number of coupled entries per row (the matrix-wide
   // maximum, rounded up to a supported count)
-  std::vector<IluChunk> ch = P.chunks;
-  int kmax = 0, maxw = 0;
-  for (const auto& c : ch) { kmax = std::max(kmax, std::max(c.KL, c.KU)); maxw = std::max(maxw, c.w); }
-  int kuni = kmax;
+  int kuni = P.kmax;
   for (int c : {1, 2, 3, 4, 6, 8})
-    if (kmax <= c) { kuni = c; break; }
-  for (auto& c : ch) { c.KL = kuni; c.KU = kuni; }
+    if (P.kmax <= c) { kuni = c; break; }
+  std::vector<int> blk_chunk;
+  std::vector<IluChunk> ch = plan_chunks(P, kuni, blk_chunk);
   D.K = kuni;
   RingMap ring;
-  D.grp = kuni <= 8 && grp_layout<T>(P, ch, kuni, maxw, D, ring);
+  D.grp = kuni <= 8 && grp_layout<T>(P, ch, blk_chunk, kuni, D, ring);
   if (!D.grp) {
     // the general sweep: its ring holds the last W levels when they fit 64 KB
     const int budget = sweep_smem_budget();
@@ -2107,7 +2113,7 @@ int ilu_setup_device(const IluPlan& P, const DevMat<double>& A, int ilu_method,
   D.chunks.alloc(sizeof(IluChunk) * std::max<size_t>(ch.size(), 1));
   h2d(D.chunks.p, ch.data(), sizeof(IluChunk) * ch.size());
   D.blk_chunk.alloc(sizeof(int) * (P.nb + 1));
-  h2d(D.blk_chunk.p, P.blk_chunk.data(), sizeof(int) * (P.nb + 1));
+  h2d(D.blk_chunk.p, blk_chunk.data(), sizeof(int) * (P.nb + 1));
   DBuf blo(sizeof(int) * P.nb), bhi(sizeof(int) * P.nb);
   h2d(blo.p, P.blk_lo.data(), sizeof(int) * P.nb);
   h2d(bhi.p, P.blk_hi.data(), sizeof(int) * P.nb);
@@ -2120,7 +2126,7 @@ int ilu_setup_device(const IluPlan& P, const DevMat<double>& A, int ilu_method,
   trace_mark("ilu: tables to device");
   // factorisation in natural CSR order
   Factor F;
-  F.run_plan(P, kmax, A, ilu_method, LevelTab{dp<int>(blvl), dp<int>(lst), dp<int>(lend)}, dp<int>(blo), dp<int>(bhi),
+  F.run_plan(P, P.kmax, A, ilu_method, LevelTab{dp<int>(blvl), dp<int>(lst), dp<int>(lend)}, dp<int>(blo), dp<int>(bhi),
              d_pos, d_rowAt, d_lev, st);
   trace_mark("ilu: factor");
   // every byte of them that is read is packed below
@@ -2423,19 +2429,17 @@ bool ilu_setup_dd(const IluPlan& P, const DevMat<double>& A, const double* al, c
   D.dilu = true;
   D.W = P.W;
   D.maxWp = std::max(4, P.maxWp);
-  std::vector<IluChunk> ch = P.chunks;
-  int kmax = 0, maxw = 0;
-  for (const auto& c : ch) { kmax = std::max(kmax, std::max(c.KL, c.KU)); maxw = std::max(maxw, c.w); }
   int kuni = 0;
   for (int c : {6, 4, 3, 2, 1})
-    if (kmax <= c) kuni = c;
+    if (P.kmax <= c) kuni = c;
   // a stage ring takes most of an SM: with eight blocks per SM and more the unstaged sweep,
   // several CTAs to an SM, is the better one
   if (kuni == 0 || P.nb >= 8 * num_sms()) return false;
-  for (auto& c : ch) { c.KL = kuni; c.KU = kuni; }
+  std::vector<int> blk_chunk;
+  const std::vector<IluChunk> ch = plan_chunks(P, kuni, blk_chunk);
   D.K = kuni;
   RingMap ring;
-  if (!grp_layout<dd>(P, ch, kuni, maxw, D, ring)) return false;
+  if (!grp_layout<dd>(P, ch, blk_chunk, kuni, D, ring)) return false;
   D.grp = true;
   DBuf chunks(sizeof(IluChunk) * std::max<size_t>(ch.size(), 1)), blo(sizeof(int) * P.nb), bhi(sizeof(int) * P.nb),
       blvl(sizeof(int) * (P.nb + 1)), lst(sizeof(int) * std::max<size_t>(P.lvl_start.size(), 1));

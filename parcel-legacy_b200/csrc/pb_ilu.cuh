@@ -81,8 +81,7 @@ struct IluPlan {
   int W = 1;            // ring depth in levels
   int maxWp = 0;        // widest level (padded)
   int max_levels = 0;
-  std::vector<IluChunk> chunks;
-  std::vector<int> blk_chunk;   // nb + 1
+  int kmax = 0;         // strictly-lower or strictly-upper in-block entries of a row, the larger
   std::vector<int> blk_lo, blk_hi;   // natural row ranges [lo, hi)
   std::vector<int> lvl_start;   // per block-level (global index) permuted start
   std::vector<int> lvl_end;     // per block-level permuted end (start + width)

@@ -321,3 +321,16 @@ def test_short_vector_cg_is_for_few_entries(n, k, one_launch):
     assert res["niter"] == no == 30
     assert (res["stats"]["kernel_launches"] < 20) == one_launch
     assert np.abs(res["x"] - xo).max() < 1e-9 * np.abs(xo).max()
+
+
+def test_dd_setup_of_many_small_blocks():
+    """4,096 lines of 64 rows, each row its own level: the set-up makes no table of the sweep with staged
+    records, which these blocks do not take (with it 1.5 applications' time, without 0.9)."""
+    import torch
+    A = problems.poisson3d_reference(64, 64, 64)[0]
+    rp, ci, va, b = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (A.rowptr, A.col, A.val, np.ones(A.n)))
+    torch.cuda.synchronize()
+    st = [api.ddcg(A, b, rowptr=rp, col=ci, val=va, itrmax=8, rtolmax=1e-30, ipreflag=2, ILU_method=1,
+                   precon_thblock=4096)["stats"] for _ in range(5)]
+    assert min(s["setup_s"] for s in st) < 1.25 * min(s["solve_s"] for s in st) / 8
+
