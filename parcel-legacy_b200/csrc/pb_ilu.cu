@@ -66,246 +66,326 @@ void ilu_block_rows(int b, int nb, int n, int* lo, int* hi) {
 // forward and the backward sweep.  The dependency window W is the largest level gap of any
 // coupling + 1.
 //
-// One CTA per block walks the block's rows kPlanRows at a time.  Levels of earlier rows are
-// final; among the rows at hand, every row takes the largest level of what it waits for plus
+// k_plan_levels: one CTA per block walks the block's rows PR at a time.  Levels of earlier rows
+// are final; among the rows at hand, every row takes the largest level of what it waits for plus
 // one until nothing changes.  The equations are acyclic and the levels only grow, so the
-// reads of rows that change at the same time do no harm.  A chunk takes as many rounds as the
-// longest chain in it, about the line length for a stencil.  The same work on the host
-// cores, with the structure's copy back and the maps' copy out, was 3 to 11 ms of a solve's
-// set-up (128^3 to 160^3, 16 cores).
+// reads of rows that change at the same time do no harm.  Rows that each wait for the row before
+// them, as along a grid line, are taken in one prefix maximum per warp, and a row's neighbour in
+// the plane before is final already, so a stencil's chunk takes few rounds.  What a round
+// costs is block barriers and shared-memory latency: a row's couplings within the chunk are
+// listed in shared memory once, and those that the other row lists as well (all, in a symmetric
+// pattern) are read and not also pushed.  Where couplings make longer chains (a random band) a
+// chunk gives up the rounds, after fewer of them than the chunk before if that did, and its warps
+// take turns instead, each until its 32 rows are final.
+// Everything that is not a chain is done for all rows at once by other kernels: gaps, positions.
+// With positions and gaps inside one CTA or warp a block, two passes over the levels where the
+// gap was 1 already, and a round per row on chains, the plan of few blocks took longer than on
+// the host (copies of the structure and of the maps included): 160^3 in one block 71 ms on the
+// host, 106 ms so, 17 ms now; 1,024 x 1,024 triangulated 13.7, 21.1, 4.0 ms; 100,000
+// rows tridiagonal 2.1, 74.9, 3.0 ms; a random band of 9 in a million rows 16.7, about 390, 128
+// ms (of a set-up of 1.4 s).
 //
 // When the early levels' gap makes the ring too long, they are moved as late as the rows'
 // dependents allow, rows without dependents left where they are (every row with dependents to
-// one below its lowest dependent).  The number of levels and the validity of the order are
+// one below its lowest dependent): the same kernel on the mirrored order (LATE) finds every
+// row's distance from the last level.  The number of levels and the validity of the order are
 // unchanged (the longest chain has no slack); what changes is the largest gap.  A block that
 // starts in the middle of a grid plane has rows that could start at once but are only needed
 // a hundred levels later; with the levels taken as early as possible the ring of a
 // 12,000-row block of a 61 x 53 x 47 stencil would hold 58 levels, tightened it holds 2, as for
 // a block of whole planes, and the grouped sweep takes it instead of the general one, which
-// gathers coupled values from global memory: 147 -> 33 us per application there (16 blocks),
-// 248 -> 53 us on 97 x 89 x 83 in 48 blocks.  The late levels are kept when they shorten the gap.
-constexpr int kPlanRows = 1024;
-constexpr int kPlanReg = 8;   // entries of a row kept in registers
+// gathers coupled values from global memory: 119 -> 26 us per application there (16 blocks, in
+// a solve), 245 -> 53 us on 97 x 89 x 83 in 48 blocks.  The late levels are kept when they shorten
+// the gap, which in no case tried (400 grids of 5 to 27 points, 1 to 24 blocks) made the ring
+// longer.
+constexpr int kPlanRounds = 48;
+constexpr int kPlanRetry = 8;
+constexpr int kPlanList = 16;      // couplings of a row within its chunk, each way, that are listed
+constexpr int kPlanFar = 4;        // couplings to later chunks kept in registers
+constexpr int kPlanBatch = 8;      // entries of a row loaded at once
 
 struct PlanStat {
-  int kmax, gap, missing;   // missing: a block without a diagonal entry, or INT_MAX
-  int long_ring;            // a block's early levels make its ring too long
+  int kmax, missing;   // missing: a block without a diagonal entry, or INT_MAX
 };
 
-// The in-block entries of a row, from registers when it has at most kPlanReg entries.
-struct PlanRow {
-  int col[kPlanReg];
-  int a, z;
-  template <class F>
-  __device__ __forceinline__ void each(const int* ci, int cbase, F&& f) const {
-    if (z - a <= kPlanReg) {
-#pragma unroll
-      for (int e = 0; e < kPlanReg; ++e)
-        if (col[e] >= 0) f(col[e]);
-    } else {
-      for (int j = a; j < z; ++j) f(ci[j] - cbase);
-    }
-  }
-};
+// A block's early levels make its ring too long, and another order can help.
+__host__ __device__ inline bool plan_loose(int gap, int rows, int nlev) {
+  return gap > 1 && (int64_t)(gap + 1) * rows > kTightenRing * (int64_t)nlev;
+}
 
-// lev: levels out.  low (zeroed), first (all INT_MAX) and late: scratch, one int per row; dep
-// (zeroed): one byte.  wid (zeroed): level widths, block b's from its first row on.
-__global__ void __launch_bounds__(kPlanRows) k_plan_levels(const int* __restrict__ starts, const int* __restrict__ rp,
-                                                           const int* __restrict__ ci, int rbase, int cbase, int* lev,
-                                                           int* low, int* first, int* late, unsigned char* dep,
-                                                           int* wid, int* __restrict__ nlev, PlanStat* stat, bool tighten) {
-  __shared__ volatile int cur[kPlanRows];   // level of the chunk's rows
-  __shared__ int push[kPlanRows];           // forced on them by rows whose entries point at them
-  __shared__ int s_max, s_gap, s_kmax;
+// val: levels out (LATE: distances from the last level).  far (zeroed): scratch, one int per
+// row.  wid (zeroed): level widths, block b's from its first row on.  LATE: lev, nlev and gap of
+// the early levels, dep: rows that have dependents; blocks that are not loose are left out.
+template <bool LATE, int PR>
+__global__ void __launch_bounds__(PR, PR == 1024 ? 1 : 4)
+    k_plan_levels(const int* __restrict__ starts, const int* __restrict__ rp, const int* __restrict__ ci, int rbase,
+                  int cbase, int* val, int* far, int* wid, const int* __restrict__ lev,
+                  const unsigned char* __restrict__ dep, const int* __restrict__ gap, int* nlev, PlanStat* stat) {
+  extern __shared__ unsigned short plan_smem[];
+  unsigned short(*before)[PR] = reinterpret_cast<unsigned short(*)[PR]>(plan_smem);
+  unsigned short(*after)[PR] = before + kPlanList;
+  __shared__ volatile int cur[PR];   // level of the chunk's rows
+  __shared__ int push[PR];           // forced on them by couplings only the other row lists
+  __shared__ unsigned short nbef[PR];   // listed couplings; kPlanList + 1: the row is read
+  __shared__ int s_max, s_kmax;
   const int b = blockIdx.x, t = threadIdx.x;
-  const int lo = starts[b], hi = starts[b + 1];
-  if (t == 0) s_max = s_gap = s_kmax = 0;
-  __syncthreads();
-  auto row_at = [&](int i, PlanRow& R) {
-    R.a = R.z = 0;
-    if (i < hi) {
-      R.a = rp[i] - rbase;
-      R.z = rp[i + 1] - rbase;
-    }
-#pragma unroll
-    for (int e = 0; e < kPlanReg; ++e) {
-      const int c = e < R.z - R.a ? ci[R.a + e] - cbase : -1;
-      R.col[e] = c;
-    }
-  };
-  int kmax = 0, maxlev = 0;
+  const int lo = starts[b], hi = starts[b + 1], m = hi - lo;
+  if (LATE && !plan_loose(gap[b], m, nlev[b])) return;
+  const int last = LATE ? nlev[b] - 1 : 0;
+  if (t == 0) s_max = s_kmax = 0;
+  auto row_of = [&](int u) { return LATE ? hi - 1 - u : lo + u; };   // u-th row of the walk
+  auto walk_of = [&](int c) { return LATE ? hi - 1 - c : c - lo; };
+  int kmax = 0, maxlev = 0, rounds = kPlanRounds;
   bool missing = false;
-  // ---- early levels, chunk by chunk
-  for (int base = lo; base < hi; base += kPlanRows) {
-    const int i = base + t;
-    const bool on = i < hi;
-    PlanRow R;
-    row_at(i, R);
-    int L0 = on ? __ldcg(low + i) : 0;
-    int nl = 0, nu = 0;
+  for (int base = 0; base < m; base += PR) {
+    const int u = base + t;
+    const bool on = u < m;
+    const int i = on ? row_of(u) : 0;
+    const int a = on ? rp[i] - rbase : 0, z = on ? rp[i + 1] - rbase : 0;
+    int L0 = on ? __ldcg(far + i) : 0;
+    if (LATE && on && !dep[i]) L0 = last - lev[i];
+    int nb = 0, na = 0, nf = 0, kl = 0, ku = 0, farc[kPlanFar];
     bool diag = false;
-    R.each(ci, cbase, [&](int c) {
-      if (c < lo || c >= hi) return;
-      if (c < i) {
-        ++nl;
-        if (c < base) L0 = max(L0, __ldcg(lev + c) + 1);
-      } else if (c > i) {
-        ++nu;
-      } else {
-        diag = true;
+    // f(walk position) for every in-block entry off the diagonal
+    auto entries = [&](int from, int to, int self, auto&& f) {
+      for (int j0 = from; j0 < to; j0 += kPlanBatch) {
+        int c[kPlanBatch];
+#pragma unroll
+        for (int e = 0; e < kPlanBatch; ++e) c[e] = j0 + e < to ? ci[j0 + e] - cbase : -1;
+#pragma unroll
+        for (int e = 0; e < kPlanBatch; ++e)
+          if (c[e] >= lo && c[e] < hi && c[e] != self) f(walk_of(c[e]));
       }
-    });
-    kmax = max(kmax, max(nl, nu));
-    missing |= on && !diag;
-    cur[t] = -1;
-    push[t] = L0;
-    __syncthreads();
-    int mine = -1;
-    int changed;
-    do {
-      changed = 0;
-      if (on) {
-        int L = *(volatile int*)&push[t];
-        R.each(ci, cbase, [&](int c) {
-          if (c >= base && c < i) L = max(L, cur[c - base] + 1);
-        });
-        if (L > mine) {
-          mine = L;
-          cur[t] = L;
-          changed = 1;
-          R.each(ci, cbase, [&](int c) {
-            if (c > i && c < hi && c < base + kPlanRows) atomicMax(&push[c - base], L + 1);
-          });
+    };
+    for (int j0 = a; j0 < z; j0 += kPlanBatch) {
+      int c[kPlanBatch], lv[kPlanBatch];
+#pragma unroll
+      for (int e = 0; e < kPlanBatch; ++e) c[e] = j0 + e < z ? ci[j0 + e] - cbase : -1;
+#pragma unroll
+      for (int e = 0; e < kPlanBatch; ++e) {
+        const bool done = c[e] >= lo && c[e] < hi && walk_of(c[e]) < base;
+        lv[e] = done ? __ldcg(val + c[e]) : -1;
+      }
+#pragma unroll
+      for (int e = 0; e < kPlanBatch; ++e) {
+        if (c[e] < lo || c[e] >= hi) continue;
+        if (c[e] == i) { diag = true; continue; }
+        const int v = walk_of(c[e]);
+        L0 = max(L0, lv[e] + 1);
+        if (v < u) {
+          ++kl;
+          if (v >= base) {
+            if (nb < kPlanList) before[nb][t] = (unsigned short)(v - base);
+            ++nb;
+          }
+        } else {
+          ++ku;
+          if (v < base + PR) {
+            if (na < kPlanList) after[na][t] = (unsigned short)(v - base);
+            ++na;
+          } else {
+#pragma unroll
+            for (int q = 0; q < kPlanFar; ++q)
+              if (q == nf) farc[q] = c[e];
+            ++nf;
+          }
         }
       }
-    } while (__syncthreads_or(changed));
+    }
+    kmax = max(kmax, max(kl, ku));
+    missing |= on && !diag;
+    const bool listed = nb <= kPlanList && na <= kPlanList;
+    cur[t] = -1;
+    push[t] = L0;
+    nbef[t] = listed ? nb : kPlanList + 1;
+    __syncthreads();
+    if (listed) {   // drop the couplings that the other row reads
+      int k = 0;
+      for (int e = 0; e < na; ++e) {
+        const int v = after[e][t], n = nbef[v];
+        bool seen = n > kPlanList;   // it reads its whole row
+        if (seen) {
+          seen = false;
+          entries(rp[row_of(base + v)] - rbase, rp[row_of(base + v) + 1] - rbase, -1, [&](int w) { seen |= w == u; });
+        } else {
+          for (int q = 0; q < n; ++q) seen |= before[q][v] == t;
+        }
+        if (!seen) after[k++][t] = (unsigned short)v;
+      }
+      na = k;
+    }
+    // how many rows before this one in the warp each wait for the one before them
+    bool link = false;
+    for (int e = 0; listed && e < nb; ++e) link |= before[e][t] == t - 1;
+    const int run = __clz(~(__ballot_sync(kFull, link && (t & 31) != 0) << (31 - (t & 31))));
+    const int longest = __reduce_max_sync(kFull, run);
+    int mine = -1, changed, left = rounds;
+    auto round = [&]() -> int {   // whole warps
+      int L = on ? max(mine, *(volatile int*)&push[t]) : -1;
+      if (listed) {
+        for (int e = 0; e < nb; ++e) L = max(L, cur[before[e][t]] + 1);
+      } else {
+        entries(a, z, i, [&](int v) { if (v >= base && v < u) L = max(L, cur[v - base] + 1); });
+      }
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        if (o > longest) break;   // the same in every lane
+        const int up = __shfl_up_sync(kFull, L, o);
+        if (o <= run) L = max(L, up + o);
+      }
+      if (!on || L <= mine) return 0;
+      mine = L;
+      cur[t] = L;
+      if (listed) {
+        for (int e = 0; e < na; ++e) atomicMax(&push[after[e][t]], L + 1);
+      } else {
+        entries(a, z, i, [&](int v) { if (v > u && v < base + PR) atomicMax(&push[v - base], L + 1); });
+      }
+      return 1;
+    };
+    do changed = __syncthreads_or(round()); while (changed && --left > 0);
+    rounds = changed ? kPlanRetry : kPlanRounds;
+    if (changed) {   // a long chain: the warps in order, each until its rows are final
+      for (int w = 0; w < PR / 32; ++w) {
+        if ((t >> 5) == w) {
+          int c;
+          do {
+            c = round();
+            __syncwarp();
+          } while (__any_sync(kFull, c));
+        }
+        __syncthreads();
+      }
+    }
     if (on) {
-      lev[i] = mine;
+      val[i] = mine;
       maxlev = max(maxlev, mine);
-      R.each(ci, cbase, [&](int c) {
-        if (c >= base + kPlanRows && c < hi) atomicMax(low + c, mine + 1);
-      });
+      atomicAdd(wid + lo + (LATE ? last - mine : mine), 1);
+      if (nf <= kPlanFar) {
+#pragma unroll
+        for (int q = 0; q < kPlanFar; ++q)
+          if (q < nf) atomicMax(far + farc[q], mine + 1);
+      } else {
+        entries(a, z, i, [&](int v) { if (v >= base + PR) atomicMax(far + row_of(v), mine + 1); });
+      }
     }
     __syncthreads();
   }
+  if (LATE) return;
   atomicMax(&s_max, maxlev);
   atomicMax(&s_kmax, kmax);
   if (missing) atomicMin(&stat->missing, b);
   __syncthreads();
-  maxlev = s_max;
-  // largest gap of a coupling; which rows have dependents
-  auto gap_of = [&](const int* lv) {
-    int g = 0;
-    for (int base = lo; base < hi; base += kPlanRows) {
-      const int i = base + t;
-      if (i >= hi) continue;
-      PlanRow R;
-      row_at(i, R);
-      const int L = __ldcg(lv + i);
-      R.each(ci, cbase, [&](int c) {
-        if (c < lo || c >= hi || c == i) return;
-        g = max(g, abs(__ldcg(lv + c) - L));
-        dep[min(c, i)] = 1;
-      });
-    }
-    __syncthreads();
-    if (t == 0) s_gap = 0;
-    __syncthreads();
-    atomicMax(&s_gap, g);
-    __syncthreads();
-    return s_gap;
-  };
-  int gap = gap_of(lev);
-  const int* use = lev;
-  const bool long_ring = (int64_t)(gap + 1) * (hi - lo) > kTightenRing * (int64_t)(maxlev + 1);
-  if (long_ring && t == 0) stat->long_ring = 1;
-  if (long_ring && tighten) {
-    // ---- late levels, from the last chunk back; they fall from the largest level
-    const int nch = (hi - lo + kPlanRows - 1) / kPlanRows;
-    for (int k = nch - 1; k >= 0; --k) {
-      const int base = lo + k * kPlanRows, i = base + t;
-      const bool on = i < hi;
-      PlanRow R;
-      row_at(i, R);
-      const bool has = on && *(volatile unsigned char*)(dep + i) != 0;
-      const int own = on ? __ldcg(lev + i) : 0;
-      int F = on ? __ldcg(first + i) : INT_MAX;
-      R.each(ci, cbase, [&](int c) {
-        if (c >= base + kPlanRows && c < hi) F = min(F, __ldcg(late + c));
-      });
-      cur[t] = has ? maxlev : own;
-      push[t] = F;
-      __syncthreads();
-      int mine = INT_MAX;
-      int changed;
-      do {
-        changed = 0;
-        if (on) {
-          int m = *(volatile int*)&push[t];
-          R.each(ci, cbase, [&](int c) {
-            if (c > i && c < hi && c < base + kPlanRows) m = min(m, cur[c - base]);
-          });
-          const int L = has ? m - 1 : own;
-          if (L < mine) {
-            mine = L;
-            cur[t] = L;
-            changed = 1;
-            R.each(ci, cbase, [&](int c) {
-              if (c >= base && c < i) atomicMin(&push[c - base], L);
-            });
-          }
-        }
-      } while (__syncthreads_or(changed));
-      if (on) {
-        late[i] = mine;
-        R.each(ci, cbase, [&](int c) {
-          if (c >= lo && c < base) atomicMin(first + c, mine);
-        });
-      }
-      __syncthreads();
-    }
-    const int g2 = gap_of(late);
-    if (g2 < gap) {
-      gap = g2;
-      use = late;
-    }
-  }
-  // level widths
-  for (int i = lo + t; i < hi; i += kPlanRows) {
-    const int L = __ldcg(use + i);
-    if (use != lev) lev[i] = L;
-    atomicAdd(wid + lo + L, 1);
-  }
   if (t == 0) {
-    nlev[b] = maxlev + 1;
-    atomicMax(&stat->gap, gap);
+    nlev[b] = s_max + 1;
     atomicMax(&stat->kmax, s_kmax);
   }
 }
 
-// Block b's level widths from wid (from its first row on) to width[blvl[b]..].
-__global__ void k_plan_widths(const int* __restrict__ starts, const int* __restrict__ blvl,
-                              const int* __restrict__ wid, int* __restrict__ width) {
-  const int b = blockIdx.x, l0 = blvl[b], n = blvl[b + 1] - l0;
-  for (int l = threadIdx.x; l < n; l += blockDim.x) width[l0 + l] = wid[starts[b] + l];
+__device__ __forceinline__ int plan_block(const int* __restrict__ starts, int nb, int i) {
+  int a = 0, z = nb - 1;   // the last block that starts at or before row i
+  while (a < z) {
+    const int mid = (a + z + 1) >> 1;
+    if (starts[mid] <= i) a = mid; else z = mid - 1;
+  }
+  return a;
 }
 
-// Positions: the rows of a level in natural order.  One warp per block takes 32 rows at a time;
-// rows of one level among them are ranked by lane, and next[level] is where the level goes on.
-__global__ void __launch_bounds__(32) k_plan_pos(const int* __restrict__ starts, const int* __restrict__ blvl,
-                                                 const int* __restrict__ lev, int* next, int* __restrict__ pos,
-                                                 int* __restrict__ rowAt) {
-  const int b = blockIdx.x, lane = threadIdx.x;
-  const int lo = starts[b], hi = starts[b + 1];
-  int* nx = next + blvl[b];
-  int L = lo + lane < hi ? lev[lo + lane] : -1;
-  for (int base = lo; base < hi; base += 32) {
+// Largest level difference of a coupling of each block (gap, zeroed); dep, if given: the rows
+// that have dependents.  only: the blocks that are loose by it (with nlev) are looked at.
+__global__ void k_plan_gap(int n, int nb, const int* __restrict__ starts, const int* __restrict__ rp,
+                           const int* __restrict__ ci, int rbase, int cbase, const int* __restrict__ val,
+                           int* gap, unsigned char* __restrict__ dep, const int* __restrict__ only,
+                           const int* __restrict__ nlev) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int b = plan_block(starts, nb, i), lo = starts[b], hi = starts[b + 1];
+    if (only && !plan_loose(only[b], hi - lo, nlev[b])) continue;
+    const int L = val[i];
+    int g = 0;
+    for (int j = rp[i] - rbase; j < rp[i + 1] - rbase; ++j) {
+      const int c = ci[j] - cbase;
+      if (c < lo || c >= hi || c == i) continue;
+      if (dep) dep[min(c, i)] = 1;
+      else g = max(g, abs(val[c] - L));
+    }
+    if (!dep && g > *(volatile int*)(gap + b)) atomicMax(gap + b, g);
+  }
+}
+
+// Blocks whose late levels have the smaller gap take them.
+__global__ void k_plan_take(int n, int nb, const int* __restrict__ starts, const int* __restrict__ gap,
+                            const int* __restrict__ gap_late, const int* __restrict__ nlev,
+                            const int* __restrict__ late, int* __restrict__ lev) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int b = plan_block(starts, nb, i);
+    if (plan_loose(gap[b], starts[b + 1] - starts[b], nlev[b]) && gap_late[b] < gap[b])
+      lev[i] = nlev[b] - 1 - late[i];
+  }
+}
+
+// Block b's level widths from wid (wid_late where its late levels are taken), from its first row
+// on, to width[blvl[b]..].
+__global__ void k_plan_widths(const int* __restrict__ starts, const int* __restrict__ blvl,
+                              const int* __restrict__ wid, const int* __restrict__ wid_late,
+                              const int* __restrict__ gap, const int* __restrict__ gap_late,
+                              int* __restrict__ width) {
+  const int b = blockIdx.x, lo = starts[b], l0 = blvl[b], n = blvl[b + 1] - l0;
+  const bool late = wid_late && plan_loose(gap[b], starts[b + 1] - lo, n) && gap_late[b] < gap[b];
+  for (int l = threadIdx.x; l < n; l += blockDim.x) width[l0 + l] = (late ? wid_late : wid)[lo + l];
+}
+
+// Positions: the rows of a level in natural order.  A segment is a run of one block's rows; its
+// counters, one per level of the block, end as the position where the segment's rows of the
+// level start: counted per segment, then summed over the segments of a block, level by level.
+struct PlanSeg {
+  int row0, row1;   // rows [row0, row1)
+  int64_t ctr;      // first counter
+};
+
+__global__ void k_plan_count(int nseg, const PlanSeg* __restrict__ seg, const int* __restrict__ lev, int* ctr) {
+  const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (s >= nseg) return;
+  const PlanSeg S = seg[s];
+  for (int i = S.row0 + lane; i < S.row1; i += 32) atomicAdd(ctr + S.ctr + lev[i], 1);
+}
+
+__global__ void k_plan_scan(int totlev, int nb, const int* __restrict__ blvl, const int* __restrict__ blk_seg,
+                            const PlanSeg* __restrict__ seg, const int* __restrict__ lst, int* __restrict__ ctr) {
+  const int gl = blockIdx.x * blockDim.x + threadIdx.x;
+  if (gl >= totlev) return;
+  const int b = plan_block(blvl, nb, gl), l = gl - blvl[b], nl = blvl[b + 1] - blvl[b];
+  const int s0 = blk_seg[b], ns = blk_seg[b + 1] - s0;
+  int* c = ctr + seg[s0].ctr + l;   // a block's segments have their counters one after another
+  int at = lst[gl];
+  for (int s = 0; s < ns; s += 8) {
+    int w[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) w[u] = s + u < ns ? c[(int64_t)(s + u) * nl] : 0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (s + u < ns) {
+        c[(int64_t)(s + u) * nl] = at;
+        at += w[u];
+      }
+  }
+}
+
+// One warp per segment takes 32 rows at a time; rows of one level among them are ranked by
+// lane, and the level's counter is where it goes on.
+__global__ void k_plan_pos(int nseg, const PlanSeg* __restrict__ seg, const int* __restrict__ lev, int* ctr,
+                           int* __restrict__ pos, int* __restrict__ rowAt) {
+  const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (s >= nseg) return;
+  const PlanSeg S = seg[s];
+  int* nx = ctr + S.ctr;
+  int L = S.row0 + lane < S.row1 ? lev[S.row0 + lane] : -1;
+  for (int base = S.row0; base < S.row1; base += 32) {
     const int i = base + lane;
-    const int Ln = i + 32 < hi ? lev[i + 32] : -1;   // on its way while this step runs
+    const int Ln = i + 32 < S.row1 ? lev[i + 32] : -1;   // on its way while this step runs
     const unsigned same = __match_any_sync(kFull, L);
     const int lead = __ffs(same) - 1, rank = __popc(same & ((1u << lane) - 1u));
     int at = 0;
-    if (lane == lead && L >= 0) {   // one lane per level, this warp alone on the block's counters
+    if (lane == lead && L >= 0) {   // one lane per level, this warp alone on the counters
       at = *(volatile int*)(nx + L);
       *(volatile int*)(nx + L) = at + __popc(same);
     }
@@ -319,6 +399,61 @@ __global__ void __launch_bounds__(32) k_plan_pos(const int* __restrict__ starts,
   }
 }
 
+static int row_grid(int n) { return std::max(1, std::min((n + 255) / 256, 8 * num_sms())); }
+
+template <bool LATE>
+static void plan_levels(const DevMat<double>& A, int nb, int max_rows, const int* starts, int* val, int* far, int* wid,
+                        const int* lev, const unsigned char* dep, const int* gap, int* nlev, PlanStat* stat) {
+  auto go = [&](auto kern, int pr) {
+    const size_t smem = sizeof(unsigned short) * 2 * kPlanList * pr;
+    PB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<nb, pr, smem, stream()>>>(starts, A.rowptr, A.col, A.rbase, A.cbase, val, far, wid, lev, dep, gap, nlev, stat);
+    PB_CUDA(cudaGetLastError());
+  };
+  // more than two blocks per SM: narrower CTAs, several to an SM
+  if (max_rows <= 256 || nb > 2 * num_sms()) go(k_plan_levels<LATE, 256>, 256);
+  else go(k_plan_levels<LATE, 1024>, 1024);
+}
+
+// pos and rowAt from the levels and their starts.
+static void plan_positions(int nb, const std::vector<int>& starts, const std::vector<int>& blk_lvl, const int* d_blvl,
+                           const int* d_lst, int totlev, const int* lev, int* pos, int* rowAt) {
+  cudaStream_t st = stream();
+  std::vector<PlanSeg> seg;
+  std::vector<int> blk_seg(nb + 1, 0);
+  seg.reserve(nb);
+  int64_t ctrs = 0;
+  for (int b = 0; b < nb; ++b) {
+    blk_seg[b] = (int)seg.size();
+    const int nl = blk_lvl[b + 1] - blk_lvl[b];
+    const int len = std::max(1024, nl);   // so there are never more counters than rows and levels together
+    for (int r = starts[b]; r < starts[b + 1]; r += len) {
+      seg.push_back(PlanSeg{r, std::min(r + len, starts[b + 1]), ctrs});
+      ctrs += nl;
+    }
+  }
+  blk_seg[nb] = (int)seg.size();
+  const int ns = (int)seg.size(), grid = (ns + 7) / 8;
+  DBuf dseg, ctr;
+  dseg.alloc(sizeof(PlanSeg) * seg.size(), false);
+  h2d(dseg.p, seg.data(), sizeof(PlanSeg) * seg.size());
+  ctr.alloc(sizeof(int) * (size_t)ctrs, ns > nb);
+  if (ns > nb) {
+    DBuf dbs;
+    dbs.alloc(sizeof(int) * blk_seg.size(), false);
+    h2d(dbs.p, blk_seg.data(), sizeof(int) * blk_seg.size());
+    k_plan_count<<<grid, 256, 0, st>>>(ns, dp<PlanSeg>(dseg), lev, dp<int>(ctr));
+    PB_CUDA(cudaGetLastError());
+    k_plan_scan<<<(totlev + 255) / 256, 256, 0, st>>>(totlev, nb, d_blvl, dp<int>(dbs), dp<PlanSeg>(dseg), d_lst,
+                                                      dp<int>(ctr));
+    PB_CUDA(cudaGetLastError());
+  } else {   // a segment per block: its counters are the level starts
+    d2d(ctr.p, d_lst, sizeof(int) * (size_t)totlev);
+  }
+  k_plan_pos<<<grid, 256, 0, st>>>(ns, dp<PlanSeg>(dseg), lev, dp<int>(ctr), pos, rowAt);
+  PB_CUDA(cudaGetLastError());
+}
+
 bool ilu_build_plan(const DevMat<double>& A, const BlockSplit& blocks, bool tighten, IluPlan& P, DBuf& pos,
                     DBuf& rowAt, DBuf& lev) {
   cudaStream_t st = stream();
@@ -328,35 +463,65 @@ bool ilu_build_plan(const DevMat<double>& A, const BlockSplit& blocks, bool tigh
   P.blk_lo.resize(nb);
   P.blk_hi.resize(nb);
   std::vector<int> starts(nb + 1, n);
+  int max_rows = 0;
   for (int b = 0; b < nb; ++b) {
     blocks.rows(b, n, &P.blk_lo[b], &P.blk_hi[b]);
     starts[b] = P.blk_lo[b];
+    max_rows = std::max(max_rows, P.blk_hi[b] - P.blk_lo[b]);
   }
   const size_t ib = sizeof(int) * (size_t)n;
-  DBuf dstarts(sizeof(int) * (nb + 1)), low(ib), dep(n), wid(ib), dnlev(sizeof(int) * nb), dstat(sizeof(PlanStat)),
-      first, late;
-  first.alloc(ib, false);
-  late.alloc(ib, false);
+  DBuf dstarts(sizeof(int) * (nb + 1)), far(ib), wid(ib), dnlev(sizeof(int) * nb), dgap(sizeof(int) * nb),
+      dstat(sizeof(PlanStat));
   lev.alloc(ib, false);
-  PB_CUDA(cudaMemsetAsync(first.p, 0x7f, ib, st));   // 0x7f7f7f7f: above every level
-  PlanStat h{0, 0, INT_MAX, 0};
+  PlanStat h{0, INT_MAX};
   h2d(dstarts.p, starts.data(), sizeof(int) * (nb + 1));
   h2d(dstat.p, &h, sizeof(h));
-  k_plan_levels<<<nb, kPlanRows, 0, st>>>(dp<int>(dstarts), A.rowptr, A.col, A.rbase, A.cbase, dp<int>(lev),
-                                          dp<int>(low), dp<int>(first), dp<int>(late), dp<unsigned char>(dep),
-                                          dp<int>(wid), dp<int>(dnlev), dp<PlanStat>(dstat), tighten);
+  plan_levels<false>(A, nb, max_rows, dp<int>(dstarts), dp<int>(lev), dp<int>(far), dp<int>(wid), nullptr, nullptr,
+                     nullptr, dp<int>(dnlev), dp<PlanStat>(dstat));
+  k_plan_gap<<<row_grid(n), 256, 0, st>>>(n, nb, dp<int>(dstarts), A.rowptr, A.col, A.rbase, A.cbase, dp<int>(lev),
+                                          dp<int>(dgap), nullptr, nullptr, nullptr);
   PB_CUDA(cudaGetLastError());
-  std::vector<int> nlev(nb);
+  std::vector<int> nlev(nb), gap(nb);
   PB_CUDA(cudaMemcpyAsync(nlev.data(), dnlev.p, sizeof(int) * nb, cudaMemcpyDeviceToHost, st));
+  PB_CUDA(cudaMemcpyAsync(gap.data(), dgap.p, sizeof(int) * nb, cudaMemcpyDeviceToHost, st));
   d2h(&h, dstat.p, sizeof(h));
   PB_CHECK(h.missing == INT_MAX, PARCEL_B_E_ZERO_PIVOT,
            "block-Jacobi block %d has a row without an in-block diagonal entry", h.missing);
+  bool loose = false, moved = false;
+  for (int b = 0; b < nb; ++b) loose |= plan_loose(gap[b], starts[b + 1] - starts[b], nlev[b]);
+  DBuf late, wid_late, gap_late;
+  if (loose && tighten) {
+    DBuf dep(n);
+    late.alloc(ib, false);
+    wid_late.alloc(ib);
+    gap_late.alloc(sizeof(int) * nb);
+    far.zero_fill();
+    k_plan_gap<<<row_grid(n), 256, 0, st>>>(n, nb, dp<int>(dstarts), A.rowptr, A.col, A.rbase, A.cbase, dp<int>(lev),
+                                            dp<int>(dgap), dp<unsigned char>(dep), dp<int>(dgap), dp<int>(dnlev));
+    PB_CUDA(cudaGetLastError());
+    plan_levels<true>(A, nb, max_rows, dp<int>(dstarts), dp<int>(late), dp<int>(far), dp<int>(wid_late), dp<int>(lev),
+                      dp<unsigned char>(dep), dp<int>(dgap), dp<int>(dnlev), nullptr);
+    k_plan_gap<<<row_grid(n), 256, 0, st>>>(n, nb, dp<int>(dstarts), A.rowptr, A.col, A.rbase, A.cbase, dp<int>(late),
+                                            dp<int>(gap_late), nullptr, dp<int>(dgap), dp<int>(dnlev));
+    PB_CUDA(cudaGetLastError());
+    k_plan_take<<<row_grid(n), 256, 0, st>>>(n, nb, dp<int>(dstarts), dp<int>(dgap), dp<int>(gap_late), dp<int>(dnlev),
+                                             dp<int>(late), dp<int>(lev));
+    PB_CUDA(cudaGetLastError());
+    std::vector<int> g2(nb);
+    d2h(g2.data(), gap_late.p, sizeof(int) * nb);
+    for (int b = 0; b < nb; ++b)
+      if (plan_loose(gap[b], starts[b + 1] - starts[b], nlev[b]) && g2[b] < gap[b]) {
+        gap[b] = g2[b];
+        moved = true;
+      }
+  }
   P.blk_lvl.assign(nb + 1, 0);
   for (int b = 0; b < nb; ++b) P.blk_lvl[b + 1] = P.blk_lvl[b] + nlev[b];
   const int totlev = P.blk_lvl[nb];
   DBuf dblvl(sizeof(int) * (nb + 1)), dwidth(sizeof(int) * std::max(totlev, 1));
   h2d(dblvl.p, P.blk_lvl.data(), sizeof(int) * (nb + 1));
-  k_plan_widths<<<nb, 256, 0, st>>>(dp<int>(dstarts), dp<int>(dblvl), dp<int>(wid), dp<int>(dwidth));
+  k_plan_widths<<<nb, 256, 0, st>>>(dp<int>(dstarts), dp<int>(dblvl), dp<int>(wid), dp<int>(wid_late), dp<int>(dgap),
+                                    dp<int>(gap_late), dp<int>(dwidth));
   PB_CUDA(cudaGetLastError());
   std::vector<int> width(totlev);
   d2h(width.data(), dwidth.p, sizeof(int) * totlev);
@@ -366,8 +531,7 @@ bool ilu_build_plan(const DevMat<double>& A, const BlockSplit& blocks, bool tigh
   PB_CHECK(total <= INT_MAX - 3, PARCEL_B_E_ARG, "the permuted layout of %d rows exceeds 2^31 entries", n);
   P.lvl_start.resize(totlev);
   P.lvl_end.resize(totlev);
-  int cursor = 0, maxw = 0, maxl = 0;
-  for (int b = 0; b < nb; ++b) maxl = std::max(maxl, nlev[b]);
+  int cursor = 0, maxw = 0;
   for (int l = 0; l < totlev; ++l) {
     P.lvl_start[l] = cursor;
     P.lvl_end[l] = cursor + width[l];
@@ -376,19 +540,18 @@ bool ilu_build_plan(const DevMat<double>& A, const BlockSplit& blocks, bool tigh
   }
   P.np = (int)total;   // the last level is padded as well
   P.maxWp = align4(maxw);
-  P.max_levels = maxl;
+  P.max_levels = *std::max_element(nlev.begin(), nlev.end());
   P.kmax = h.kmax;
-  P.W = h.gap + 1;
+  P.W = *std::max_element(gap.begin(), gap.end()) + 1;
   pos.alloc(ib, false);
   rowAt.alloc(sizeof(int) * (size_t)P.np, false);
   PB_CUDA(cudaMemsetAsync(rowAt.p, 0xFF, sizeof(int) * (size_t)P.np, st));   // padding: -1
-  DBuf next(sizeof(int) * std::max(totlev, 1));
-  h2d(next.p, P.lvl_start.data(), sizeof(int) * totlev);
-  k_plan_pos<<<nb, 32, 0, st>>>(dp<int>(dstarts), dp<int>(dblvl), dp<int>(lev), dp<int>(next), dp<int>(pos),
-                                dp<int>(rowAt));
-  PB_CUDA(cudaGetLastError());
+  DBuf dlst(sizeof(int) * std::max(totlev, 1));
+  h2d(dlst.p, P.lvl_start.data(), sizeof(int) * totlev);
+  plan_positions(nb, starts, P.blk_lvl, dp<int>(dblvl), dp<int>(dlst), totlev, dp<int>(lev), dp<int>(pos),
+                 dp<int>(rowAt));
   sync();   // the temporaries above are released on return
-  return h.long_ring != 0;
+  return tighten ? moved : loose;
 }
 
 // The plan's chunks (a level split at kIluChunk rows), in block order; K couplings per row in
@@ -1668,24 +1831,40 @@ static int sweep_smem_budget() {
   return std::min(dev_smem, 220 * 1024);
 }
 
+// Couplings per row of the records: the matrix's largest number rounded up to a supported one.
+static int record_couplings(int kmax) {
+  for (int c : {1, 2, 3, 4, 6, 8})
+    if (kmax <= c) return c;
+  return kmax;
+}
+
+// Whether the grouped sweep takes plan P with kuni couplings per row and sweep, and its ring: the
+// last W levels or the largest block by position, whichever is smaller; its byte offsets are
+// 16-bit and two stages of a widest chunk must fit beside it.  elems: the zero slot included.
+static bool grp_fits(const IluPlan& P, int tsize, int kuni, RingMap& ring, int64_t& elems) {
+  if (kuni > 8) return false;
+  int max_span = 0;
+  for (int b = 0; b < P.nb; ++b)
+    max_span = std::max(max_span, align4(P.lvl_end[P.blk_lvl[b + 1] - 1]) - P.lvl_start[P.blk_lvl[b]]);
+  const int maxWp = std::max(4, P.maxWp);
+  const int64_t by_level = (int64_t)P.W * maxWp;
+  ring = by_level <= max_span ? RingMap{P.W, maxWp} : RingMap{0, 0};
+  elems = std::min<int64_t>(by_level, max_span) + 1;
+  const int64_t ring_alloc = (elems * tsize + 127) & ~int64_t(127);
+  const int64_t widest = kGrpHdr + align4(std::min(P.maxWp, kIluChunk)) * (int64_t)(rec_stride(tsize, true, kuni) + tsize) + 256;
+  return elems * tsize <= 65536 && 128 + ring_alloc + 2 * widest <= sweep_smem_budget();
+}
+
 // Lays out the grouped sweep of plan P (chunks ch, kuni couplings per row and sweep) if it fits:
-// ring, groups, stages and the producer tables.  The ring holds the last W levels or the
-// largest block by position, whichever is smaller; its byte offsets are 16-bit and two
-// stages of a widest chunk must fit beside it.
+// ring, groups, stages and the producer tables.
 template <class T>
 static bool grp_layout(const IluPlan& P, const std::vector<IluChunk>& ch, const std::vector<int>& blk_chunk, int kuni,
                        IluDev<T>& D, RingMap& ring) {
   const int budget = sweep_smem_budget();
   const int maxw = std::min(P.maxWp, kIluChunk);
-  int max_span = 0;
-  for (int b = 0; b < P.nb; ++b)
-    max_span = std::max(max_span, align4(P.lvl_end[P.blk_lvl[b + 1] - 1]) - P.lvl_start[P.blk_lvl[b]]);
-  const int64_t by_level = (int64_t)D.W * D.maxWp;
-  ring = by_level <= max_span ? RingMap{D.W, D.maxWp} : RingMap{0, 0};
-  const int64_t elems = std::min<int64_t>(by_level, max_span) + 1;
+  int64_t elems = 0;
+  if (!grp_fits(P, (int)sizeof(T), kuni, ring, elems)) return false;
   const int64_t ring_alloc = (elems * (int64_t)sizeof(T) + 127) & ~int64_t(127);
-  const int64_t widest = kGrpHdr + align4(maxw) * (int64_t)(rec_stride((int)sizeof(T), true, kuni) + sizeof(T)) + 256;
-  if (elems * (int64_t)sizeof(T) > 65536 || 128 + ring_alloc + 2 * widest > budget) return false;
   D.ring_elems = (int)elems;
   // consumer threads: one row per thread, as many warps as the widest chunk needs (chunks
   // have at most kIluChunk = 512 rows): every warp more lengthens the level barrier
@@ -2062,14 +2241,12 @@ int ilu_setup_device(const IluPlan& P, const DevMat<double>& A, int ilu_method,
   D.maxWp = std::max(4, P.maxWp);
   // every chunk carries the same number of coupled entries per row (the matrix-wide
   // maximum, rounded up to a supported count)
-  int kuni = P.kmax;
-  for (int c : {1, 2, 3, 4, 6, 8})
-    if (P.kmax <= c) { kuni = c; break; }
+  const int kuni = record_couplings(P.kmax);
   std::vector<int> blk_chunk;
   std::vector<IluChunk> ch = plan_chunks(P, kuni, blk_chunk);
   D.K = kuni;
   RingMap ring;
-  D.grp = kuni <= 8 && grp_layout<T>(P, ch, blk_chunk, kuni, D, ring);
+  D.grp = grp_layout<T>(P, ch, blk_chunk, kuni, D, ring);
   if (!D.grp) {
     // the general sweep: its ring holds the last W levels when they fit 64 KB
     const int budget = sweep_smem_budget();
@@ -2162,15 +2339,18 @@ int ilu_setup_device(const IluPlan& P, const DevMat<double>& A, int ilu_method,
 // ------------------------------------------------------------------ many small blocks, set-up
 // The wavefront plan of tens of thousands of small blocks, one thread per block walking its
 // rows in order; no per-chunk tables go out (64,000 boxes of 4^3: 28 ms with the plan and the
-// tables made on the host, 0.8 ms so).  A block's rows are few, so its thread's dependent loads (row pointer, column,
-// level: about 1.5 us a row) end after 0.1 to 1.5 ms whatever the number of blocks.
+// tables made on the host, 0.8 ms so).  A thread's dependent loads (row pointer, column, level)
+// take 1 to 2 us a row, so blocks of more than kSmallWalk rows get a CTA each (k_plan_levels):
+// 1,200 blocks of 1,000 rows 1.7 ms on the host, 4.9 ms walked by threads, 0.25 ms so.
+constexpr int kSmallWalk = 128;
+
 struct SmallStat {
-  int maxw, max_levels, kmax, span, missing;   // missing: a block without a diagonal entry, or INT_MAX
+  int maxw, max_levels, span;
 };
 
 __global__ void k_small_levels(int nb, const int* __restrict__ starts, const int* __restrict__ rp,
                                const int* __restrict__ ci, int rbase, int cbase, int* lev, int* low, int* wid,
-                               int* __restrict__ nlev, int* __restrict__ span, SmallStat* stat) {
+                               int* __restrict__ nlev, PlanStat* stat) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nb) return;
   const int lo = starts[b], hi = starts[b + 1];
@@ -2206,43 +2386,52 @@ __global__ void k_small_levels(int nb, const int* __restrict__ starts, const int
     maxlev = max(maxlev, L);
     kmax = max(kmax, max(nl, nu));
   }
+  nlev[b] = maxlev + 1;
+  atomicMax(&stat->kmax, kmax);
+  if (missing) atomicMin(&stat->missing, b);
+}
+
+// Every block's stretch of the layout, and the largest values.
+__global__ void k_small_spans(int nb, const int* __restrict__ starts, const int* __restrict__ wid,
+                              const int* __restrict__ nlev, int* __restrict__ span, SmallStat* stat) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= nb) return;
+  const int lo = starts[b], nl = nlev[b];
   int sp = 0, maxw = 0;
-  for (int l = 0; l <= maxlev; ++l) {
+  for (int l = 0; l < nl; ++l) {
     const int w = wid[lo + l];
     sp += (w + 3) & ~3;
     maxw = max(maxw, w);
   }
-  nlev[b] = maxlev + 1;
   span[b] = sp;
   atomicMax(&stat->maxw, maxw);
-  atomicMax(&stat->max_levels, maxlev + 1);
-  atomicMax(&stat->kmax, kmax);
+  atomicMax(&stat->max_levels, nl);
   atomicMax(&stat->span, sp);
-  if (missing) atomicMin(&stat->missing, b);
 }
 
-// Level ranges and positions (stable by row within a level), block by block.
+// Level ranges, block by block.
 __global__ void k_small_layout(int nb, const int* __restrict__ starts, const int* __restrict__ blvl,
                                const int* __restrict__ first, const int* __restrict__ span,
-                               const int* __restrict__ lev, int* wid, int* __restrict__ lst, int* __restrict__ lend,
-                               int* __restrict__ pos, int* __restrict__ rowAt, int2* __restrict__ box) {
+                               const int* __restrict__ wid, int* __restrict__ lst, int* __restrict__ lend,
+                               int2* __restrict__ box) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nb) return;
-  const int lo = starts[b], hi = starts[b + 1], l0 = blvl[b], nl = blvl[b + 1] - l0;
+  const int lo = starts[b], l0 = blvl[b], nl = blvl[b + 1] - l0;
   int cur = first[b];
   for (int l = 0; l < nl; ++l) {
     const int w = wid[lo + l];
     lst[l0 + l] = cur;
     lend[l0 + l] = cur + w;
-    wid[lo + l] = cur;   // from here on the level's next free position
     cur = (cur + w + 3) & ~3;
   }
-  for (int i = lo; i < hi; ++i) {
-    const int p = wid[lo + lev[i]]++;
-    pos[i] = p;
-    rowAt[p] = i;
-  }
   box[b] = make_int2(first[b], span[b]);
+}
+
+// One segment per block for k_plan_pos.
+__global__ void k_small_segs(int nb, const int* __restrict__ starts, const int* __restrict__ blvl,
+                             PlanSeg* __restrict__ seg) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b < nb) seg[b] = PlanSeg{starts[b], starts[b + 1], blvl[b]};
 }
 
 bool ilu_small_blocks(const BlockSplit& bs, int n) {
@@ -2267,13 +2456,23 @@ bool ilu_small_plan(const BlockSplit& bs, const DevMat<double>& A, SmallPlan& P)
   }
   P.starts.alloc(sizeof(int) * (nb + 1));
   h2d(P.starts.p, starts.data(), sizeof(int) * (nb + 1));
-  DBuf lev(sizeof(int) * n), low(sizeof(int) * n), wid(sizeof(int) * n), stat(sizeof(SmallStat)),
+  DBuf lev(sizeof(int) * n), low(sizeof(int) * n), wid(sizeof(int) * n), stat(sizeof(SmallStat)), pstat(sizeof(PlanStat)),
       nlev(sizeof(int) * (nb + 1)), span(sizeof(int) * (nb + 1)), first(sizeof(int) * (nb + 1));   // zero-filled
-  SmallStat h{0, 0, 0, 0, INT_MAX};
-  h2d(stat.p, &h, sizeof(h));
+  PlanStat ph{0, INT_MAX};
+  h2d(pstat.p, &ph, sizeof(ph));
   const int grid = (nb + 127) / 128;
-  k_small_levels<<<grid, 128, 0, st>>>(nb, dp<int>(P.starts), A.rowptr, A.col, A.rbase, A.cbase, dp<int>(lev),
-                                       dp<int>(low), dp<int>(wid), dp<int>(nlev), dp<int>(span), dp<SmallStat>(stat));
+  int max_rows = 0;
+  for (int b = 0; b < nb; ++b) max_rows = std::max(max_rows, starts[b + 1] - starts[b]);
+  if (max_rows <= kSmallWalk) {
+    k_small_levels<<<grid, 128, 0, st>>>(nb, dp<int>(P.starts), A.rowptr, A.col, A.rbase, A.cbase, dp<int>(lev),
+                                         dp<int>(low), dp<int>(wid), dp<int>(nlev), dp<PlanStat>(pstat));
+    PB_CUDA(cudaGetLastError());
+  } else {
+    plan_levels<false>(A, nb, max_rows, dp<int>(P.starts), dp<int>(lev), dp<int>(low), dp<int>(wid), nullptr, nullptr,
+                       nullptr, dp<int>(nlev), dp<PlanStat>(pstat));
+  }
+  k_small_spans<<<grid, 128, 0, st>>>(nb, dp<int>(P.starts), dp<int>(wid), dp<int>(nlev), dp<int>(span),
+                                      dp<SmallStat>(stat));
   PB_CUDA(cudaGetLastError());
   P.blvl.alloc(sizeof(int) * (nb + 1));
   size_t tmp_bytes = 0;
@@ -2282,18 +2481,20 @@ bool ilu_small_plan(const BlockSplit& bs, const DevMat<double>& A, SmallPlan& P)
   PB_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tmp_bytes, dp<int>(nlev), dp<int>(P.blvl), nb + 1, st));
   PB_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tmp_bytes, dp<int>(span), dp<int>(first), nb + 1, st));
   int totals[2];
+  SmallStat h;
   PB_CUDA(cudaMemcpyAsync(&h, stat.p, sizeof(h), cudaMemcpyDeviceToHost, st));
+  PB_CUDA(cudaMemcpyAsync(&ph, pstat.p, sizeof(ph), cudaMemcpyDeviceToHost, st));
   PB_CUDA(cudaMemcpyAsync(&totals[0], dp<int>(P.blvl) + nb, sizeof(int), cudaMemcpyDeviceToHost, st));
   PB_CUDA(cudaMemcpyAsync(&totals[1], dp<int>(first) + nb, sizeof(int), cudaMemcpyDeviceToHost, st));
   sync();
-  PB_CHECK(h.missing == INT_MAX, PARCEL_B_E_ZERO_PIVOT,
-           "block-Jacobi block %d has a row without an in-block diagonal entry", h.missing);
-  if (h.kmax > 8) return false;   // more couplings than the records hold
+  PB_CHECK(ph.missing == INT_MAX, PARCEL_B_E_ZERO_PIVOT,
+           "block-Jacobi block %d has a row without an in-block diagonal entry", ph.missing);
+  if (ph.kmax > 8) return false;   // more couplings than the records hold
   P.totlev = totals[0];
   P.np = totals[1];
   P.maxw = h.maxw;
   P.max_levels = h.max_levels;
-  P.kmax = h.kmax;
+  P.kmax = ph.kmax;
   P.span = h.span;
   P.lo.alloc(sizeof(int) * P.totlev);
   P.hi.alloc(sizeof(int) * P.totlev);
@@ -2302,8 +2503,16 @@ bool ilu_small_plan(const BlockSplit& bs, const DevMat<double>& A, SmallPlan& P)
   PB_CUDA(cudaMemsetAsync(P.rowAt.p, 0xFF, sizeof(int) * P.np, st));   // padding: -1
   P.box.alloc(sizeof(int2) * nb);
   k_small_layout<<<grid, 128, 0, st>>>(nb, dp<int>(P.starts), dp<int>(P.blvl), dp<int>(first), dp<int>(span),
-                                       dp<int>(lev), dp<int>(wid), dp<int>(P.lo), dp<int>(P.hi), dp<int>(P.pos),
-                                       dp<int>(P.rowAt), dp<int2>(P.box));
+                                       dp<int>(wid), dp<int>(P.lo), dp<int>(P.hi), dp<int2>(P.box));
+  PB_CUDA(cudaGetLastError());
+  DBuf seg, next;
+  seg.alloc(sizeof(PlanSeg) * nb, false);
+  next.alloc(sizeof(int) * P.totlev, false);
+  d2d(next.p, P.lo.p, sizeof(int) * P.totlev);
+  k_small_segs<<<grid, 128, 0, st>>>(nb, dp<int>(P.starts), dp<int>(P.blvl), dp<PlanSeg>(seg));
+  PB_CUDA(cudaGetLastError());
+  k_plan_pos<<<(nb + 7) / 8, 256, 0, st>>>(nb, dp<PlanSeg>(seg), dp<int>(lev), dp<int>(next), dp<int>(P.pos),
+                                          dp<int>(P.rowAt));
   PB_CUDA(cudaGetLastError());
   sync();   // the temporaries above are released on return
   return true;

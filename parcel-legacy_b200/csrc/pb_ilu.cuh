@@ -149,8 +149,9 @@ inline int ilu_factor_threads(int maxWp) { return std::min(256, std::max(32, (ma
 
 // Wavefront plan of the block-Jacobi blocks of the natural matrix A (device arrays).  pos and
 // lev (n entries) receive every row's permuted position and its level within its block, rowAt
-// (np entries) the row at every position, -1 for padding.  Returns whether the early levels of
-// a block make its sweep's ring too long; with tighten they are then moved later.
+// (np entries) the row at every position, -1 for padding.  With tighten, the early levels of a
+// block that make its sweep's ring too long are moved later where that shortens it; returns
+// whether any were (without: whether a block has such levels).
 bool ilu_build_plan(const DevMat<double>& A, const BlockSplit& blocks, bool tighten, IluPlan& P, DBuf& pos,
                     DBuf& rowAt, DBuf& lev);
 

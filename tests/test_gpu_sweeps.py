@@ -334,3 +334,91 @@ def test_dd_setup_of_many_small_blocks():
                    precon_thblock=4096)["stats"] for _ in range(5)]
     assert min(s["setup_s"] for s in st) < 1.25 * min(s["solve_s"] for s in st) / 8
 
+
+# ---- the wavefront plan -----------------------------------------------------------------------------
+def _from_pairs(n, r, c, seed):
+    """A diagonally dominant matrix with the given entries (r, c) and the diagonal, pattern as given."""
+    rng = np.random.default_rng(seed)
+    key = np.unique(np.concatenate([np.arange(n, dtype=np.int64) * (n + 1), np.asarray(r, np.int64) * n + np.asarray(c, np.int64)]))
+    r, c = key // n, key % n
+    v = rng.uniform(-1, 1, r.size)
+    cnt = np.bincount(r, minlength=n)
+    v[r == c] = 2.0 * cnt + np.bincount(c, minlength=n)
+    rp = np.concatenate([[0], np.cumsum(cnt)]) + 1
+    return problems.CRS(n=n, rowptr=rp.astype(np.int32), col=(c + 1).astype(np.int32), val=v)
+
+
+def _chain(n):
+    i = np.arange(n - 1)
+    return np.concatenate([i, i + 1]), np.concatenate([i + 1, i])
+
+
+@pytest.mark.parametrize("ilu", [0, 1])
+@pytest.mark.parametrize("n,blocks", [(130, 1), (1024, 1), (5000, 1), (5000, 3), (4000, 900)])
+def test_plan_of_chains(n, blocks, ilu):
+    """Tridiagonal blocks: every row its own level, more rounds than a chunk of rows is given."""
+    assert _apply_both(_from_pairs(n, *_chain(n), 1), ipreflag=2, ILU_method=ilu, precon_thblock=blocks) < 1e-11
+
+
+@pytest.mark.parametrize("chain", [False, True])
+@pytest.mark.parametrize("n,blocks", [(700, 1), (3000, 1), (6000, 4), (9000, 600), (60000, 1300)])
+def test_plan_of_one_sided_couplings(n, blocks, chain):
+    """Entries whose transposes are missing, near (same chunk of rows) and far, with and without a
+    chain through all rows; some rows with more near couplings than are listed."""
+    rng = np.random.default_rng(n)
+    r = rng.integers(0, n, 2 * n)
+    c = np.clip(r + rng.integers(-90, 91, 2 * n), 0, n - 1)
+    r2, c2 = rng.integers(0, n, n // 4), rng.integers(0, n, n // 4)
+    dense = rng.choice(n, max(1, n // 200), replace=False)
+    r3 = np.repeat(dense, 41)
+    c3 = np.clip(r3 + np.tile(np.arange(-20, 21), dense.size), 0, n - 1)
+    r, c = np.concatenate([r, r2, r3]), np.concatenate([c, c2, c3])
+    if chain:
+        a, b = _chain(n)
+        r, c = np.concatenate([r, a]), np.concatenate([c, b])
+    A = _from_pairs(n, r, c, 2)
+    for ilu in (0, 1):
+        assert _apply_both(A, ipreflag=2, ILU_method=ilu, precon_thblock=blocks) < 1e-11
+
+
+@pytest.mark.parametrize("ilu", [0, 1])
+def test_plan_moves_levels_along_a_chain(ilu):
+    """A chain of 6,000 rows and 3,000 rows between that could start at once but are coupled to its end:
+    late levels over chunks that need a round per row."""
+    n = 9000
+    link = np.concatenate([np.arange(3000), np.arange(6000, 9000)])
+    single = np.arange(3000, 6000)
+    end = 8999 - np.arange(3000) % 1500
+    r = np.concatenate([link[:-1], link[1:], single, end])
+    c = np.concatenate([link[1:], link[:-1], end, single])
+    assert _apply_both(_from_pairs(n, r, c, 3), ipreflag=2, ILU_method=ilu, precon_thblock=1) < 1e-11
+
+
+_TRACE = """
+import sys, numpy as np, torch
+sys.path[:0] = %r
+import test_gpu_sweeps as t
+from parcel_b import api, problems
+A = t._from_pairs(100000, *t._chain(100000), 1) if sys.argv[1] == "chain" else problems.poisson3d_reference(100, 100, 120)[0]
+rp, ci, va, b = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (A.rowptr, A.col, A.val, np.ones(A.n)))
+torch.cuda.synchronize()
+for _ in range(3):
+    api.solve(A, b, rowptr=rp, col=ci, val=va, solver=3, ipreflag=2, ILU_method=0, precon_thblock=int(sys.argv[2]), itrmax=1, rtolmax=1e-30)
+"""
+
+
+@pytest.mark.parametrize("matrix,blocks", [("chain", 1), ("grid", 1200)])
+def test_plan_takes_less_than_the_factorisation(matrix, blocks):
+    """One long chain, and 1,200 blocks of 1,000 rows: plans that took 1.4 and five times as long as
+    the factorisation when a round went to every row or a thread to every block."""
+    import os
+    import re
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    path = [here, os.path.join(here, "..", "parcel-legacy_b200"), os.path.join(here, "..", "oracle")]
+    out = subprocess.run([sys.executable, "-c", _TRACE % path, matrix, str(blocks)], capture_output=True, text=True,
+                         timeout=300, env=dict(os.environ, PARCEL_B_TRACE="1"))
+    assert out.returncode == 0, out.stderr[-2000:]
+    ms = lambda label: min(float(x) for x in re.findall(re.escape(label) + r"\s+([\d.]+) ms", out.stderr))
+    assert ms("setup: wavefront plan") < ms("ilu: factor" if blocks == 1 else "setup: ILU factor + pack")
