@@ -1838,6 +1838,12 @@ static int record_couplings(int kmax) {
   return kmax;
 }
 
+// The general sweep's ring of the last W levels, and the most it takes of shared memory.
+constexpr int64_t kGeneralRing = 64 * 1024;
+static int64_t general_ring_bytes(const IluPlan& P, int tsize) {
+  return ((int64_t)P.W * std::max(4, P.maxWp) + 1) * tsize;
+}
+
 // Whether the grouped sweep takes plan P with kuni couplings per row and sweep, and its ring: the
 // last W levels or the largest block by position, whichever is smaller; its byte offsets are
 // 16-bit and two stages of a widest chunk must fit beside it.  elems: the zero slot included.
@@ -1853,6 +1859,13 @@ static bool grp_fits(const IluPlan& P, int tsize, int kuni, RingMap& ring, int64
   const int64_t ring_alloc = (elems * tsize + 127) & ~int64_t(127);
   const int64_t widest = kGrpHdr + align4(std::min(P.maxWp, kIluChunk)) * (int64_t)(rec_stride(tsize, true, kuni) + tsize) + 256;
   return elems * tsize <= 65536 && 128 + ring_alloc + 2 * widest <= sweep_smem_budget();
+}
+
+int ilu_sweep_rank(const IluPlan& P, int tsize) {
+  RingMap ring;
+  int64_t elems;
+  if (grp_fits(P, tsize, record_couplings(P.kmax), ring, elems)) return 2;
+  return general_ring_bytes(P, tsize) <= kGeneralRing ? 1 : 0;
 }
 
 // Lays out the grouped sweep of plan P (chunks ch, kuni couplings per row and sweep) if it fits:
@@ -2248,10 +2261,10 @@ int ilu_setup_device(const IluPlan& P, const DevMat<double>& A, int ilu_method,
   RingMap ring;
   D.grp = grp_layout<T>(P, ch, blk_chunk, kuni, D, ring);
   if (!D.grp) {
-    // the general sweep: its ring holds the last W levels when they fit 64 KB
+    // the general sweep: its ring holds the last W levels when they fit
     const int budget = sweep_smem_budget();
-    const int64_t ring_bytes = ((int64_t)D.W * D.maxWp + 1) * (int64_t)sizeof(T);
-    D.ring = ring_bytes <= 64 * 1024;
+    const int64_t ring_bytes = general_ring_bytes(P, (int)sizeof(T));
+    D.ring = ring_bytes <= kGeneralRing;
     const int64_t ring_alloc = D.ring ? ((ring_bytes + 127) & ~int64_t(127)) : 0;
     // per-chunk records for the general sweep
     int64_t oF = 0, oB = 0;

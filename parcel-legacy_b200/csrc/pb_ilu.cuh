@@ -155,6 +155,10 @@ inline int ilu_factor_threads(int maxWp) { return std::min(256, std::max(32, (ma
 bool ilu_build_plan(const DevMat<double>& A, const BlockSplit& blocks, bool tighten, IluPlan& P, DBuf& pos,
                     DBuf& rowAt, DBuf& lev);
 
+// The sweep a plan gets for values of tsize bytes: 2 the grouped one, 1 the general one with its
+// ring in shared memory, 0 without.
+int ilu_sweep_rank(const IluPlan& P, int tsize);
+
 // Factorises (ILU(0)) or computes the D-ILU diagonal on the device and packs the sweep
 // data.  ilu_method: 0 ILU(0), 1 ILUD, 2 MLUD (define.f90:40-42).  Returns a status.
 template <class T>

@@ -180,10 +180,15 @@ void build_system(const Options& o, const parcel_b_crs& A, bool dev, System<T>& 
     }
     IluPlan P;
     // BiCGStab's recurrences amplify the order of a sum to 1e-3 of its residual history, so its
-    // vectors keep the early levels' order whatever order the sweep takes; the two copies per
-    // application are 6 of 60 us where levels are moved at all (97 x 89 x 83, 48 blocks)
+    // vectors keep the early levels' order whatever order the sweep takes.  A sweep in another
+    // order costs two copies per application (6 of 60 us on 97 x 89 x 83 in 48 blocks), so it is
+    // taken only where levels were moved and the sweep got a better form by it.
     const bool keep_order = o.solver == PARCEL_B_SOLVER_BICG;
-    const bool long_ring = ilu_build_plan(S.Anat, bs, !keep_order, P, S.pos, S.rowAt, S.lev);
+    const bool loose = ilu_build_plan(S.Anat, bs, !keep_order, P, S.pos, S.rowAt, S.lev);
+    IluPlan Q;
+    DBuf qpos, qrowAt, qlev;
+    const bool reorder = keep_order && loose && ilu_build_plan(S.Anat, bs, true, Q, qpos, qrowAt, qlev) &&
+                         ilu_sweep_rank(Q, sizeof(T)) > ilu_sweep_rank(P, sizeof(T));
     trace_mark("setup: wavefront plan");
     S.np = P.np;
     S.permuted = true;
@@ -193,12 +198,9 @@ void build_system(const Options& o, const parcel_b_crs& A, bool dev, System<T>& 
     S.A.nnz = A.nnz;
     build_sell<T>(S.Anat, P.np, dp<int>(S.rowAt), dp<int>(S.pos), S.Asell, S.A);
     trace_mark("setup: sliced ELLPACK");
-    if (keep_order && long_ring) {
-      IluPlan Q;
-      DBuf pos, rowAt, lev;
-      ilu_build_plan(S.Anat, bs, true, Q, pos, rowAt, lev);
-      ilu_setup_device<T>(Q, S.Anat, o.ilu_method, dp<int>(pos), dp<int>(rowAt), dp<int>(lev), S.M.ilu);
-      ilu_reorder<T>(S.M.ilu, dp<int>(rowAt), dp<int>(S.pos));
+    if (reorder) {
+      ilu_setup_device<T>(Q, S.Anat, o.ilu_method, dp<int>(qpos), dp<int>(qrowAt), dp<int>(qlev), S.M.ilu);
+      ilu_reorder<T>(S.M.ilu, dp<int>(qrowAt), dp<int>(S.pos));
     } else {
       ilu_setup_device<T>(P, S.Anat, o.ilu_method, dp<int>(S.pos), dp<int>(S.rowAt), dp<int>(S.lev), S.M.ilu);
     }

@@ -422,3 +422,44 @@ def test_plan_takes_less_than_the_factorisation(matrix, blocks):
     assert out.returncode == 0, out.stderr[-2000:]
     ms = lambda label: min(float(x) for x in re.findall(re.escape(label) + r"\s+([\d.]+) ms", out.stderr))
     assert ms("setup: wavefront plan") < ms("ilu: factor" if blocks == 1 else "setup: ILU factor + pack")
+
+
+# ---- BiCGStab on a sweep in another order than its vectors' --------------------------------------------
+@pytest.mark.parametrize("inner", [0, 1])
+@pytest.mark.parametrize("ilu", [0, 1])
+@pytest.mark.parametrize("N,blocks", [(31, 7), (41, 3), (33, 1)])
+def test_bicgstab_on_ragged_blocks(N, blocks, ilu, inner):
+    """Blocks of more than 2,048 rows that start inside a plane: their levels are moved for the sweep,
+    the vectors keep the early levels' order (33^3 in one block: nothing to move)."""
+    A = problems.convdiff3d_upwind(N)
+    pre = dict(ipreflag=2, ILU_method=ilu, precon_thblock=blocks)
+    b = problems.rhs_normal(A.n, N)
+    if inner:
+        res = api.solve(A, b, solver=2, itrmax=500, rtolmax=1e-11, inner_precision=1, inner_rtol=1e-4, max_refine=40, **pre)
+        xo, _, _, _ = oracle.solve(A, b, solver=2, itrmax=500, rtolmax=1e-12, **pre)
+        assert res["iret"] == 0 and res["stats"]["true_relres"] < 1e-11
+        # 1.1e-11 cond(A), cond(A) as below
+        assert np.linalg.norm(res["x"] - xo) < 1.1e-11 * 0.41 * (N + 1) ** 2 * np.linalg.norm(xo)
+        return
+    assert _apply_both(A, solver=2, **pre) < 1e-11
+    kw = dict(solver=2, itrmax=400, rtolmax=1e-9, **pre)
+    xo, ho, no, io = oracle.solve(A, b, **kw)
+    res = api.solve(A, b, **kw)
+    assert abs(res["niter"] - no) <= 1 and res["iret"] == io
+    k = min(5, len(ho))   # its recurrences amplify rounding: the first steps agree closely, then x does
+    assert (np.abs(res["reshistory"][:k] - ho[:k]) / ho[:k]).max() < 1e-9
+    # both residuals are below 1e-9 |b|, so x differs by at most 2e-9 cond(A), 4 (N + 1)^2 / pi^2
+    assert np.linalg.norm(res["x"] - xo) < 2e-9 * 0.41 * (N + 1) ** 2 * np.linalg.norm(xo)
+
+
+def test_bicgstab_sets_up_one_order_where_levels_do_not_move():
+    """One block of whole planes: its levels cannot move, so BiCGStab plans and factors once, as GMRES."""
+    import torch
+    A = problems.convdiff3d_upwind(64)
+    rp, ci, va, b = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (A.rowptr, A.col, A.val, np.ones(A.n)))
+    torch.cuda.synchronize()
+    t = {}
+    for solver in (2, 3):
+        kw = dict(solver=solver, ipreflag=2, ILU_method=1, precon_thblock=1, itrmax=1, rtolmax=1e-30)
+        t[solver] = min(api.solve(A, b, rowptr=rp, col=ci, val=va, **kw)["stats"]["setup_s"] for _ in range(6))
+    assert t[2] < 1.35 * t[3]
