@@ -554,11 +554,24 @@ bool ilu_build_plan(const DevMat<double>& A, const BlockSplit& blocks, bool tigh
   return tighten ? moved : loose;
 }
 
-// The plan's chunks (a level split at kIluChunk rows), in block order; K couplings per row in
+// Largest chunk, and the most consumer threads of the grouped sweep, for records of K couplings
+// of tsize bytes.  A thread holds two rows' operands.  With 512 consumers and the producer warp an
+// SM partition has five warps and a thread 96 registers, with 480 four warps and 128, with 352
+// three and 168.  At 96 the wide records spilled 172 to 1,164 bytes: 15-point stencil, 96^3 in 24
+// blocks (seven couplings, levels of up to 372 rows), 264 us per application, 168 at 128 registers
+// (178 before rows were staged ahead); double-double 13-point, 48 x 48 x 96 in 8 blocks (levels of
+// up to 540 rows), 20 iterations 14.5 ms at 96, 9.7 at 128, 8.9 at 168.  Narrower records fit 96
+// registers and keep the longer chunk.
+constexpr int grp_rows(int tsize, int K) {
+  if (tsize == 16 && K <= 6) return K > 4 ? 352 : (K > 2 ? 480 : kIluChunk);
+  return tsize == 8 && (K == 7 || K == 8) ? 480 : kIluChunk;
+}
+
+// The plan's chunks (a level split at `rows` rows), in block order; K couplings per row in
 // their records.  blk_chunk: nb + 1.
-static std::vector<IluChunk> plan_chunks(const IluPlan& P, int K, std::vector<int>& blk_chunk) {
+static std::vector<IluChunk> plan_chunks(const IluPlan& P, int rows, int K, std::vector<int>& blk_chunk) {
   size_t n = 0;
-  for (size_t l = 0; l < P.lvl_start.size(); ++l) n += (P.lvl_end[l] - P.lvl_start[l] + kIluChunk - 1) / kIluChunk;
+  for (size_t l = 0; l < P.lvl_start.size(); ++l) n += (P.lvl_end[l] - P.lvl_start[l] + rows - 1) / rows;
   std::vector<IluChunk> ch(n);
   blk_chunk.assign(P.nb + 1, 0);
   int c = 0;
@@ -566,10 +579,10 @@ static std::vector<IluChunk> plan_chunks(const IluPlan& P, int K, std::vector<in
     blk_chunk[b] = c;
     for (int gl = P.blk_lvl[b]; gl < P.blk_lvl[b + 1]; ++gl) {
       const int w = P.lvl_end[gl] - P.lvl_start[gl];
-      for (int o = 0; o < w; o += kIluChunk) {
+      for (int o = 0; o < w; o += rows) {
         IluChunk& C = ch[c++];
         C.start = P.lvl_start[gl] + o;
-        C.w = std::min(kIluChunk, w - o);
+        C.w = std::min(rows, w - o);
         C.wpad = align4(C.w);
         C.KL = C.KU = K;
         C.lvl = gl - P.blk_lvl[b];
@@ -1857,7 +1870,7 @@ static bool grp_fits(const IluPlan& P, int tsize, int kuni, RingMap& ring, int64
   ring = by_level <= max_span ? RingMap{P.W, maxWp} : RingMap{0, 0};
   elems = std::min<int64_t>(by_level, max_span) + 1;
   const int64_t ring_alloc = (elems * tsize + 127) & ~int64_t(127);
-  const int64_t widest = kGrpHdr + align4(std::min(P.maxWp, kIluChunk)) * (int64_t)(rec_stride(tsize, true, kuni) + tsize) + 256;
+  const int64_t widest = kGrpHdr + align4(std::min(P.maxWp, grp_rows(tsize, kuni))) * (int64_t)(rec_stride(tsize, true, kuni) + tsize) + 256;
   return elems * tsize <= 65536 && 128 + ring_alloc + 2 * widest <= sweep_smem_budget();
 }
 
@@ -1874,13 +1887,13 @@ template <class T>
 static bool grp_layout(const IluPlan& P, const std::vector<IluChunk>& ch, const std::vector<int>& blk_chunk, int kuni,
                        IluDev<T>& D, RingMap& ring) {
   const int budget = sweep_smem_budget();
-  const int maxw = std::min(P.maxWp, kIluChunk);
+  const int maxw = std::min(P.maxWp, grp_rows((int)sizeof(T), kuni));
   int64_t elems = 0;
   if (!grp_fits(P, (int)sizeof(T), kuni, ring, elems)) return false;
   const int64_t ring_alloc = (elems * (int64_t)sizeof(T) + 127) & ~int64_t(127);
   D.ring_elems = (int)elems;
-  // consumer threads: one row per thread, as many warps as the widest chunk needs (chunks
-  // have at most kIluChunk = 512 rows): every warp more lengthens the level barrier
+  // consumer threads: one row per thread, as many warps as the widest chunk needs: every warp more
+  // lengthens the level barrier
   D.nc = std::max(32, (maxw + 31) & ~31);
   // Groups of consecutive chunks of one block, each at most kGrpMax chunks and about a
   // quarter of the stage budget (a chunk larger than that forms a group of its own).
@@ -2256,7 +2269,7 @@ int ilu_setup_device(const IluPlan& P, const DevMat<double>& A, int ilu_method,
   // maximum, rounded up to a supported count)
   const int kuni = record_couplings(P.kmax);
   std::vector<int> blk_chunk;
-  std::vector<IluChunk> ch = plan_chunks(P, kuni, blk_chunk);
+  std::vector<IluChunk> ch = plan_chunks(P, grp_rows((int)sizeof(T), kuni), kuni, blk_chunk);
   D.K = kuni;
   RingMap ring;
   D.grp = grp_layout<T>(P, ch, blk_chunk, kuni, D, ring);
@@ -2658,7 +2671,7 @@ bool ilu_setup_dd(const IluPlan& P, const DevMat<double>& A, const double* al, c
   // several CTAs to an SM, is the better one
   if (kuni == 0 || P.nb >= 8 * num_sms()) return false;
   std::vector<int> blk_chunk;
-  const std::vector<IluChunk> ch = plan_chunks(P, kuni, blk_chunk);
+  const std::vector<IluChunk> ch = plan_chunks(P, grp_rows((int)sizeof(dd), kuni), kuni, blk_chunk);
   D.K = kuni;
   RingMap ring;
   if (!grp_layout<dd>(P, ch, blk_chunk, kuni, D, ring)) return false;
@@ -2708,7 +2721,7 @@ void ilu_apply_dd(const IluDev<dd>& D, const dd* r, dd* s, cudaStream_t st) {
 #define GRP_DD(KM_)                                                                                \
   case KM_:                                                                                        \
     if (D.nc <= 256) launch_grp<dd, true, KM_, 256>(D, g, st);                                     \
-    else launch_grp<dd, true, KM_, 512>(D, g, st);                                                 \
+    else launch_grp<dd, true, KM_, grp_rows(sizeof(dd), KM_)>(D, g, st);                           \
     break;
   switch (D.K) {
     GRP_DD(1) GRP_DD(2) GRP_DD(3) GRP_DD(4) GRP_DD(6)
@@ -2829,12 +2842,12 @@ static void ilu_sweep(const IluDev<T>& D, const T* r, T* s, T* accum, const int*
   }
   if (D.grp && !accum) {
     const GrpArgs<T> g = grp_args<T>(D, r, s, gate);
-    // 256 consumers leave each thread twice the registers of 512
+    // 256 consumers leave each thread twice the registers of 512 (grp_rows)
 #define GRP_C(KM_, MAXC_)                                                                          \
   if (D.dilu) launch_grp<T, true, KM_, MAXC_>(D, g, st); else launch_grp<T, false, KM_, MAXC_>(D, g, st);
 #define GRP(KM_)                                                                                   \
   case KM_:                                                                                        \
-    if (D.nc <= 256) { GRP_C(KM_, 256) } else { GRP_C(KM_, 512) }                                  \
+    if (D.nc <= 256) { GRP_C(KM_, 256) } else { GRP_C(KM_, grp_rows(sizeof(T), KM_)) }             \
     break;
     switch (D.K) {
       GRP(1) GRP(2) GRP(3) GRP(4) GRP(6) GRP(8)

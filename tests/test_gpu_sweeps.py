@@ -463,3 +463,46 @@ def test_bicgstab_sets_up_one_order_where_levels_do_not_move():
         kw = dict(solver=solver, ipreflag=2, ILU_method=1, precon_thblock=1, itrmax=1, rtolmax=1e-30)
         t[solver] = min(api.solve(A, b, rowptr=rp, col=ci, val=va, **kw)["stats"]["setup_s"] for _ in range(6))
     assert t[2] < 1.35 * t[3]
+
+
+# ---- records of many couplings on wide levels, and of one -----------------------------------------------
+def _stencil15(nx, ny, nz, corners=4):
+    """The 7-point stencil and the first `corners` pairs of cube corners: 3 + corners couplings each way."""
+    i = np.arange(nx * ny * nz).reshape(nz, ny, nx)
+    sh = [(0, 0, 1), (0, 1, 0), (1, 0, 0)] + [(1, 1, 1), (1, 1, -1), (1, -1, 1), (1, -1, -1)][4 - corners:]
+    cut = lambda d, n, up: slice(max(d, 0), n + min(d, 0)) if up else slice(max(-d, 0), n + min(-d, 0))
+    r = np.concatenate([i[cut(a, nz, 0), cut(b, ny, 0), cut(c, nx, 0)].ravel() for a, b, c in sh])
+    c = np.concatenate([i[cut(a, nz, 1), cut(b, ny, 1), cut(c, nx, 1)].ravel() for a, b, c in sh])
+    return _from_pairs(nx * ny * nz, np.concatenate([r, c]), np.concatenate([c, r]), 7)
+
+
+@pytest.mark.parametrize("dims,blocks,corners", [((96, 96, 8), 2, 4), ((140, 140, 4), 1, 4), ((140, 140, 4), 1, 2),
+                                                 ((200, 180, 5), 1, 4)])
+def test_many_couplings_on_wide_levels(dims, blocks, corners):
+    """Five to seven couplings on levels of 372 rows and of more than one chunk (480 rows of seven
+    couplings, 512 of fewer; in double-double 352 of five and six)."""
+    A = _stencil15(*dims, corners=corners)
+    pre = dict(ipreflag=2, precon_thblock=blocks)
+    for ilu in (0, 1):
+        assert _apply_both(A, ILU_method=ilu, **pre) < 1e-11
+    if corners == 2:
+        _dd_both(A, problems.rhs_normal(A.n, 5), solver=1, itrmax=6, rtolmax=1e-25, ILU_method=1, **pre)
+
+
+def _apply_ms(A, **pre):
+    import torch
+    rp, ci, va = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (A.rowptr, A.col, A.val))
+    torch.cuda.synchronize()
+    p, S, a, b = _lib.new_input(**pre), api.crs_struct(A, rp, ci, va), C.c_double(), C.c_double()
+    best = np.inf
+    for _ in range(5):
+        assert _lib.load().parcel_b_bench_kernels(C.byref(p), C.byref(S), 20, C.byref(a), C.byref(b)) == 0
+        best = min(best, b.value)
+    return best
+
+
+def test_many_couplings_on_wide_levels_stay_in_registers():
+    """Levels of 372 rows: eight couplings a row cost 1.2 times as much as six when a thread's two rows are
+    in registers, twice as much when they spill."""
+    pre = dict(solver=3, ipreflag=2, ILU_method=0, precon_thblock=24)
+    assert _apply_ms(_stencil15(96, 96, 96), **pre) < 1.6 * _apply_ms(_stencil15(96, 96, 96, corners=3), **pre)
