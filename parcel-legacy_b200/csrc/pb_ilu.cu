@@ -1492,9 +1492,10 @@ __global__ void k_ilu_small_pack(int n, int nb, const int* __restrict__ blk_lo, 
     inblock_range(rp, ci, rbase, cbase, i, blk_lo[a], blk_hi[a], &ia, &iz, &idg);
     const int64_t p = pos[i];
     // entry k of a sweep's record: permuted column (unstaged records) or position in the
-    // block's stretch (staged ones), -1 and 0xffff for none
+    // block's stretch (staged ones; 32 bits where it is the only one), -1 and 0xffff for none
     auto put = [&](int* c, unsigned short* h, int k, int q) {
-      if (h) h[p * KC + k] = q < 0 ? (unsigned short)0xffff : (unsigned short)(q - box[a].x);
+      if (h && K == 1) reinterpret_cast<int*>(h)[p] = q < 0 ? -1 : q - box[a].x;
+      else if (h) h[p * KC + k] = q < 0 ? (unsigned short)0xffff : (unsigned short)(q - box[a].x);
       else c[p * K + k] = q;
     };
     int k = 0;
@@ -1636,10 +1637,14 @@ k_ilu_small(int nb, const int* __restrict__ blvl, const int* __restrict__ lo, co
 // in flight on an SM, which is what the sweep waits on.  Same records, same expressions, same
 // order as k_ilu_small.
 // The staged records hold a coupling as its 16-bit position in the stretch, a row's entries
-// padded to a multiple of four (small_kc): 8 bytes of indices per row and sweep instead of 12
-// for a 7-point stencil, read in one load, and a 4^3 box takes 3.9 KB instead of 4.3.
+// padded to two or a multiple of four (small_kc): 8 bytes of indices per row and sweep instead of
+// 12 for a 7-point stencil, read in one load, and a 4^3 box takes 3.9 KB instead of 4.3.  One coupling,
+// as in lines of a grid, is 32 bits as it stands: the same 4 bytes as two positions, and a level
+// does not wait for them to be unpacked.  64,000 lines of 64 rows, ILU(0) / D-ILU: 589 / 435 us per
+// application (598 / 443 with 32-bit columns; 653 / 562 with one position padded to four, which
+// also leaves room for fewer blocks on an SM; 665 / 486 padded to two).
 constexpr int kStageWarps = 4;
-__host__ __device__ constexpr int small_kc(int K) { return (K + 3) & ~3; }
+__host__ __device__ constexpr int small_kc(int K) { return K <= 2 ? 2 : (K + 3) & ~3; }
 constexpr int kStageBoxBytes = 12 * 1024;
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
@@ -1656,15 +1661,29 @@ __device__ __forceinline__ void group_stage(void* dst, const void* src, int byte
   for (int o = li * 16; o < bytes; o += lanes * 16) cp_async16(d + o, g + o);
 }
 
-template <int KC>
-__device__ __forceinline__ void small_cols16(unsigned short (&c)[KC], const unsigned short* p) {
+// The positions of row q's K couplings, negative for none.
+template <int K>
+__device__ __forceinline__ void small_at(int (&c)[K], const unsigned short* Cc, int q) {
+  if constexpr (K == 1) {
+    c[0] = reinterpret_cast<const int*>(Cc)[q];
+  } else {
+    constexpr int KC = small_kc(K), W = KC / 2;
+    unsigned w[W];
+    if constexpr (KC == 2) {
+      w[0] = reinterpret_cast<const unsigned*>(Cc)[q];
+    } else {
 #pragma unroll
-  for (int k = 0; k < KC; k += 4) {
-    const uint2 v = *reinterpret_cast<const uint2*>(p + k);
-    c[k] = (unsigned short)(v.x & 0xffffu);
-    c[k + 1] = (unsigned short)(v.x >> 16);
-    c[k + 2] = (unsigned short)(v.y & 0xffffu);
-    c[k + 3] = (unsigned short)(v.y >> 16);
+      for (int k = 0; k < W; k += 2) {
+        const uint2 v = *reinterpret_cast<const uint2*>(Cc + q * KC + 2 * k);
+        w[k] = v.x;
+        w[k + 1] = v.y;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const unsigned h = (k & 1) ? w[k / 2] >> 16 : w[k / 2] & 0xffffu;
+      c[k] = h == 0xffffu ? -1 : (int)h;
+    }
   }
 }
 
@@ -1759,11 +1778,11 @@ k_ilu_small_staged(int nb, const int2* __restrict__ box, const int* __restrict__
         const int e = Hi[t];
         for (int q = Lo[t] + li; q < e; q += LPB) {
           T acc = X[q];
-          unsigned short cc[KC];
-          small_cols16<KC>(cc, Cc + q * KC);
+          int cc[K];
+          small_at<K>(cc, Cc, q);
 #pragma unroll
           for (int k = 0; k < K; ++k)
-            if (cc[k] != 0xffff) acc = acc - V[q * K + k] * X[cc[k]];
+            if (cc[k] >= 0) acc = acc - V[q * K + k] * X[cc[k]];
           X[q] = DILU ? Fd[q] * acc : acc;
         }
       }
@@ -1795,11 +1814,11 @@ k_ilu_small_staged(int nb, const int2* __restrict__ box, const int* __restrict__
         for (int q = Lo[tl] + li; q < e; q += LPB) {
           const T xp = X[q], d = Bd[q];
           T acc = DILU ? T(0) : xp;
-          unsigned short cc[KC];
-          small_cols16<KC>(cc, Cc + q * KC);
+          int cc[K];
+          small_at<K>(cc, Cc, q);
 #pragma unroll
           for (int k = 0; k < K; ++k) {
-            if (cc[k] != 0xffff) {
+            if (cc[k] >= 0) {
               if (DILU) acc = acc + X[cc[k]] * V[q * K + k];
               else acc = acc - X[cc[k]] * V[q * K + k];
             }
