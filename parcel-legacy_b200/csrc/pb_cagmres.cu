@@ -728,6 +728,7 @@ SolveOut solve_cagmres(const Options& o, System<double>& S, const double* b_nat,
   Dev D;
   D.part.alloc(sizeof(double) * (size_t)tsgemm_blocks() * kTsMaxPQ);
   D.out.alloc(sizeof(double) * kTsMaxPQ);
+  ilu_clear_error<double>(S.M.ilu, o.fail_sweep);
   sync();
   if (setup_t) *setup_t = now_s();
 
@@ -751,7 +752,7 @@ SolveOut solve_cagmres(const Options& o, System<double>& S, const double* b_nat,
     const double rnorm0 = std::sqrt(dot(r, r));
     launches += 2;
     if (rnorm0 < o.abstol || rnorm0 / bnorm < o.rtol) break;
-    if (rnorm0 != rnorm0) { SolveOut so; so.niter = itr; so.iret = PARCEL_B_E_BREAKDOWN; return so; }
+    if (rnorm0 != rnorm0) { ilu_check_error<double>(S.M.ilu); SolveOut so; so.niter = itr; so.iret = PARCEL_B_E_BREAKDOWN; return so; }
     if (itr == 1) hist[0] = rnorm0 / bnorm;
     ze[0] = -rnorm0;
     lincomb<double>(np, V, r, cimm(-1.0 / rnorm0), nullptr, cimm(0), nullptr, cimm(0), nullptr, st);
@@ -839,6 +840,7 @@ SolveOut solve_cagmres(const Options& o, System<double>& S, const double* b_nat,
   }
   if (S.permuted) gather_perm<double>(S.n, x_nat, x, dp<int>(S.pos), st);
   sync();
+  ilu_check_error<double>(S.M.ilu);
   SolveOut so;
   so.niter = std::min(o.itrmax, itr0);
   so.iret = (o.itrmax <= itr) ? 1 : 0;

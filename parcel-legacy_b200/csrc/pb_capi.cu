@@ -461,6 +461,7 @@ int parcel_b_precon_apply(const parcel_b_input* prm, const parcel_b_crs* A, cons
     double* sp = s;
     if (!sdev) { sown.alloc(sizeof(double) * n); sp = dp<double>(sown); }
     cudaStream_t st = stream();
+    ilu_clear_error<double>(S.M.ilu, o.fail_sweep);
     if (S.permuted) {
       DBuf rp(sizeof(double) * S.np), spp(sizeof(double) * S.np);
       PB_CUDA(cudaMemsetAsync(rp.p, 0, sizeof(double) * S.np, st));
@@ -471,9 +472,7 @@ int parcel_b_precon_apply(const parcel_b_input* prm, const parcel_b_crs* A, cons
     } else {
       S.M.apply(n, rv.p, sp, nullptr, st);
     }
-    int err = 0;
-    if (S.permuted) d2h(&err, S.M.ilu.err.p, sizeof(int));
-    PB_CHECK(err == 0, PARCEL_B_E_CUDA, "ILU sweep kernel reported wait timeout %d", err);
+    ilu_check_error<double>(S.M.ilu);
     if (!sdev) d2h(s, sp, sizeof(double) * n);
     sync();
     return 0;

@@ -113,7 +113,8 @@ struct KState {
   int stop_after_update;                   // GMRES: exit the solve after update_xVec
   int last_inner;                          // GMRES: Fortran `inner` after the last cycle
   int itrmax;                              // iteration limit of this solve
-  int pad[4];
+  int sweep_err;                           // the block-Jacobi sweeps' error flag, copied at the end
+  int pad[3];
   __host__ __device__ int mm_prev_inner() const { return last_inner; }
 };
 

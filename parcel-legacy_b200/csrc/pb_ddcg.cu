@@ -1553,15 +1553,12 @@ int dd_krylov(int solver, const parcel_b_input* prm, const parcel_b_crs* A, cons
       h2d(dcst, h, sizeof(h));
     }
     const DdRun R{S, P, st, n, grid_for(n), dp<dd>(part), dcst, dcst + 1, dcst + 2};
+    ilu_clear_error<dd>(P.grp, o.fail_sweep);
     DdLoop L;
     if (solver == PARCEL_B_SOLVER_BICG) L = dd_bicg_loop(R, o, x, b, reshistory);
     else if (solver == PARCEL_B_SOLVER_GMRES) L = dd_gmres_loop(R, o, x, b, reshistory);
     else L = dd_cg_loop(R, o, x, b, reshistory);
-    if (P.grp.grp) {
-      int err = 0;
-      d2h(&err, P.grp.err.p, sizeof(int));
-      PB_CHECK(err == 0, PARCEL_B_E_CUDA, "dd D-ILU sweep reported wait timeout %d", err);
-    }
+    ilu_check_error<dd>(P.grp);
     used = L.used;
     ir = L.iret;
     auto store = [&](double* dst, const double* src) {

@@ -2828,6 +2828,26 @@ template void ilu_reorder<double>(IluDev<double>&, const int*, const int*);
 template void ilu_reorder<float>(IluDev<float>&, const int*, const int*);
 
 template <class T>
+void ilu_clear_error(const IluDev<T>& D, bool fail) {
+  if (D.err.p) PB_CUDA(cudaMemsetAsync(D.err.p, fail ? 1 : 0, sizeof(int), stream()));
+}
+void ilu_raise_error(int flag) {
+  PB_CHECK(flag == 0, PARCEL_B_E_CUDA, "block-Jacobi sweep gave up waiting (code %d)", flag);
+}
+template <class T>
+void ilu_check_error(const IluDev<T>& D) {
+  int flag = 0;
+  if (D.err.p) d2h(&flag, D.err.p, sizeof(int));
+  ilu_raise_error(flag);
+}
+template void ilu_clear_error<double>(const IluDev<double>&, bool);
+template void ilu_clear_error<float>(const IluDev<float>&, bool);
+template void ilu_clear_error<dd>(const IluDev<dd>&, bool);
+template void ilu_check_error<double>(const IluDev<double>&);
+template void ilu_check_error<float>(const IluDev<float>&);
+template void ilu_check_error<dd>(const IluDev<dd>&);
+
+template <class T>
 static void ilu_sweep(const IluDev<T>& D, const T* r, T* s, T* accum, const int* gate, cudaStream_t st);
 
 template <class T>

@@ -203,6 +203,15 @@ template <class T>
 bool ilu_apply_cg(const IluDev<T>& D, T* r, const T* q, const double* c, T* s, const Red& red, const int* gate,
                   cudaStream_t st);
 
+// The sweeps' error flag: a sweep whose bounded wait runs out sets it and leaves its output
+// incomplete.  Every call that runs sweeps clears it first (fail: sets it instead, as if one had
+// given up; tests only) and raises an error if it is set at the end.
+template <class T>
+void ilu_clear_error(const IluDev<T>& D, bool fail = false);
+void ilu_raise_error(int flag);
+template <class T>
+void ilu_check_error(const IluDev<T>& D);   // waits for the stream
+
 // Makes ilu_apply take and give vectors in another layout than the sweep's own order.
 template <class T>
 void ilu_reorder(IluDev<T>& D, const int* sweep_rowAt, const int* layout_pos);

@@ -128,12 +128,11 @@ int parcel_b_local_precon(parcel_b_local h, const double* r, double* z) {
     if (!L.has_precon) {
       d2d(z, r, sizeof(double) * L.n);
     } else if (L.S.permuted) {
+      ilu_clear_error<double>(L.S.M.ilu);
       scatter_perm<double>(L.n, dp<double>(L.rperm), r, dp<int>(L.S.pos), st);
       L.S.M.apply(L.S.np, dp<double>(L.rperm), dp<double>(L.zperm), nullptr, st);
       gather_perm<double>(L.n, z, dp<double>(L.zperm), dp<int>(L.S.pos), st);
-      int err = 0;
-      d2h(&err, L.S.M.ilu.err.p, sizeof(int));
-      PB_CHECK(err == 0, PARCEL_B_E_CUDA, "ILU sweep kernel reported wait timeout %d", err);
+      ilu_check_error<double>(L.S.M.ilu);
     } else {
       L.S.M.apply(L.n, r, z, nullptr, st);
     }

@@ -77,6 +77,7 @@ Options resolve_options(const parcel_b_input* p) {
   if (p->independ_nvec > 0) o.independ_nvec = p->independ_nvec;
   if (p->reserved[0] == 1) o.use_graphs = false;
   if (p->reserved[1] == 1) o.fused_mgs = false;
+  if (p->reserved[2] == 1) o.fail_sweep = true;
   return o;
 }
 
@@ -239,9 +240,13 @@ static int read_done(const KState* st, cudaStream_t s) {
   return *pinned;
 }
 
-static KState read_state(const KState* st) {
+// The state at the end of a solve; an error if a preconditioner sweep gave up.
+template <class T>
+static KState read_state(KState* st, const System<T>& S) {
   KState h;
+  if (S.M.ilu.err.p) d2d(&st->sweep_err, S.M.ilu.err.p, sizeof(int));
   d2h(&h, st, sizeof(KState));
+  ilu_raise_error(h.sweep_err);
   return h;
 }
 
@@ -289,7 +294,7 @@ static SolveOut run_pcg(const Options& o, const System<T>& S, const T* b, T* x, 
   auto finish = [&]() -> SolveOut {
     // x = alpha p + x   (pcg.f90:733)
     lincomb<T>(np, x, P, cdev(&K->alpha), x, cimm(1.0), nullptr, cimm(0), nullptr, st);
-    KState h = read_state(K);
+    KState h = read_state(K, S);
     SolveOut out;
     out.niter = h.niter;
     out.iret = h.iret;
@@ -410,7 +415,7 @@ static SolveOut run_bicg(const Options& o, const System<T>& S, const T* b, T* x,
     G.launch(iterations, o.use_graphs, st);
     launches += 8 * chunk;
   }
-  KState h = read_state(K);
+  KState h = read_state(K, S);
   SolveOut out;
   out.niter = h.niter;
   out.iret = h.iret;
@@ -565,7 +570,7 @@ static SolveOut run_gmres(const Options& o, const System<T>& S, const T* b, T* x
     launches += per_cycle;
     if (o.on_cycle) (*o.on_cycle)(c);
   }
-  KState h = read_state(K);
+  KState h = read_state(K, S);
   int merr_h = 0;
   d2h(&merr_h, merr, sizeof(int));
   PB_CHECK(merr_h == 0, PARCEL_B_E_CUDA, "MGS grid barrier timed out");
@@ -582,6 +587,7 @@ SolveOut run_krylov(const Options& o, const System<T>& S, const T* b, T* x, doub
   KrylovWork own;
   KrylovWork& kw = keep ? *keep : own;
   kw.begin(&S, b, x, hist_dev);
+  ilu_clear_error<T>(S.M.ilu, o.fail_sweep);
   switch (o.solver) {
     case PARCEL_B_SOLVER_CG: return run_pcg<T>(o, S, b, x, hist_dev, kw);
     case PARCEL_B_SOLVER_BICG: return run_bicg<T>(o, S, b, x, hist_dev, kw);

@@ -32,6 +32,7 @@ struct Options {
   std::vector<int> block_starts;                       // explicit block-Jacobi blocks (BlockSplit)
   bool use_graphs = true;
   bool fused_mgs = true;
+  bool fail_sweep = false;                             // tests: the sweeps' error flag starts set
   bool flexible = false;                               // GMRES: flexible variant (keeps M^-1 v_j)
   const std::function<void(int)>* on_cycle = nullptr;  // GMRES: called after each restart cycle
 };

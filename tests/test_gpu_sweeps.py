@@ -514,3 +514,44 @@ def test_lines_as_blocks_keep_their_shared_memory():
     A = problems.poisson3d_reference(64, 64, 64)[0]
     pre = dict(solver=1, ipreflag=2, precon_thblock=4096)
     assert _apply_ms(A, ILU_method=1, **pre) < 0.8 * _apply_ms(A, ILU_method=0, **pre)
+
+
+# ---- a sweep that gives up --------------------------------------------------------------------------
+_FAIL = (C.c_int * 7)(0, 0, 1)   # the sweeps' error flag starts set, as if a bounded wait had run out
+
+
+@pytest.mark.parametrize("blocks", [3, 1200])
+@pytest.mark.parametrize("kw", [dict(solver=1), dict(solver=2), dict(solver=3), dict(solver=3, GMRES_GSflag=2),
+                                dict(solver=4, CAGMRES_sstep=4, CAGMRES_tstep=4),
+                                dict(solver=1, inner_precision=1), dict(solver=3, inner_precision=1)])
+def test_solves_report_a_sweep_that_gave_up(kw, blocks):
+    A = problems.poisson3d_reference(14, 14, 14)[0]
+    b = problems.rhs_normal(A.n, 2)
+    kw = dict(kw, ipreflag=2, ILU_method=1, precon_thblock=blocks, itrmax=500, rtolmax=1e-6)
+    with pytest.raises(RuntimeError, match="gave up waiting"):
+        api.solve(A, b, reserved=_FAIL, **kw)
+    assert api.solve(A, b, **kw)["iret"] == 0
+
+
+@pytest.mark.parametrize("solver", [1, 2, 3])
+def test_dd_solves_report_a_sweep_that_gave_up(solver):
+    A = problems.poisson3d_reference(10, 10, 10)[0]
+    kw = dict(solver=solver, ipreflag=2, ILU_method=1, precon_thblock=3, itrmax=60, rtolmax=1e-6)
+    with pytest.raises(RuntimeError, match="gave up waiting"):
+        api.ddcg(A, problems.rhs_normal(A.n, 2), reserved=_FAIL, **kw)
+    assert api.ddcg(A, problems.rhs_normal(A.n, 2), **kw)["iret"] == 0
+
+
+def test_a_handle_reports_a_sweep_that_gave_up_in_every_start():
+    """parcel_b_start clears the flag at its start: the next one reports its own outcome alone."""
+    A = problems.poisson3d_reference(14, 14, 14)[0]
+    L, n, i, h = _lib.load(), C.c_int(), C.c_int(), C.c_void_p()
+    p = _lib.new_input(solver=3, ipreflag=2, ILU_method=0, precon_thblock=3, itrmax=60, rtolmax=1e-6, reserved=_FAIL)
+    S = api.crs_struct(A)
+    assert L.parcel_b_setup(C.byref(p), C.byref(S), C.byref(h)) == 0, _lib.last_error()
+    b, hist = problems.rhs_normal(A.n, 2), np.zeros(60)
+    for _ in range(2):
+        x = np.zeros(A.n)
+        assert L.parcel_b_start(h, b.ctypes.data, x.ctypes.data, hist.ctypes.data, C.byref(n), C.byref(i)) < 0
+        assert "gave up waiting" in _lib.last_error()
+    assert L.parcel_b_release(h) == 0
