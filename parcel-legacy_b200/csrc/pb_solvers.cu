@@ -586,7 +586,7 @@ template <class T>
 SolveOut run_krylov(const Options& o, const System<T>& S, const T* b, T* x, double* hist_dev, KrylovWork* keep) {
   KrylovWork own;
   KrylovWork& kw = keep ? *keep : own;
-  kw.begin(&S, b, x, hist_dev);
+  kw.begin(o, &S, S.extra, b, x, hist_dev);
   ilu_clear_error<T>(S.M.ilu, o.fail_sweep);
   switch (o.solver) {
     case PARCEL_B_SOLVER_CG: return run_pcg<T>(o, S, b, x, hist_dev, kw);

@@ -5,6 +5,7 @@
 #include <deque>
 #include <functional>
 #include <memory>
+#include <tuple>
 
 #include "pb_blas.cuh"
 #include "pb_ilu.cuh"
@@ -153,27 +154,36 @@ struct GraphRunner {
 // iteration.  A caller that solves on the same system, right-hand side and solution buffers
 // again (the corrections of a refinement loop) passes the same object each time: the vectors
 // stay and the graph is replayed (instantiating and destroying one of a 40-column cycle with
-// the learned stage took 7 ms a time).  Options other than itrmax must be the same.
+// the learned stage took 7 ms a time).  The graph and the buffers' sizes hang on the options too:
+// all but itrmax, which the device reads from KState, must be the same.
 struct KrylovWork {
   Workspace W;
   GraphRunner G;
   int per_cycle = 0;
   std::deque<DBuf> bufs;
   size_t next = 0;
-  const void* key[4] = {};
-  void begin(const void* S, const void* b, const void* x, const void* hist) {
-    const void* k[4] = {S, b, x, hist};
-    if (!key[0]) {
-      W.init();
-      memcpy(key, k, sizeof(key));
+  struct Key {
+    const void *S, *b, *x, *hist, *extra;
+    int solver, m, gs, flexible, fused_mgs, use_graphs;
+    double rtol, abstol;
+    auto tie() const {
+      return std::tie(S, b, x, hist, extra, solver, m, gs, flexible, fused_mgs, use_graphs, rtol, abstol);
     }
-    PB_CHECK(memcmp(key, k, sizeof(key)) == 0, PARCEL_B_E_ARG, "Krylov workspace used with other vectors");
+  } key{};
+  void begin(const Options& o, const void* S, const void* extra, const void* b, const void* x, const void* hist) {
+    const Key k{S, b, x, hist, extra, o.solver, o.m, o.gs, o.flexible, o.fused_mgs, o.use_graphs, o.rtol, o.abstol};
+    if (!key.S) {
+      W.init();
+      key = k;
+    }
+    PB_CHECK(key.tie() == k.tie(), PARCEL_B_E_ARG, "Krylov workspace used with other vectors or options");
     next = 0;
   }
   // The buffers are asked for in the same order every time; zero-filled when first allocated.
   template <class T>
   T* buf(size_t bytes) {
     if (next == bufs.size()) bufs.emplace_back(bytes);
+    PB_CHECK(bytes <= bufs[next].bytes, PARCEL_B_E_ARG, "Krylov workspace used with longer vectors");
     return dp<T>(bufs[next++]);
   }
 };
