@@ -891,9 +891,6 @@ struct RingMap {
   }
 };
 
-// Packs the group records of the grouped sweep (layout above): one CTA per group;
-// gi[g] = {first chunk, end chunk, sstart, sspan}, goff[g] = byte offsets of the forward
-// and backward records.
 // Sweep coefficients of the packed records: L and U entries by position in the natural
 // matrix, and the diagonal factors of row nat (diagonal entry jd).
 template <class T>
@@ -918,6 +915,9 @@ struct DdSrc {
 template <class T> __device__ __forceinline__ T pad_coef() { return T(0); }
 template <> __device__ __forceinline__ dd pad_coef<dd>() { return dd{1.0, 0.0}; }
 
+// Packs the group records of the grouped sweep (layout above): one CTA per group;
+// gi[g] = {first chunk, end chunk, sstart, sspan}, goff[g] = byte offsets of the forward
+// and backward records.
 template <class T, class Src>
 __global__ void k_ilu_pack_grp(const int4* __restrict__ gi, const int64_t* __restrict__ goff, int ngroups,
                                const IluChunk* __restrict__ ch, const int* __restrict__ blk_lo,
@@ -1020,7 +1020,6 @@ struct IluSolveArgs {
   const T* r;
   T* y;
   T* s;
-  T* accum;
   int W, maxWp, stage_bytes, nstages, ring_elems;
   const int* gate;
   int* err;
@@ -1439,7 +1438,6 @@ __global__ void __launch_bounds__(kIluThreads, 1) k_ilu_solve(IluSolveArgs<T> a)
             else out = acc * dg[p];
             if (RING) rslot[p] = out;
             vout[start + p] = out;
-            if (!fwd && a.accum) a.accum[start + p] += out;
           }
         }
         named_bar_sync(1, kIluConsumerThreads);
@@ -2848,25 +2846,24 @@ template void ilu_check_error<float>(const IluDev<float>&);
 template void ilu_check_error<dd>(const IluDev<dd>&);
 
 template <class T>
-static void ilu_sweep(const IluDev<T>& D, const T* r, T* s, T* accum, const int* gate, cudaStream_t st);
+static void ilu_sweep(const IluDev<T>& D, const T* r, T* s, const int* gate, cudaStream_t st);
 
 template <class T>
-void ilu_apply(const IluDev<T>& D, const T* r, T* s, T* accum, const int* gate, cudaStream_t st) {
+void ilu_apply(const IluDev<T>& D, const T* r, T* s, const int* gate, cudaStream_t st) {
   if (!D.perm.p) {
-    ilu_sweep<T>(D, r, s, accum, gate, st);
+    ilu_sweep<T>(D, r, s, gate, st);
     return;
   }
-  PB_CHECK(!accum, PARCEL_B_E_UNSUPPORTED, "accumulating block-Jacobi apply on a reordered sweep");
   const int grid = std::max(1, std::min((D.np + 255) / 256, 8 * num_sms()));
   k_to_sweep<T><<<grid, 256, 0, st>>>(D.np, dp<int>(D.perm), r, dp<T>(D.rq), gate);
-  ilu_sweep<T>(D, dp<T>(D.rq), dp<T>(D.sq), nullptr, gate, st);
+  ilu_sweep<T>(D, dp<T>(D.rq), dp<T>(D.sq), gate, st);
   k_from_sweep<T><<<grid, 256, 0, st>>>(D.np, dp<int>(D.perm), dp<T>(D.sq), s, gate);
   PB_CUDA(cudaGetLastError());
 }
 
 template <class T>
-static void ilu_sweep(const IluDev<T>& D, const T* r, T* s, T* accum, const int* gate, cudaStream_t st) {
-  if (D.small && !accum) {
+static void ilu_sweep(const IluDev<T>& D, const T* r, T* s, const int* gate, cudaStream_t st) {
+  if (D.small) {
 #define SMALL(K_)                                                                                  \
   case K_:                                                                                         \
     if (D.dilu) launch_small<T, true, K_>(D, r, s, gate, st); else launch_small<T, false, K_>(D, r, s, gate, st); \
@@ -2879,7 +2876,7 @@ static void ilu_sweep(const IluDev<T>& D, const T* r, T* s, T* accum, const int*
     PB_CUDA(cudaGetLastError());
     return;
   }
-  if (D.grp && !accum) {
+  if (D.grp) {
     const GrpArgs<T> g = grp_args<T>(D, r, s, gate);
     // 256 consumers leave each thread twice the registers of 512 (grp_rows)
 #define GRP_C(KM_, MAXC_)                                                                          \
@@ -2897,7 +2894,6 @@ static void ilu_sweep(const IluDev<T>& D, const T* r, T* s, T* accum, const int*
     PB_CUDA(cudaGetLastError());
     return;
   }
-  PB_CHECK(!D.grp && !D.small, PARCEL_B_E_UNSUPPORTED, "accumulating block-Jacobi apply needs the general sweep");
   IluSolveArgs<T> a;
   a.tabF = dp<ProdDesc>(D.tabF);
   a.tabB = dp<ProdDesc>(D.tabB);
@@ -2907,7 +2903,6 @@ static void ilu_sweep(const IluDev<T>& D, const T* r, T* s, T* accum, const int*
   a.r = r;
   a.y = dp<T>(D.ytmp);
   a.s = s;
-  a.accum = accum;
   a.W = D.W;
   a.maxWp = D.maxWp;
   a.stage_bytes = D.stage_bytes;
@@ -2927,9 +2922,7 @@ template int ilu_setup_device<double>(const IluPlan&, const DevMat<double>&, int
                                       const int*, const int*, IluDev<double>&);
 template int ilu_setup_device<float>(const IluPlan&, const DevMat<double>&, int, const int*,
                                      const int*, const int*, IluDev<float>&);
-template void ilu_apply<double>(const IluDev<double>&, const double*, double*, double*,
-                                const int*, cudaStream_t);
-template void ilu_apply<float>(const IluDev<float>&, const float*, float*, float*, const int*,
-                               cudaStream_t);
+template void ilu_apply<double>(const IluDev<double>&, const double*, double*, const int*, cudaStream_t);
+template void ilu_apply<float>(const IluDev<float>&, const float*, float*, const int*, cudaStream_t);
 
 }  // namespace pb

@@ -216,9 +216,8 @@ void ilu_check_error(const IluDev<T>& D);   // waits for the stream
 template <class T>
 void ilu_reorder(IluDev<T>& D, const int* sweep_rowAt, const int* layout_pos);
 
-// s = M^-1 r on permuted vectors (np entries each).  If `accum` is non-null the result
-// is added into it instead of being written to s (s may then be null).
+// s = M^-1 r on permuted vectors (np entries each).
 template <class T>
-void ilu_apply(const IluDev<T>& D, const T* r, T* s, T* accum, const int* gate, cudaStream_t st);
+void ilu_apply(const IluDev<T>& D, const T* r, T* s, const int* gate, cudaStream_t st);
 
 }  // namespace pb

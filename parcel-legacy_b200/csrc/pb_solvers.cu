@@ -125,7 +125,7 @@ void Precon<T>::apply(int64_t np, const T* r, T* s, const int* gate, cudaStream_
       // the sweeps may read r over the whole padded iteration layout
       PB_CHECK(ilu.perm.p || np >= ilu.np, PARCEL_B_E_ARG, "vector of %lld entries, the iteration layout has %d", (long long)np,
                ilu.np);
-      ilu_apply<T>(ilu, r, s, nullptr, gate, st);
+      ilu_apply<T>(ilu, r, s, gate, st);
       break;
   }
 }
