@@ -110,7 +110,7 @@ typedef struct parcel_b_input {
   int residual_dd;        /* 1: outer residual b - A x in double-double            */
   double inner_rtol;      /* relative tolerance of each inner solve (FP32 path)     */
   int max_refine;         /* outer refinement steps (FP32 path)                     */
-  int reserved[7];
+  int reserved[7];        /* zero; 1 for tests: [0] no graphs, [1] separate MGS kernels, [2] the sweeps' error flag starts set */
 } parcel_b_input;
 
 /* Fills every field with -1 / defaults (INIT_PARCEL_INPUT, wrapper.f90:5-45). */

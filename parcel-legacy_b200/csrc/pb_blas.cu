@@ -78,7 +78,8 @@ __global__ void __launch_bounds__(kRedThreads, 4) k_lincomb_dot(int64_t n, T* __
 #pragma unroll
   for (int k = 0; k < ND; ++k) acc[k] = 0.0;
   // three elements per thread and step (a thread still visits its elements in increasing
-  // order): four CTAs of 256 threads per SM then fit the registers without spilling
+  // order): the loop of four CTAs of 256 threads per SM then fits the registers (the sums of the
+  // last block, reduce_and_finish, spill up to 24 bytes with one and with three products)
   constexpr int kUD = 3;
   const int64_t st = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += kUD * st) {

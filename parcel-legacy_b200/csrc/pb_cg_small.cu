@@ -30,6 +30,9 @@ constexpr int kCgThreads = 512;
 constexpr int kCgWarps = kCgThreads / 32;
 constexpr int kCgMaxElems = 4;             // rows per thread
 constexpr unsigned kCgWaitLimit = 1u << 21;
+// Up to this many CTAs read one another's words, beyond it CTA 0 hands the total back.  Five-point
+// stencil, us an iteration, read directly / through CTA 0: 16 CTAs 5.7 / 7.0, 32 5.7 / 6.8, 64 6.4 /
+// 6.8, 96 7.5 / 6.9, 128 8.6 / 6.8.
 constexpr int kCgDirect = 32;
 
 // Both words of a value in one access; each word is single-copy atomic by itself, and each

@@ -254,7 +254,8 @@ __device__ __forceinline__ bool reduce_block(double (&v)[K], const Red& r, doubl
 // and run the epilogue.  Every thread of the block must call it.  Deterministic for a fixed
 // grid size.  Warp k sums value k, a lane's loads (19 for four blocks on each of 148 SMs) all
 // in flight before the first is added: four at a time straight from L2 they took 3 of the 5 us
-// that a sum added to a short kernel.  (Staged in 5 KB of shared memory they were as fast, but
+// that a sum added to a short kernel.  (At 64 registers the 20 of them make the kernels of one
+// sum spill 4 to 24 bytes, once, in the last block.  Staged in 5 KB of shared memory they were as fast, but
 // the space came out of the L1 cache: a product on the diagonal copy went from 61 to 65 us at
 // 160^3.)
 template <int K>

@@ -94,8 +94,8 @@ void ilu_block_rows(int b, int nb, int n, int* lo, int* hi) {
 // a hundred levels later; with the levels taken as early as possible the ring of a
 // 12,000-row block of a 61 x 53 x 47 stencil would hold 58 levels, tightened it holds 2, as for
 // a block of whole planes, and the grouped sweep takes it instead of the general one, which
-// gathers coupled values from global memory: 119 -> 26 us per application there (16 blocks, in
-// a solve), 245 -> 53 us on 97 x 89 x 83 in 48 blocks.  The late levels are kept when they shorten
+// gathers coupled values from global memory: applications back to back 147 -> 33 us there (16
+// blocks; 119 -> 26 us inside a solve), 247 -> 53 us on 97 x 89 x 83 in 48 blocks.  The late levels are kept when they shorten
 // the gap, which in no case tried (400 grids of 5 to 27 points, 1 to 24 blocks) made the ring
 // longer.
 constexpr int kPlanRounds = 48;
@@ -1139,15 +1139,17 @@ __device__ __forceinline__ T gsolve(const GOps<T, KM>& c, const T (&dv)[KM], uin
 // Consumer side of one sweep over groups [g0, g0 + ng) of the sequence (NG groups over both
 // sweeps).  Per chunk: gather the coupled values from the ring, load the next chunk's
 // operands (through its descriptor, read one chunk earlier still) and finish the row, then
-// pass the level barrier.  What a level costs is the number of instructions a warp issues
-// between two barriers -- each waits about four cycles for the one before it -- so
+// pass the level barrier.  What a level costs is the instructions a warp issues between two
+// barriers: about 50 a warp and level, 317 cycles, 6.8 cycles each of which 1.9 wait for a fixed
+// latency, 1.5 for shared memory and 1.5 at the barrier (counters, 128^3 in 64 blocks).  So
 // descriptors come ready to add, the group's bookkeeping runs once per group and threads
 // without a row repeat the last one instead of branching around the work (a warp-uniform
-// branch per level cost 14 us of the 84 below).  Measured, 128^3 convection-diffusion, 64
-// blocks, 2 x 256 levels: 125 us with the descriptors and records read in one dependent chain
-// under predicates, 84 us so (118 -> 72 us in FP32; 160^3 D-ILU, 80 blocks, 170 -> 128 us;
-// four 1,024-row blocks of a 16^3 grid, 18.5 -> 10.8 us).  The level's own chain (gather 29
-// cycles, four dependent FMAs 36, store and barrier about 45) is half of what remains.  A
+// branch per level cost 14 us of the 86 below).  Measured, applications back to back, 128^3
+// convection-diffusion, 64 blocks, 2 x 256 levels: 126 us with the descriptors and records read in
+// one dependent chain under predicates, 86 us so (119 -> 70 us in FP32; 160^3 D-ILU, 80 blocks,
+// 170 -> 124 us; four 1,024-row blocks of a 16^3 grid, 18.5 -> 10.3 us); inside a solve, where the
+// vectors come from L2, 125 -> 77 us.  The level's own chain (gather 29 cycles, four dependent FMAs
+// 36, store and barrier about 45) is a third of what remains.  A
 // stage that never landed sets the abort flag; every consumer reads it after the barrier that follows a
 // stage wait, so all return together (`arrived` tells how far each released stages).
 template <class T, bool DILU, bool FWD, int KM>
