@@ -702,7 +702,6 @@ __global__ void k_dd_dilu_diag(const DdChunk* __restrict__ ch, const int* __rest
 // gathers of s_c, the dd chain and the stores remain.
 constexpr int kPre = 3;       // couplings per row held in the records
 constexpr int kRowsPer = 2;   // rows per thread staged ahead (levels of up to 512 rows)
-constexpr int kDdRingBytes = 160 * 1024;   // largest shared-memory ring of the sweep
 
 struct DdRecords {
   int np = 0;
@@ -1078,7 +1077,7 @@ void dd_setup_precon(const Options& o, const parcel_b_crs& A, const DdSystem& S,
   M.n = S.n; M.nnz = A.nnz; M.rowptr = S.rp; M.col = S.ci; M.val = S.ah; M.rbase = 1; M.cbase = S.cbase;
   IluPlan plan;
   DBuf dpos, dlev;
-  ilu_build_plan(M, block_split(o, A.n), true, plan, dpos, P.rowAt, dlev);
+  ilu_build_plan(M, block_split(o, A.n), Tighten::shorter, sizeof(dd), plan, dpos, P.rowAt, dlev);
   P.nb = plan.nb;
   DBuf blo(sizeof(int) * plan.nb), bhi(sizeof(int) * plan.nb), bof(sizeof(int) * A.n);
   h2d(blo.p, plan.blk_lo.data(), sizeof(int) * plan.nb);

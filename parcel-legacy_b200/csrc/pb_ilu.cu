@@ -60,6 +60,14 @@ void ilu_block_rows(int b, int nb, int n, int* lo, int* hi) {
   *hi = (int)h;
 }
 
+// How a plan's sweep runs for values of one size: 2 grouped, 1 general with its ring in shared
+// memory, 0 general without, -1 too wide for it; ring: entries of the grouped sweep's ring.
+struct SweepForm {
+  int rank;
+  int64_t ring;
+};
+static SweepForm sweep_form(const IluPlan& P, int tsize);
+
 // ------------------------------------------------------------------ wavefront plan
 // Levels: row x waits for every in-block row y < x coupled to it in either direction
 // (a lower entry of x, or an upper entry (y, x) of y), so one level order serves the
@@ -95,9 +103,10 @@ void ilu_block_rows(int b, int nb, int n, int* lo, int* hi) {
 // 12,000-row block of a 61 x 53 x 47 stencil would hold 58 levels, tightened it holds 2, as for
 // a block of whole planes, and the grouped sweep takes it instead of the general one, which
 // gathers coupled values from global memory: applications back to back 147 -> 33 us there (16
-// blocks; 119 -> 26 us inside a solve), 247 -> 53 us on 97 x 89 x 83 in 48 blocks.  The late levels are kept when they shorten
-// the gap, which in no case tried (400 grids of 5 to 27 points, 1 to 24 blocks) made the ring
-// longer.
+// blocks; 119 -> 26 us inside a solve), 247 -> 53 us on 97 x 89 x 83 in 48 blocks.  The late levels are kept where they get
+// the sweep a better form (sweep_form), or a grouped sweep a shorter ring: a shorter gap alone can
+// come with levels so wide that the ring is longer, or that no sweep takes them (rows all over a
+// chain whose only dependents are at its end move into one level).
 constexpr int kPlanRounds = 48;
 constexpr int kPlanRetry = 8;
 constexpr int kPlanList = 16;      // couplings of a row within its chunk, each way, that are listed
@@ -312,7 +321,7 @@ __global__ void k_plan_gap(int n, int nb, const int* __restrict__ starts, const 
   }
 }
 
-// Blocks whose late levels have the smaller gap take them.
+// Blocks whose late levels have the smaller gap take them (once the host has chosen that plan).
 __global__ void k_plan_take(int n, int nb, const int* __restrict__ starts, const int* __restrict__ gap,
                             const int* __restrict__ gap_late, const int* __restrict__ nlev,
                             const int* __restrict__ late, int* __restrict__ lev) {
@@ -454,8 +463,28 @@ static void plan_positions(int nb, const std::vector<int>& starts, const std::ve
   PB_CUDA(cudaGetLastError());
 }
 
-bool ilu_build_plan(const DevMat<double>& A, const BlockSplit& blocks, bool tighten, IluPlan& P, DBuf& pos,
-                    DBuf& rowAt, DBuf& lev) {
+// What depends on the levels' widths and gaps: level starts (multiples of 4, in block order) and the
+// sizes of ring and layout.
+static void plan_layout(IluPlan& P, const std::vector<int>& width, const std::vector<int>& gap) {
+  int64_t total = 0;
+  for (int w : width) total += align4(w);
+  PB_CHECK(total <= INT_MAX - 3, PARCEL_B_E_ARG, "the permuted layout of %d rows exceeds 2^31 entries", P.n);
+  P.lvl_start.resize(width.size());
+  P.lvl_end.resize(width.size());
+  int cursor = 0, maxw = 0;
+  for (size_t l = 0; l < width.size(); ++l) {
+    P.lvl_start[l] = cursor;
+    P.lvl_end[l] = cursor + width[l];
+    maxw = std::max(maxw, width[l]);
+    cursor = align4(cursor + width[l]);
+  }
+  P.np = (int)total;   // the last level is padded as well
+  P.maxWp = align4(maxw);
+  P.W = *std::max_element(gap.begin(), gap.end()) + 1;
+}
+
+bool ilu_build_plan(const DevMat<double>& A, const BlockSplit& blocks, Tighten tighten, int tsize, IluPlan& P,
+                    DBuf& pos, DBuf& rowAt, DBuf& lev) {
   cudaStream_t st = stream();
   const int n = A.n, nb = blocks.nb;
   P.n = n;
@@ -487,14 +516,27 @@ bool ilu_build_plan(const DevMat<double>& A, const BlockSplit& blocks, bool tigh
   d2h(&h, dstat.p, sizeof(h));
   PB_CHECK(h.missing == INT_MAX, PARCEL_B_E_ZERO_PIVOT,
            "block-Jacobi block %d has a row without an in-block diagonal entry", h.missing);
+  P.kmax = h.kmax;
+  P.max_levels = *std::max_element(nlev.begin(), nlev.end());
+  P.blk_lvl.assign(nb + 1, 0);
+  for (int b = 0; b < nb; ++b) P.blk_lvl[b + 1] = P.blk_lvl[b] + nlev[b];
+  const int totlev = P.blk_lvl[nb];
+  DBuf dblvl(sizeof(int) * (nb + 1)), dwidth(sizeof(int) * std::max(totlev, 1));
+  h2d(dblvl.p, P.blk_lvl.data(), sizeof(int) * (nb + 1));
+  std::vector<int> width(totlev);
+  auto widths = [&](const int* wid_late, const int* gap_late) {
+    k_plan_widths<<<nb, 256, 0, st>>>(dp<int>(dstarts), dp<int>(dblvl), dp<int>(wid), wid_late, dp<int>(dgap), gap_late,
+                                      dp<int>(dwidth));
+    PB_CUDA(cudaGetLastError());
+    d2h(width.data(), dwidth.p, sizeof(int) * totlev);
+  };
+  widths(nullptr, nullptr);
+  plan_layout(P, width, gap);
   bool loose = false, moved = false;
   for (int b = 0; b < nb; ++b) loose |= plan_loose(gap[b], starts[b + 1] - starts[b], nlev[b]);
-  DBuf late, wid_late, gap_late;
-  if (loose && tighten) {
-    DBuf dep(n);
+  if (loose && tighten != Tighten::no) {
+    DBuf dep(n), wid_late(ib), gap_late(sizeof(int) * nb), late;
     late.alloc(ib, false);
-    wid_late.alloc(ib);
-    gap_late.alloc(sizeof(int) * nb);
     far.zero_fill();
     k_plan_gap<<<row_grid(n), 256, 0, st>>>(n, nb, dp<int>(dstarts), A.rowptr, A.col, A.rbase, A.cbase, dp<int>(lev),
                                             dp<int>(dgap), dp<unsigned char>(dep), dp<int>(dgap), dp<int>(dnlev));
@@ -504,45 +546,28 @@ bool ilu_build_plan(const DevMat<double>& A, const BlockSplit& blocks, bool tigh
     k_plan_gap<<<row_grid(n), 256, 0, st>>>(n, nb, dp<int>(dstarts), A.rowptr, A.col, A.rbase, A.cbase, dp<int>(late),
                                             dp<int>(gap_late), nullptr, dp<int>(dgap), dp<int>(dnlev));
     PB_CUDA(cudaGetLastError());
-    k_plan_take<<<row_grid(n), 256, 0, st>>>(n, nb, dp<int>(dstarts), dp<int>(dgap), dp<int>(gap_late), dp<int>(dnlev),
-                                             dp<int>(late), dp<int>(lev));
-    PB_CUDA(cudaGetLastError());
     std::vector<int> g2(nb);
     d2h(g2.data(), gap_late.p, sizeof(int) * nb);
+    bool any = false;
     for (int b = 0; b < nb; ++b)
       if (plan_loose(gap[b], starts[b + 1] - starts[b], nlev[b]) && g2[b] < gap[b]) {
         gap[b] = g2[b];
-        moved = true;
+        any = true;
       }
+    if (any) {
+      IluPlan Q = P;
+      widths(dp<int>(wid_late), dp<int>(gap_late));
+      plan_layout(Q, width, gap);
+      const SweepForm f = sweep_form(P, tsize), g = sweep_form(Q, tsize);
+      moved = g.rank > f.rank || (tighten == Tighten::shorter && g.rank == 2 && f.rank == 2 && g.ring < f.ring);
+      if (moved) {
+        P = std::move(Q);
+        k_plan_take<<<row_grid(n), 256, 0, st>>>(n, nb, dp<int>(dstarts), dp<int>(dgap), dp<int>(gap_late),
+                                                 dp<int>(dnlev), dp<int>(late), dp<int>(lev));
+        PB_CUDA(cudaGetLastError());
+      }
+    }
   }
-  P.blk_lvl.assign(nb + 1, 0);
-  for (int b = 0; b < nb; ++b) P.blk_lvl[b + 1] = P.blk_lvl[b] + nlev[b];
-  const int totlev = P.blk_lvl[nb];
-  DBuf dblvl(sizeof(int) * (nb + 1)), dwidth(sizeof(int) * std::max(totlev, 1));
-  h2d(dblvl.p, P.blk_lvl.data(), sizeof(int) * (nb + 1));
-  k_plan_widths<<<nb, 256, 0, st>>>(dp<int>(dstarts), dp<int>(dblvl), dp<int>(wid), dp<int>(wid_late), dp<int>(dgap),
-                                    dp<int>(gap_late), dp<int>(dwidth));
-  PB_CUDA(cudaGetLastError());
-  std::vector<int> width(totlev);
-  d2h(width.data(), dwidth.p, sizeof(int) * totlev);
-  // level starts (multiples of 4), in block order
-  int64_t total = 0;
-  for (int w : width) total += align4(w);
-  PB_CHECK(total <= INT_MAX - 3, PARCEL_B_E_ARG, "the permuted layout of %d rows exceeds 2^31 entries", n);
-  P.lvl_start.resize(totlev);
-  P.lvl_end.resize(totlev);
-  int cursor = 0, maxw = 0;
-  for (int l = 0; l < totlev; ++l) {
-    P.lvl_start[l] = cursor;
-    P.lvl_end[l] = cursor + width[l];
-    maxw = std::max(maxw, width[l]);
-    cursor = align4(cursor + width[l]);
-  }
-  P.np = (int)total;   // the last level is padded as well
-  P.maxWp = align4(maxw);
-  P.max_levels = *std::max_element(nlev.begin(), nlev.end());
-  P.kmax = h.kmax;
-  P.W = *std::max_element(gap.begin(), gap.end()) + 1;
   pos.alloc(ib, false);
   rowAt.alloc(sizeof(int) * (size_t)P.np, false);
   PB_CUDA(cudaMemsetAsync(rowAt.p, 0xFF, sizeof(int) * (size_t)P.np, st));   // padding: -1
@@ -551,7 +576,7 @@ bool ilu_build_plan(const DevMat<double>& A, const BlockSplit& blocks, bool tigh
   plan_positions(nb, starts, P.blk_lvl, dp<int>(dblvl), dp<int>(dlst), totlev, dp<int>(lev), dp<int>(pos),
                  dp<int>(rowAt));
   sync();   // the temporaries above are released on return
-  return tighten ? moved : loose;
+  return tighten == Tighten::no ? loose : moved;
 }
 
 // Largest chunk, and the most consumer threads of the grouped sweep, for records of K couplings
@@ -1875,6 +1900,13 @@ constexpr int64_t kGeneralRing = 64 * 1024;
 static int64_t general_ring_bytes(const IluPlan& P, int tsize) {
   return ((int64_t)P.W * std::max(4, P.maxWp) + 1) * tsize;
 }
+// Shared memory of the general sweep with `stages` stages of a widest chunk.
+static int64_t general_smem(const IluPlan& P, int tsize, int K, bool ring, int stages) {
+  const int64_t ring_alloc = ring ? ((general_ring_bytes(P, tsize) + 127) & ~int64_t(127)) : 0;
+  const int64_t wpad = align4(std::min(P.maxWp, grp_rows(tsize, K)));
+  const int64_t stage = (kIluHeader + wpad * tsize * (1 + K) + 4 * K * wpad + wpad * tsize + 127) & ~int64_t(127);
+  return ((16 * stages + 16 + 127) & ~127) + ring_alloc + stages * stage;
+}
 
 // Whether the grouped sweep takes plan P with kuni couplings per row and sweep, and its ring: the
 // last W levels or the largest block by position, whichever is smaller; its byte offsets are
@@ -1893,11 +1925,18 @@ static bool grp_fits(const IluPlan& P, int tsize, int kuni, RingMap& ring, int64
   return elems * tsize <= 65536 && 128 + ring_alloc + 2 * widest <= sweep_smem_budget();
 }
 
-int ilu_sweep_rank(const IluPlan& P, int tsize) {
+// The double-double sweep without staged records (pb_ddcg.cu) has no stages; its ring is larger.
+static SweepForm sweep_form(const IluPlan& P, int tsize) {
+  const bool is_dd = tsize == (int)sizeof(dd);
+  const int K = record_couplings(P.kmax);
   RingMap ring;
-  int64_t elems;
-  if (grp_fits(P, tsize, record_couplings(P.kmax), ring, elems)) return 2;
-  return general_ring_bytes(P, tsize) <= kGeneralRing ? 1 : 0;
+  int64_t elems = 0;
+  if (!(is_dd && (K > 6 || P.nb >= 8 * num_sms())) && grp_fits(P, tsize, K, ring, elems)) return SweepForm{2, elems};
+  const int64_t bytes = general_ring_bytes(P, tsize);
+  if (is_dd) return SweepForm{bytes <= kDdRingBytes ? 1 : 0, bytes};
+  const bool with_ring = bytes <= kGeneralRing;
+  if (general_smem(P, tsize, K, with_ring, 2) > sweep_smem_budget()) return SweepForm{-1, bytes};
+  return SweepForm{with_ring ? 1 : 0, bytes};
 }
 
 // Lays out the grouped sweep of plan P (chunks ch, kuni couplings per row and sweep) if it fits:

@@ -71,6 +71,7 @@ struct IluChunk {
   __host__ __device__ IluChunk() {}
 };
 constexpr int kIluChunk = 512;      // rows per chunk (multiple of 4)
+constexpr int kDdRingBytes = 160 * 1024;   // largest shared-memory ring of the double-double sweep without staged records
 constexpr int kIluHeader = 32;      // bytes of the per-chunk header in the packed data
 
 // Wavefront levels of every block and the permuted, padded layout: what the host keeps of it.
@@ -147,17 +148,16 @@ struct BlockSplit {
 // gives the same result; small blocks with narrow levels then fit many more CTAs per SM).
 inline int ilu_factor_threads(int maxWp) { return std::min(256, std::max(32, (maxWp + 31) & ~31)); }
 
-// Wavefront plan of the block-Jacobi blocks of the natural matrix A (device arrays).  pos and
-// lev (n entries) receive every row's permuted position and its level within its block, rowAt
-// (np entries) the row at every position, -1 for padding.  With tighten, the early levels of a
-// block that make its sweep's ring too long are moved later where that shortens it; returns
-// whether any were (without: whether a block has such levels).
-bool ilu_build_plan(const DevMat<double>& A, const BlockSplit& blocks, bool tighten, IluPlan& P, DBuf& pos,
-                    DBuf& rowAt, DBuf& lev);
+// Whether levels may be moved later than the early ones: not at all, where that shortens the ring of
+// the sweep, or only where the sweep gets a better form by it.
+enum class Tighten { no, shorter, better_form };
 
-// The sweep a plan gets for values of tsize bytes: 2 the grouped one, 1 the general one with its
-// ring in shared memory, 0 without.
-int ilu_sweep_rank(const IluPlan& P, int tsize);
+// Wavefront plan of the block-Jacobi blocks of the natural matrix A (device arrays), for a sweep on
+// values of tsize bytes.  pos and lev (n entries) receive every row's permuted position and its
+// level within its block, rowAt (np entries) the row at every position, -1 for padding.  Returns
+// whether levels were moved (Tighten::no: whether a block's early levels make its ring too long).
+bool ilu_build_plan(const DevMat<double>& A, const BlockSplit& blocks, Tighten tighten, int tsize, IluPlan& P,
+                    DBuf& pos, DBuf& rowAt, DBuf& lev);
 
 // Factorises (ILU(0)) or computes the D-ILU diagonal on the device and packs the sweep
 // data.  ilu_method: 0 ILU(0), 1 ILUD, 2 MLUD (define.f90:40-42).  Returns a status.

@@ -185,11 +185,12 @@ void build_system(const Options& o, const parcel_b_crs& A, bool dev, System<T>& 
     // order costs two copies per application (6 of 60 us on 97 x 89 x 83 in 48 blocks), so it is
     // taken only where levels were moved and the sweep got a better form by it.
     const bool keep_order = o.solver == PARCEL_B_SOLVER_BICG;
-    const bool loose = ilu_build_plan(S.Anat, bs, !keep_order, P, S.pos, S.rowAt, S.lev);
+    const bool loose = ilu_build_plan(S.Anat, bs, keep_order ? Tighten::no : Tighten::shorter, sizeof(T), P, S.pos,
+                                      S.rowAt, S.lev);
     IluPlan Q;
     DBuf qpos, qrowAt, qlev;
-    const bool reorder = keep_order && loose && ilu_build_plan(S.Anat, bs, true, Q, qpos, qrowAt, qlev) &&
-                         ilu_sweep_rank(Q, sizeof(T)) > ilu_sweep_rank(P, sizeof(T));
+    const bool reorder = keep_order && loose &&
+                         ilu_build_plan(S.Anat, bs, Tighten::better_form, sizeof(T), Q, qpos, qrowAt, qlev);
     trace_mark("setup: wavefront plan");
     S.np = P.np;
     S.permuted = true;

@@ -555,3 +555,19 @@ def test_a_handle_reports_a_sweep_that_gave_up_in_every_start():
         assert L.parcel_b_start(h, b.ctypes.data, x.ctypes.data, hist.ctypes.data, C.byref(n), C.byref(i)) < 0
         assert "gave up waiting" in _lib.last_error()
     assert L.parcel_b_release(h) == 0
+
+
+@pytest.mark.parametrize("ilu", [0, 1])
+def test_plan_keeps_levels_that_the_sweep_can_take(ilu):
+    """A chain of 2,500 rows, a row hanging on each, and the 84 rows at the end that are all those rows'
+    only dependents: moved late they would form one level of 2,500 rows of 30 couplings, which no
+    sweep takes, for a gap shorter by one."""
+    m, per = 2500, 30
+    chain = np.arange(m)
+    side = m + chain
+    end = 2 * m + 1 + chain // per
+    last = np.unique(end)
+    r = np.concatenate([chain[:-1], chain, side, [2 * m], last])
+    c = np.concatenate([chain[1:], side, end, [2 * m + 1], np.full(last.size, m - 1)])
+    A = _from_pairs(int(last[-1]) + 1, np.concatenate([r, c]), np.concatenate([c, r]), 4)
+    assert _apply_both(A, ipreflag=2, ILU_method=ilu, precon_thblock=1) < 1e-11
