@@ -752,7 +752,13 @@ SolveOut solve_cagmres(const Options& o, System<double>& S, const double* b_nat,
     const double rnorm0 = std::sqrt(dot(r, r));
     launches += 2;
     if (rnorm0 < o.abstol || rnorm0 / bnorm < o.rtol) break;
-    if (rnorm0 != rnorm0) { ilu_check_error<double>(S.M.ilu); SolveOut so; so.niter = itr; so.iret = PARCEL_B_E_BREAKDOWN; return so; }
+    if (rnorm0 != rnorm0) {
+      ilu_check_error<double>(S.M.ilu);
+      SolveOut so;
+      so.niter = itr;
+      so.iret = PARCEL_B_E_BREAKDOWN;
+      return so;
+    }
     if (itr == 1) hist[0] = rnorm0 / bnorm;
     ze[0] = -rnorm0;
     lincomb<double>(np, V, r, cimm(-1.0 / rnorm0), nullptr, cimm(0), nullptr, cimm(0), nullptr, st);

@@ -103,10 +103,11 @@ static SweepForm sweep_form(const IluPlan& P, int tsize);
 // 12,000-row block of a 61 x 53 x 47 stencil would hold 58 levels, tightened it holds 2, as for
 // a block of whole planes, and the grouped sweep takes it instead of the general one, which
 // gathers coupled values from global memory: applications back to back 147 -> 33 us there (16
-// blocks; 119 -> 26 us inside a solve), 247 -> 53 us on 97 x 89 x 83 in 48 blocks.  The late levels are kept where they get
-// the sweep a better form (sweep_form), or a grouped sweep a shorter ring: a shorter gap alone can
-// come with levels so wide that the ring is longer, or that no sweep takes them (rows all over a
-// chain whose only dependents are at its end move into one level).
+// blocks; 119 -> 26 us inside a solve), 247 -> 53 us on 97 x 89 x 83 in 48 blocks.  The late
+// levels are kept where they get the sweep a better form (sweep_form), or a grouped sweep a
+// shorter ring: a shorter gap alone can come with levels so wide that the ring is longer, or that
+// no sweep takes them (rows all over a chain whose only dependents are at its end move into one
+// level).
 constexpr int kPlanRounds = 48;
 constexpr int kPlanRetry = 8;
 constexpr int kPlanList = 16;      // couplings of a row within its chunk, each way, that are listed
@@ -352,7 +353,7 @@ struct PlanSeg {
 };
 
 __global__ void k_plan_count(int nseg, const PlanSeg* __restrict__ seg, const int* __restrict__ lev, int* ctr) {
-  const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  const int s = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (s >= nseg) return;
   const PlanSeg S = seg[s];
   for (int i = S.row0 + lane; i < S.row1; i += 32) atomicAdd(ctr + S.ctr + lev[i], 1);
@@ -383,7 +384,7 @@ __global__ void k_plan_scan(int totlev, int nb, const int* __restrict__ blvl, co
 // lane, and the level's counter is where it goes on.
 __global__ void k_plan_pos(int nseg, const PlanSeg* __restrict__ seg, const int* __restrict__ lev, int* ctr,
                            int* __restrict__ pos, int* __restrict__ rowAt) {
-  const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  const int s = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (s >= nseg) return;
   const PlanSeg S = seg[s];
   int* nx = ctr + S.ctr;

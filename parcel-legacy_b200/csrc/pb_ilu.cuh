@@ -71,7 +71,8 @@ struct IluChunk {
   __host__ __device__ IluChunk() {}
 };
 constexpr int kIluChunk = 512;      // rows per chunk (multiple of 4)
-constexpr int kDdRingBytes = 160 * 1024;   // largest shared-memory ring of the double-double sweep without staged records
+// largest shared-memory ring of the double-double sweep without staged records
+constexpr int kDdRingBytes = 160 * 1024;
 constexpr int kIluHeader = 32;      // bytes of the per-chunk header in the packed data
 
 // Wavefront levels of every block and the permuted, padded layout: what the host keeps of it.
