@@ -2878,6 +2878,7 @@ template <class T>
 void ilu_check_error(const IluDev<T>& D) {
   int flag = 0;
   if (D.err.p) d2h(&flag, D.err.p, sizeof(int));
+  if (flag) ilu_clear_error<T>(D);   // reported once: a kept operator's next call starts clean
   ilu_raise_error(flag);
 }
 template void ilu_clear_error<double>(const IluDev<double>&, bool);

@@ -205,8 +205,8 @@ bool ilu_apply_cg(const IluDev<T>& D, T* r, const T* q, const double* c, T* s, c
                   cudaStream_t st);
 
 // The sweeps' error flag: a sweep whose bounded wait runs out sets it and leaves its output
-// incomplete.  Every call that runs sweeps clears it first (fail: sets it instead, as if one had
-// given up; tests only) and raises an error if it is set at the end.
+// incomplete.  A solve clears it first (fail: sets it instead, as if one had given up; tests only),
+// and every call that runs sweeps raises an error if it is set at the end.
 template <class T>
 void ilu_clear_error(const IluDev<T>& D, bool fail = false);
 void ilu_raise_error(int flag);

@@ -128,7 +128,6 @@ int parcel_b_local_precon(parcel_b_local h, const double* r, double* z) {
     if (!L.has_precon) {
       d2d(z, r, sizeof(double) * L.n);
     } else if (L.S.permuted) {
-      ilu_clear_error<double>(L.S.M.ilu);
       scatter_perm<double>(L.n, dp<double>(L.rperm), r, dp<int>(L.S.pos), st);
       L.S.M.apply(L.S.np, dp<double>(L.rperm), dp<double>(L.zperm), nullptr, st);
       gather_perm<double>(L.n, z, dp<double>(L.zperm), dp<int>(L.S.pos), st);
